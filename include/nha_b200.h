@@ -247,6 +247,8 @@ int64_t nha_chunk_bwd_workspace_bytes(const nha_chunk_desc* d);
 
 /* fills desc->plan from cu_seqlens on the device (no host synchronisation) */
 int nha_chunk_plan(const nha_chunk_desc* d, void* stream);
+/* as nha_chunk_plan for N sequences of T tokens each; also WRITES cu_seqlens (the caller's buffer of N+1 ints) */
+int nha_chunk_plan_dense(const nha_chunk_desc* d, int T, void* stream);
 /* state pass: chunk-start states hk_chunks/hv_chunks (+ final states hkt/hvt when non-NULL) */
 int nha_chunk_state_pass(const nha_chunk_desc* d, void* stream);
 /* The two halves of nha_chunk_state_pass, for callers that have part of their inputs early (the sequence-parallel
@@ -318,6 +320,8 @@ int nha_chunk_output_pass(const nha_chunk_desc* d, void* stream);
 int nha_chunk_device_error(const nha_chunk_desc* d, void* stream);
 /* plan + state pass + output pass */
 int nha_chunk_fwd(const nha_chunk_desc* d, void* stream);
+/* nha_chunk_fwd with nha_chunk_plan_dense in front: a batch of N sequences of T tokens needs no cu_seqlens upfront */
+int nha_chunk_fwd_dense(const nha_chunk_desc* d, int T, void* stream);
 /* backward: needs the forward's o, lse_swa, lse_gsa, hk_chunks, hv_chunks, plan (and hkt/hvt
    when d_hkt/d_hvt are given); writes dq_*, dk_*, dv, ds, dg (+ dhk0/dhv0 when non-NULL) */
 int nha_chunk_bwd(const nha_chunk_desc* d, void* stream);
@@ -346,6 +350,13 @@ int nha_chunk_state_pass_static(const nha_chunk_desc* d, void* stream);
    (dk_gsa, dv, ds, dg).  The stages of one backward must run in this order; running all five
    equals nha_chunk_bwd.  No counterpart in the reference (it has no timing hooks). */
 int nha_chunk_bwd_stage(const nha_chunk_desc* d, int stage, void* stream);
+
+/* dst[i] = src[i] in another type, n[i] elements each, up to eight tensors in one launch (host arrays of device
+ * pointers).  Types: bf16 <-> fp32, bf16 <-> fp16, rounded to nearest even.  The callers' tensors may be fp32 or fp16
+ * (the reference casts too, nha_fla/ops/nha/chunk.py:232-235); the kernels take bf16. */
+enum { NHA_BF16 = 0, NHA_FP16 = 1, NHA_FP32 = 2 };
+int nha_cast_many(const void* const* src, void* const* dst, const int64_t* n, int count, int src_type, int dst_type,
+                  void* stream);
 
 /* ------------------------------------------------------------------------------------------
  * Slot gates of the callers, fused.  The layers turn the gate projection f [.., H, M] into the

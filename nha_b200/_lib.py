@@ -1,4 +1,5 @@
-"""ctypes binding of ``libnha_b200.so`` (the C ABI declared in ``include/nha_b200.h``).
+"""Loading of ``libnha_b200.so`` (the C ABI declared in ``include/nha_b200.h``, bound by ctypes) and of the host module
+that the operators call.
 
 The library is the only implementation: loading fails loudly when it is
 missing and cannot be built, and every op raises when the library reports a
@@ -67,6 +68,9 @@ SYMBOLS = {
     'nha_chunk_fwd_workspace_bytes': (C.c_int64, [C.POINTER(ChunkDesc)]),
     'nha_chunk_bwd_workspace_bytes': (C.c_int64, [C.POINTER(ChunkDesc)]),
     'nha_chunk_plan': (C.c_int, [C.POINTER(ChunkDesc), c_void_p]),
+    'nha_chunk_plan_dense': (C.c_int, [C.POINTER(ChunkDesc), C.c_int, c_void_p]),
+    'nha_chunk_fwd_dense': (C.c_int, [C.POINTER(ChunkDesc), C.c_int, c_void_p]),
+    'nha_cast_many': (C.c_int, [c_void_p, c_void_p, c_void_p, C.c_int, C.c_int, C.c_int, c_void_p]),
     'nha_chunk_state_pass': (C.c_int, [C.POINTER(ChunkDesc), c_void_p]),
     'nha_chunk_state_terms': (C.c_int, [C.POINTER(ChunkDesc), C.c_int, C.c_int, c_void_p]),
     'nha_chunk_state_scan': (C.c_int, [C.POINTER(ChunkDesc), c_void_p]),
@@ -132,6 +136,22 @@ def load():
             raise NHALibraryError('nha_chunk_desc layout mismatch between the binding and the library')
         _lib = lib
         return lib
+
+
+class _Host:
+    """The host module ``_nha_host`` (csrc/host), loaded at the first use: its functions become attributes of this object,
+    so a later access is one dictionary lookup."""
+
+    def __getattr__(self, name):
+        load()                                   # builds what is missing, binds the library the module links to
+        import importlib
+        m = importlib.import_module('nha_b200._nha_host')
+        m.set_error(NHALibraryError)
+        self.__dict__.update({k: v for k, v in vars(m).items() if not k.startswith('_')})
+        return self.__dict__[name]
+
+
+host = _Host()
 
 
 def check(status: int, what: str):

@@ -17,6 +17,7 @@ from typing import Optional, Tuple, Union
 import torch
 
 from . import _lib
+from ._lib import host as _host
 
 _BF16 = torch.bfloat16
 IntOrTensor = Union[int, torch.Tensor]
@@ -136,47 +137,6 @@ def chunk_backward(q_gsa, q_swa, k_gsa, k_swa, v, s, g, cu_seqlens, scale, saved
             t.get('dhk0'), t.get('dhv0'))
 
 
-class ChunkNativeHybridAttentionFunction(torch.autograd.Function):
-    """Autograd node of ``chunk_nha`` on flat packed tensors.
-
-    Mirrors nha_fla/ops/nha/chunk.py:352-564: gradients flow to q_swa, k_swa, q_gsa,
-    k_gsa, v, s, g and the initial states; a gradient arriving on ``lse_gsa`` is
-    honoured, one arriving on ``lse_swa`` is dropped exactly as the reference drops it
-    (chunk.py:491-512)."""
-
-    @staticmethod
-    def forward(ctx, q_swa, k_swa, q_gsa, k_gsa, v, s, g, cu_seqlens, max_seqlen, scale, window_left, shift,
-                hk0, hv0, output_final_state, q_offset):
-        o, lse_swa, lse_gsa, hkt, hvt, saved = chunk_forward(
-            q_gsa, q_swa, k_gsa, k_swa, v, s, g, cu_seqlens, max_seqlen, scale, window_left, shift,
-            hk0, hv0, output_final_state, q_offset)
-        ctx.save_for_backward(q_swa, k_swa, q_gsa, k_gsa, v, s, g, cu_seqlens, o, lse_swa, lse_gsa,
-                              saved['hk_chunks'], saved['hv_chunks'], hk0, hv0, hkt, hvt)
-        ctx.saved_meta = saved
-        ctx.scale = scale
-        ctx.state_grad = hk0 is not None and (hk0.requires_grad or hv0.requires_grad)
-        ctx.mark_non_differentiable(lse_swa)
-        if hkt is None:
-            return o, lse_swa, lse_gsa, None, None
-        return o, lse_swa, lse_gsa, hkt, hvt
-
-    @staticmethod
-    def backward(ctx, d_o, d_lse_swa, d_lse_gsa, d_hkt, d_hvt):
-        (q_swa, k_swa, q_gsa, k_gsa, v, s, g, cu_seqlens, o, lse_swa, lse_gsa, hk_chunks, hv_chunks, hk0, hv0,
-         hkt, hvt) = ctx.saved_tensors
-        saved = dict(ctx.saved_meta, hk_chunks=hk_chunks, hv_chunks=hv_chunks)
-        d_o = d_o.contiguous().to(_BF16)
-        if d_lse_gsa is not None:
-            d_lse_gsa = d_lse_gsa.float().contiguous()
-        if d_hkt is not None or d_hvt is not None:
-            d_hkt = torch.zeros_like(hkt) if d_hkt is None else d_hkt.float().contiguous()
-            d_hvt = torch.zeros_like(hvt) if d_hvt is None else d_hvt.float().contiguous()
-        grads = chunk_backward(q_gsa, q_swa, k_gsa, k_swa, v, s, g, cu_seqlens, ctx.scale, saved, o, lse_swa, lse_gsa,
-                               d_o, d_lse_gsa, d_hkt, d_hvt, hkt, hvt, hk0, hv0, need_state_grad=ctx.state_grad)
-        dq_swa, dk_swa, dq_gsa, dk_gsa, dv, ds, dg, dhk0, dhv0 = grads
-        return (dq_swa, dk_swa, dq_gsa, dk_gsa, dv, ds, dg, None, None, None, None, None, dhk0, dhv0, None, None)
-
-
 @torch.compiler.disable
 def chunk_nha(
     q_swa: torch.Tensor,
@@ -218,43 +178,8 @@ def chunk_nha(
             "head_first is deprecated and will be removed in a future version. "
             "Please use head_first=False for now instead.",
         )
-    if scale is None:
-        scale = q_swa.shape[-1] ** -0.5
-    assert q_swa.dim() == 4, "Expected [B, T, H, D] for input"
-    assert window_size_right in (0, -1), "the window branch is causal: window_size_right must be 0 or -1"
-    B, T, HQ, D = q_swa.shape
-    dev = q_swa.device
-    is_varlen = cu_seqlens is not None
-    if is_varlen:
-        assert B == 1, "varlen inputs must be packed into a single batch row"
-        cu = cu_seqlens.to(device=dev, dtype=torch.int32).contiguous()
-        if max_seqlen is None:
-            max_seqlen = int((cu[1:] - cu[:-1]).max().item())
-    else:
-        cu = torch.arange(0, (B + 1) * T, T, dtype=torch.int32, device=dev)
-        max_seqlen = T
-    out_dtype = q_swa.dtype
-
-    def flat(x):
-        x = x.reshape(B * T, *x.shape[2:])
-        if x.dtype != _BF16:
-            x = x.to(_BF16)
-        return x.contiguous()
-
-    hk0, hv0 = (None, None) if initial_state is None else initial_state
-    if hk0 is not None:
-        hk0, hv0 = hk0.float().contiguous(), hv0.float().contiguous()
-    o, lse_swa, lse_gsa, hkt, hvt = ChunkNativeHybridAttentionFunction.apply(
-        flat(q_swa), flat(k_swa), flat(q_gsa), flat(k_gsa), flat(v), flat(s), flat(g), cu, max_seqlen, scale,
-        window_size_left, gsa_kv_shift, hk0, hv0, output_final_state, 0)
-    o = o.view(B, T, HQ, -1)
-    if out_dtype != _BF16:
-        o = o.to(out_dtype)
-    lse_swa = lse_swa.view(B, T, HQ)
-    lse_gsa = lse_gsa.view(B, T, HQ)
-    if output_final_state:
-        return o, lse_swa, lse_gsa, (hkt, hvt)
-    return o, lse_swa, lse_gsa
+    return _host.chunk_nha(q_swa, k_swa, q_gsa, k_gsa, v, s, g, cu_seqlens, max_seqlen, scale, window_size_left, window_size_right,
+                           gsa_kv_shift, initial_state, output_final_state)
 
 
 def chunk_final_state(k_gsa, v, s, g, cu_seqlens, max_seqlen, shift, hk0=None, hv0=None):

@@ -469,10 +469,14 @@ extern "C" int nha_chunk_device_error(const nha_chunk_desc* d, void* stream) {
   return v;
 }
 
-extern "C" int nha_chunk_fwd(const nha_chunk_desc* d, void* stream) {
-  int st = nha_chunk_plan(d, stream);
+static int fwd_after_plan(const nha_chunk_desc* d, int st, void* stream) {
   if (st != NHA_OK) return st;
   st = nha_chunk_state_pass(d, stream);
   if (st != NHA_OK) return st;
   return nha_chunk_output_pass(d, stream);
+}
+
+extern "C" int nha_chunk_fwd(const nha_chunk_desc* d, void* stream) { return fwd_after_plan(d, nha_chunk_plan(d, stream), stream); }
+extern "C" int nha_chunk_fwd_dense(const nha_chunk_desc* d, int T, void* stream) {
+  return fwd_after_plan(d, nha_chunk_plan_dense(d, T, stream), stream);
 }

@@ -31,34 +31,71 @@ constexpr int kStThreads = 256;
 constexpr int kStWarps = kStThreads / 32;
 
 // ---------------------------------------------------------------------------------------------
-__global__ void nha_plan_kernel(const int32_t* __restrict__ cu, int32_t* __restrict__ plan, int N, int NCB, int H) {
-  if (threadIdx.x == 0) plan[N + 1 + NCB + (size_t)NCB * H] = 0;   // device-side error word
-  // plan[0..N]: first chunk of each sequence; plan[N+1+c]: sequence of chunk c (-1 = unused)
-  __shared__ int total;
-  if (threadIdx.x == 0) {
-    int acc = 0;
-    for (int n = 0; n < N; ++n) {
-      plan[n] = acc;
-      const int len = cu[n + 1] - cu[n];
-      acc += (len + kChunk - 1) / kChunk;
-    }
-    plan[N] = acc;
-    total = acc;
-  }
-  __syncthreads();
-  for (int c = total + threadIdx.x; c < NCB; c += blockDim.x) plan[N + 1 + c] = -1;
+// One CTA.  With T >= 0 the plan is of N sequences of T tokens each and the kernel writes their boundaries too (no launch
+// for them); otherwise it reads `cu`.  The offsets of packed sequences are a running sum over the CTA's threads, so many
+// short sequences cost no serial walk.
+constexpr int kPlanThreads = 512;
+__global__ void __launch_bounds__(kPlanThreads) nha_plan_kernel(int32_t* __restrict__ cu, int32_t* __restrict__ plan, int N, int NCB, int H,
+                                                                int T) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) plan[N + 1 + NCB + (size_t)NCB * H] = 0;           // device-side error word
   int4* rec = reinterpret_cast<int4*>(plan + plan_rec_offset(N, NCB, H));
-  for (int c = total + threadIdx.x; c < NCB; c += blockDim.x) rec[c] = make_int4(-1, 0, 0, 0);
-  // one thread per chunk: its sequence is the last one whose first chunk is <= c (binary search over plan[0..N])
-  for (int c = threadIdx.x; c < total; c += blockDim.x) {
-    int lo = 0, hi = N - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (plan[mid] <= c) lo = mid; else hi = mid - 1;
+  int total;
+  // plan[0..N]: first chunk of each sequence; plan[N+1+c]: sequence of chunk c (-1 = unused)
+  if (T >= 0) {
+    const int per = (T + kChunk - 1) / kChunk;
+    total = N * per;
+    for (int n = tid; n <= N; n += kPlanThreads) {
+      plan[n] = n * per;
+      cu[n] = n * T;
     }
-    while (lo + 1 < N && plan[lo + 1] <= c) ++lo;      // empty sequences share their first chunk with the next one
-    plan[N + 1 + c] = lo;
-    rec[c] = make_int4(lo, c - plan[lo], cu[lo], cu[lo + 1] - cu[lo]);
+    for (int c = tid; c < total; c += kPlanThreads) {
+      const int n = c / per;
+      plan[N + 1 + c] = n;
+      rec[c] = make_int4(n, c - n * per, n * T, T);
+    }
+  } else {
+    __shared__ int part[kPlanThreads / 32];
+    int base = 0;
+    for (int n0 = 0; n0 < N; n0 += kPlanThreads) {
+      const int n = n0 + tid;
+      const int mine = n < N ? (cu[n + 1] - cu[n] + kChunk - 1) / kChunk : 0;
+      int incl = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+      }
+      if (lane == 31) part[warp] = incl;
+      __syncthreads();
+      int before = 0, all = 0;
+#pragma unroll
+      for (int w = 0; w < kPlanThreads / 32; ++w) {
+        before += w < warp ? part[w] : 0;
+        all += part[w];
+      }
+      if (n < N) plan[n] = base + before + incl - mine;
+      base += all;
+      __syncthreads();
+    }
+    total = base;
+    if (tid == 0) plan[N] = total;
+    __syncthreads();
+    // one thread per chunk: its sequence is the last one whose first chunk is <= c (binary search over plan[0..N])
+    for (int c = tid; c < total; c += kPlanThreads) {
+      int lo = 0, hi = N - 1;
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (plan[mid] <= c) lo = mid; else hi = mid - 1;
+      }
+      while (lo + 1 < N && plan[lo + 1] <= c) ++lo;      // empty sequences share their first chunk with the next one
+      plan[N + 1 + c] = lo;
+      rec[c] = make_int4(lo, c - plan[lo], cu[lo], cu[lo + 1] - cu[lo]);
+    }
+  }
+  for (int c = total + tid; c < NCB; c += kPlanThreads) {
+    plan[N + 1 + c] = -1;
+    rec[c] = make_int4(-1, 0, 0, 0);
   }
 }
 
@@ -586,11 +623,16 @@ extern "C" int64_t nha_chunk_plan_ints(int64_t Ttot, int64_t N, int64_t H) {
   return plan_rec_offset(N, ncb, H) + 4 * ncb;
 }
 
-extern "C" int nha_chunk_plan(const nha_chunk_desc* d, void* stream) {
+static int plan_launch(const nha_chunk_desc* d, int T, void* stream) {
   if (!d || !d->cu_seqlens || !d->plan || d->N <= 0) return NHA_ERR_BAD_ARG;
   const int NCB = (int)nha_chunk_count_bound(d->Ttot, d->N);
-  nha_plan_kernel<<<1, 256, 0, (cudaStream_t)stream>>>(d->cu_seqlens, d->plan, d->N, NCB, d->H);
+  nha_plan_kernel<<<1, kPlanThreads, 0, (cudaStream_t)stream>>>(const_cast<int32_t*>(d->cu_seqlens), d->plan, d->N, NCB, d->H, T);
   return check_launch();
+}
+extern "C" int nha_chunk_plan(const nha_chunk_desc* d, void* stream) { return plan_launch(d, -1, stream); }
+extern "C" int nha_chunk_plan_dense(const nha_chunk_desc* d, int T, void* stream) {
+  if (!d || T < 0 || (int64_t)T * d->N != d->Ttot) return NHA_ERR_BAD_ARG;
+  return plan_launch(d, T, stream);
 }
 
 extern "C" int nha_chunk_state_pass(const nha_chunk_desc* d, void* stream) {

@@ -21,7 +21,8 @@ from typing import List, Optional, Tuple
 import torch
 
 from . import _lib
-from .fused_recurrent import _decode_workspace, _stream
+from ._lib import host as _host
+from .fused_recurrent import _stream
 
 _BF16 = torch.bfloat16
 
@@ -144,44 +145,17 @@ def fused_recurrent_nha_decode_ring(q: torch.Tensor, k: torch.Tensor, v: torch.T
     ``cos/sin [1|B, W, K]`` for the W window positions (row W-1 = the query's position); while the rings are
     still filling (``layer.fill < W``) the window is ``layer.fill + 1`` long and so are the tables.
     """
-    lib = _lib.load()
-    B, one, HQ, K = q.shape
-    if one != 1:
+    if q.shape[1] != 1:
         raise ValueError('decode takes one token per sequence')
-    H, V, M, W = k.shape[2], v.shape[3], g.shape[3], layer.window
-    fill = layer.fill
-    wlen = W if fill >= W else fill + 1
     if layer.ring_kr is not None:
         return _decode_ring_rot(q, k, v, g, layer, cos, sin, scale)
-    assert cos.shape[-2] == wlen and cos.shape[-1] == K, 'cos/sin must cover the window positions'
-    dev = q.device
-    qc, kc, vc, gc = (x.to(_BF16).contiguous() for x in (q, k, v, g))
-    cosc, sinc = cos.to(_BF16).contiguous(), sin.to(_BF16).contiguous()
-    cs_batch = cosc.stride(0) if (cosc.dim() == 3 and cosc.shape[0] > 1) else 0
-    o = torch.empty(B, 1, HQ, V, dtype=_BF16, device=dev)
-    sc = float(K ** -0.5 if scale is None else scale)
-    with torch.cuda.device(dev):                       # split count and launches follow the tensors' device
-        ws = _decode_workspace(dev, B, HQ, H, V, W)
-        st = _stream(dev)
-        if layer.fused:
-            if layer.head.shape[1] != H:               # rings made through update(): the kv-head count is known only now
-                layer.head = layer.head[:, :1].repeat(1, H)
-            _lib.check(lib.nha_decode_step_ring_fused(
-                qc.data_ptr(), kc.data_ptr(), vc.data_ptr(), gc.data_ptr(), layer.ring_k.data_ptr(), layer.ring_v.data_ptr(),
-                layer.ring_g.data_ptr(), layer.head.data_ptr(), cosc.data_ptr(), sinc.data_ptr(), cs_batch, cosc.stride(-2),
-                layer.hk.data_ptr(), layer.hv.data_ptr(), o.data_ptr(), ws.data_ptr(), ws.numel(), B, HQ, H, K, V, M, W, fill,
-                sc, st), 'nha_decode_step_ring_fused')
-        else:
-            _lib.check(lib.nha_decode_step_ring(qc.data_ptr(), kc.data_ptr(), vc.data_ptr(), layer.ring_k.data_ptr(),
-                                                layer.ring_v.data_ptr(), layer.ring_g.data_ptr(), layer.head.data_ptr(),
-                                                cosc.data_ptr(), sinc.data_ptr(), cs_batch, cosc.stride(-2),
-                                                layer.hk.data_ptr(), layer.hv.data_ptr(), o.data_ptr(), ws.data_ptr(),
-                                                ws.numel(), B, HQ, H, K, V, M, W, fill, sc, st), 'nha_decode_step_ring')
-            _lib.check(lib.nha_ring_append(layer.ring_k.data_ptr(), layer.ring_v.data_ptr(), layer.ring_g.data_ptr(),
-                                           kc.data_ptr(), vc.data_ptr(), gc.data_ptr(), layer.head.data_ptr(), B, H, K, V, M,
-                                           W, fill, st), 'nha_ring_append')
-        _lib.check_decode_device(lib, ws, B, H, st, 'nha_decode_step_ring')
-    layer.fill = min(fill + 1, W)
+    fill, head = layer.fill, layer.head
+    if layer.fused and head.shape[1] != k.shape[2]:    # rings made through update(): the kv-head count is known only now
+        head = layer.head = head[:, :1].repeat(1, k.shape[2])
+    ring_k = layer.ring_k
+    o = _host.decode_ring(q, k, v, g, ring_k, layer.ring_v, layer.ring_g, head, cos, sin, layer.hk, layer.hv, fill, layer.fused, scale)
+    if fill < ring_k.shape[1]:
+        layer.fill = fill + 1
     return o
 
 
@@ -200,7 +174,7 @@ def _decode_ring_rot(q, k, v, g, layer: RingLayer, cos, sin, scale) -> torch.Ten
     o = torch.empty(B, 1, HQ, V, device=dev, dtype=_BF16)
     fill = layer.fill
     with torch.cuda.device(dev):
-        ws = _decode_workspace(dev, B, HQ, H, V, W)
+        ws = _host.decode_workspace(q, B, HQ, H, V, W)
         st = _stream(dev)
         _lib.check(lib.nha_decode_step_ring_rot(qc.data_ptr(), kc.data_ptr(), vc.data_ptr(), layer.ring_k.data_ptr(),
                                                 layer.ring_kr.data_ptr(), layer.ring_v.data_ptr(), layer.ring_g.data_ptr(),
