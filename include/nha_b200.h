@@ -230,7 +230,7 @@ typedef struct nha_chunk_desc {
                                    kv-head tensors hold all Ttot positions.  The state pass covers every position; the output
                                    pass skips the chunks below q_offset.  Used by the sequence-parallel prefill, whose ranks
                                    prepend the last window of the rank before them to their kv-head tensors only.  Honoured by
-                                   the pipelined output pass (K == V == 128, M == 64, even HQ / H); other shapes return
+                                   the pipelined output pass (K == V == 128, M == 64); other shapes return
                                    NHA_ERR_UNSUPPORTED */
   float scale;
 } nha_chunk_desc;

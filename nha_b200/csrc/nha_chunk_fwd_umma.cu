@@ -151,14 +151,16 @@ __global__ void __launch_bounds__(UmmaLayout<D, R>::kThreads, (D == 64 && R == 6
   load_sw<D, kUThreads>(sm + L::tV, 8192, (const bf16*)d.v + ((size_t)t0 * H + h) * D, (int64_t)H * D, c0 - shift, lo, hi, 64, 0, tid);
   load_sw<64, kUThreads>(sm + L::tHk, 0, (const bf16*)d.hk_chunks + ((size_t)cg * H + h) * D * M, M, 0, 0, D, D, 0, tid);
   load_sw<D, kUThreads>(sm + L::tHv, 8192, (const bf16*)d.hv_chunks + ((size_t)cg * H + h) * M * D, D, 0, 0, M, M, 0, tid);
+// an odd group's last 128-row tile holds one head: its other 64 rows are zeros and never stored
+#define NHA_HEAD_ROWS(hq_) (R == 64 || (hq_) < (h + 1) * NG ? len : 0)
 #define NHA_LOAD_HEAD_TILE(ht_)                                                                                       \
   do {                                                                                                                \
     const int hq0_ = h * NG + (ht_) * TH;                                                                             \
     _Pragma("unroll") for (int t2 = 0; t2 < TH; ++t2) {                                                               \
       load_sw<D, kUThreads>(sm + L::tQ, L::kATile, (const bf16*)d.q_gsa + ((size_t)t0 * HQ + hq0_ + t2) * D, (int64_t)HQ * D,    \
-                 c0, 0, len, 64, 64 * t2, tid);                                                                       \
+                 c0, 0, NHA_HEAD_ROWS(hq0_ + t2), 64, 64 * t2, tid);                                                  \
       load_sw<D, kUThreads>(sm + L::tQS, L::kATile, (const bf16*)d.q_swa + ((size_t)t0 * HQ + hq0_ + t2) * D, (int64_t)HQ * D,   \
-                 c0, 0, len, 64, 64 * t2, tid);                                                                       \
+                 c0, 0, NHA_HEAD_ROWS(hq0_ + t2), 64, 64 * t2, tid);                                                  \
     }                                                                                                                 \
     if (L::kPipe && !L::kAlias && (ht_) > 0) {     /* the second window buffer set has overwritten k' and Hk */       \
       load_sw<D, kUThreads>(sm + L::tK, 8192, (const bf16*)d.k_gsa + ((size_t)t0 * H + h) * D, (int64_t)H * D,          \
@@ -257,13 +259,8 @@ __global__ void __launch_bounds__(UmmaLayout<D, R>::kThreads, (D == 64 && R == 6
   const int tk = row & 63;                          // token inside the chunk
   const int th = row >> 6;                          // head inside the tile
   const int pos = c0 + tk;
-  const bool in_seq = pos < len;
   float* xch = (float*)(sm + L::oX);                // [4 exchange points][NS parts][128 rows]
-  // visible keys of this row: klo <= key <= pos, tested as (unsigned)(key - klo) <= kspan; a row past the
-  // sequence end sees nothing
   constexpr float kLog2e = 1.4426950408889634f;
-  const int klo = in_seq ? (wl < 0 ? 0 : max(0, pos - wl)) : (1 << 30);
-  const unsigned kspan = in_seq ? (unsigned)(pos - klo) : 0u;
   const float sc2 = d.scale * kLog2e;
   const uint32_t aQ = smem_u32(sm + L::tQ), aQS = smem_u32(sm + L::tQS), aK = smem_u32(sm + L::tK);
   const uint32_t aV = smem_u32(sm + L::tV), aHk = smem_u32(sm + L::tHk), aHv = smem_u32(sm + L::tHv);
@@ -403,9 +400,14 @@ __global__ void __launch_bounds__(UmmaLayout<D, R>::kThreads, (D == 64 && R == 6
   } while (0)
   uint32_t phases = 0u;                               // parities: bits 0-1 loads, 2-3 S products, 4 P~ V product
 
-  for (int ht = 0; ht < NG / TH; ++ht) {
+  for (int ht = 0; ht < (NG + TH - 1) / TH; ++ht) {
     const int hq0 = h * NG + ht * TH;
     const int hq = hq0 + th;
+    const bool in_seq = pos < NHA_HEAD_ROWS(hq);
+    // visible keys of this row: klo <= key <= pos, tested as (unsigned)(key - klo) <= kspan; a row past the
+    // sequence end sees nothing
+    const int klo = in_seq ? (wl < 0 ? 0 : max(0, pos - wl)) : (1 << 30);
+    const unsigned kspan = in_seq ? (unsigned)(pos - klo) : 0u;
     if (ht > 0) NHA_LOAD_HEAD_TILE(ht);
     cp_wait_all();
     NHA_SMEM_TO_MMA();
@@ -639,6 +641,7 @@ __global__ void __launch_bounds__(UmmaLayout<D, R>::kThreads, (D == 64 && R == 6
 #undef NHA_ISSUE_PV
 #undef NHA_XCHG
 #undef NHA_LOAD_HEAD_TILE
+#undef NHA_HEAD_ROWS
 #undef NHA_KBASE
   if (failed) atomicExch(err, 1);
   cp_wait_all();
@@ -664,8 +667,8 @@ static int launch_umma(const nha_chunk_desc* d, int* flags, int* err, cudaStream
   return check_launch();
 }
 
-// Runs the tensor-memory output pass when the shape has one (K == V in {64, 128}, M == 64, one or an
-// even number of query heads per kv head, positive scale).  Returns NHA_ERR_UNSUPPORTED otherwise.
+// Runs the tensor-memory output pass when the shape has one (K == V in {64, 128}, M == 64, positive
+// scale).  Returns NHA_ERR_UNSUPPORTED otherwise.
 bool fwd_pipe_supported(const nha_chunk_desc* d);
 int fwd_pipe_launch(const nha_chunk_desc* d, int* flags, int* err, cudaStream_t cs);
 
@@ -673,15 +676,15 @@ int chunk_output_pass_umma(const nha_chunk_desc* d, int* flags, int* err, cudaSt
   const int NG = d->HQ / d->H;
   if (d->K != d->V || d->M != 64) return NHA_ERR_UNSUPPORTED;
   if (!(d->scale > 0.f)) return NHA_ERR_UNSUPPORTED;     // row maxima are taken before scaling
-  // head dim 128 with groups of four query heads: the warp-specialised pipeline (nha_chunk_fwd_pipe.cu)
+  // head dim 128: the warp-specialised pipeline (nha_chunk_fwd_pipe.cu)
   if (fwd_pipe_supported(d)) {
     const int st = fwd_pipe_launch(d, flags, err, cs);
     if (st != NHA_ERR_UNSUPPORTED) return st;
   }
   if (d->K == 64 && NG == 1) return launch_umma<64, 64>(d, flags, err, cs);
-  if (d->K == 64 && NG % 2 == 0) return launch_umma<64, 128>(d, flags, err, cs);
+  if (d->K == 64) return launch_umma<64, 128>(d, flags, err, cs);
   if (d->K == 128 && NG == 1) return launch_umma<128, 64>(d, flags, err, cs);
-  if (d->K == 128 && NG % 2 == 0) return launch_umma<128, 128>(d, flags, err, cs);
+  if (d->K == 128) return launch_umma<128, 128>(d, flags, err, cs);
   return NHA_ERR_UNSUPPORTED;
 }
 
