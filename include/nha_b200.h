@@ -73,7 +73,7 @@ int nha_abi_version(void);
  *            int32 is a device error word (nha_decode_device_error): they must be zero before the
  *            first call and every call leaves the counters zero, so one zero-initialised buffer can
  *            be reused by all calls with the same B*H that do not overlap on the GPU.  May be NULL
- *            for W <= 64.
+ *            for W <= 64 (M > 64 then takes the general kernel).
  * K == V in {64, 128} with window keys takes a streaming kernel (ring of asynchronous copies, whole
  * grid resident in one wave; 2, 4 or 8 splits run as a thread-block cluster and merge through shared
  * memory without touching the workspace, which must be passed all the same); other shapes and the

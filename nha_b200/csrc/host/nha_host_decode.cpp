@@ -115,7 +115,7 @@ NHA_METHOD(decode) {
     State st(hk0, hv0, B, H, K, V, M, keep, bf16_state ? at::kBFloat16 : at::kFloat, q);
     o = empty({B, 1, HQ, V}, at::kBFloat16, q);
     Tensor ws;
-    if (W > 64 || bf16_state) ws = decode_workspace(q, B, HQ, H, V, W);
+    if (W > 64 || M > 64 || bf16_state) ws = decode_workspace(q, B, HQ, H, V, W);
     void* stream = stream_of(q);
     const char* cp = rotary ? (const char*)cos.data_ptr() + 2 * skip * cs_row : nullptr;
     const char* sp = rotary ? (const char*)sin.data_ptr() + 2 * skip * cs_row : nullptr;

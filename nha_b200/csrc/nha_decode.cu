@@ -473,7 +473,8 @@ int decode_stream_try(const void* q, const void* sq, const void* k, const void* 
 // every split.  Sized for whichever kernel cuts a (sequence, kv head) into more splits.
 static int decode_max_splits(int B, int H, int W) {
   const int a = decode_splits(W, false), b = decode_stream_splits(B, H, W, 1 << 20);
-  return a > b ? a : b;
+  const int c = a > b ? a : b;
+  return c > 2 ? c : 2;               // more than 64 slots take two splits of the streaming kernel, whatever the window
 }
 
 }  // namespace nha
@@ -529,7 +530,8 @@ static int decode_step_impl(const void* q, const void* sq, const void* k, const 
   a.B = B; a.HQ = HQ; a.H = H; a.K = K; a.V = V; a.M = M; a.W = W; a.NG = NG;
   // common shapes take the streaming kernel (ring of bulk copies, whole grid resident in one wave)
   const char* force_general = getenv("NHA_B200_DECODE_GENERAL");
-  const bool stream_ok = decode_stream_supported(K, V, M, W, NG, logits_mode) && !(force_general && force_general[0] == '1');
+  const bool stream_ok = decode_stream_supported(K, V, M, W, NG, logits_mode) && !(force_general && force_general[0] == '1') &&
+                         (M <= 64 || workspace);                  // more than 64 slots are split, and splits may merge through it
   if (state_bf16 && !stream_ok) return NHA_ERR_UNSUPPORTED;      // bf16 slot memory: streaming kernel only
   a.SPLITS = stream_ok ? decode_stream_splits(B, H, W, M) : decode_splits(W, logits_mode);
   if (a.SPLITS > kMaxSplits) return NHA_ERR_UNSUPPORTED;

@@ -1,33 +1,39 @@
 // Streaming variant of the fused NHA decode step (sm_100a) for the common shapes: K == V in {64, 128},
-// window keys in the cache (not caller-supplied logits).  Same arithmetic and the same split / merge
-// protocol as nha_decode.cu, organised so that the whole grid is resident at once and every byte a CTA
-// needs is requested as early as shared memory allows:
+// window keys in the cache (not caller-supplied logits).
 //
-//   * a (sequence, kv head) is cut into SPLITS CTAs chosen so that B*H*SPLITS CTAs fit the GPU in ONE
-//     wave (two CTAs per SM); split s owns a contiguous range of window keys and of slots;
-//   * the small inputs (queries, gates, the token that enters the slot memory, the rotary row of the query) and the
-//     CTA's hk columns are requested first, into registers, so that they are not queued behind the window;
-//   * window keys and values stream through a ring of four 64-key slots filled by 16-byte asynchronous
-//     copies with one commit group per stage (the rows of one kv head are 2 D bytes long and H times that
-//     apart, too short for bulk copies to pay: one cp.async.bulk per row measured slower): first every key
-//     stage, then - into slots as their keys have been used - the value stages.  A warp owns eight rows of every
-//     stage: it copies them, rotates them in place (rotate-half on packed bf16 pairs), multiplies them
-//     (ldmatrix + mma.sync m16n8k16 for the logits, m16n8k8 over its eight keys for the value readout) and refills
-//     them, so the stage loops synchronise with cp.async.wait_group and __syncwarp only - no block-wide barrier.
-//     All logits of the CTA are kept ([16][keys] fp32), so the softmax is exact in one pass and the value readout
-//     accumulates in registers without rescaling; the eight warps' partial outputs are summed at the end;
-//   * the hk columns of the split never touch shared memory: a thread updates its elements in registers,
-//     stores them back and contributes to the slot logits of all query heads, which are then summed over
-//     the warps; the hv rows, contiguous in memory, arrive by ONE bulk copy (cp.async.bulk on an mbarrier)
-//     and are updated and read out before the value stages, while those stream in;
-//   * splits are merged by the last CTA of a (sequence, kv head) to arrive (a ticket in global memory); with up
-//     to four splits every thread fetches the partial results of its output element in one trip to L2.
+// A (sequence, kv head) is cut into SPLITS CTAs so that the GPU is filled (two CTAs per SM); split s owns a contiguous
+// range of window keys and of slots.  Inside a CTA every WARP works on its own, with a softmax of its own (running maximum,
+// unnormalised weights); the only block barriers are the one behind the small inputs and those of the final merge.
+//   * Slot memory: a warp takes eight slots.  Its hk columns and hv rows are updated in registers and stored; the slot
+//     logits of all query heads are summed over the lanes by a halving exchange, and the readout of the warp's slots joins
+//     the warp's window output.
+//   * Window: the warps share the split's keys, those with slots taking fewer (a task of eight slots counts as kSlotCost
+//     groups of eight keys).  A warp walks its keys eight at a time, keys and values side by side, each fetched by 16-byte
+//     asynchronous copies into rings of two key and two value slots that only this warp touches.  S = q K^T by mma.sync
+//     m16n8k16 with the keys as the n dimension: the order of the features inside a product is free as long as q and K
+//     agree, so a lane takes 16 consecutive bytes of its key row (two k steps), no ldmatrix is needed, and the two halves
+//     that rotate-half pairs up lie in the same lane, where they are rotated on their way from shared memory to the product.
+//     O^T = V^T P^T by m16n8k8: the accumulator layout of S is the B fragment of P^T as it stands, the heads are the n
+//     dimension (a group of up to eight heads wastes nothing), V^T is packed from two value rows by byte permutes.
+//   * Under dependent launch a CTA asks for its share of the window and of the slot memory (contiguous pieces, bulk prefetch
+//     into L2) before it waits for the kernel in front: a prefetch has no value to get wrong.  The slot memory is therefore
+//     read last, from L2, while the first window loads go out at once.
+//   * The warps' outputs are merged in shared memory, the splits through the cluster's shared memory (2, 4 or 8 splits)
+//     or by the last CTA of a (sequence, kv head) to arrive (a ticket in global memory).
+//
+// What bounds it: the instructions of the warps (6.0 M a launch at 32 sequences, HQ 32, H 4, D 128, W 512, issue slots 30 %
+// busy) and the chain of a CTA, about 4 us whatever it holds; HBM is at half its rate.  Measured per layer in a stack, against
+// a version that formed all logits of a CTA first and requested the values only when the keys had been used: 32 sequences,
+// HQ 32, H 4, D 128, W 512: 18.8 -> 17.3 us; H 8: 41.8 -> 25.9 us (3.9 TB/s); the same on rings 47.1 -> 28.7 us; 64 sequences,
+// H 8, W 64: 41.4 -> 26.1 us; one sequence, H 16, D 64, W 64: 7.3 -> 5.0 us.
 //
 // Replaces the two Triton launches of fused_recurrent_nha_decode
 // (nha_fla/ops/nha/fused_recurrent.py:229-353 k-kernel, :356-428 v-kernel).
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
+#include <type_traits>
 #include <atomic>
 
 #include "nha_common.cuh"
@@ -37,8 +43,10 @@ namespace nha {
 
 constexpr int kStrThreads = 256;
 constexpr int kStrWarps = kStrThreads / 32;
-constexpr int kStrStage = 64;            // keys per ring slot
-constexpr int kStrSlots = 4;
+constexpr int kGroup = 8;                // keys of one step of a warp, slots of one task of a warp
+constexpr int kAhead = 4;                // loads a warp keeps in flight: keys and values of two steps
+constexpr int kMinKeys = 128;            // a split holds at least this many window keys: a CTA costs about 4 us whatever it holds
+constexpr int kSlotCost = 4;             // eight slots cost a warp about as much as this many groups of eight keys
 
 struct DecodeStreamArgs {
   const bf16* q; const bf16* sq; const bf16* k; const bf16* v; const bf16* g; const bf16* s;
@@ -76,44 +84,31 @@ struct DecodeStreamArgs {
   // window of this call are requested BEFORE that wait (the caller asserts that the kernel in front writes neither)
   int pdl;
   float scale;
-  int off_ring, off_hv, off_S, off_red, off_q, off_sqA, off_oks, off_eg, off_sv, off_kpop, off_vpop, off_ml, off_bar;
+  int off_ring, off_q, off_sqA, off_p, off_eg, off_sv, off_kpop, off_vpop, off_wml, off_ml, off_out;
 };
 
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* mbar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   umma::smem_u32(dst)),
-               "l"(src), "r"(bytes), "r"(umma::smem_u32(mbar))
-               : "memory");
+// four elements of the slot memory, fp32 or bf16 storage
+template <bool SB16>
+__device__ __forceinline__ float4 ld_state4(const float* base, size_t idx) {
+  if (!SB16) return *reinterpret_cast<const float4*>(base + idx);
+  const uint2 raw = *reinterpret_cast<const uint2*>(reinterpret_cast<const bf16*>(base) + idx);
+  const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
+  const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+  return make_float4(lo.x, lo.y, hi.x, hi.y);
 }
-// one element of the slot memory, fp32 or bf16 storage
-__device__ __forceinline__ float ld_state(const float* base, size_t idx, int is_bf16) {
-  return is_bf16 ? __bfloat162float(reinterpret_cast<const bf16*>(base)[idx]) : base[idx];
-}
-__device__ __forceinline__ void st_state(float* base, size_t idx, float& v, int is_bf16) {
-  if (is_bf16) {
-    const bf16 r = __float2bfloat16_rn(v);
-    reinterpret_cast<bf16*>(base)[idx] = r;
-    v = __bfloat162float(r);                 // the rounded value is the state from here on
-  } else {
-    base[idx] = v;
+template <bool SB16>
+__device__ __forceinline__ void st_state4(float* base, size_t idx, float4& v) {
+  if (!SB16) {
+    *reinterpret_cast<float4*>(base + idx) = v;
+    return;
   }
-}
-__device__ __forceinline__ void mbar_expect(uint64_t* mbar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(umma::smem_u32(mbar)), "r"(bytes) : "memory");
-}
-
-// warp-level matrix fragments straight from shared memory, and the two mma.sync shapes the kernel uses
-__device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], const void* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(umma::smem_u32(p)) : "memory");
-}
-__device__ __forceinline__ void ldsm_x4_trans(uint32_t (&r)[4], const void* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(umma::smem_u32(p)) : "memory");
-}
-__device__ __forceinline__ void ldsm_x2(uint32_t (&r)[2], const void* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];"
-               : "=r"(r[0]), "=r"(r[1]) : "r"(umma::smem_u32(p)) : "memory");
+  uint2 pk;
+  *reinterpret_cast<__nv_bfloat162*>(&pk.x) = __floats2bfloat162_rn(v.x, v.y);
+  *reinterpret_cast<__nv_bfloat162*>(&pk.y) = __floats2bfloat162_rn(v.z, v.w);
+  *reinterpret_cast<uint2*>(reinterpret_cast<bf16*>(base) + idx) = pk;
+  const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pk.x));
+  const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pk.y));
+  v = make_float4(lo.x, lo.y, hi.x, hi.y);       // the rounded value is the state from here on
 }
 // thread-block cluster: barrier over all threads of all CTAs, and loads from another CTA's shared memory
 __device__ __forceinline__ void cluster_sync_all() {
@@ -140,11 +135,16 @@ __device__ __forceinline__ float2 ld_cluster_f2(uint32_t addr) {
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// start of a 16-byte aligned range into L2
+__device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
 // c[16x8] += a[16x16] b[16x8]
-__device__ __forceinline__ void mma_16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+__device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 // c[16x8] += a[16x8] b[8x8]
 __device__ __forceinline__ void mma_1688(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
@@ -152,56 +152,84 @@ __device__ __forceinline__ void mma_1688(float (&c)[4], uint32_t a0, uint32_t a1
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(b0));
 }
 
-template <int D, bool SB16>
-__global__ void __launch_bounds__(kStrThreads, 2) nha_decode_stream_kernel(const DecodeStreamArgs a) {
-  using namespace nvcuda::wmma;
+// shared-memory row pitches of a warp's ring slots, in bytes: 16-byte pieces of eight lanes (rows gq, pieces tq for keys;
+// rows 2 tq, pieces gq for values) fall into eight different bank groups
+template <int D> struct DecodeRing {
+  static constexpr int kKRow = D * 2 + 64, kVRow = D * 2 + 16;
+  static constexpr int kKSlot = kGroup * kKRow, kVSlot = kGroup * kVRow;
+  static constexpr int kWarp = 2 * (kKSlot + kVSlot);              // two key slots, two value slots
+};
+
+template <int D, int NT, bool SB16, bool RING>
+__global__ void __launch_bounds__(kStrThreads, NT == 1 ? 2 : 1) nha_decode_stream_kernel(const DecodeStreamArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
-  constexpr int K = D, V = D, ldk = D + 8, ldq = D + 8, ldo = D + 8;
-  constexpr int kSlotBytes = kStrStage * ldk * 2;
-  unsigned char* ring = smem + a.off_ring;                         // [4 slots][64][D+8] bf16
-  float* hvS = reinterpret_cast<float*>(smem + a.off_hv);          // [MQ][V] my rows of hv
-  float* S = reinterpret_cast<float*>(smem + a.off_S);             // [16][nkp+8] logits, then bf16 weights in place
-  float* red = reinterpret_cast<float*>(smem + a.off_red);         // [warps][NG][32] partial slot logits
-  float* qs = reinterpret_cast<float*>(smem + a.off_q);            // [NG][K] raw query, fp32
+  typedef DecodeRing<D> RG;
+  constexpr int K = D, V = D, ldq = D + 8, NH = 8 * NT;            // NH: heads, padded to the products' n tiles
+  constexpr int V4 = V / 4, kRowsI = 32 / V4;                      // lanes of an hv row; hv rows a warp touches at once
+  constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
+  float* qT = reinterpret_cast<float*>(smem + a.off_q);            // [K][NH] raw query, fp32 (columns >= NG zero)
   bf16* sqA = reinterpret_cast<bf16*>(smem + a.off_sqA);           // [16][K+8] rotated query (rows >= NG zero)
-  float* oks = reinterpret_cast<float*>(smem + a.off_oks);         // [NG][MQ] slot logits -> unnormalised weights
   float* eg = reinterpret_cast<float*>(smem + a.off_eg);
   float* sv = reinterpret_cast<float*>(smem + a.off_sv);
   float* kpop = reinterpret_cast<float*>(smem + a.off_kpop);
   float* vpop = reinterpret_cast<float*>(smem + a.off_vpop);
-  float* ml = reinterpret_cast<float*>(smem + a.off_ml);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + a.off_bar);  // [4] ring slots, [4] = hv rows
+  float* wml = reinterpret_cast<float*>(smem + a.off_wml);         // [warps][NH][4] max and sum of the slots, of the window
+  float* ml = reinterpret_cast<float*>(smem + a.off_ml);           // [NG][2] of the split (natural units)
+  float* outp = reinterpret_cast<float*>(smem + a.off_out);        // [NG][V] partial output of the split
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int SPL = a.SPLITS, NG = a.NG, M = a.M, W = a.W, MQ = a.MQ;
   const int bh = blockIdx.x / SPL, sp = blockIdx.x % SPL;
   const int b = bh / a.H, h = bh % a.H;
   const bool rotary = a.cosp != nullptr;
-  const int w0 = sp * a.KSPL;
-  const int nkeys = max(0, min(a.KSPL, W - w0));
-  const int nst = (nkeys + kStrStage - 1) / kStrStage;
-  const int nkp = nst * kStrStage;
-  const int lds = nkp + 8;
   const int m0 = sp * MQ;
   const int nslots = max(0, min(MQ, M - m0));
-  const int nloads = 2 * nst;                                      // key stages, then value stages
-  const bool isring = a.head != nullptr;
+  const int ntask = (nslots + kGroup - 1) / kGroup;                // tasks of eight slots, at most one a warp
+  // this warp's keys: logical window positions [wk0, wk0 + nk), eight at a time
+  int wk0, nk;
+  {
+    const int skeys = max(0, min(a.KSPL, W - sp * a.KSPL)), sgrp = (skeys + kGroup - 1) / kGroup;
+    const int busy = min(ntask, kStrWarps), free_ = kStrWarps - busy;
+    // groups of a warp without slots and of one with: the difference is kSlotCost as far as there are groups for it
+    int gf = (sgrp + busy * kSlotCost + kStrWarps - 1) / kStrWarps;
+    int gb = max(0, gf - kSlotCost);
+    if (free_ * gf + busy * gb < sgrp) gb = (sgrp - free_ * gf + busy - 1) / max(busy, 1);
+    const int first = warp < busy ? warp * gb : busy * gb + (warp - busy) * gf;
+    const int last = min(sgrp, first + (warp < busy ? gb : gf));
+    wk0 = sp * a.KSPL + min(first, sgrp) * kGroup;
+    nk = max(0, min(last * kGroup, skeys) - first * kGroup);
+  }
+  const int ngrp = (nk + kGroup - 1) / kGroup;
   const int WR = a.WR;
+  if (a.pdl) {
+    // The window and the slot memory of this call go into L2 while the kernel in front is still draining.  A prefetch has
+    // no value to get wrong, L2 is where the kernel in front writes, and it also brings the address translations in.
+    // The CTAs of a sequence share its window, which is contiguous over the heads, and those of a (sequence, kv head) its state.
+    const int64_t wbytes = (int64_t)WR * a.H * D * 2, part = (wbytes / (a.H * SPL)) & ~(int64_t)15;
+    const int64_t sbytes = (int64_t)K * M * (SB16 ? 2 : 4), spart = (sbytes / SPL) & ~(int64_t)15;
+    const int idx = h * SPL + sp;
+    if (warp < 4) {
+      const bool win = warp < 2;
+      const char* base = win ? (const char*)(warp == 0 ? a.sw_k : a.sw_v) + b * wbytes + idx * part
+                             : (const char*)(warp == 2 ? a.hk : a.hv) + bh * sbytes + sp * spart;
+      const int64_t n = win ? part : (a.zero_state ? 0 : spart);
+      for (int64_t at = lane * 4096; at < n; at += 32 * 4096) prefetch_l2(base + at, (uint32_t)min((int64_t)4096, n - at));
+    }
+  }
   if (a.pdl == 1) {                                                // before the first global read
     grid_dep_wait();
     grid_dep_launch();
   }
-  const int hd = isring ? (a.nopop ? -1 : a.head[a.g_new ? bh : b]) : 0;   // physical row of the oldest ring entry
+  const int hd = RING ? (a.nopop ? -1 : a.head[a.g_new ? bh : b]) : 0;   // physical row of the oldest ring entry
   // the token that enters the slot memory: separate small tensors, or the oldest ring entry
-  const bool prerot = a.ring_kraw != nullptr;
-  const bf16* kpop_g = isring ? (prerot ? a.ring_kraw : a.sw_k) + (((size_t)b * WR + max(hd, 0)) * a.H + h) * D
+  const bool prerot = RING && a.ring_kraw != nullptr;
+  const bf16* kpop_g = RING ? (prerot ? a.ring_kraw : a.sw_k) + (((size_t)b * WR + max(hd, 0)) * a.H + h) * D
                               : a.k + (size_t)bh * D;
-  const bf16* vpop_g = isring ? a.sw_v + (((size_t)b * WR + max(hd, 0)) * a.H + h) * D : a.v + (size_t)bh * D;
-  const bf16* gpop_g = isring ? a.ring_g + (((size_t)b * WR + max(hd, 0)) * a.H + h) * M : a.g + (size_t)bh * M;
-  bool failed = false;
+  const bf16* vpop_g = RING ? a.sw_v + (((size_t)b * WR + max(hd, 0)) * a.H + h) * D : a.v + (size_t)bh * D;
+  const bf16* gpop_g = RING ? a.ring_g + (((size_t)b * WR + max(hd, 0)) * a.H + h) * M : a.g + (size_t)bh * M;
   // the step's token into the rings (called by the one CTA that finishes this (sequence, kv head))
   auto append_token = [&]() {
-    if (!a.g_new) return;
+    if (!RING || !a.g_new) return;
     const int row = a.nopop ? W - 1 : hd;                          // a filling ring holds W - 1 entries: next free row
     const size_t at = ((size_t)b * WR + row) * a.H + h;
     uint4* rk = reinterpret_cast<uint4*>(const_cast<bf16*>(a.sw_k) + at * D);
@@ -219,91 +247,76 @@ __global__ void __launch_bounds__(kStrThreads, 2) nha_decode_stream_kernel(const
     if (tid == 0 && !a.nopop) const_cast<int*>(a.head)[bh] = hd + 1 == WR ? 0 : hd + 1;
   };
 
-  if (tid == 0) {
-    for (int i = 0; i < kStrSlots + 1; ++i) umma::mbar_init(&bars[i], 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
-
-  // ring load j (j < nst: keys of stage j; else values of stage j - nst) into slot j % 4 by 16-byte asynchronous
-  // copies.  A warp copies, rotates and multiplies only ITS OWN eight rows of every stage (rows 8 warp .. 8 warp + 7),
-  // so a stage is handed from the copies to the arithmetic by cp.async.wait_group + __syncwarp alone and the loops
-  // below hold no block-wide barrier.  A lane always copies the same 16-byte column, so the address arithmetic
-  // is one add per copy; rows past the end of the split are zero-filled.  One commit group per load and thread:
-  // groups complete in order, which is the order the stages are consumed in.
+  // Load j of this warp: keys (j even) or values (j odd) of its group j / 2, into slot (j / 2) & 1 of that kind.  A lane
+  // always copies the same 16-byte column; rows past the warp's keys are zero-filled.  One commit group per load: groups
+  // complete in order, which is the order they are used in.
+  unsigned char* ring = smem + a.off_ring + warp * RG::kWarp;
   constexpr int kC8 = D / 8;                                       // 16-byte columns of a row
   constexpr int kRStep = 32 / kC8;                                 // rows between two copies of a lane
-  const int lc = lane % kC8, lr = 8 * warp + lane / kC8;
-#define NHA_ISSUE_LOAD(j_)                                                                          \
-  do {                                                                                              \
-    const int j__ = (j_);                                                                           \
-    const int st__ = j__ < nst ? j__ : j__ - nst;                                                   \
-    const bf16* base__ = (j__ < nst ? a.sw_k : a.sw_v) + ((size_t)b * WR * a.H + h) * D + 8 * lc;   \
-    const bf16* new__ = (j__ < nst ? a.k : a.v) + (size_t)bh * D + 8 * lc;                          \
-    unsigned char* dst__ = ring + (j__ % kStrSlots) * kSlotBytes + 16 * lc;                         \
-    const int rows__ = min(kStrStage, nkeys - st__ * kStrStage);                                    \
-    _Pragma("unroll") for (int i__ = 0; i__ < kC8 / 4; ++i__) {                                     \
-      const int r__ = lr + i__ * kRStep;                                                            \
-      const bool ok__ = r__ < rows__;                                                               \
-      const int lw__ = w0 + st__ * kStrStage + (ok__ ? r__ : 0);      /* logical window index */    \
-      const bf16* src__;                                                                            \
-      if (!isring) src__ = base__ + (size_t)lw__ * a.H * D;                                         \
-      else if (lw__ == W - 1) src__ = new__;                          /* the token of this step */  \
-      else { int pr__ = hd + 1 + lw__; if (pr__ >= WR) pr__ -= WR; src__ = base__ + (size_t)pr__ * a.H * D; } \
-      umma::cp16(dst__ + r__ * ldk * 2, src__, ok__);                                               \
-    }                                                                                               \
-    umma::cp_commit();                                                                              \
-  } while (0)
-// wait until ring load j_ has landed: the loads issued after it may stay in flight
-#define NHA_WAIT_LOAD(j_, issued_)                                                                  \
-  do {                                                                                              \
-    const int pend__ = (issued_) - (j_) - 1;                                                        \
-    if (pend__ >= 3) asm volatile("cp.async.wait_group 3;\n" ::);                                   \
-    else if (pend__ == 2) asm volatile("cp.async.wait_group 2;\n" ::);                              \
-    else if (pend__ == 1) asm volatile("cp.async.wait_group 1;\n" ::);                              \
-    else asm volatile("cp.async.wait_group 0;\n" ::);                                               \
-  } while (0)
+  const int lc = lane % kC8, lr = lane / kC8;
+  const uint32_t rpitch = a.H * D;
+  const bf16* kbase = a.sw_k + ((size_t)b * WR * a.H + h) * D + 8 * lc;
+  const bf16* vbase = a.sw_v + ((size_t)b * WR * a.H + h) * D + 8 * lc;
+  // (rows past the warp's keys repeat its last one: their logits are masked and their weights are zero.  Every call commits
+  // a group, empty past the last load: a warp always has kAhead groups behind the one it waits for.)
+  const int rlast = wk0 + nk - 1;
+  auto issue = [&](int g, auto kind) {
+    constexpr int kv = decltype(kind)::value, pitch = kv ? RG::kVRow : RG::kKRow;
+    if (g < ngrp) {
+      const bf16* base = kv ? vbase : kbase;
+      unsigned char* dst = ring + (kv ? 2 * RG::kKSlot : 0) + (g & 1) * (kv ? RG::kVSlot : RG::kKSlot) + 16 * lc + lr * pitch;
+      const int r0 = wk0 + g * kGroup + lr;
+#pragma unroll
+      for (int i = 0; i < kGroup / kRStep; ++i) {
+        int row = min(r0 + i * kRStep, rlast);                     // logical window index, then physical row
+        const bf16* src;
+        if (RING) {
+          const bool fresh = row == W - 1;                         // the token of this step
+          row += hd + 1;
+          row -= row >= WR ? WR : 0;
+          src = fresh ? (kv ? a.v : a.k) + (size_t)bh * D + 8 * lc : base + (uint64_t)((uint32_t)row) * rpitch;
+        } else {
+          src = base + (uint64_t)((uint32_t)row) * rpitch;
+        }
+        umma::cp16(dst + i * kRStep * pitch, src, true);
+      }
+    }
+    umma::cp_commit();
+  };
+  constexpr std::integral_constant<int, 0> kKeys{};
+  constexpr std::integral_constant<int, 1> kValues{};
+  // wait until the oldest load in flight has landed: the kAhead - 1 issued after it may stay
+  auto wait_load = [&]() {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(kAhead - 1) : "memory");
+    __syncwarp();                                                  // every lane's copies have landed
+  };
 
-  // ---- the small inputs first, into registers, so that they are not queued behind the window in the memory system;
-  //      then everything that fits goes in flight: my columns of hk, the first ring loads, my rows of hv.
-  //      Disjoint groups of threads fetch the four small inputs, so that their loads overlap. ----------------------
-  // my columns of hk: thread -> column m = lane (+32 per block of columns), rows k = kRowsPer warp + j.  The first
-  // block of columns (all of them unless the split owns more than 32 slots) is fetched in the prologue.
-  constexpr int kRowsPer = K / kStrWarps;
-  float hreg[kRowsPer];
-  const int ncb = (nslots + 31) / 32;
-#define NHA_LOAD_HK_FIRST()                                                                         \
-  do {                                                                                              \
-    if (!a.zero_state && nslots > 0) {                                                              \
-      _Pragma("unroll") for (int j = 0; j < kRowsPer; ++j)                                          \
-        hreg[j] = lane < nslots ? ld_state(a.hk, ((size_t)bh * K + kRowsPer * warp + j) * M + m0 + lane, SB16) : 0.f; \
-    }                                                                                               \
-  } while (0)
-#define NHA_LOAD_HV_ROWS()                                                                          \
-  do {                                                                                              \
-    if (nslots > 0 && !a.zero_state && tid == 0) {                                                  \
-      if (SB16) {     /* bf16 rows land in the second half of their fp32 home */                \
-        mbar_expect(&bars[kStrSlots], (uint32_t)nslots * V * 2);                                    \
-        bulk_g2s(reinterpret_cast<bf16*>(hvS) + (size_t)nslots * V,                                 \
-                 reinterpret_cast<const bf16*>(a.hv) + ((size_t)bh * M + m0) * V, (uint32_t)nslots * V * 2, &bars[kStrSlots]); \
-      } else {                                                                                      \
-        mbar_expect(&bars[kStrSlots], (uint32_t)nslots * V * 4);                                    \
-        bulk_g2s(hvS, a.hv + ((size_t)bh * M + m0) * V, (uint32_t)nslots * V * 4, &bars[kStrSlots]); \
-      }                                                                                             \
-    }                                                                                               \
-  } while (0)
+  // ---- requests: the small inputs, the first task's slot memory into registers, the first window loads ------------------
+  // hk of a task: lane -> slots 4 (lane & 1) .. + 3 of the eight, rows 16 i + lane / 2; hv: rows (slots) kRowsI u + lane / V4
+  constexpr int kHk = K / 16, kHv = kGroup / kRowsI;
+  const int hs = 4 * (lane & 1), hr = lane >> 1;
+  const int vsub = lane / V4, vcol = 4 * (lane % V4);
+  float4 hreg[kHk], vreg[kHv];
+  auto load_state = [&]() {
+    const int ms = kGroup * warp;
+#pragma unroll
+    for (int i = 0; i < kHk; ++i)
+      hreg[i] = !a.zero_state && ms + hs < nslots ? ld_state4<SB16>(a.hk, ((size_t)bh * K + 16 * i + hr) * M + m0 + ms + hs)
+                                                  : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int u = 0; u < kHv; ++u)
+      vreg[u] = !a.zero_state && ms + kRowsI * u + vsub < nslots
+                    ? ld_state4<SB16>(a.hv, ((size_t)bh * M + m0 + ms + kRowsI * u + vsub) * V + vcol) : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
   // Dependent launch with early requests (pdl == 2): the state and the window of this call do not depend on the
   // kernel in front, so they go in flight before the wait.  In ring mode the newest window entry is the token of
-  // this step (a.k / a.v, written by the caller's projections): the ring loads from the first one that holds it on
-  // are issued after the wait, in the same order as always (groups complete in issue order).
-  const int ninit = min(nloads, kStrSlots);
-  int npre = 0;
+  // this step (a.k / a.v, written by the caller's projections): the loads from the first one that holds it on
+  // are issued after the wait, in the same order as always.
+  int npre = 0;                                                    // groups requested before the wait
   if (a.pdl == 2) {
-    npre = ninit;
-    if (isring && w0 + nkeys == W && nst > 0) npre = min(npre, nst - 1);
-    NHA_LOAD_HK_FIRST();
-    for (int j = 0; j < npre; ++j) NHA_ISSUE_LOAD(j);
-    NHA_LOAD_HV_ROWS();
+    npre = kAhead / 2;
+    if (RING && nk > 0 && wk0 + nk == W) npre = min(npre, ngrp - 1);
+    for (int g = 0; g < npre; ++g) { issue(g, kKeys); issue(g, kValues); }
     grid_dep_wait();
     grid_dep_launch();
   }
@@ -329,7 +342,6 @@ __global__ void __launch_bounds__(kStrThreads, 2) nha_decode_stream_kernel(const
       rq_c2 = __ldg(reinterpret_cast<const uint4*>(srow + 8 * (q_c + c8h)));
     }
   }
-  if (a.pdl != 2) NHA_LOAD_HK_FIRST();
   // the gates (threads 0..63) and the popped token (one warp each for k and v)
   bf16 gb[2], sb[2];
   gb[0] = gb[1] = sb[0] = sb[1] = f2bf(0.f);
@@ -348,10 +360,7 @@ __global__ void __launch_bounds__(kStrThreads, 2) nha_decode_stream_kernel(const
   } else if (tid < 128) {
     if (tid - 96 < (V >> 3) && !a.nopop) rpop = __ldg(reinterpret_cast<const uint4*>(vpop_g + 8 * (tid - 96)));
   }
-  for (int j = npre; j < ninit; ++j) NHA_ISSUE_LOAD(j);
-  if (a.pdl != 2) NHA_LOAD_HV_ROWS();
-#undef NHA_LOAD_HK_FIRST
-#undef NHA_LOAD_HV_ROWS
+  for (int g = npre; g < kAhead / 2; ++g) { issue(g, kKeys); issue(g, kValues); }
   // registers -> shared memory
   if (tid < 64) {
 #pragma unroll
@@ -378,10 +387,11 @@ __global__ void __launch_bounds__(kStrThreads, 2) nha_decode_stream_kernel(const
     }
   } else if (qthread) {
     uint4 o1 = make_uint4(0u, 0u, 0u, 0u), o2 = o1;
+    float x[8], y[8];
+    unpack8(rq_x, x); unpack8(rq_y, y);
     if (qlive) {
       if (rotary) {
-        float x[8], y[8], c1[8], s1[8], c2[8], s2[8], p1[8], p2[8];
-        unpack8(rq_x, x); unpack8(rq_y, y);
+        float c1[8], s1[8], c2[8], s2[8], p1[8], p2[8];
         unpack8(rq_c1, c1); unpack8(rq_s1, s1); unpack8(rq_c2, c2); unpack8(rq_s2, s2);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
@@ -392,330 +402,317 @@ __global__ void __launch_bounds__(kStrThreads, 2) nha_decode_stream_kernel(const
       } else {
         o1 = rq_c1; o2 = rq_c2;
       }
-      float fx[8], fy[8];
-      unpack8(rq_x, fx); unpack8(rq_y, fy);
-      float4* qd = reinterpret_cast<float4*>(qs + q_r * K + 8 * q_c);
-      qd[0] = make_float4(fx[0], fx[1], fx[2], fx[3]);
-      qd[1] = make_float4(fx[4], fx[5], fx[6], fx[7]);
-      qd = reinterpret_cast<float4*>(qs + q_r * K + 8 * (q_c + c8h));
-      qd[0] = make_float4(fy[0], fy[1], fy[2], fy[3]);
-      qd[1] = make_float4(fy[4], fy[5], fy[6], fy[7]);
+    }
+    if (q_r < NH) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        qT[(8 * q_c + e) * NH + q_r] = x[e];
+        qT[(8 * (q_c + c8h) + e) * NH + q_r] = y[e];
+      }
     }
     *reinterpret_cast<uint4*>(sqA + q_r * ldq + 8 * q_c) = o1;
     *reinterpret_cast<uint4*>(sqA + q_r * ldq + 8 * (q_c + c8h)) = o2;
   }
   __syncthreads();
-  // ---- my columns of hk <- hk exp(g) + k s^T (registers -> global), partial slot logits of every query head ----
-  for (int cb = 0; cb < ncb; ++cb) {
-    const int m = 32 * cb + lane;
-    if (cb > 0 && !a.zero_state) {
-#pragma unroll
-      for (int j = 0; j < kRowsPer; ++j)
-        hreg[j] = m < nslots ? ld_state(a.hk, ((size_t)bh * K + kRowsPer * warp + j) * M + m0 + m, SB16) : 0.f;
-    }
-    const float e = m < MQ ? eg[m] : 1.f, sm = m < MQ ? sv[m] : 0.f;
-    float hval[kRowsPer];
-#pragma unroll
-    for (int j = 0; j < kRowsPer; ++j) {
-      const int kk = kRowsPer * warp + j;
-      hval[j] = (a.zero_state ? 0.f : hreg[j]) * e + kpop[kk] * sm;
-      if (m < nslots) st_state(a.hk, ((size_t)bh * K + kk) * M + m0 + m, hval[j], SB16);
-    }
-    // this warp's rows of every query head: 16-byte loads of the query (the same address for all lanes)
-#pragma unroll
-    for (int qh = 0; qh < 16; ++qh) {
-      if (qh < NG) {
-        float acc = 0.f;
-#pragma unroll
-        for (int c4 = 0; c4 < kRowsPer / 4; ++c4) {
-          const float4 q4 = *reinterpret_cast<const float4*>(qs + qh * K + kRowsPer * warp + 4 * c4);
-          acc += q4.x * hval[4 * c4] + q4.y * hval[4 * c4 + 1] + q4.z * hval[4 * c4 + 2] + q4.w * hval[4 * c4 + 3];
-        }
-        red[(warp * NG + qh) * 32 + lane] = acc;
-      }
-    }
-    __syncthreads();
-    for (int i = tid; i < NG * 32; i += kStrThreads) {
-      const int qh = i >> 5, l = i & 31;
-      float sum = 0.f;
-#pragma unroll
-      for (int w8 = 0; w8 < kStrWarps; ++w8) sum += red[(w8 * NG + qh) * 32 + l];
-      if (32 * cb + l < MQ) oks[qh * MQ + 32 * cb + l] = sum * a.scale;
-    }
-    __syncthreads();
-  }
+  const float sc2 = a.scale * kLog2e;
+  constexpr float kRaise = 8.f;
 
-  // ---- key stages, warp-private: wait for my rows, rotate-half in place, S[:, my 8 keys] = sq K^T by m16n8k16 MMAs
-  //      with the query fragments held in registers; the freed rows take the next ring load -------------------------
-  constexpr int kTasks = 8 * c8h / 32;                             // rotary tasks per lane (8 values x 2 halves each)
+
+  // ---- the window, eight keys at a time --------------------------------------------------------------------------------
   const int gq = lane >> 2, tq = lane & 3;                         // fragment coordinates of the lane
-  uint32_t afr[K / 16][4];
+  float oacc[NT][D / 64][4][4];                                    // [heads 2 tq, 2 tq + 1 of tile t][columns 64 j + 8 gq + 2 u, + 1]
+  float m_run[NT], l_run[NT];                                      // of head gq + 8 t
 #pragma unroll
-  for (int ks = 0; ks < K / 16; ++ks) ldsm_x4(afr[ks], sqA + (lane & 15) * ldq + 16 * ks + 8 * (lane >> 4));
-  uint4 cs[kTasks][4];                                             // rotate-half table entries of the stage being rotated
-#define NHA_LOAD_TABLE(st_)                                                                         \
-  _Pragma("unroll") for (int u = 0; u < kTasks; ++u) {                                              \
-    const int i = lane + 32 * u;                                                                    \
-    const int r = i / c8h, c = i - r * c8h;                                                         \
-    const int wraw = w0 + (st_) * kStrStage + 8 * warp + r;                                         \
-    const int wpos = min(wraw, W - 1);                                                              \
-    if (!prerot || wraw == W - 1) {                     /* rotated ring: only the token of this step */ \
-      const bf16* crow = a.cosp + b * a.cs_batch + (int64_t)wpos * a.cs_row;                        \
-      const bf16* srow = a.sinp + b * a.cs_batch + (int64_t)wpos * a.cs_row;                        \
-      cs[u][0] = __ldg(reinterpret_cast<const uint4*>(crow + 8 * c));                               \
-      cs[u][1] = __ldg(reinterpret_cast<const uint4*>(srow + 8 * c));                               \
-      cs[u][2] = __ldg(reinterpret_cast<const uint4*>(crow + 8 * (c + c8h)));                       \
-      cs[u][3] = __ldg(reinterpret_cast<const uint4*>(srow + 8 * (c + c8h)));                       \
-    }                                                                                               \
+  for (int t = 0; t < NT; ++t) {
+    m_run[t] = -INFINITY;
+    l_run[t] = 0.f;
+#pragma unroll
+    for (int j = 0; j < D / 64; ++j)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) oacc[t][j][u][0] = oacc[t][j][u][1] = oacc[t][j][u][2] = oacc[t][j][u][3] = 0.f;
   }
-  if (rotary && nst > 0) { NHA_LOAD_TABLE(0) }
-  for (int st = 0; st < nst; ++st) {
-    const int slot = st % kStrSlots;
-    bf16* kst = reinterpret_cast<bf16*>(ring + slot * kSlotBytes) + (size_t)8 * warp * ldk;   // my rows of the stage
-    NHA_WAIT_LOAD(st, min(nloads, kStrSlots + st));
-    __syncwarp();                                                  // every lane's copies of my rows have landed
+  constexpr int kHalf = D / 64;                                    // 16-byte pieces of a lane in each half of a key row
+  uint4 cs[kHalf][4];                                              // rotate-half table entries of the group's key gq
+  const bf16* ctab = rotary ? a.cosp + b * a.cs_batch + 8 * tq : nullptr;
+  const bf16* stab = rotary ? a.sinp + b * a.cs_batch + 8 * tq : nullptr;
+  auto load_table = [&](int g) {
+    const int lw = wk0 + min(g * kGroup + gq, nk - 1);
+    if (prerot && lw != W - 1) return;                             // rotated ring: only the token of this step is rotated
+    const uint64_t at = (uint64_t)(uint32_t)lw * (uint32_t)a.cs_row;
+#pragma unroll
+    for (int i = 0; i < kHalf; ++i) {
+      cs[i][0] = __ldg(reinterpret_cast<const uint4*>(ctab + at + 32 * i));
+      cs[i][1] = __ldg(reinterpret_cast<const uint4*>(stab + at + 32 * i));
+      cs[i][2] = __ldg(reinterpret_cast<const uint4*>(ctab + at + 32 * i + D / 2));
+      cs[i][3] = __ldg(reinterpret_cast<const uint4*>(stab + at + 32 * i + D / 2));
+    }
+  };
+  if (rotary && ngrp > 0) load_table(0);
+#pragma unroll 1
+  for (int g = 0; g < ngrp; ++g) {
+    const unsigned char* kst = ring + (g & 1) * RG::kKSlot + gq * RG::kKRow + 16 * tq;
+    wait_load();
+    uint4 kf[2 * kHalf];
+#pragma unroll
+    for (int i = 0; i < 2 * kHalf; ++i) kf[i] = *reinterpret_cast<const uint4*>(kst + 64 * i);
     if (rotary) {
+      if (!prerot || wk0 + g * kGroup + gq == W - 1) {
 #pragma unroll
-      for (int u = 0; u < kTasks; ++u) {
-        const int i = lane + 32 * u;
-        const int r = i / c8h, c = i - r * c8h;
-        if (prerot && w0 + st * kStrStage + 8 * warp + r != W - 1) continue;
-        // packed bf16 arithmetic: x c1 - y s1 and y c2 + x s2 on pairs, the first product rounded to bf16
-        uint4 xu = *reinterpret_cast<const uint4*>(kst + r * ldk + 8 * c);
-        uint4 yu = *reinterpret_cast<const uint4*>(kst + r * ldk + 8 * (c + c8h));
-        uint4 o1u, o2u;
-        const __nv_bfloat162* xv = reinterpret_cast<const __nv_bfloat162*>(&xu);
-        const __nv_bfloat162* yv = reinterpret_cast<const __nv_bfloat162*>(&yu);
-        const __nv_bfloat162* c1v = reinterpret_cast<const __nv_bfloat162*>(&cs[u][0]);
-        const __nv_bfloat162* s1v = reinterpret_cast<const __nv_bfloat162*>(&cs[u][1]);
-        const __nv_bfloat162* c2v = reinterpret_cast<const __nv_bfloat162*>(&cs[u][2]);
-        const __nv_bfloat162* s2v = reinterpret_cast<const __nv_bfloat162*>(&cs[u][3]);
-        __nv_bfloat162* o1v = reinterpret_cast<__nv_bfloat162*>(&o1u);
-        __nv_bfloat162* o2v = reinterpret_cast<__nv_bfloat162*>(&o2u);
+        for (int i = 0; i < kHalf; ++i) {
+          // packed bf16 arithmetic: x c1 - y s1 and y c2 + x s2 on pairs, the first product rounded to bf16
+          const __nv_bfloat162* c1v = reinterpret_cast<const __nv_bfloat162*>(&cs[i][0]);
+          const __nv_bfloat162* s1v = reinterpret_cast<const __nv_bfloat162*>(&cs[i][1]);
+          const __nv_bfloat162* c2v = reinterpret_cast<const __nv_bfloat162*>(&cs[i][2]);
+          const __nv_bfloat162* s2v = reinterpret_cast<const __nv_bfloat162*>(&cs[i][3]);
+          __nv_bfloat162* xv = reinterpret_cast<__nv_bfloat162*>(&kf[i]);
+          __nv_bfloat162* yv = reinterpret_cast<__nv_bfloat162*>(&kf[i + kHalf]);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          o1v[e] = __hfma2(xv[e], c1v[e], __hneg2(__hmul2(yv[e], s1v[e])));
-          o2v[e] = __hfma2(yv[e], c2v[e], __hmul2(xv[e], s2v[e]));
+          for (int e = 0; e < 4; ++e) {
+            const __nv_bfloat162 x = xv[e], y = yv[e];
+            xv[e] = __hfma2(x, c1v[e], __hneg2(__hmul2(y, s1v[e])));
+            yv[e] = __hfma2(y, c2v[e], __hmul2(x, s2v[e]));
+          }
         }
-        *reinterpret_cast<uint4*>(kst + r * ldk + 8 * c) = o1u;
-        *reinterpret_cast<uint4*>(kst + r * ldk + 8 * (c + c8h)) = o2u;
       }
-      // the next stage's table entries travel while this stage's logits are formed
-      if (st + 1 < nst) { NHA_LOAD_TABLE(st + 1) }
-      __syncwarp();
+      if (g + 1 < ngrp) load_table(g + 1);                         // travels while this group is worked on
     }
     float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int k2 = 0; k2 < K / 32; ++k2) {
-      uint32_t bfr[4];                                             // my 8 keys x 32 features: two k-steps
-      ldsm_x4(bfr, kst + (lane & 7) * ldk + 32 * k2 + 8 * (lane >> 3));
-      mma_16816(c0, afr[2 * k2], bfr[0], bfr[1]);
-      mma_16816(c1, afr[2 * k2 + 1], bfr[2], bfr[3]);
+    for (int jj = 0; jj < D / 32; ++jj) {
+      // the query fragments are read anew for every group: they would not fit the registers beside the table entries
+      const uint4 qh0 = *reinterpret_cast<const uint4*>(sqA + gq * ldq + 8 * (tq + 4 * jj));
+      const uint4 qh1 = NT > 1 ? *reinterpret_cast<const uint4*>(sqA + (gq + 8) * ldq + 8 * (tq + 4 * jj)) : make_uint4(0u, 0u, 0u, 0u);
+      mma_16816(c0, qh0.x, qh1.x, qh0.y, qh1.y, kf[jj].x, kf[jj].y);
+      mma_16816(c1, qh0.z, qh1.z, qh0.w, qh1.w, kf[jj].z, kf[jj].w);
     }
-    float* sdst = S + st * kStrStage + 8 * warp + 2 * tq;
-    *reinterpret_cast<float2*>(sdst + (size_t)gq * lds) = make_float2(c0[0] + c1[0], c0[1] + c1[1]);
-    *reinterpret_cast<float2*>(sdst + (size_t)(gq + 8) * lds) = make_float2(c0[2] + c1[2], c0[3] + c1[3]);
-    __syncwarp();                                                  // every lane is done with my rows of the slot
-    if (st + kStrSlots < nloads) NHA_ISSUE_LOAD(st + kStrSlots);
-  }
-#undef NHA_LOAD_TABLE
-  __syncthreads();                                                 // all logits of the CTA are in S
-
-  // ---- my rows of hv <- diag(exp(g)) hv + s v^T (in place; they arrived behind the keys) ----------------------------
-  constexpr int V4 = V >> 2;
-  if (nslots > 0) {
-    if (!a.zero_state && !umma::mbar_wait(&bars[kStrSlots], 0)) failed = true;
-    float4* hg = reinterpret_cast<float4*>(a.hv + ((size_t)bh * M + m0) * V);
-    uint2* hg16 = reinterpret_cast<uint2*>(reinterpret_cast<bf16*>(a.hv) + ((size_t)bh * M + m0) * V);
-    const uint2* stage16 = reinterpret_cast<const uint2*>(reinterpret_cast<const bf16*>(hvS) + (size_t)nslots * V);
-    // four elements per thread and round: all loads of a round before its stores.  bf16 states: the rows were staged
-    // in the second half of the fp32 rows they are expanded into, so a block barrier separates a round's loads from its
-    // stores (round r writes the bytes [16 KB r, 16 KB (r + 1)), the staging of the later rounds lies behind them)
-    for (int i0 = tid; i0 - tid < nslots * V4; i0 += 4 * kStrThreads) {
-      float4 hh[4], vp4[4];
-      float e[4], sm[4];
+    // softmax step of head gq (+ 8): this lane has keys 2 tq, 2 tq + 1 of the group
+    const int left = nk - g * kGroup - 2 * tq;
+    uint32_t pb[NT];
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+      const float x0 = left > 0 ? (c0[2 * t] + c1[2 * t]) * sc2 : -INFINITY;
+      const float x1 = left > 1 ? (c0[2 * t + 1] + c1[2 * t + 1]) * sc2 : -INFINITY;
+      float mx = fmaxf(x0, x1);
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+      const bool raise = mx > m_run[t] + kRaise;                   // weights stay below 2^8, exact enough in fp32 sums
+      if (__any_sync(0xffffffffu, raise)) {
+        const float f = raise ? exp2f(m_run[t] - mx) : 1.f;        // 0 when nothing came before
+        if (raise) m_run[t] = mx;
+        l_run[t] *= f;
+        const float f0 = __shfl_sync(0xffffffffu, f, 8 * tq), f1 = __shfl_sync(0xffffffffu, f, 8 * tq + 4);
+#pragma unroll
+        for (int j = 0; j < D / 64; ++j)
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            oacc[t][j][u][0] *= f0; oacc[t][j][u][1] *= f1;
+            oacc[t][j][u][2] *= f0; oacc[t][j][u][3] *= f1;
+          }
+      }
+      const float p0 = exp2f(x0 - m_run[t]), p1 = exp2f(x1 - m_run[t]);
+      l_run[t] += p0 + p1;
+      const __nv_bfloat162 pk = __floats2bfloat162_rn(p0, p1);
+      pb[t] = *reinterpret_cast<const uint32_t*>(&pk);
+    }
+    __syncwarp();                                                  // every lane is done with the key slot
+    issue(g + kAhead / 2, kKeys);
+    wait_load();
+    const unsigned char* vst = ring + 2 * RG::kKSlot + (g & 1) * RG::kVSlot + 2 * tq * RG::kVRow + 16 * gq;
+#pragma unroll
+    for (int j = 0; j < D / 64; ++j) {
+      const uint4 va = *reinterpret_cast<const uint4*>(vst + 128 * j), vb = *reinterpret_cast<const uint4*>(vst + RG::kVRow + 128 * j);
+      const uint32_t ea[4] = {va.x, va.y, va.z, va.w}, eb[4] = {vb.x, vb.y, vb.z, vb.w};
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const int i = i0 + u * kStrThreads;
-        if (i < nslots * V4) {
-          const int m = i / V4, c = i - m * V4;
-          if (a.zero_state) {
-            hh[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-          } else if (SB16) {
-            const uint2 raw = stage16[i];
-            const float2 lo2 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
-            const float2 hi2 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
-            hh[u] = make_float4(lo2.x, lo2.y, hi2.x, hi2.y);
-          } else {
-            hh[u] = *reinterpret_cast<const float4*>(hvS + m * V + 4 * c);
-          }
-          vp4[u] = *reinterpret_cast<const float4*>(vpop + 4 * c);
-          e[u] = eg[m]; sm[u] = sv[m];
-        }
-      }
-      if (SB16) __syncthreads();
+        const uint32_t a0 = __byte_perm(ea[u], eb[u], 0x5410), a1 = __byte_perm(ea[u], eb[u], 0x7632);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int i = i0 + u * kStrThreads;
-        if (i < nslots * V4) {
-          hh[u].x = hh[u].x * e[u] + sm[u] * vp4[u].x;
-          hh[u].y = hh[u].y * e[u] + sm[u] * vp4[u].y;
-          hh[u].z = hh[u].z * e[u] + sm[u] * vp4[u].z;
-          hh[u].w = hh[u].w * e[u] + sm[u] * vp4[u].w;
-          if (SB16) {
-            // the rounded value is the state from here on: the readout uses what the next step will read
-            uint2 pk;
-            *reinterpret_cast<__nv_bfloat162*>(&pk.x) = __floats2bfloat162_rn(hh[u].x, hh[u].y);
-            *reinterpret_cast<__nv_bfloat162*>(&pk.y) = __floats2bfloat162_rn(hh[u].z, hh[u].w);
-            hg16[i] = pk;
-            const float2 lo2 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pk.x));
-            const float2 hi2 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pk.y));
-            reinterpret_cast<float4*>(hvS)[i] = make_float4(lo2.x, lo2.y, hi2.x, hi2.y);
-          } else {
-            reinterpret_cast<float4*>(hvS)[i] = hh[u];
-            hg[i] = hh[u];
-          }
+        for (int t = 0; t < NT; ++t) mma_1688(oacc[t][j][u], a0, a1, pb[t]);
+      }
+    }
+    __syncwarp();                                                  // every lane is done with the value slot
+    issue(g + kAhead / 2, kValues);
+  }
+
+  // ---- the window output into the warp's own (now dead) ring memory: [NG][ldo] ----------------------------------------
+  constexpr int ldo = V + 4, kOut = RG::kWarp / 4;
+  static_assert(16 * ldo * 4 <= RG::kWarp || NT == 1, "a warp's output fits its ring");
+  static_assert(8 * ldo * 4 <= RG::kWarp, "a warp's output fits its ring");
+  float* osm = reinterpret_cast<float*>(smem + a.off_ring);        // warp w: at w kOut
+  float* myml = wml + warp * NH * 4;
+  __syncwarp();
+#pragma unroll
+  for (int t = 0; t < NT; ++t) {
+    float l = l_run[t];
+    l += __shfl_xor_sync(0xffffffffu, l, 1);
+    l += __shfl_xor_sync(0xffffffffu, l, 2);
+    if (tq == 0) *reinterpret_cast<float4*>(myml + 4 * (8 * t + gq)) = make_float4(-INFINITY, 0.f, m_run[t], l);
+#pragma unroll
+    for (int hf = 0; hf < 2; ++hf) {
+      const int qh = 8 * t + 2 * tq + hf;
+      if (qh < NG) {
+        float* orow = osm + warp * kOut + qh * ldo + 8 * gq;
+#pragma unroll
+        for (int j = 0; j < D / 64; ++j) {
+          *reinterpret_cast<float4*>(orow + 64 * j) = make_float4(oacc[t][j][0][hf], oacc[t][j][0][2 + hf], oacc[t][j][1][hf], oacc[t][j][1][2 + hf]);
+          *reinterpret_cast<float4*>(orow + 64 * j + 4) = make_float4(oacc[t][j][2][hf], oacc[t][j][2][2 + hf], oacc[t][j][3][hf], oacc[t][j][3][2 + hf]);
         }
       }
     }
   }
+  __syncwarp();
 
-  // ---- partial softmax over [my slots | my keys], one warp per query head; weights replace the logits in place ---
-  for (int qh = warp; qh < NG; qh += kStrWarps) {
-    float* srow = S + (size_t)qh * lds;
-    bf16* prow = reinterpret_cast<bf16*>(srow);
-    float mx = -INFINITY;
-    for (int m = lane; m < nslots; m += 32) mx = fmaxf(mx, oks[qh * MQ + m]);
-    // a lane takes 8 consecutive keys of every block of 256
-    for (int w8 = 8 * lane; w8 < nkp; w8 += 256) {
-      const float4 x0 = *reinterpret_cast<const float4*>(srow + w8), x1 = *reinterpret_cast<const float4*>(srow + w8 + 4);
-      const float xs[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+  // ---- slot memory: the warp's eight slots (their lines were brought into L2 by the prefetch at the start) -------------
+  float* pS = reinterpret_cast<float*>(smem + a.off_p) + warp * kGroup * NH;     // [8 slots][NH] weights of the task
+  if (warp < ntask) {
+    const int ms = kGroup * warp;
+    load_state();
+    {
+      const float4 e4 = *reinterpret_cast<const float4*>(eg + ms + hs), s4 = *reinterpret_cast<const float4*>(sv + ms + hs);
 #pragma unroll
-      for (int e8 = 0; e8 < 8; ++e8)
-        if (w8 + e8 < nkeys) mx = fmaxf(mx, xs[e8] * a.scale);
+      for (int i = 0; i < kHk; ++i) {
+        const float kk = kpop[16 * i + hr];
+        hreg[i].x = hreg[i].x * e4.x + kk * s4.x;
+        hreg[i].y = hreg[i].y * e4.y + kk * s4.y;
+        hreg[i].z = hreg[i].z * e4.z + kk * s4.z;
+        hreg[i].w = hreg[i].w * e4.w + kk * s4.w;
+        if (ms + hs < nslots) st_state4<SB16>(a.hk, ((size_t)bh * K + 16 * i + hr) * M + m0 + ms + hs, hreg[i]);
+      }
     }
-    mx = warp_max(mx);
-    float sum = 0.f;
-    for (int m = lane; m < nslots; m += 32) {
-      const float e = __expf(oks[qh * MQ + m] - mx);
-      oks[qh * MQ + m] = e;
-      sum += e;
-    }
-    // the bf16 weight of key w lands inside the fp32 logit of key w / 2: convert a block of 256 keys at a time,
-    // blocks in ascending order, reading all of a block before any of it is written
-    for (int blk = 0; blk < nkp; blk += 256) {
-      const int w8 = blk + 8 * lane;
-      float es[8];
-      if (w8 < nkp) {
-        const float4 x0 = *reinterpret_cast<const float4*>(srow + w8), x1 = *reinterpret_cast<const float4*>(srow + w8 + 4);
-        const float xs[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
 #pragma unroll
-        for (int e8 = 0; e8 < 8; ++e8) {
-          es[e8] = w8 + e8 < nkeys ? __expf(xs[e8] * a.scale - mx) : 0.f;
-          sum += es[e8];
+    for (int t = 0; t < NT; ++t) {
+      // logits: acc[4 head + slot], summed over the sixteen lanes that share a slot quad by exchanging halves, after which
+      // a lane holds two neighbouring slots of one head
+      float acc[32];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) acc[i] = 0.f;
+#pragma unroll
+      for (int i = 0; i < kHk; ++i) {
+        const float4 q0 = *reinterpret_cast<const float4*>(qT + (16 * i + hr) * NH + 8 * t);
+        const float4 q1 = *reinterpret_cast<const float4*>(qT + (16 * i + hr) * NH + 8 * t + 4);
+        const float qv[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+#pragma unroll
+        for (int qh = 0; qh < 8; ++qh) {
+          acc[4 * qh] += qv[qh] * hreg[i].x;
+          acc[4 * qh + 1] += qv[qh] * hreg[i].y;
+          acc[4 * qh + 2] += qv[qh] * hreg[i].z;
+          acc[4 * qh + 3] += qv[qh] * hreg[i].w;
         }
       }
-      __syncwarp();
-      if (w8 < nkp) *reinterpret_cast<uint4*>(prow + w8) = pack8(es);
-      __syncwarp();
-    }
-    sum = warp_sum(sum);
-    if (lane == 0) {
-      ml[2 * qh] = (nslots + nkeys) > 0 ? mx : -INFINITY;
-      ml[2 * qh + 1] = sum;
-    }
-  }
-  __syncthreads();
-
-  // ---- slot readout of my output elements, kept in registers while the values stream in ---------------------------
-  float4 sacc[2];
 #pragma unroll
-  for (int u = 0; u < 2; ++u) {
-    sacc[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-    const int i = tid + u * kStrThreads;
-    if (i < NG * V4) {
-      const int qh = i / V4, c = i - qh * V4;
-      // nslots is a multiple of four: four slots at a time, all loads of a block before its arithmetic
-#pragma unroll 2
-      for (int m = 0; m < nslots; m += 4) {
-        const float4 pm = *reinterpret_cast<const float4*>(oks + qh * MQ + m);
-        const float4 h0 = *reinterpret_cast<const float4*>(hvS + m * V + 4 * c);
-        const float4 h1 = *reinterpret_cast<const float4*>(hvS + (m + 1) * V + 4 * c);
-        const float4 h2 = *reinterpret_cast<const float4*>(hvS + (m + 2) * V + 4 * c);
-        const float4 h3 = *reinterpret_cast<const float4*>(hvS + (m + 3) * V + 4 * c);
-        sacc[u].x += pm.x * h0.x; sacc[u].y += pm.x * h0.y; sacc[u].z += pm.x * h0.z; sacc[u].w += pm.x * h0.w;
-        sacc[u].x += pm.y * h1.x; sacc[u].y += pm.y * h1.y; sacc[u].z += pm.y * h1.z; sacc[u].w += pm.y * h1.w;
-        sacc[u].x += pm.z * h2.x; sacc[u].y += pm.z * h2.y; sacc[u].z += pm.z * h2.z; sacc[u].w += pm.z * h2.w;
-        sacc[u].x += pm.w * h3.x; sacc[u].y += pm.w * h3.y; sacc[u].z += pm.w * h3.z; sacc[u].w += pm.w * h3.w;
+      for (int st = 0; st < 4; ++st) {                             // lane bits 4, 3, 2: head; bit 1: slot pair of the quad
+        const int n = 16 >> st, bit = 16 >> st;
+        const bool up = lane & bit;
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+          const float keep = up ? acc[i + n] : acc[i], give = up ? acc[i] : acc[i + n];
+          acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
+        }
       }
-    }
-  }
-
-  // ---- value stages, warp-private: O_w += P[:, my 8 keys] V[my 8 keys, :] by m16n8k8 MMAs, all V columns per warp,
-  //      accumulated in registers; the partial outputs of the eight warps are summed at the end ---------------------
-  float oacc[V / 8][4];
-#pragma unroll
-  for (int nt = 0; nt < V / 8; ++nt) oacc[nt][0] = oacc[nt][1] = oacc[nt][2] = oacc[nt][3] = 0.f;
-  const bf16* P = reinterpret_cast<const bf16*>(S);
-  const int ldp = 2 * lds;
-  for (int st = 0; st < nst; ++st) {
-    const int j = nst + st, slot = j % kStrSlots;
-    const bf16* vst = reinterpret_cast<const bf16*>(ring + slot * kSlotBytes) + (size_t)8 * warp * ldk;
-    NHA_WAIT_LOAD(j, min(nloads, kStrSlots + j));
-    __syncwarp();
-    uint32_t pa[2];
-    ldsm_x2(pa, P + (size_t)(lane & 15) * ldp + st * kStrStage + 8 * warp);
-#pragma unroll
-    for (int n4 = 0; n4 < V / 32; ++n4) {
-      uint32_t vb[4];                                              // my 8 keys x 32 value columns, transposed
-      ldsm_x4_trans(vb, vst + (lane & 7) * ldk + 32 * n4 + 8 * (lane >> 3));
-#pragma unroll
-      for (int t = 0; t < 4; ++t) mma_1688(oacc[4 * n4 + t], pa[0], pa[1], vb[t]);
+      const int qh = 8 * t + (lane >> 2), sl = hs + (lane & 2);    // this lane's head, first of its two slots
+      const float x0 = ms + sl < nslots ? acc[0] * sc2 : -INFINITY, x1 = ms + sl + 1 < nslots ? acc[1] * sc2 : -INFINITY;
+      float mx = fmaxf(x0, x1);
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+      const float p0 = exp2f(x0 - mx), p1 = exp2f(x1 - mx);
+      pS[sl * NH + qh] = p0;
+      pS[(sl + 1) * NH + qh] = p1;
+      float sum = p0 + p1;
+      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+      if ((lane & 3) == 0) {
+        myml[4 * qh] = mx;
+        myml[4 * qh + 1] = sum;
+      }
     }
     __syncwarp();
-    if (j + kStrSlots < nloads) NHA_ISSUE_LOAD(j + kStrSlots);
-  }
-#undef NHA_ISSUE_LOAD
-#undef NHA_WAIT_LOAD
-  __syncthreads();                                                 // the logits / weights and the ring are dead
-  float* osm = reinterpret_cast<float*>(ring);                     // [8 warps][16][V+8] window parts of the output
-  {
-    float* ow = osm + (size_t)warp * 16 * ldo + 2 * tq;
+    float sacc[NT][8][4];                                          // readout of the warp's slots: heads 8 t + i, columns vcol ..
 #pragma unroll
-    for (int nt = 0; nt < V / 8; ++nt) {
-      *reinterpret_cast<float2*>(ow + gq * ldo + 8 * nt) = make_float2(oacc[nt][0], oacc[nt][1]);
-      *reinterpret_cast<float2*>(ow + (gq + 8) * ldo + 8 * nt) = make_float2(oacc[nt][2], oacc[nt][3]);
+    for (int t = 0; t < NT; ++t)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) sacc[t][i][0] = sacc[t][i][1] = sacc[t][i][2] = sacc[t][i][3] = 0.f;
+    const float4 vp = *reinterpret_cast<const float4*>(vpop + vcol);
+#pragma unroll
+    for (int u = 0; u < kHv; ++u) {
+      const int m = ms + kRowsI * u + vsub;
+      if (m < nslots) {
+        const float e = eg[m], sm = sv[m];
+        vreg[u].x = vreg[u].x * e + sm * vp.x;
+        vreg[u].y = vreg[u].y * e + sm * vp.y;
+        vreg[u].z = vreg[u].z * e + sm * vp.z;
+        vreg[u].w = vreg[u].w * e + sm * vp.w;
+        st_state4<SB16>(a.hv, ((size_t)bh * M + m0 + m) * V + vcol, vreg[u]);
+      }
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        const float4 p0 = *reinterpret_cast<const float4*>(pS + (kRowsI * u + vsub) * NH + 8 * t);
+        const float4 p1 = *reinterpret_cast<const float4*>(pS + (kRowsI * u + vsub) * NH + 8 * t + 4);
+        const float p[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          sacc[t][i][0] += p[i] * vreg[u].x; sacc[t][i][1] += p[i] * vreg[u].y;
+          sacc[t][i][2] += p[i] * vreg[u].z; sacc[t][i][3] += p[i] * vreg[u].w;
+        }
+      }
     }
+    // slots and window of the warp together
+#pragma unroll
+    for (int t = 0; t < NT; ++t)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int qh = 8 * t + i;
+        float4 x = make_float4(sacc[t][i][0], sacc[t][i][1], sacc[t][i][2], sacc[t][i][3]);
+        if (kRowsI == 2) {                                         // D = 64: the two halves of the warp hold different slots
+          x.x += __shfl_xor_sync(0xffffffffu, x.x, 16); x.y += __shfl_xor_sync(0xffffffffu, x.y, 16);
+          x.z += __shfl_xor_sync(0xffffffffu, x.z, 16); x.w += __shfl_xor_sync(0xffffffffu, x.w, 16);
+        }
+        if (qh < NG && (kRowsI == 1 || lane < 16)) {
+          const float m1 = myml[4 * qh], m2 = myml[4 * qh + 2], mx = fmaxf(m1, m2);
+          const float f1 = exp2f(m1 - mx), f2 = exp2f(m2 - mx);    // the slots' maximum is finite
+          float4* o4 = reinterpret_cast<float4*>(osm + warp * kOut + qh * ldo + vcol);
+          const float4 w4 = *o4;
+          *o4 = make_float4(f1 * x.x + f2 * w4.x, f1 * x.y + f2 * w4.y, f1 * x.z + f2 * w4.z, f1 * x.w + f2 * w4.w);
+        }
+      }
   }
-
   __syncthreads();
-  // partial output of this split: slot part + window part, unnormalised
   float* po = a.part_o + ((size_t)bh * SPL + sp) * NG * V;
+  auto store_row = [&](int qh, int c, const float4& x) {
+    uint2 pk;
+    *reinterpret_cast<__nv_bfloat162*>(&pk.x) = __floats2bfloat162_rn(x.x, x.y);
+    *reinterpret_cast<__nv_bfloat162*>(&pk.y) = __floats2bfloat162_rn(x.z, x.w);
+    *reinterpret_cast<uint2*>(a.o + ((size_t)b * a.HQ + h * NG + qh) * V + 4 * c) = pk;
+  };
+  for (int i = tid; i < NG * V4; i += kStrThreads) {
+    const int qh = i / V4, c = i - qh * V4;
+    float mw[kStrWarps], lw[kStrWarps], mx = -INFINITY;
 #pragma unroll
-  for (int u = 0; u < 2; ++u) {
-    const int i = tid + u * kStrThreads;
-    if (i < NG * V4) {
-      const int qh = i / V4, c = i - qh * V4;
-      float4 acc = sacc[u];
-      if (nkeys > 0) {
+    for (int w8 = 0; w8 < kStrWarps; ++w8) {
+      const float4 s4 = *reinterpret_cast<const float4*>(wml + (w8 * NH + qh) * 4);
+      mw[w8] = fmaxf(s4.x, s4.z);
+      lw[w8] = (s4.x > -INFINITY ? s4.y * exp2f(s4.x - mw[w8]) : 0.f) + (s4.z > -INFINITY ? s4.w * exp2f(s4.z - mw[w8]) : 0.f);
+      mx = fmaxf(mx, mw[w8]);
+    }
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    float den = 0.f;
 #pragma unroll
-        for (int w8 = 0; w8 < kStrWarps; ++w8) {
-          const float4 wv = *reinterpret_cast<const float4*>(osm + ((size_t)w8 * 16 + qh) * ldo + 4 * c);
-          acc.x += wv.x; acc.y += wv.y; acc.z += wv.z; acc.w += wv.w;
-        }
-      }
-      if (SPL == 1) {
-        const float inv = 1.0f / ml[2 * qh + 1];
-        bf16* orow = a.o + ((size_t)b * a.HQ + h * NG + qh) * V + 4 * c;
-        orow[0] = f2bf(acc.x * inv); orow[1] = f2bf(acc.y * inv); orow[2] = f2bf(acc.z * inv); orow[3] = f2bf(acc.w * inv);
-      } else if (a.cluster) {
-        *reinterpret_cast<float4*>(hvS + qh * V + 4 * c) = acc;      // my rows of hv are dead: the partial output goes there
-      } else {
-        *reinterpret_cast<float4*>(po + qh * V + 4 * c) = acc;
+    for (int w8 = 0; w8 < kStrWarps; ++w8) {
+      const float wgt = mw[w8] > -INFINITY ? exp2f(mw[w8] - mx) : 0.f;
+      const float4 wv = *reinterpret_cast<const float4*>(osm + w8 * kOut + qh * ldo + 4 * c);
+      den += wgt * lw[w8];
+      acc.x += wgt * wv.x; acc.y += wgt * wv.y; acc.z += wgt * wv.z; acc.w += wgt * wv.w;
+    }
+    if (SPL == 1) {
+      const float inv = 1.0f / den;
+      store_row(qh, c, make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv));
+    } else {
+      if (a.cluster) *reinterpret_cast<float4*>(outp + qh * V + 4 * c) = acc;
+      else *reinterpret_cast<float4*>(po + qh * V + 4 * c) = acc;
+      if (c == 0) {
+        ml[2 * qh] = mx * kLn2;
+        ml[2 * qh + 1] = den;
       }
     }
   }
-  if (failed && tid == 0 && a.err) atomicExch(a.err, 1);
   if (SPL == 1) {
     append_token();
     return;
@@ -738,14 +735,13 @@ __global__ void __launch_bounds__(kStrThreads, 2) nha_decode_stream_kernel(const
           float den = 0.f;
           for (int s2 = 0; s2 < SPL; ++s2) {
             const float2 t2 = ld_cluster_f2(cluster_map(ml + 2 * qh, s2));
-            const float4 pv = ld_cluster_f4(cluster_map(hvS + qh * V + 4 * c, s2));
+            const float4 pv = ld_cluster_f4(cluster_map(outp + qh * V + 4 * c, s2));
             const float w2 = t2.x > -INFINITY ? __expf(t2.x - mx) : 0.f;
             den += t2.y * w2;
             acc.x += w2 * pv.x; acc.y += w2 * pv.y; acc.z += w2 * pv.z; acc.w += w2 * pv.w;
           }
           const float inv = 1.0f / den;
-          bf16* orow = a.o + ((size_t)b * a.HQ + h * NG + qh) * V + 4 * c;
-          orow[0] = f2bf(acc.x * inv); orow[1] = f2bf(acc.y * inv); orow[2] = f2bf(acc.z * inv); orow[3] = f2bf(acc.w * inv);
+          store_row(qh, c, make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv));
         }
       }
     }
@@ -755,6 +751,7 @@ __global__ void __launch_bounds__(kStrThreads, 2) nha_decode_stream_kernel(const
 
   // ---- merge: the last split of this (sequence, kv head) to arrive combines all partials ------------
   float* pml = a.part_ml + ((size_t)bh * SPL + sp) * NG * 2;
+  __syncthreads();                      // ml is complete
   for (int i = tid; i < NG * 2; i += kStrThreads) pml[i] = ml[i];
   __syncthreads();
   __shared__ int s_last;
@@ -804,13 +801,12 @@ __global__ void __launch_bounds__(kStrThreads, 2) nha_decode_stream_kernel(const
           const float w2 = wq[s2] / den;
           acc.x += w2 * pv[s2].x; acc.y += w2 * pv[s2].y; acc.z += w2 * pv[s2].z; acc.w += w2 * pv[s2].w;
         }
-        bf16* orow = a.o + ((size_t)b * a.HQ + h * NG + qh) * V + 4 * c;
-        orow[0] = f2bf(acc.x); orow[1] = f2bf(acc.y); orow[2] = f2bf(acc.z); orow[3] = f2bf(acc.w);
+        store_row(qh, c, acc);
       }
     }
     return;
   }
-  float* wgt = red;                     // [SPL][NG] merge weights exp(m_s - m) / denominator
+  float* wgt = outp;                    // [SPL][NG] merge weights exp(m_s - m) / denominator
   for (int qh = tid; qh < NG; qh += kStrThreads) {
     float mx = -INFINITY;
     for (int s2 = 0; s2 < SPL; ++s2) mx = fmaxf(mx, __ldcg(all_ml + ((size_t)s2 * NG + qh) * 2));
@@ -834,44 +830,37 @@ __global__ void __launch_bounds__(kStrThreads, 2) nha_decode_stream_kernel(const
       const float4 pv = __ldcg(reinterpret_cast<const float4*>(all_o + ((size_t)s2 * NG + qh) * V + 4 * c));
       acc.x += wq * pv.x; acc.y += wq * pv.y; acc.z += wq * pv.z; acc.w += wq * pv.w;
     }
-    bf16* orow = a.o + ((size_t)b * a.HQ + h * NG + qh) * V + 4 * c;
-    orow[0] = f2bf(acc.x); orow[1] = f2bf(acc.y); orow[2] = f2bf(acc.z); orow[3] = f2bf(acc.w);
+    store_row(qh, c, acc);
   }
 }
 
-static int stream_layout(DecodeStreamArgs& a, int D, int nkp) {
-  const int NG = a.NG, MQ = a.MQ;
+static int stream_layout(DecodeStreamArgs& a, int D) {
+  const int NG = a.NG, MQ = a.MQ, NH = NG > 8 ? 16 : 8;
   int off = 0;
   auto take = [&](int bytes) { int o = off; off = (off + bytes + 127) / 128 * 128; return o; };
-  a.off_ring = take(kStrSlots * kStrStage * (D + 8) * 2);
-  a.off_hv = take(MQ * D * 4);
-  const int s_bytes = 16 * (nkp + 8) * 4, red_bytes = kStrWarps * NG * 32 * 4;
-  a.off_S = take(s_bytes > red_bytes ? s_bytes : red_bytes);
-  a.off_red = a.off_S;                               // the partial slot logits are summed before the first S tile lands
-  a.off_q = take(NG * D * 4);
+  a.off_ring = take(kStrWarps * (D == 128 ? DecodeRing<128>::kWarp : DecodeRing<64>::kWarp));
+  a.off_out = take(std::max(NG * D, a.SPLITS * NG) * 4);
+  a.off_q = take(D * NH * 4);
   a.off_sqA = take(16 * (D + 8) * 2);
-  a.off_oks = take(NG * MQ * 4);
+  a.off_p = take(kStrWarps * kGroup * NH * 4);
   a.off_eg = take(MQ * 4);
   a.off_sv = take(MQ * 4);
   a.off_kpop = take(D * 4);
   a.off_vpop = take(D * 4);
+  a.off_wml = take(kStrWarps * NH * 4 * 4);
   a.off_ml = take(NG * 2 * 4);
-  a.off_bar = take((kStrSlots + 1) * 8);
   return off;
 }
 
 // Splits of a (sequence, kv head) for the streaming kernel: as many as keep the whole grid in one wave of two
-// CTAs per SM, each split keeping at least 64 keys and 4 slots.
+// CTAs per SM, each split keeping at least kMinKeys keys and 4 slots.
 int decode_stream_splits(int B, int H, int W, int M) {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  int spl = 1;
-  while (spl < 16 && (int64_t)B * H * spl * 2 <= 2 * (int64_t)sms && W / (spl * 2) >= kStrStage && M / (spl * 2) >= 4 &&
+  int spl = M > 64 && M <= 128 ? 2 : 1;            // a split has at most 64 slots: eight a warp
+  while (spl < 16 && (int64_t)B * H * spl * 2 <= 2 * (int64_t)sms && W / (spl * 2) >= kMinKeys && M / (spl * 2) >= 4 &&
          M % (spl * 2 * 4) == 0)
     spl *= 2;
-  // a CTA keeps all logits of its key range in shared memory: very wide windows are split further (more than one wave
-  // then) so that a split holds at most 512 keys
-  while (spl < 16 && (W + spl - 1) / spl > 512 && M / (spl * 2) >= 4 && M % (spl * 2 * 4) == 0) spl *= 2;
   return spl;
 }
 
@@ -898,20 +887,24 @@ bool decode_stream_supported(int K, int V, int M, int W, int NG, bool logits_mod
 // The caller has checked decode_stream_supported() and sized the workspace for `splits`.
 int decode_stream_launch(const DecodeStreamArgs& in, int D, cudaStream_t st) {
   DecodeStreamArgs a = in;
-  a.KSPL = ((a.W + a.SPLITS - 1) / a.SPLITS + kStrStage - 1) / kStrStage * kStrStage;
-  a.MQ = ((a.M + a.SPLITS - 1) / a.SPLITS + 3) / 4 * 4;
-  const int nkp = a.KSPL;
-  const int smem = stream_layout(a, D, nkp);
+  a.KSPL = ((a.W + a.SPLITS - 1) / a.SPLITS + kGroup - 1) / kGroup * kGroup;
+  a.MQ = ((a.M + a.SPLITS - 1) / a.SPLITS + kGroup - 1) / kGroup * kGroup;
+  const int smem = stream_layout(a, D);
   if (smem > kMaxSmem) return NHA_ERR_SMEM;
   dim3 grid(a.B * a.H * a.SPLITS), block(kStrThreads);
-  // 2, 4 or 8 splits whose partial outputs fit the (dead) hv rows merge through the cluster's shared memory
-  a.cluster = (a.SPLITS == 2 || a.SPLITS == 4 || a.SPLITS == 8) && a.NG <= a.MQ;
+  // 2, 4 or 8 splits merge through the cluster's shared memory
+  a.cluster = a.SPLITS == 2 || a.SPLITS == 4 || a.SPLITS == 8;
   if (const char* nc = getenv("NHA_B200_DECODE_NO_CLUSTER")) {
     if (nc[0] == '1') a.cluster = 0;                 // merge through the workspace instead
   }
-  const void* fn = a.state_bf16 ? (D == 128 ? (const void*)nha_decode_stream_kernel<128, true> : (const void*)nha_decode_stream_kernel<64, true>)
-                                : (D == 128 ? (const void*)nha_decode_stream_kernel<128, false>
-                                            : (const void*)nha_decode_stream_kernel<64, false>);
+  const void* fn;
+#define NHA_PICK(D_, T_)                                                                                   \
+  (a.state_bf16 ? (const void*)nha_decode_stream_kernel<D_, T_, true, false>                               \
+                : a.head ? (const void*)nha_decode_stream_kernel<D_, T_, false, true>                      \
+                         : (const void*)nha_decode_stream_kernel<D_, T_, false, false>)
+  if (D == 128) fn = a.NG > 8 ? NHA_PICK(128, 2) : NHA_PICK(128, 1);
+  else fn = a.NG > 8 ? NHA_PICK(64, 2) : NHA_PICK(64, 1);
+#undef NHA_PICK
   cudaError_t e = set_max_smem(fn, smem);
   if (e != cudaSuccess) return record_cuda_error(e);
   cudaLaunchConfig_t cfg;
