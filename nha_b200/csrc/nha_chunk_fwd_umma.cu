@@ -1,4 +1,4 @@
-// Output pass of the chunked NHA forward on the sm_100a tensor-core path: tcgen05.mma with operands in
+// Output pass of the chunked NHA forward for head dim 128 where the pipelined kernel (nha_chunk_fwd_pipe.cu) is not available: tcgen05.mma with operands in
 // 128-byte-swizzled shared memory, accumulators in tensor memory (TMEM), two (D = 64) or four (D = 128)
 // threads per query row for the softmax: tcgen05.ld hands a thread 32 or 16 columns of its row, the warps
 // that share a TMEM lane quarter (w, w + 4, ...) take alternate parts of the columns and combine row maxima
@@ -669,11 +669,15 @@ static int launch_umma(const nha_chunk_desc* d, int* flags, int* err, cudaStream
 
 // Runs the tensor-memory output pass when the shape has one (K == V in {64, 128}, M == 64, positive
 // scale).  Returns NHA_ERR_UNSUPPORTED otherwise.
+bool fwd64_supported(const nha_chunk_desc* d);
+int fwd64_launch(const nha_chunk_desc* d, int* flags, int* err, cudaStream_t cs);
 bool fwd_pipe_supported(const nha_chunk_desc* d);
 int fwd_pipe_launch(const nha_chunk_desc* d, int* flags, int* err, cudaStream_t cs);
 
 int chunk_output_pass_umma(const nha_chunk_desc* d, int* flags, int* err, cudaStream_t cs) {
   const int NG = d->HQ / d->H;
+  // head dim 64: 64-row products with full lanes, whatever the group (nha_chunk_fwd64.cu)
+  if (fwd64_supported(d)) return fwd64_launch(d, flags, err, cs);
   if (d->K != d->V || d->M != 64) return NHA_ERR_UNSUPPORTED;
   if (!(d->scale > 0.f)) return NHA_ERR_UNSUPPORTED;     // row maxima are taken before scaling
   // head dim 128: the warp-specialised pipeline (nha_chunk_fwd_pipe.cu)
@@ -681,8 +685,6 @@ int chunk_output_pass_umma(const nha_chunk_desc* d, int* flags, int* err, cudaSt
     const int st = fwd_pipe_launch(d, flags, err, cs);
     if (st != NHA_ERR_UNSUPPORTED) return st;
   }
-  if (d->K == 64 && NG == 1) return launch_umma<64, 64>(d, flags, err, cs);
-  if (d->K == 64) return launch_umma<64, 128>(d, flags, err, cs);
   if (d->K == 128 && NG == 1) return launch_umma<128, 64>(d, flags, err, cs);
   if (d->K == 128) return launch_umma<128, 128>(d, flags, err, cs);
   return NHA_ERR_UNSUPPORTED;

@@ -1,0 +1,24 @@
+"""GPU: the head-dim-64 kernels with full lanes: every slot count they take, ragged last chunks, windows of one and of several
+steps, window logits that grow towards older keys (the running reference of the softmax is raised), against the oracle."""
+import pytest
+import torch
+
+from oracle import nha_oracle as orc
+from tests import inputs as gen
+from tests.gpu_util import TOL_OUT, assert_close
+
+pytestmark = pytest.mark.gpu
+NAMES = ('q_swa', 'k_swa', 'q_gsa', 'k_gsa', 'v', 's', 'g')
+
+
+@pytest.mark.parametrize('M', [16, 32, 48, 64])
+@pytest.mark.parametrize('HQ,H,T,wl,shift', [(2, 2, 129, 64, 0), (6, 2, 65, 63, 64), (2, 1, 400, 300, 0), (1, 1, 700, -1, 70)])
+def test_forward(M, HQ, H, T, wl, shift):
+    from nha_b200 import chunk_nha
+    d = gen.layer_inputs(50 + M + T, 1, T, HQ, H, 64, 64, M, gate_div=2.0, val_scale=1.0)
+    grow = torch.linspace(6.0, 0.2, T)[None, :, None, None]
+    d['k_swa'] = (d['k_swa'].float() * grow).bfloat16()            # older keys have the larger logits
+    want = orc.nha_varlen(*(d[n][0].double() for n in ('q_gsa', 'q_swa', 'k_gsa', 'k_swa', 'v', 's', 'g')), [0, T], 0.125, wl, shift, None, None)
+    got = chunk_nha(*(d[n].cuda() for n in NAMES), window_size_left=wl, window_size_right=0, gsa_kv_shift=shift, output_final_state=True)
+    for x, y, name in zip((got[0][0], got[1][0], got[2][0], *got[3]), want, ('o', 'lse_swa', 'lse_gsa', 'hk', 'hv')):
+        assert_close(x, y, TOL_OUT, name)
