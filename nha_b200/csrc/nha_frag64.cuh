@@ -38,6 +38,14 @@ __device__ __forceinline__ void frag_ld(uint32_t taddr, float (&v)[16]) {
   frag_ld_nowait(taddr, v);
   tmem_ld_wait();
 }
+// 16 columns: v[4 j + e], j = 0, 1
+__device__ __forceinline__ void frag_ld8_nowait(uint32_t taddr, float (&v)[8]) {
+  uint32_t* r = reinterpret_cast<uint32_t*>(v);
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
 // the reverse (rescaling an accumulator in place)
 __device__ __forceinline__ void frag_st(uint32_t taddr, const float (&v)[16]) {
   const uint32_t* r = reinterpret_cast<const uint32_t*>(v);
@@ -67,6 +75,10 @@ __device__ __forceinline__ void stm4(uint32_t saddr, uint32_t a, uint32_t b, uin
 __device__ __forceinline__ void ldm4(uint32_t saddr, uint32_t (&r)[4]) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(saddr) : "memory");
+}
+// 16 x 16: one column pair
+__device__ __forceinline__ void frag8_to_tile(uint32_t o, const float (&v)[8]) {
+  stm4(o, pair_bf16(v[0], v[1]), pair_bf16(v[2], v[3]), pair_bf16(v[4], v[5]), pair_bf16(v[6], v[7]));
 }
 // the warp's 16 x 32 block of a tile from fp32 fragments (o0, o1: frag_off of the two column pairs + the tile's address)
 __device__ __forceinline__ void frag_to_tile(uint32_t o0, uint32_t o1, const float (&v)[16]) {
