@@ -1141,10 +1141,12 @@ static int launch_cols(const nha_chunk_desc* d, const BwdWs& w, int* err, cudaSt
 
 bool bwd64_supported(const nha_chunk_desc* d);
 int bwd_rows64_launch(const nha_chunk_desc* d, const BwdWs& w, int* err, cudaStream_t cs);
+int bwd_cols64_launch(const nha_chunk_desc* d, const BwdWs& w, int* err, cudaStream_t cs);
 
 bool bwd_umma_supported(const nha_chunk_desc* d) {
   const int NG = d->HQ / d->H;
-  return d->K == d->V && d->M == 64 && (d->K == 64 || d->K == 128) && (NG == 1 || NG % 2 == 0);
+  if (d->K == 64) return bwd64_supported(d);
+  return d->K == d->V && d->M == 64 && d->K == 128 && (NG == 1 || NG % 2 == 0);
 }
 
 // which: 0 = rows pass, 1 = columns pass.  The caller has checked bwd_umma_supported().
@@ -1153,7 +1155,7 @@ int bwd_umma_launch(const nha_chunk_desc* d, const BwdWs& w, int which, int* err
   const bool one = NG == 1;
   if (d->K == 64) {
     if (which == 0) return bwd_rows64_launch(d, w, err, cs);
-    return one ? launch_cols<64, 64>(d, w, err, cs) : launch_cols<64, 128>(d, w, err, cs);
+    return bwd_cols64_launch(d, w, err, cs);
   }
   if (which == 0) return one ? launch_rows<128, 64>(d, w, err, cs) : launch_rows<128, 128>(d, w, err, cs);
   return one ? launch_cols<128, 64>(d, w, err, cs) : launch_cols<128, 128>(d, w, err, cs);
