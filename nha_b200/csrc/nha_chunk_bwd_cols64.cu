@@ -12,6 +12,8 @@
 // a quarter, shared memory across the quarters) plus the carry <DK, hk_next> + <DV, hv_next>, formed in fp32 from the same loads.
 //
 // Replaces, with the other backward kernels, ChunkNativeHybridAttentionFunction.backward (nha_fla/ops/nha/chunk.py:491-564).
+#include <string.h>
+
 #include "nha_bwd_common.cuh"
 #include "nha_frag64.cuh"
 
@@ -26,16 +28,29 @@ constexpr int oTot = oPart + 9 * 64 * 4;                      // fp32 [4 quarter
 constexpr int oBar = oTot + 4 * 64 * 4;
 constexpr int total = oBar + 64 + 1024;
 static_assert(total <= 113 * 1024, "two CTAs per SM");
+// The pass is bound by how early its loads start: it reads 32 KB of fp32 states and 64 KB of rows per CTA, and two CTAs an SM keep
+// too few bytes in flight.  Tiles by TMA, the states in registers before the first wait, and an L2 prefetch of the CTA that starts
+// one wave of SMs later: B16 T2048 H16 W64 386 -> 325 us (without the prefetch 350; 296 or 74 CTAs ahead 330-340).
+constexpr int kAhead = 148;                                   // CTAs by which the prefetch runs ahead: one per SM
 }  // namespace cl64
+
+// Tensor maps of the call's tensors (this GPU's own memory).  A tile whose 64 rows lie inside its sequence comes by TMA; the
+// others (ragged ends, rows in front of a sequence) are copied piece by piece with zero fill.  use == 0: all tiles are copied
+// (fewer than 64 slots, or no tensor maps).
+struct ColsMaps {
+  CUtensorMap qg, kg, v, g, s, dout, za, pa;
+  int use;
+};
 
 // ONE: one query head per kv head.  Several heads accumulate in columns of their own (512 columns, one CTA per SM).
 template <bool ONE>
-__global__ void __launch_bounds__(kThreads, ONE ? 2 : 1) nha_bwd_cols64_kernel(const nha_chunk_desc d, const BwdWs w, int* __restrict__ err) {
+__global__ void __launch_bounds__(kThreads, ONE ? 2 : 1) nha_bwd_cols64_kernel(const nha_chunk_desc d, const BwdWs w, int* __restrict__ err,
+                                                                                 const __grid_constant__ ColsMaps maps) {
   using namespace cl64;
   constexpr int c0_ = 0, c1_ = 64, c2_ = 128, c3_ = 192, kTmemCols = ONE ? 256 : 512;
   constexpr int cDS = ONE ? 0 : 256, cDK = ONE ? 64 : 320, cDV = ONE ? 128 : 384, cDS2 = ONE ? 192 : 448;
   const int H = d.H, HQ = d.HQ, M = d.M, NG = ONE ? 1 : HQ / H;
-  const int cg = blockIdx.x, h = blockIdx.y;
+  const int cg = blockIdx.x / H, h = blockIdx.x - cg * H;
   const ChunkRec rc = chunk_rec(d, cg);
   if (rc.n < 0) return;
   if (!chunk_gate(w, cg, h, H)) return;
@@ -50,32 +65,109 @@ __global__ void __launch_bounds__(kThreads, ONE ? 2 : 1) nha_bwd_cols64_kernel(c
   float* part = (float*)(sm + oPart);
   float* tot = (float*)(sm + oTot);
   uint64_t* mbar = (uint64_t*)(sm + oBar);
-  uint32_t* tslot = (uint32_t*)(mbar + 1);
+  uint32_t* tslot = (uint32_t*)(mbar + 1);   // then the load barriers
   auto tile = [&](int i) { return sm + i * kTile; };
 
   // ---- loads: gates and write weights first, then the first head's tiles -------------------------------------------------
   const int lr = tid >> 3, lc = tid & 7;
   const uint32_t loff = sw_off(lr, lc);
   const int64_t rq = (int64_t)HQ * 64, rp = (int64_t)H * 64, rm = (int64_t)H * M, rz = (int64_t)HQ * M;
-  auto load_tokens = [&](int t, const void* base, int64_t pitch, int col, int row, int lo, int hi, bool col_ok) {
-    const bf16* p = (const bf16*)base + (int64_t)t0 * pitch + col + 8 * lc;
-    const bool ok0 = col_ok && row + lr >= lo && row + lr < hi, ok1 = col_ok && row + lr + 32 >= lo && row + lr + 32 < hi;
-    tile_in(tile(t), loff, p + (ok0 ? row + lr : 0) * pitch, ok0, p + (ok1 ? row + lr + 32 : 0) * pitch, ok1);
+  // load barriers: each phase is closed by one arrival of thread 0 behind its last TMA; bits of lph: their parities
+  uint64_t* bl = mbar + 2;
+  uint32_t lph = 0;
+  auto loads_done = [&](int bar) {
+    cp_commit();
+    if (tid == 0) mbar_arrive(&bl[bar]);
+  };
+  bool failed = false;
+  auto loads_wait = [&](int bar, bool newest) {                // newest == false: a later group may stay in flight
+    if (newest) cp_wait_all(); else cp_wait_but_one();
+    if (!failed && !mbar_wait(&bl[bar], (lph >> bar) & 1u)) failed = true;
+    lph ^= 1u << bar;
+  };
+  auto load_tokens = [&](int t, const CUtensorMap& map, int head, const void* base, int64_t pitch, int width, int row, int lo, int hi, int bar) {
+    if (maps.use && row >= lo && row + kChunk <= hi) {
+      if (tid == 0) {
+        mbar_expect_more(&bl[bar], kTile);
+        tma_load_3d(tile(t), &map, 0, head, t0 + row, &bl[bar]);
+      }
+    } else {
+      const bf16* p = (const bf16*)base + (int64_t)t0 * pitch + head * width + 8 * lc;
+      const bool cok = 8 * lc < width;
+      const bool ok0 = cok && row + lr >= lo && row + lr < hi, ok1 = cok && row + lr + 32 >= lo && row + lr + 32 < hi;
+      tile_in(tile(t), loff, p + (ok0 ? row + lr : 0) * pitch, ok0, p + (ok1 ? row + lr + 32 : 0) * pitch, ok1);
+    }
   };
   const bool mcol = 8 * lc < M;
-  load_tokens(b2, d.g, rm, h * M, c0 - shift, 0, len - shift, mcol);
-  load_tokens(tSB, d.s, rm, h * M, c0 - shift, 0, len - shift, mcol);
-  cp_commit();
+  if (tid == 0) {
+    mbar_init(mbar, 1);
+    mbar_init(&bl[0], 1);
+    mbar_init(&bl[1], 1);
+    mbar_init(&bl[2], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    fence_async_smem();
+  }
+  load_tokens(b2, maps.g, h, d.g, rm, M, c0 - shift, 0, len - shift, 0);
+  load_tokens(tSB, maps.s, h, d.s, rm, M, c0 - shift, 0, len - shift, 0);
+  loads_done(0);
   auto load_head = [&](int hq) {
-    load_tokens(tQ, d.q_gsa, rq, hq * 64, c0, 0, len, true);
-    load_tokens(tDO, d.d_o, rq, hq * 64, c0, 0, len, true);
-    load_tokens(tZA, w.dza, rz, hq * M, c0, 0, len, mcol);
-    load_tokens(tPA, w.paq, rz, hq * M, c0, 0, len, mcol);
-    cp_commit();
+    load_tokens(tQ, maps.qg, hq, d.q_gsa, rq, 64, c0, 0, len, 1);
+    load_tokens(tDO, maps.dout, hq, d.d_o, rq, 64, c0, 0, len, 1);
+    load_tokens(tZA, maps.za, hq, w.dza, rz, M, c0, 0, len, 1);
+    load_tokens(tPA, maps.pa, hq, w.paq, rz, M, c0, 0, len, 1);
+    loads_done(1);
   };
-  load_tokens(tK, d.k_gsa, rp, h * 64, c0 - shift, 0, len - shift, true);
-  load_tokens(tV, d.v, rp, h * 64, c0 - shift, 0, len - shift, true);
+  load_tokens(tK, maps.kg, h, d.k_gsa, rp, 64, c0 - shift, 0, len - shift, 1);
+  load_tokens(tV, maps.v, h, d.v, rp, 64, c0 - shift, 0, len - shift, 1);
   load_head(h * NG);
+  // state gradients at the chunk end and the next chunk's start state, requested into registers beside the tiles: rows lr and
+  // lr + 32, eight columns
+  const int nchunks = (len + kChunk - 1) / kChunk;
+  const bool last = ci >= nchunks - 1, have_next = !last || (d.d_hkt && d.hkt && d.hvt);
+  const size_t nh = (size_t)rc.n * H + h;
+  const float* hkf = d.hkt ? d.hkt + nh * 64 * M : nullptr;
+  const float* hvf = d.hvt ? d.hvt + nh * M * 64 : nullptr;
+  float4 gk[2][2], gv[2][2];
+  uint4 nk[2], nv[2];
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int r = lr + 32 * u;
+    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+    gk[u][0] = gk[u][1] = gv[u][0] = gv[u][1] = z;
+    nk[u] = nv[u] = make_uint4(0u, 0u, 0u, 0u);
+    if (mcol) {
+      const float4* p = reinterpret_cast<const float4*>(w.dkc + ch * 64 * M + r * M + 8 * lc);
+      gk[u][0] = p[0]; gk[u][1] = p[1];
+      if (!last) nk[u] = *reinterpret_cast<const uint4*>((const bf16*)d.hk_chunks + ((size_t)(cg + 1) * H + h) * 64 * M + r * M + 8 * lc);
+    }
+    if (r < M) {
+      const float4* p = reinterpret_cast<const float4*>(w.dvc + ch * M * 64 + r * 64 + 8 * lc);
+      gv[u][0] = p[0]; gv[u][1] = p[1];
+      if (!last) nv[u] = *reinterpret_cast<const uint4*>((const bf16*)d.hv_chunks + ((size_t)(cg + 1) * H + h) * M * 64 + r * 64 + 8 * lc);
+    }
+  }
+  // What the CTA that follows on this SM will read goes into L2 now: the loads are what the pass waits for (B16 T2048 H16: 386 us
+  // without, 325 us with it; two or three CTAs ahead 341 and 374 us).
+  if (maps.use && tid == 64 && blockIdx.x + kAhead < gridDim.x) {
+    const int ncg = (blockIdx.x + kAhead) / H, nhd = blockIdx.x + kAhead - ncg * H;
+    const ChunkRec nr = chunk_rec(d, ncg);
+    if (nr.n >= 0) {
+      const int row = nr.t0 + nr.ci * kChunk;
+      const size_t nch = (size_t)ncg * H + nhd;
+      prefetch_tile(maps.g, nhd, row);
+      prefetch_tile(maps.s, nhd, row);
+      prefetch_tile(maps.kg, nhd, row);
+      prefetch_tile(maps.v, nhd, row);
+      prefetch_tile(maps.qg, nhd * NG, row);
+      prefetch_tile(maps.dout, nhd * NG, row);
+      prefetch_tile(maps.za, nhd * NG, row);
+      prefetch_tile(maps.pa, nhd * NG, row);
+      prefetch_bytes(w.dkc + nch * 4096, 16384);
+      prefetch_bytes(w.dvc + nch * 4096, 16384);
+      prefetch_bytes((const bf16*)d.hk_chunks + nch * 4096, kTile);
+      prefetch_bytes((const bf16*)d.hv_chunks + nch * 4096, kTile);
+    }
+  }
   fill_half_signs(tile(b1), tid);
   {
     // strictly upper triangular ones: row t of y sums the gates of the rows after t
@@ -92,12 +184,9 @@ __global__ void __launch_bounds__(kThreads, ONE ? 2 : 1) nha_bwd_cols64_kernel(c
       *reinterpret_cast<uint4*>(tile(b3) + sw_off(r, c)) = make_uint4(pr[0], pr[1], pr[2], pr[3]);
     }
   }
-  if (tid == 0) {
-    mbar_init(mbar, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
   if (warp == 0) tmem_alloc(tslot, kTmemCols);
-  cp_wait_but_one();
+  __syncthreads();                                             // the barriers are initialised
+  loads_wait(0, false);
   fence_async_smem();
   tc_fence_before();
   __syncthreads();
@@ -105,7 +194,6 @@ __global__ void __launch_bounds__(kThreads, ONE ? 2 : 1) nha_bwd_cols64_kernel(c
   const uint32_t tbase = *tslot;
   const uint32_t tl = tbase + ((uint32_t)(quarter * 32) << 16) + 32 * half;       // this warp's columns of an accumulator at +0
   uint32_t phase = 0;
-  bool failed = false;
   auto mma_wait = [&]() {
     if (tid == 0) commit(mbar);
     if (!failed && !mbar_wait(mbar, phase)) failed = true;
@@ -130,27 +218,12 @@ __global__ void __launch_bounds__(kThreads, ONE ? 2 : 1) nha_bwd_cols64_kernel(c
   // ---- state gradients at the chunk end: bf16 operands, and the carry's dot products with the next chunk's start state --------
   uint4 dkp[2];                                                        // rows lr, lr + 32 of DK, columns 8 lc .. + 7
   {
-    const int nchunks = (len + kChunk - 1) / kChunk;
-    const bool last = ci >= nchunks - 1, have_next = !last || (d.d_hkt && d.hkt && d.hvt);
-    const size_t nh = (size_t)rc.n * H + h;
-    const float* dk = w.dkc + ch * 64 * M;
-    const float* dv = w.dvc + ch * M * 64;
-    const bf16* hkn = (const bf16*)d.hk_chunks + ((size_t)(cg + 1) * H + h) * 64 * M;
-    const bf16* hvn = (const bf16*)d.hv_chunks + ((size_t)(cg + 1) * H + h) * M * 64;
-    const float* hkf = d.hkt ? d.hkt + nh * 64 * M : nullptr;
-    const float* hvf = d.hvt ? d.hvt + nh * M * 64 : nullptr;
-    auto eight = [&](const float* p, float (&f)[8]) {
-      const float4 x = *reinterpret_cast<const float4*>(p), y = *reinterpret_cast<const float4*>(p + 4);
-      f[0] = x.x; f[1] = x.y; f[2] = x.z; f[3] = x.w; f[4] = y.x; f[5] = y.y; f[6] = y.z; f[7] = y.w;
-    };
-    auto next = [&](const bf16* n, const float* fin, int64_t at_, float (&f)[8]) {
-      if (!have_next) {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) f[e] = 0.f;
-      } else if (last) {
-        eight(fin + at_, f);
+    auto next = [&](const uint4& n, const float* fin, int64_t at_, float (&f)[8]) {
+      if (last && have_next) {                                         // the fp32 final state stands in for a next chunk's start
+        const float4 x = *reinterpret_cast<const float4*>(fin + at_), y = *reinterpret_cast<const float4*>(fin + at_ + 4);
+        f[0] = x.x; f[1] = x.y; f[2] = x.z; f[3] = x.w; f[4] = y.x; f[5] = y.y; f[6] = y.z; f[7] = y.w;
       } else {
-        unpack8(*reinterpret_cast<const uint4*>(n + at_), f);
+        unpack8(n, f);
       }
     };
     float ck[8];
@@ -161,9 +234,9 @@ __global__ void __launch_bounds__(kThreads, ONE ? 2 : 1) nha_bwd_cols64_kernel(c
       const int r = lr + 32 * u;
       dkp[u] = make_uint4(0u, 0u, 0u, 0u);
       if (mcol) {
-        float f[8], n[8];
-        eight(dk + r * M + 8 * lc, f);
-        next(hkn, hkf, r * M + 8 * lc, n);
+        const float f[8] = {gk[u][0].x, gk[u][0].y, gk[u][0].z, gk[u][0].w, gk[u][1].x, gk[u][1].y, gk[u][1].z, gk[u][1].w};
+        float n[8];
+        next(nk[u], hkf, r * M + 8 * lc, n);
 #pragma unroll
         for (int e = 0; e < 8; ++e) ck[e] += f[e] * n[e];
         dkp[u] = pack8(f);
@@ -171,9 +244,9 @@ __global__ void __launch_bounds__(kThreads, ONE ? 2 : 1) nha_bwd_cols64_kernel(c
       float cv = 0.f;
       uint4 dvp = make_uint4(0u, 0u, 0u, 0u);
       if (r < M) {
-        float f[8], n[8];
-        eight(dv + r * 64 + 8 * lc, f);
-        next(hvn, hvf, r * 64 + 8 * lc, n);
+        const float f[8] = {gv[u][0].x, gv[u][0].y, gv[u][0].z, gv[u][0].w, gv[u][1].x, gv[u][1].y, gv[u][1].z, gv[u][1].w};
+        float n[8];
+        next(nv[u], hvf, r * 64 + 8 * lc, n);
 #pragma unroll
         for (int e = 0; e < 8; ++e) cv += f[e] * n[e];
         dvp = pack8(f);
@@ -248,7 +321,7 @@ __global__ void __launch_bounds__(kThreads, ONE ? 2 : 1) nha_bwd_cols64_kernel(c
   for (int ht = 0; ht < NG; ++ht) {
     const bool fin = ht + 1 == NG;
     if (!ONE && ht > 0) load_head(h * NG + ht);
-    cp_wait_all();
+    loads_wait(1, true);
     hand_over();
     if (tid == 0) {
       mma64<0, 0>(tbase + c0_, desc(tQ), desc(tK), iKK, false);
@@ -387,9 +460,15 @@ int bwd_cols64_launch(const nha_chunk_desc* d, const BwdWs& w, int* err, cudaStr
   const void* fn = d->HQ == d->H ? (const void*)nha_bwd_cols64_kernel<true> : (const void*)nha_bwd_cols64_kernel<false>;
   cudaError_t e = set_max_smem(fn, cl64::total);
   if (e != cudaSuccess) return record_cuda_error(e);
-  const dim3 grid((unsigned)nha_chunk_count_bound(d->Ttot, d->N), d->H);
-  if (d->HQ == d->H) nha_bwd_cols64_kernel<true><<<grid, kThreads, cl64::total, cs>>>(*d, w, err);
-  else nha_bwd_cols64_kernel<false><<<grid, kThreads, cl64::total, cs>>>(*d, w, err);
+  ColsMaps maps;
+  memset(&maps, 0, sizeof(maps));
+  maps.use = d->M == 64 && make_map_rows_heads(&maps.qg, d->q_gsa, d->Ttot, d->HQ, 64) && make_map_rows_heads(&maps.kg, d->k_gsa, d->Ttot, d->H, 64) &&
+             make_map_rows_heads(&maps.v, d->v, d->Ttot, d->H, 64) && make_map_rows_heads(&maps.g, d->g, d->Ttot, d->H, 64) &&
+             make_map_rows_heads(&maps.s, d->s, d->Ttot, d->H, 64) && make_map_rows_heads(&maps.dout, d->d_o, d->Ttot, d->HQ, 64) &&
+             make_map_rows_heads(&maps.za, w.dza, d->Ttot, d->HQ, 64) && make_map_rows_heads(&maps.pa, w.paq, d->Ttot, d->HQ, 64);
+  const dim3 grid((unsigned)(nha_chunk_count_bound(d->Ttot, d->N) * d->H));
+  if (d->HQ == d->H) nha_bwd_cols64_kernel<true><<<grid, kThreads, cl64::total, cs>>>(*d, w, err, maps);
+  else nha_bwd_cols64_kernel<false><<<grid, kThreads, cl64::total, cs>>>(*d, w, err, maps);
   return check_launch();
 }
 

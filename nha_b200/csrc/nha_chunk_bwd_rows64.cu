@@ -40,7 +40,7 @@ static_assert(total <= 113 * 1024, "two CTAs per SM");
 __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows64_kernel(const nha_chunk_desc d, const BwdWs w, int* __restrict__ err) {
   using namespace rw64;
   const int H = d.H, HQ = d.HQ, M = d.M, NG = HQ / H;
-  const int cg = blockIdx.x, h = blockIdx.y;
+  const int cg = blockIdx.x / H, h = blockIdx.x - cg * H;
   const ChunkRec rc = chunk_rec(d, cg);
   if (rc.n < 0) return;
   if (!chunk_gate(w, cg, h, H)) return;
@@ -93,29 +93,36 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows64_kernel(const nha_c
     const int o0 = lr * M + 8 * lc, o1 = o0 + 32 * M;
     tile_in(tile(tHk), loff, hk + (mcol ? o0 : 0), mcol, hk + (mcol ? o1 : 0), mcol);
   }
-  load_head(h * NG);
-  // row statistics of a head: delta = <do, o> by four threads per row, the joint log-sum-exp by one
-  auto row_stats = [&](int hq) {
+  // row statistics of a head: delta = <do, o> by four threads per row, the joint log-sum-exp by one (requested first, formed later)
+  uint4 o0, o1, g0, g1;
+  float lsw, lgs, dl;
+  auto row_request = [&](int hq) {
     const int r = tid >> 2, part = tid & 3, pos = c0 + r;
-    float del = 0.f, lsw = 0.f, lgs = 0.f, dl = 0.f;
+    o0 = o1 = g0 = g1 = make_uint4(0u, 0u, 0u, 0u);
+    lsw = lgs = dl = 0.f;
     if (pos < len) {
       const size_t at = (size_t)(t0 + pos) * HQ + hq;
       const uint4* o = reinterpret_cast<const uint4*>((const bf16*)d.o + at * 64 + 16 * part);
       const uint4* g = reinterpret_cast<const uint4*>((const bf16*)d.d_o + at * 64 + 16 * part);
-      const uint4 o0 = __ldg(o), o1 = __ldg(o + 1), g0 = __ldg(g), g1 = __ldg(g + 1);
+      o0 = __ldg(o); o1 = __ldg(o + 1); g0 = __ldg(g); g1 = __ldg(g + 1);
       if (part == 0) {
         lsw = d.lse_swa[at];
         lgs = d.lse_gsa[at];
         dl = d.d_lse_gsa ? d.d_lse_gsa[at] : 0.f;
       }
-      float x[8], y[8];
-      unpack8(o0, x); unpack8(g0, y);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) del += x[e] * y[e];
-      unpack8(o1, x); unpack8(g1, y);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) del += x[e] * y[e];
     }
+  };
+  row_request(h * NG);
+  load_head(h * NG);
+  auto row_stats = [&](int hq) {
+    const int r = tid >> 2, part = tid & 3, pos = c0 + r;
+    float del = 0.f, x[8], y[8];
+    unpack8(o0, x); unpack8(g0, y);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) del += x[e] * y[e];
+    unpack8(o1, x); unpack8(g1, y);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) del += x[e] * y[e];
     del += __shfl_xor_sync(0xffffffffu, del, 1);
     del += __shfl_xor_sync(0xffffffffu, del, 2);
     if (part == 0) {
@@ -240,6 +247,7 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows64_kernel(const nha_c
     const int hq = h * NG + ht;
     if (ht > 0) {
       load_head(hq);
+      row_request(hq);
       row_stats(hq);
     }
     cp_wait_all();
@@ -424,7 +432,7 @@ bool bwd64_supported(const nha_chunk_desc* d) { return d->K == 64 && d->V == 64 
 int bwd_rows64_launch(const nha_chunk_desc* d, const BwdWs& w, int* err, cudaStream_t cs) {
   cudaError_t e = set_max_smem((const void*)nha_bwd_rows64_kernel, rw64::total);
   if (e != cudaSuccess) return record_cuda_error(e);
-  nha_bwd_rows64_kernel<<<dim3((unsigned)nha_chunk_count_bound(d->Ttot, d->N), d->H), kThreads, rw64::total, cs>>>(*d, w, err);
+  nha_bwd_rows64_kernel<<<dim3((unsigned)(nha_chunk_count_bound(d->Ttot, d->N) * d->H)), kThreads, rw64::total, cs>>>(*d, w, err);
   return check_launch();
 }
 

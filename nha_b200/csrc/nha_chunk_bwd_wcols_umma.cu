@@ -42,7 +42,7 @@ __global__ void __launch_bounds__(kWCThreads, D == 64 ? 2 : 1) nha_bwd_wcols_umm
   typedef WColsLayout<D> L;
   constexpr int KT = L::KT;
   const int H = d.H, HQ = d.HQ, NG = HQ / H, N = d.N;
-  const int cg = blockIdx.x, h = blockIdx.y;
+  const int cg = blockIdx.x / H, h = blockIdx.x - cg * H;
   const ChunkRec rc = chunk_rec(d, cg);
   const int n = rc.n;
   if (n < 0) return;
@@ -204,7 +204,7 @@ static int launch_wcols(const nha_chunk_desc* d, const BwdWs& w, int* err, cudaS
   cudaError_t e = set_max_smem((const void*)nha_bwd_wcols_umma_kernel<D>, L::total);
   if (e != cudaSuccess) return record_cuda_error(e);
   const int NCB = (int)nha_chunk_count_bound(d->Ttot, d->N);
-  nha_bwd_wcols_umma_kernel<D><<<dim3(NCB, d->H), kWCThreads, L::total, cs>>>(*d, w, err);
+  nha_bwd_wcols_umma_kernel<D><<<dim3(NCB * d->H), kWCThreads, L::total, cs>>>(*d, w, err);
   return check_launch();
 }
 
