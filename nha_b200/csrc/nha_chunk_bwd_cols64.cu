@@ -28,9 +28,9 @@ constexpr int oTot = oPart + 9 * 64 * 4;                      // fp32 [4 quarter
 constexpr int oBar = oTot + 4 * 64 * 4;
 constexpr int total = oBar + 64 + 1024;
 static_assert(total <= 113 * 1024, "two CTAs per SM");
-// The pass is bound by how early its loads start: it reads 32 KB of fp32 states and 64 KB of rows per CTA, and two CTAs an SM keep
-// too few bytes in flight.  Tiles by TMA, the states in registers before the first wait, and an L2 prefetch of the CTA that starts
-// one wave of SMs later: B16 T2048 H16 W64 386 -> 325 us (without the prefetch 350; 296 or 74 CTAs ahead 330-340).
+// The pass waits for its loads: two CTAs an SM keep too few bytes in flight, so each prefetches the inputs of a later CTA into L2.
+// B16 T2048 H16 W64: 386 us with TMA tiles alone (392 before them), 325-330 with the prefetch 148 CTAs ahead, 341 with 296, 374
+// with 444.
 constexpr int kAhead = 148;                                   // CTAs by which the prefetch runs ahead: one per SM
 }  // namespace cl64
 
