@@ -1,4 +1,4 @@
-// Key side of the sliding-window backward on the sm_100a tensor-core path: dk_swa and the window part of
+// Key side of the sliding-window backward on the sm_100a tensor-core path, head dim 128: dk_swa and the window part of
 // dv.  One CTA per (key chunk, kv head).  The query rows that can see the chunk - every (query chunk,
 // query head of the group) pair - are taken two 64-row blocks at a time as the 128 rows of
 //     S = q_swa k_swa^T,   dP = do v^T                           (tcgen05.mma, accumulators in TMEM)
@@ -20,8 +20,8 @@ using namespace umma;
 
 constexpr int kWCThreads = 256;          // two threads per query row (alternate 32-key halves)
 
-template <int D>
 struct WColsLayout {
+  static constexpr int D = 128;
   static constexpr int KT = D / 64;
   static constexpr int kATile = 128 * 128;              // one 64-wide k tile of a 128-row operand
   static constexpr int tK = 0;                           // k_swa of the chunk [64][D]
@@ -32,15 +32,13 @@ struct WColsLayout {
   static constexpr int tZ = tP + kATile;                 // dz [128][64]
   static constexpr int oBar = tZ + kATile;
   static constexpr int total = oBar + 64 + 1024;
-  static constexpr int kTmemCols = D == 64 ? 256 : 512;
+  static constexpr int kTmemCols = 512;
   static constexpr int cS = 0, cDP = 64, cDV = 128, cDK = 128 + D;
 };
 
-template <int D>
-__global__ void __launch_bounds__(kWCThreads, D == 64 ? 2 : 1) nha_bwd_wcols_umma_kernel(const nha_chunk_desc d, const BwdWs w,
-                                                                        int* __restrict__ err) {
-  typedef WColsLayout<D> L;
-  constexpr int KT = L::KT;
+__global__ void __launch_bounds__(kWCThreads, 1) nha_bwd_wcols_umma_kernel(const nha_chunk_desc d, const BwdWs w, int* __restrict__ err) {
+  typedef WColsLayout L;
+  constexpr int D = L::D, KT = L::KT;
   const int H = d.H, HQ = d.HQ, NG = HQ / H, N = d.N;
   const int cg = blockIdx.x / H, h = blockIdx.x - cg * H;
   const ChunkRec rc = chunk_rec(d, cg);
@@ -198,21 +196,18 @@ __global__ void __launch_bounds__(kWCThreads, D == 64 ? 2 : 1) nha_bwd_wcols_umm
   if (warp == 0) tmem_dealloc(tbase, L::kTmemCols);
 }
 
-template <int D>
-static int launch_wcols(const nha_chunk_desc* d, const BwdWs& w, int* err, cudaStream_t cs) {
-  typedef WColsLayout<D> L;
-  cudaError_t e = set_max_smem((const void*)nha_bwd_wcols_umma_kernel<D>, L::total);
-  if (e != cudaSuccess) return record_cuda_error(e);
-  const int NCB = (int)nha_chunk_count_bound(d->Ttot, d->N);
-  nha_bwd_wcols_umma_kernel<D><<<dim3(NCB * d->H), kWCThreads, L::total, cs>>>(*d, w, err);
-  return check_launch();
-}
-
 bool bwd_wcols_umma_supported(const nha_chunk_desc* d) { return d->K == d->V && (d->K == 64 || d->K == 128); }
+
+int bwd_wcols64_launch(const nha_chunk_desc* d, const BwdWs& w, int* err, cudaStream_t cs);
 
 // The caller has checked bwd_wcols_umma_supported().
 int bwd_wcols_umma_launch(const nha_chunk_desc* d, const BwdWs& w, int* err, cudaStream_t cs) {
-  return d->K == 64 ? launch_wcols<64>(d, w, err, cs) : launch_wcols<128>(d, w, err, cs);
+  if (d->K == 64) return bwd_wcols64_launch(d, w, err, cs);
+  cudaError_t e = set_max_smem((const void*)nha_bwd_wcols_umma_kernel, WColsLayout::total);
+  if (e != cudaSuccess) return record_cuda_error(e);
+  const int NCB = (int)nha_chunk_count_bound(d->Ttot, d->N);
+  nha_bwd_wcols_umma_kernel<<<dim3(NCB * d->H), kWCThreads, WColsLayout::total, cs>>>(*d, w, err);
+  return check_launch();
 }
 
 }  // namespace nha

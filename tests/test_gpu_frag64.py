@@ -6,6 +6,7 @@ import torch
 from oracle import nha_oracle as orc
 from tests import inputs as gen
 from tests.gpu_util import TOL_OUT, assert_close
+from tests.test_gpu_chunk import compare, run_gpu, run_oracle
 
 pytestmark = pytest.mark.gpu
 NAMES = ('q_swa', 'k_swa', 'q_gsa', 'k_gsa', 'v', 's', 'g')
@@ -22,3 +23,19 @@ def test_forward(M, HQ, H, T, wl, shift):
     got = chunk_nha(*(d[n].cuda() for n in NAMES), window_size_left=wl, window_size_right=0, gsa_kv_shift=shift, output_final_state=True)
     for x, y, name in zip((got[0][0], got[1][0], got[2][0], *got[3]), want, ('o', 'lse_swa', 'lse_gsa', 'hk', 'hv')):
         assert_close(x, y, TOL_OUT, name)
+
+
+@pytest.mark.parametrize('M', [16, 32, 48, 64])
+@pytest.mark.parametrize('HQ,H,cu,wl,shift', [(2, 2, [0, 64, 193], 64, 0), (3, 1, [0, 1, 130], [0, 63], 64), (4, 2, [0, 321], 200, 65),
+                                              (1, 1, [0, 257], -1, 0)])
+def test_backward(M, HQ, H, cu, wl, shift):
+    T = cu[-1]
+    d = {n: x[0] for n, x in gen.layer_inputs(70 + M + T, 1, T, HQ, H, 64, 64, M, gate_div=2.0, val_scale=1.0).items() if torch.is_tensor(x)}
+    ge = torch.Generator().manual_seed(M + T)
+    do, dlse = torch.randn(T, HQ, 64, generator=ge).bfloat16(), 0.1 * torch.randn(T, HQ, generator=ge)
+    N = len(cu) - 1
+    dhk, dhv = 0.1 * torch.randn(N, H, 64, M, generator=ge), 0.1 * torch.randn(N, H, M, 64, generator=ge)
+    wls = wl if isinstance(wl, list) else [wl] * N
+    want, gwant = run_oracle(d, cu, 0.125, wls, [shift] * N, None, None, do, dlse, dhk, dhv)
+    got, ggot = run_gpu(d, cu, max(b - a for a, b in zip(cu, cu[1:])), 0.125, wls, [shift] * N, None, None, do, dlse, dhk, dhv)
+    compare(got, ggot, want, gwant)
