@@ -28,14 +28,20 @@ def test_forward(M, HQ, H, T, wl, shift):
 @pytest.mark.parametrize('M', [16, 32, 48, 64])
 @pytest.mark.parametrize('HQ,H,cu,wl,shift', [(2, 2, [0, 64, 193], 64, 0), (3, 1, [0, 1, 130], [0, 63], 64), (4, 2, [0, 321], 200, 65),
                                               (1, 1, [0, 257], -1, 0)])
-def test_backward(M, HQ, H, cu, wl, shift):
+def test_backward(M, HQ, H, cu, wl, shift, D=64):
     T = cu[-1]
-    d = {n: x[0] for n, x in gen.layer_inputs(70 + M + T, 1, T, HQ, H, 64, 64, M, gate_div=2.0, val_scale=1.0).items() if torch.is_tensor(x)}
+    d = {n: x[0] for n, x in gen.layer_inputs(70 + M + T, 1, T, HQ, H, D, D, M, gate_div=2.0, val_scale=1.0).items() if torch.is_tensor(x)}
     ge = torch.Generator().manual_seed(M + T)
-    do, dlse = torch.randn(T, HQ, 64, generator=ge).bfloat16(), 0.1 * torch.randn(T, HQ, generator=ge)
+    do, dlse = torch.randn(T, HQ, D, generator=ge).bfloat16(), 0.1 * torch.randn(T, HQ, generator=ge)
     N = len(cu) - 1
-    dhk, dhv = 0.1 * torch.randn(N, H, 64, M, generator=ge), 0.1 * torch.randn(N, H, M, 64, generator=ge)
+    dhk, dhv = 0.1 * torch.randn(N, H, D, M, generator=ge), 0.1 * torch.randn(N, H, M, D, generator=ge)
     wls = wl if isinstance(wl, list) else [wl] * N
-    want, gwant = run_oracle(d, cu, 0.125, wls, [shift] * N, None, None, do, dlse, dhk, dhv)
-    got, ggot = run_gpu(d, cu, max(b - a for a, b in zip(cu, cu[1:])), 0.125, wls, [shift] * N, None, None, do, dlse, dhk, dhv)
+    want, gwant = run_oracle(d, cu, D ** -0.5, wls, [shift] * N, None, None, do, dlse, dhk, dhv)
+    got, ggot = run_gpu(d, cu, max(b - a for a, b in zip(cu, cu[1:])), D ** -0.5, wls, [shift] * N, None, None, do, dlse, dhk, dhv)
     compare(got, ggot, want, gwant)
+
+
+@pytest.mark.parametrize('HQ,H,cu,wl,shift', [(2, 2, [0, 64, 193], 64, 0), (4, 1, [0, 1, 130], [0, 63], 64), (4, 2, [0, 321], 200, 65),
+                                              (2, 1, [0, 257], -1, 0), (3, 1, [0, 191], 127, 128)])
+def test_backward_128(HQ, H, cu, wl, shift):
+    test_backward(64, HQ, H, cu, wl, shift, D=128)
