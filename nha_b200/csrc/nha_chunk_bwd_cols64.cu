@@ -154,14 +154,14 @@ __global__ void __launch_bounds__(kThreads, ONE ? 2 : 1) nha_bwd_cols64_kernel(c
     if (nr.n >= 0) {
       const int row = nr.t0 + nr.ci * kChunk;
       const size_t nch = (size_t)ncg * H + nhd;
-      prefetch_tile(maps.g, nhd, row);
-      prefetch_tile(maps.s, nhd, row);
-      prefetch_tile(maps.kg, nhd, row);
-      prefetch_tile(maps.v, nhd, row);
-      prefetch_tile(maps.qg, nhd * NG, row);
-      prefetch_tile(maps.dout, nhd * NG, row);
-      prefetch_tile(maps.za, nhd * NG, row);
-      prefetch_tile(maps.pa, nhd * NG, row);
+      prefetch_tile(maps.g, 0, nhd, row);
+      prefetch_tile(maps.s, 0, nhd, row);
+      prefetch_tile(maps.kg, 0, nhd, row);
+      prefetch_tile(maps.v, 0, nhd, row);
+      prefetch_tile(maps.qg, 0, nhd * NG, row);
+      prefetch_tile(maps.dout, 0, nhd * NG, row);
+      prefetch_tile(maps.za, 0, nhd * NG, row);
+      prefetch_tile(maps.pa, 0, nhd * NG, row);
       prefetch_bytes(w.dkc + nch * 4096, 16384);
       prefetch_bytes(w.dvc + nch * 4096, 16384);
       prefetch_bytes((const bf16*)d.hk_chunks + nch * 4096, kTile);

@@ -96,20 +96,6 @@ __device__ __forceinline__ void mma64(uint32_t d, uint64_t a, uint64_t b, uint32
 }
 __device__ __forceinline__ uint32_t idesc64(int amn, int bmn, int n = 64) { return make_idesc(64, n, bmn) | ((uint32_t)amn << 15); }
 
-// a [64][64] tile / a contiguous 16-byte aligned range into L2
-__device__ __forceinline__ void prefetch_tile(const CUtensorMap& map, int head, int row) {
-  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(reinterpret_cast<uint64_t>(&map)), "r"(0), "r"(head),
-               "r"(row)
-               : "memory");
-}
-__device__ __forceinline__ void prefetch_bytes(const void* p, uint32_t bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-}
-// adds to the bytes that the barrier's current phase waits for (no arrival)
-__device__ __forceinline__ void mbar_expect_more(uint64_t* mbar, uint32_t bytes) {
-  asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(mbar)), "r"(bytes) : "memory");
-}
-
 // rows r and r + 32 of a [64][64] tile, piece c (r = tid / 8, c = tid % 8); off = sw_off(r, c)
 __device__ __forceinline__ void tile_in(unsigned char* tile, uint32_t off, const bf16* p0, bool ok0, const bf16* p1, bool ok1) {
   cp16(tile + off, p0, ok0);
