@@ -405,14 +405,16 @@ int nha_act3_bwd(const void* const* x, const void* const* dy, void* const* dx, c
  *     o, y bf16 [rows, cols]; weight, bias (may be NULL) fp32 [cols]; rstd fp32 [rows] (may be NULL; needed by
  *     the backward).  cols a multiple of 256, at most 2048 (NHA_ERR_UNSUPPORTED otherwise).
  *   nha_silu_rmsnorm_bwd: d_o from dy (gradient of y); part_w, part_b (may be NULL) fp32
- *     [nha_silu_rmsnorm_bwd_ctas(rows), cols]: per-CTA partial sums of the weight and bias gradients, to be
- *     summed over their first axis by the caller.
+ *     [nha_silu_rmsnorm_bwd_ctas(rows), cols]: per-CTA partial sums of the weight and bias gradients, every
+ *     element written.  nha_silu_rmsnorm_part_sum adds them up over their first axis (fixed order: equal
+ *     inputs give equal bits); parts == 0 gives zeros.
  * The projection itself is a plain GEMM and stays with the GEMM library. */
 int nha_silu_rmsnorm_fwd(const void* o, const float* weight, const float* bias, void* y, float* rstd, int64_t rows,
                          int cols, float eps, void* stream);
 int nha_silu_rmsnorm_bwd_ctas(int64_t rows);
 int nha_silu_rmsnorm_bwd(const void* o, const float* weight, const float* rstd, const void* dy, void* d_o,
                          float* part_w, float* part_b, int64_t rows, int cols, void* stream);
+int nha_silu_rmsnorm_part_sum(const float* part_w, const float* part_b, float* dw, float* db, int parts, int cols, void* stream);
 
 /* ------------------------------------------------------------------------------------------
  * Layer-side consumers of lse_swa / lse_gsa, fused (the training layer's aux loss and compression

@@ -96,6 +96,7 @@ SYMBOLS = {
     'nha_silu_rmsnorm_bwd_ctas': (C.c_int, [C.c_int64]),
     'nha_silu_rmsnorm_bwd': (C.c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, C.c_int64,
                                        C.c_int, c_void_p]),
+    'nha_silu_rmsnorm_part_sum': (C.c_int, [c_void_p, c_void_p, c_void_p, c_void_p, C.c_int, C.c_int, c_void_p]),
     'nha_rope_pair': (C.c_int, [c_void_p] * 6 + [C.c_int64, C.c_int, c_void_p, C.c_int, C.c_int, C.c_int64] + [C.c_int] * 5
                       + [c_void_p]),
     'nha_lse_stats_scratch_bytes': (C.c_int64, []),

@@ -232,13 +232,16 @@ struct SiluRmsNorm : Function<SiluRmsNorm> {
     const c10::cuda::OptionalCUDAGuard guard(oc.device());
     const int64_t cols = oc.size(-1), rows = rstd.numel();
     const Tensor dy = bf16c(grads[0]), d_o = empty_same(oc);
-    const int64_t parts = std::max(1, nha_silu_rmsnorm_bwd_ctas(rows));
+    const int parts = nha_silu_rmsnorm_bwd_ctas(rows);
     const bool has_bias = ctx->saved_data["b"].toInt() >= 0;
-    const Tensor pw = zeros({parts, cols}, at::kFloat, oc), pb = has_bias ? zeros({parts, cols}, at::kFloat, oc) : Tensor();
+    const Tensor pw = empty({std::max(1, parts), cols}, at::kFloat, oc), pb = has_bias ? empty({std::max(1, parts), cols}, at::kFloat, oc) : Tensor();
+    const Tensor dw = empty({cols}, at::kFloat, oc), db = has_bias ? empty({cols}, at::kFloat, oc) : Tensor();
     check(nha_silu_rmsnorm_bwd(oc.data_ptr(), (const float*)w.data_ptr(), (const float*)rstd.data_ptr(), dy.data_ptr(), d_o.data_ptr(),
                                (float*)pw.data_ptr(), (float*)ptr(pb), rows, (int)cols, stream_of(oc)), "nha_silu_rmsnorm_bwd");
-    return {back_to(d_o, type_of(ctx->saved_data["o"])), back_to(pw.sum(0), type_of(ctx->saved_data["w"])),
-            has_bias ? back_to(pb.sum(0), type_of(ctx->saved_data["b"])) : Tensor(), Tensor()};
+    check(nha_silu_rmsnorm_part_sum((const float*)pw.data_ptr(), (const float*)ptr(pb), (float*)dw.data_ptr(), (float*)ptr(db), parts,
+                                    (int)cols, stream_of(oc)), "nha_silu_rmsnorm_part_sum");
+    return {back_to(d_o, type_of(ctx->saved_data["o"])), back_to(dw, type_of(ctx->saved_data["w"])),
+            has_bias ? back_to(db, type_of(ctx->saved_data["b"])) : Tensor(), Tensor()};
   }
 };
 

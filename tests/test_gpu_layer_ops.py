@@ -72,3 +72,9 @@ def test_silu_rms_norm_refuses_widths_without_a_kernel():
     from nha_b200._lib import NHALibraryError
     with pytest.raises(NHALibraryError):
         silu_rms_norm(torch.zeros(4, 200, device='cuda', dtype=torch.bfloat16), torch.ones(200, device='cuda'))
+
+
+@pytest.mark.parametrize('rows,cols', [(1, 512), (9, 768), (4099, 512), (1201, 1536)])
+def test_silu_rms_norm_teams(rows, cols):
+    # widths with several rows or several warps to a CTA, row counts around a CTA's share
+    test_silu_rms_norm_linear_forward_and_backward(rows, cols, True)
