@@ -401,6 +401,7 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows128_kernel(const nha_
       const bool fin = i + 1 == ntile;
       if (!fin) {
         load_wv(i + 1);                                         // the values, q_swa and do of the last tile have been read
+        cp_commit();
       } else if (more) {
         load_q(d.q_gsa, tQ, hq + 1);
         load_q(d.d_o, tDO, hq + 1);

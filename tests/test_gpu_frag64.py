@@ -45,3 +45,19 @@ def test_backward(M, HQ, H, cu, wl, shift, D=64):
                                               (2, 1, [0, 257], -1, 0), (3, 1, [0, 191], 127, 128)])
 def test_backward_128(HQ, H, cu, wl, shift):
     test_backward(64, HQ, H, cu, wl, shift, D=128)
+
+
+def test_backward_128_repeatable():
+    # many chunks in flight, several window tiles, several heads a group: tiles that were read before they arrived would show as
+    # differences between two runs
+    from nha_b200 import chunk_nha
+    d = gen.layer_inputs(91, 2, 1999, 16, 4, 128, 128, 64)
+    do = d['do'].cuda()
+    runs = []
+    for _ in range(4):
+        x = [d[n].cuda().requires_grad_(True) for n in NAMES]
+        o = chunk_nha(*x, window_size_left=200, window_size_right=0, gsa_kv_shift=128)[0]
+        runs.append(torch.autograd.grad(o, x, do))
+    for other in runs[1:]:
+        for a, b, n in zip(runs[0], other, NAMES):
+            assert torch.equal(a, b), n
