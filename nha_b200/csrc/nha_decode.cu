@@ -16,6 +16,7 @@
 // (nha_fla/ops/nha/fused_recurrent.py:229-353 k-kernel, :356-428 v-kernel) and, with caller-supplied
 // window logits, the kernels of fused_recurrent_nha (:48-147).
 #include "nha_common.cuh"
+#include "nha_decode_args.cuh"
 
 namespace nha {
 
@@ -23,21 +24,6 @@ constexpr int kDecThreads = 256;
 constexpr int kDecWarps = kDecThreads / 32;
 constexpr int kMaxStageRows = 16 * kDecWarps;   // keys per CTA: one 16-key tile per warp
 constexpr int kMaxSplits = 16;
-
-struct DecodeArgs {
-  const bf16* q; const bf16* sq; const bf16* k; const bf16* v; const bf16* g; const bf16* s;
-  const bf16* sw_k; const bf16* sw_v; const bf16* cosp; const bf16* sinp; const bf16* win_logits;
-  float* hk; float* hv; bf16* o; float* win_prob;
-  float* part_o;      // [B*H, SPLITS, NG, V] unnormalised partial outputs
-  float* part_ml;     // [B*H, SPLITS, NG, 2] running max and sum of each split
-  int* tickets;       // [B*H] arrival counters, zero between calls
-  int64_t cs_batch, cs_row;
-  int B, HQ, H, K, V, M, W, NG, SPLITS, KS, KSp, MQ, zero_state;
-  float scale;
-  // shared-memory byte offsets
-  int off_qraw, off_sqA, off_oks, off_eg, off_sv, off_kpop, off_vpop, off_ml, off_P, off_hk, off_hv, off_kst, off_vst,
-      off_S;
-};
 
 __host__ __device__ inline int align_up(int x, int a) { return (x + a - 1) / a * a; }
 
@@ -469,6 +455,9 @@ int decode_stream_try(const void* q, const void* sq, const void* k, const void* 
                       cudaStream_t st, const int* head, const void* ring_g, int ring_rows, int nopop,
                       const void* ring_kraw, const void* g_new, int state_bf16);
 
+bool decode_logits_supported(const DecodeArgs& a);
+int decode_logits_launch(const DecodeArgs& a, cudaStream_t cs);
+
 // Workspace: [B*H tickets | error word] (ints, zero between calls), then the (max, sum) and the partial outputs of
 // every split.  Sized for whichever kernel cuts a (sequence, kv head) into more splits.
 static int decode_max_splits(int B, int H, int W) {
@@ -561,6 +550,7 @@ static int decode_step_impl(const void* q, const void* sq, const void* k, const 
     return decode_stream_try(q, sq, k, v, g, s, sw_k, sw_v, cosp, sinp, cs_batch, cs_row, hk, hv, zero_state, o, a.tickets,
                              errw, a.part_ml, a.part_o, a.SPLITS, B, HQ, H, K, M, W, scale, (cudaStream_t)stream, nullptr,
                              nullptr, W, 0, nullptr, nullptr, state_bf16);
+  if (decode_logits_supported(a) && !(force_general && force_general[0] == '1')) return decode_logits_launch(a, (cudaStream_t)stream);
   const int smem = decode_layout(a);
   if (smem > kMaxSmem) return NHA_ERR_SMEM;
   cudaStream_t st = (cudaStream_t)stream;

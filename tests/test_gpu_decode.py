@@ -74,6 +74,21 @@ def test_recurrent_grid(idx):
     assert_close(hv, ref_hv, 1e-5, 'hvt')
 
 
+@pytest.mark.parametrize('B,H,NG,D,W,zero', [(1, 1, 1, 64, 1, True), (3, 2, 3, 64, 33, False), (2, 1, 8, 128, 513, False), (5, 3, 2, 128, 7, True),
+                                             (1, 2, 9, 64, 40, False)])
+def test_recurrent_state_in_registers(B, H, NG, D, W, zero):
+    # the smallest and largest groups and windows, states given and absent; nine heads a group take the general kernel
+    from nha_b200 import fused_recurrent_nha
+    d = gen.recurrent_inputs(3000 + W, B, H, NG, D, D, 64, W)
+    st = (None, None) if zero else (d['hk0'], d['hv0'])
+    want = orc.recurrent_step(d['q'], d['k'], d['v'], d['sliding_window'], d['s'], d['g'], d['scale'], *st)
+    c = cuda(d)
+    o, pw, (hk, hv) = fused_recurrent_nha(c['q'], c['k'], c['v'], c['sliding_window'], c['s'], c['g'], scale=d['scale'],
+                                          initial_state=None if zero else (c['hk0'].clone(), c['hv0'].clone()), output_final_state=True)
+    for got, ref, tol, name in zip((o, pw, hk, hv), want, (TOL_OUT, TOL_OUT, 1e-5, 1e-5), ('o', 'swa_score', 'hkt', 'hvt')):
+        assert_close(got, ref, tol, name)
+
+
 @pytest.mark.parametrize('case', sorted(MAN['decode']))
 def test_decode_against_reference_fixture(case):
     from nha_b200 import fused_recurrent_nha_decode
