@@ -150,6 +150,8 @@ __device__ __forceinline__ void nha_bwd_window_rows_kernel_body(const nha_chunk_
 // One CTA walks `cpc` consecutive chunks (1 when the kernel handles every chunk; more when it is launched gated
 // on the chunk flags and most chunks return at once, so that an all-clear launch costs few CTAs).
 __global__ void __launch_bounds__(kBwThreads) nha_bwd_window_rows_kernel(const nha_chunk_desc d, const BwdWs w, const int cpc) {
+  grid_dep_wait();
+  grid_dep_launch();
   const int ncb = (int)((d.Ttot + kChunk - 1) / kChunk + d.N);
   // which of my chunks have work: one flag load per chunk, all at once (cpc <= 32)
   __shared__ unsigned todo;
@@ -191,6 +193,8 @@ __host__ __device__ inline WColLayout wcol_layout(int K, int V) {
 }
 
 __global__ void __launch_bounds__(kBwThreads) nha_bwd_window_cols_kernel(const nha_chunk_desc d, const BwdWs w) {
+  grid_dep_wait();
+  grid_dep_launch();
   ChunkCtx c;
   if (!chunk_ctx(d, blockIdx.x, c)) return;
   const int K = d.K, V = d.V, H = d.H, HQ = d.HQ, NG = HQ / H, h = blockIdx.y;
@@ -613,6 +617,8 @@ __device__ __forceinline__ void nha_bwd_slot_kernel_body(const nha_chunk_desc d,
 // One CTA walks `cpc` consecutive chunks (1 when the kernel handles every chunk; more when it is launched gated
 // on the chunk flags and most chunks return at once, so that an all-clear launch costs few CTAs).
 __global__ void __launch_bounds__(kBwThreads) nha_bwd_slot_kernel(const nha_chunk_desc d, const BwdWs w, const int cpc) {
+  grid_dep_wait();
+  grid_dep_launch();
   const int ncb = (int)((d.Ttot + kChunk - 1) / kChunk + d.N);
   // which of my chunks have work: one flag load per chunk, all at once (cpc <= 32)
   __shared__ unsigned todo;
@@ -708,6 +714,8 @@ __device__ __forceinline__ void nha_bwd_local_terms_kernel_body(const nha_chunk_
 // One CTA walks `cpc` consecutive chunks (1 when the kernel handles every chunk; more when it is launched gated
 // on the chunk flags and most chunks return at once, so that an all-clear launch costs few CTAs).
 __global__ void __launch_bounds__(kBwThreads) nha_bwd_local_terms_kernel(const nha_chunk_desc d, const BwdWs w, const int cpc) {
+  grid_dep_wait();
+  grid_dep_launch();
   const int ncb = (int)((d.Ttot + kChunk - 1) / kChunk + d.N);
   // which of my chunks have work: one flag load per chunk, all at once (cpc <= 32)
   __shared__ unsigned todo;
@@ -733,6 +741,8 @@ __global__ void __launch_bounds__(kBwThreads) nha_bwd_local_terms_kernel(const n
 // recurrence so that enough loads are in flight to cover the memory latency.
 constexpr int kScanBatch = 8;
 __global__ void __launch_bounds__(256) nha_bwd_state_scan_kernel(const nha_chunk_desc d, const BwdWs w) {
+  grid_dep_wait();
+  grid_dep_launch();
   const int K = d.K, V = d.V, M = d.M, H = d.H;
   const int KM = K * M, MV = M * V;
   const size_t nh = blockIdx.x;                     // (sequence, kv head) in x: no 65535 limit on packed batches
@@ -1004,6 +1014,8 @@ __device__ __forceinline__ void nha_bwd_inter_kernel_body(const nha_chunk_desc d
 // One CTA walks `cpc` consecutive chunks (1 when the kernel handles every chunk; more when it is launched gated
 // on the chunk flags and most chunks return at once, so that an all-clear launch costs few CTAs).
 __global__ void __launch_bounds__(kBwThreads) nha_bwd_inter_kernel(const nha_chunk_desc d, const BwdWs w, const int cpc) {
+  grid_dep_wait();
+  grid_dep_launch();
   const int ncb = (int)((d.Ttot + kChunk - 1) / kChunk + d.N);
   // which of my chunks have work: one flag load per chunk, all at once (cpc <= 32)
   __shared__ unsigned todo;
@@ -1098,8 +1110,8 @@ static int bwd_run(const nha_chunk_desc* d, int stage_mask, void* stream) {
       st = bwd_umma_launch(d, wu, 0, err, cs);
       if (st != NHA_OK) return st;
     }
-    if (umma) nha_bwd_window_rows_kernel<<<ggrid, block, L1.total, cs>>>(*d, wg, cpc);
-    else nha_bwd_window_rows_kernel<<<grid, block, L1.total, cs>>>(*d, wg, 1);
+    if (umma) launch_after(nha_bwd_window_rows_kernel, ggrid, block, L1.total, cs, *d, wg, cpc);
+    else launch_after(nha_bwd_window_rows_kernel, grid, block, L1.total, cs, *d, wg, 1);
     st = check_launch();
     if (st != NHA_OK) return st;
   }
@@ -1109,24 +1121,24 @@ static int bwd_run(const nha_chunk_desc* d, int stage_mask, void* stream) {
     if (bwd_wcols_umma_supported(d) && !(off && off[0] == '1')) {
       st = bwd_wcols_umma_launch(d, w, err, cs);
     } else {
-      nha_bwd_window_cols_kernel<<<grid, block, L2.total, cs>>>(*d, w);
+      launch_after(nha_bwd_window_cols_kernel, grid, block, L2.total, cs, *d, w);
       st = check_launch();
     }
     if (st != NHA_OK) return st;
   }
   if (stage_mask & 4) {
-    if (umma) nha_bwd_slot_kernel<<<ggrid, block, L3.total, cs>>>(*d, wg, cpc);
-    else nha_bwd_slot_kernel<<<grid, block, L3.total, cs>>>(*d, wg, 1);
+    if (umma) launch_after(nha_bwd_slot_kernel, ggrid, block, L3.total, cs, *d, wg, cpc);
+    else launch_after(nha_bwd_slot_kernel, grid, block, L3.total, cs, *d, wg, 1);
     st = check_launch();
     if (st != NHA_OK) return st;
   }
   if (stage_mask & 8) {
-    if (umma) nha_bwd_local_terms_kernel<<<ggrid, block, L5.total, cs>>>(*d, wg, cpc);
-    else nha_bwd_local_terms_kernel<<<grid, block, L5.total, cs>>>(*d, wg, 1);
+    if (umma) launch_after(nha_bwd_local_terms_kernel, ggrid, block, L5.total, cs, *d, wg, cpc);
+    else launch_after(nha_bwd_local_terms_kernel, grid, block, L5.total, cs, *d, wg, 1);
     st = check_launch();
     if (st != NHA_OK) return st;
     const int SD = d->K * d->M + d->M * d->V;
-    nha_bwd_state_scan_kernel<<<dim3(d->N * d->H, (SD / 4 + 255) / 256), 256, 0, cs>>>(*d, w);
+    launch_after(nha_bwd_state_scan_kernel, dim3(d->N * d->H, (SD / 4 + 255) / 256), 256, 0, cs, *d, w);
     st = check_launch();
     if (st != NHA_OK) return st;
   }
@@ -1135,8 +1147,8 @@ static int bwd_run(const nha_chunk_desc* d, int stage_mask, void* stream) {
       st = bwd_umma_launch(d, wu, 1, err, cs);
       if (st != NHA_OK) return st;
     }
-    if (umma) nha_bwd_inter_kernel<<<ggrid, block, L4.total, cs>>>(*d, wg, cpc);
-    else nha_bwd_inter_kernel<<<grid, block, L4.total, cs>>>(*d, wg, 1);
+    if (umma) launch_after(nha_bwd_inter_kernel, ggrid, block, L4.total, cs, *d, wg, cpc);
+    else launch_after(nha_bwd_inter_kernel, grid, block, L4.total, cs, *d, wg, 1);
     st = check_launch();
   }
   return st;

@@ -46,6 +46,8 @@ struct ColsMaps {
 template <bool ONE>
 __global__ void __launch_bounds__(kThreads, ONE ? 2 : 1) nha_bwd_cols64_kernel(const nha_chunk_desc d, const BwdWs w, int* __restrict__ err,
                                                                                  const __grid_constant__ ColsMaps maps) {
+  grid_dep_wait();
+  grid_dep_launch();
   using namespace cl64;
   constexpr int c0_ = 0, c1_ = 64, c2_ = 128, c3_ = 192, kTmemCols = ONE ? 256 : 512;
   constexpr int cDS = ONE ? 0 : 256, cDK = ONE ? 64 : 320, cDV = ONE ? 128 : 384, cDS2 = ONE ? 192 : 448;
@@ -467,8 +469,8 @@ int bwd_cols64_launch(const nha_chunk_desc* d, const BwdWs& w, int* err, cudaStr
              make_map_rows_heads(&maps.s, d->s, d->Ttot, d->H, 64) && make_map_rows_heads(&maps.dout, d->d_o, d->Ttot, d->HQ, 64) &&
              make_map_rows_heads(&maps.za, w.dza, d->Ttot, d->HQ, 64) && make_map_rows_heads(&maps.pa, w.paq, d->Ttot, d->HQ, 64);
   const dim3 grid((unsigned)(nha_chunk_count_bound(d->Ttot, d->N) * d->H));
-  if (d->HQ == d->H) nha_bwd_cols64_kernel<true><<<grid, kThreads, cl64::total, cs>>>(*d, w, err, maps);
-  else nha_bwd_cols64_kernel<false><<<grid, kThreads, cl64::total, cs>>>(*d, w, err, maps);
+  if (d->HQ == d->H) launch_after(nha_bwd_cols64_kernel<true>, grid, kThreads, cl64::total, cs, *d, w, err, maps);
+  else launch_after(nha_bwd_cols64_kernel<false>, grid, kThreads, cl64::total, cs, *d, w, err, maps);
   return check_launch();
 }
 

@@ -41,6 +41,8 @@ static_assert(total <= 113 * 1024, "two CTAs per SM");
 }  // namespace rw128
 
 __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows128_kernel(const nha_chunk_desc d, const BwdWs w, int* __restrict__ err) {
+  grid_dep_wait();
+  grid_dep_launch();
   using namespace rw128;
   const int H = d.H, HQ = d.HQ, NG = HQ / H;
   const int cg = blockIdx.x / H, h = blockIdx.x - cg * H;
@@ -458,7 +460,7 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows128_kernel(const nha_
 int bwd_rows128_launch(const nha_chunk_desc* d, const BwdWs& w, int* err, cudaStream_t cs) {
   cudaError_t e = set_max_smem((const void*)nha_bwd_rows128_kernel, rw128::total);
   if (e != cudaSuccess) return record_cuda_error(e);
-  nha_bwd_rows128_kernel<<<dim3((unsigned)(nha_chunk_count_bound(d->Ttot, d->N) * d->H)), kThreads, rw128::total, cs>>>(*d, w, err);
+  launch_after(nha_bwd_rows128_kernel, dim3((unsigned)(nha_chunk_count_bound(d->Ttot, d->N) * d->H)), kThreads, rw128::total, cs, *d, w, err);
   return check_launch();
 }
 

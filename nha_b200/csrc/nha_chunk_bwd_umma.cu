@@ -40,6 +40,8 @@ constexpr int kColsThreads = 256;        // columns pass: two threads per row
 // columns pass multiplies with.  One CTA per (chunk, kv head); M == 64.
 constexpr int kCarryThreads = 256;
 __global__ void __launch_bounds__(kCarryThreads) nha_bwd_gate_carry_kernel(const nha_chunk_desc d, const BwdWs w) {
+  grid_dep_wait();
+  grid_dep_launch();
   constexpr int M = 64;
   const int H = d.H, N = d.N, K = d.K, V = d.V;
   const int cg = blockIdx.x, h = blockIdx.y;
@@ -205,6 +207,8 @@ struct ColsLayout {
 template <int D, int R>
 __global__ void __launch_bounds__(kColsThreads, (D == 64 && R == 64) ? 2 : 1)
     nha_bwd_cols_umma_kernel(const nha_chunk_desc d, const BwdWs w, int* __restrict__ err) {
+  grid_dep_wait();
+  grid_dep_launch();
   typedef ColsLayout<D, R> L;
   constexpr int KT = L::KT, TH = R / 64, M = 64, NT = kColsThreads;
   const int H = d.H, HQ = d.HQ, NG = HQ / H, N = d.N;
@@ -544,10 +548,10 @@ static int launch_cols(const nha_chunk_desc* d, const BwdWs& w, int* err, cudaSt
   cudaError_t e = set_max_smem((const void*)nha_bwd_cols_umma_kernel<D, R>, L::total);
   if (e != cudaSuccess) return record_cuda_error(e);
   const int NCB = (int)nha_chunk_count_bound(d->Ttot, d->N);
-  nha_bwd_gate_carry_kernel<<<dim3(NCB, d->H), kCarryThreads, 0, cs>>>(*d, w);
+  launch_after(nha_bwd_gate_carry_kernel, dim3(NCB, d->H), kCarryThreads, 0, cs, *d, w);
   int st = check_launch();
   if (st != NHA_OK) return st;
-  nha_bwd_cols_umma_kernel<D, R><<<dim3(NCB, d->H), kColsThreads, L::total, cs>>>(*d, w, err);
+  launch_after(nha_bwd_cols_umma_kernel<D, R>, dim3(NCB, d->H), kColsThreads, L::total, cs, *d, w, err);
   return check_launch();
 }
 

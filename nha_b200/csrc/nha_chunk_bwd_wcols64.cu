@@ -26,6 +26,8 @@ constexpr int cS = 0, cDP = 64, cDV = 128, cDK = 192, kTmemCols = 256;
 }  // namespace wc64
 
 __global__ void __launch_bounds__(kThreads, 2) nha_bwd_wcols64_kernel(const nha_chunk_desc d, const BwdWs w, int* __restrict__ err) {
+  grid_dep_wait();
+  grid_dep_launch();
   using namespace wc64;
   const int H = d.H, HQ = d.HQ, NG = HQ / H;
   const int cg = blockIdx.x / H, h = blockIdx.x - cg * H;
@@ -183,7 +185,7 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_wcols64_kernel(const nha_
 int bwd_wcols64_launch(const nha_chunk_desc* d, const BwdWs& w, int* err, cudaStream_t cs) {
   cudaError_t e = set_max_smem((const void*)nha_bwd_wcols64_kernel, wc64::total);
   if (e != cudaSuccess) return record_cuda_error(e);
-  nha_bwd_wcols64_kernel<<<dim3((unsigned)(nha_chunk_count_bound(d->Ttot, d->N) * d->H)), kThreads, wc64::total, cs>>>(*d, w, err);
+  launch_after(nha_bwd_wcols64_kernel, dim3((unsigned)(nha_chunk_count_bound(d->Ttot, d->N) * d->H)), kThreads, wc64::total, cs, *d, w, err);
   return check_launch();
 }
 

@@ -37,6 +37,8 @@ struct WColsLayout {
 };
 
 __global__ void __launch_bounds__(kWCThreads, 1) nha_bwd_wcols_umma_kernel(const nha_chunk_desc d, const BwdWs w, int* __restrict__ err) {
+  grid_dep_wait();
+  grid_dep_launch();
   typedef WColsLayout L;
   constexpr int D = L::D, KT = L::KT;
   const int H = d.H, HQ = d.HQ, NG = HQ / H, N = d.N;
@@ -206,7 +208,7 @@ int bwd_wcols_umma_launch(const nha_chunk_desc* d, const BwdWs& w, int* err, cud
   cudaError_t e = set_max_smem((const void*)nha_bwd_wcols_umma_kernel, WColsLayout::total);
   if (e != cudaSuccess) return record_cuda_error(e);
   const int NCB = (int)nha_chunk_count_bound(d->Ttot, d->N);
-  nha_bwd_wcols_umma_kernel<<<dim3(NCB * d->H), kWCThreads, WColsLayout::total, cs>>>(*d, w, err);
+  launch_after(nha_bwd_wcols_umma_kernel, dim3(NCB * d->H), kWCThreads, WColsLayout::total, cs, *d, w, err);
   return check_launch();
 }
 

@@ -381,7 +381,9 @@ __device__ __forceinline__ void nha_chunk_fwd_kernel_body(const nha_chunk_desc d
 
 // One CTA walks `cpc` consecutive chunks (1 when the kernel handles every chunk; more when it is launched gated
 // on the chunk flags and most chunks return at once, so that an all-clear launch costs few CTAs).
-__global__ void __launch_bounds__(kFwdThreads) nha_chunk_fwd_kernel(const nha_chunk_desc d, const int* __restrict__ only_flagged, const int cpc) {
+__global__ void __launch_bounds__(kFwdThreads) nha_chunk_fwd_kernel(const nha_chunk_desc d, const int* only_flagged, const int cpc) {
+  grid_dep_wait();
+  grid_dep_launch();
   const int ncb = (int)((d.Ttot + kChunk - 1) / kChunk + d.N);
   // which of my chunks have work: one flag load per chunk, all at once (cpc <= 32)
   __shared__ unsigned todo;
@@ -449,9 +451,9 @@ extern "C" int nha_chunk_output_pass(const nha_chunk_desc* d, void* stream) {
   if (umma_done) {
     // only the flagged chunks do work: sixteen chunks per CTA keep an all-clear launch short
     const int cpc = 16;
-    nha_chunk_fwd_kernel<<<dim3((grid.x + cpc - 1) / cpc, grid.y), block, L.total, cs>>>(*d, flags, cpc);
+    launch_after(nha_chunk_fwd_kernel, dim3((grid.x + cpc - 1) / cpc, grid.y), block, L.total, cs, *d, flags, cpc);
   } else {
-    nha_chunk_fwd_kernel<<<grid, block, L.total, cs>>>(*d, nullptr, 1);
+    launch_after(nha_chunk_fwd_kernel, grid, block, L.total, cs, *d, nullptr, 1);
   }
   return check_launch();
 }

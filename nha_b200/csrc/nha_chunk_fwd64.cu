@@ -38,6 +38,8 @@ static_assert(total <= 113 * 1024, "two CTAs per SM");
 }  // namespace fw64
 
 __global__ void __launch_bounds__(kThreads, 2) nha_fwd64_kernel(const nha_chunk_desc d, int* __restrict__ flags, int* __restrict__ err) {
+  grid_dep_wait();
+  grid_dep_launch();
   using namespace fw64;
   const int H = d.H, HQ = d.HQ, M = d.M, NG = HQ / H;
   const int cg = blockIdx.x / HQ, hq = blockIdx.x - cg * HQ, h = hq / NG;
@@ -425,7 +427,7 @@ bool fwd64_supported(const nha_chunk_desc* d) {
 int fwd64_launch(const nha_chunk_desc* d, int* flags, int* err, cudaStream_t cs) {
   cudaError_t e = set_max_smem((const void*)nha_fwd64_kernel, fw64::total);
   if (e != cudaSuccess) return record_cuda_error(e);
-  nha_fwd64_kernel<<<dim3((unsigned)(nha_chunk_count_bound(d->Ttot, d->N) * d->HQ)), kThreads, fw64::total, cs>>>(*d, flags, err);
+  launch_after(nha_fwd64_kernel, dim3((unsigned)(nha_chunk_count_bound(d->Ttot, d->N) * d->HQ)), kThreads, fw64::total, cs, *d, flags, err);
   return check_launch();
 }
 

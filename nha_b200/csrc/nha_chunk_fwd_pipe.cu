@@ -115,6 +115,8 @@ __device__ __forceinline__ uint32_t bf16_pair(float lo, float hi) {
 __global__ void __launch_bounds__(pipe::kThreads, 2)
     nha_fwd_pipe_kernel(const nha_chunk_desc d, int* __restrict__ flags, int* __restrict__ err,
                         const __grid_constant__ PipeMaps maps) {
+  grid_dep_wait();
+  grid_dep_launch();
   using namespace pipe;
   const int H = d.H, HQ = d.HQ, NG = HQ / H;
   // tiles of a chunk are neighbours in the grid: two heads a tile fastest, then the kv heads
@@ -741,7 +743,7 @@ int fwd_pipe_launch(const nha_chunk_desc* d, int* flags, int* err, cudaStream_t 
   if (!ok) return NHA_ERR_UNSUPPORTED;
   cudaError_t e = set_max_smem((const void*)nha_fwd_pipe_kernel, total);
   if (e != cudaSuccess) return record_cuda_error(e);
-  nha_fwd_pipe_kernel<<<dim3((unsigned)(NCB * d->H * ((d->HQ / d->H + 1) / 2))), kThreads, total, cs>>>(*d, flags, err, maps);
+  launch_after(nha_fwd_pipe_kernel, dim3((unsigned)(NCB * d->H * ((d->HQ / d->H + 1) / 2))), kThreads, total, cs, *d, flags, err, maps);
   return check_launch();
 }
 

@@ -37,6 +37,8 @@ constexpr int kStWarps = kStThreads / 32;
 constexpr int kPlanThreads = 512;
 __global__ void __launch_bounds__(kPlanThreads) nha_plan_kernel(int32_t* __restrict__ cu, int32_t* __restrict__ plan, int N, int NCB, int H,
                                                                 int T) {
+  grid_dep_wait();
+  grid_dep_launch();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) plan[N + 1 + NCB + (size_t)NCB * H] = 0;           // device-side error word
   int4* rec = reinterpret_cast<int4*>(plan + plan_rec_offset(N, NCB, H));
@@ -142,6 +144,8 @@ __host__ __device__ inline StLocalLayout st_local_layout(int K, int V, int M) {
 
 // One CTA per (chunk, kv head): L_k, L_v and Gend of that chunk.
 __global__ void __launch_bounds__(kStThreads) nha_state_local_kernel(const nha_chunk_desc d, const StateWs w, const int chunk_lo) {
+  grid_dep_wait();
+  grid_dep_launch();
   const int cg = chunk_lo + blockIdx.x, h = blockIdx.y;
   const int NCB = gridDim.x;
   const ChunkRec rc = chunk_rec(d, cg);
@@ -298,6 +302,8 @@ __device__ __forceinline__ void scan_bulk_g2s(void* dst, const void* src, uint32
 template <int kScanElems>
 __global__ void __launch_bounds__(kScanElems / 4 + 32) nha_state_scan_kernel(const nha_chunk_desc d, const StateWs w,
                                                                              int* __restrict__ err, const int kScanStages) {
+  grid_dep_wait();
+  grid_dep_launch();
   constexpr int kScanThreads = kScanElems / 4;      // consumer threads; one more warp hosts the producer
   constexpr int kScanSlot = scan_slot_bytes(kScanElems);
   const int K = d.K, V = d.V, M = d.M, H = d.H;
@@ -458,7 +464,7 @@ static int state_terms_on(const nha_chunk_desc* d, void* scratch, int chunk_lo, 
     const StLocalLayout L = st_local_layout(d->K, d->V, d->M);
     cudaError_t e = set_max_smem((const void*)nha_state_local_kernel, L.total);
     if (e != cudaSuccess) return record_cuda_error(e);
-    nha_state_local_kernel<<<dim3(chunk_n, d->H), kStThreads, L.total, cs>>>(*d, w, chunk_lo);
+    launch_after(nha_state_local_kernel, dim3(chunk_n, d->H), kStThreads, L.total, cs, *d, w, chunk_lo);
     st = check_launch();
   }
   return st;
@@ -485,15 +491,13 @@ static int state_scan_on(const nha_chunk_desc* d, void* scratch, cudaStream_t cs
       const int smem = scan_smem_bytes(1024, stages);
       cudaError_t e = set_max_smem((const void*)nha_state_scan_kernel<1024>, smem);
       if (e != cudaSuccess) return record_cuda_error(e);
-      nha_state_scan_kernel<1024><<<dim3((unsigned)(d->N * d->H), (unsigned)((SD + 1023) / 1024)), 1024 / 4 + 32, smem, cs>>>(
-          *d, w, err, stages);
+      launch_after(nha_state_scan_kernel<1024>, dim3((unsigned)(d->N * d->H), (unsigned)((SD + 1023) / 1024)), 1024 / 4 + 32, smem, cs, *d, w, err, stages);
     } else {
       const int stages = std::max(2, std::min(5, rounds));
       const int smem = scan_smem_bytes(512, stages);
       cudaError_t e = set_max_smem((const void*)nha_state_scan_kernel<512>, smem);
       if (e != cudaSuccess) return record_cuda_error(e);
-      nha_state_scan_kernel<512><<<dim3((unsigned)(d->N * d->H), (unsigned)((SD + 511) / 512)), 512 / 4 + 32, smem, cs>>>(
-          *d, w, err, stages);
+      launch_after(nha_state_scan_kernel<512>, dim3((unsigned)(d->N * d->H), (unsigned)((SD + 511) / 512)), 512 / 4 + 32, smem, cs, *d, w, err, stages);
     }
   }
   return check_launch();
@@ -626,7 +630,7 @@ extern "C" int64_t nha_chunk_plan_ints(int64_t Ttot, int64_t N, int64_t H) {
 static int plan_launch(const nha_chunk_desc* d, int T, void* stream) {
   if (!d || !d->cu_seqlens || !d->plan || d->N <= 0) return NHA_ERR_BAD_ARG;
   const int NCB = (int)nha_chunk_count_bound(d->Ttot, d->N);
-  nha_plan_kernel<<<1, kPlanThreads, 0, (cudaStream_t)stream>>>(const_cast<int32_t*>(d->cu_seqlens), d->plan, d->N, NCB, d->H, T);
+  launch_after(nha_plan_kernel, 1, kPlanThreads, 0, (cudaStream_t)stream, const_cast<int32_t*>(d->cu_seqlens), d->plan, d->N, NCB, d->H, T);
   return check_launch();
 }
 extern "C" int nha_chunk_plan(const nha_chunk_desc* d, void* stream) { return plan_launch(d, -1, stream); }

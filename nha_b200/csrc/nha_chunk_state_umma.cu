@@ -45,6 +45,8 @@ template <int D>
 __global__ void __launch_bounds__(stu::kThreads) nha_state_local_umma_kernel(const nha_chunk_desc d, const StateWs w,
                                                                              int* __restrict__ err, const int chunk_lo,
                                                                              const __grid_constant__ StateMaps maps) {
+  grid_dep_wait();
+  grid_dep_launch();
   using namespace stu;
   constexpr int DT = D / 64;                      // 64-column tiles of k' and v'
   constexpr int M = 64;
@@ -245,8 +247,8 @@ int state_local_umma_launch(const nha_chunk_desc* d, const StateWs& w, int* err,
   const void* fn = DT == 2 ? (const void*)nha_state_local_umma_kernel<128> : (const void*)nha_state_local_umma_kernel<64>;
   cudaError_t e = set_max_smem(fn, total);
   if (e != cudaSuccess) return record_cuda_error(e);
-  if (DT == 2) nha_state_local_umma_kernel<128><<<dim3(chunk_n, d->H), kThreads, total, cs>>>(*d, w, err, chunk_lo, maps);
-  else nha_state_local_umma_kernel<64><<<dim3(chunk_n, d->H), kThreads, total, cs>>>(*d, w, err, chunk_lo, maps);
+  if (DT == 2) launch_after(nha_state_local_umma_kernel<128>, dim3(chunk_n, d->H), kThreads, total, cs, *d, w, err, chunk_lo, maps);
+  else launch_after(nha_state_local_umma_kernel<64>, dim3(chunk_n, d->H), kThreads, total, cs, *d, w, err, chunk_lo, maps);
   return check_launch();
 }
 

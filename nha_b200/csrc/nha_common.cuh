@@ -127,9 +127,32 @@ __host__ __device__ __forceinline__ int64_t plan_rec_offset(int64_t N, int64_t N
   return (N + 1 + NCB + NCB * H + 4 + 3) & ~(int64_t)3;
 }
 struct ChunkRec { int n, ci, t0, len; };
+// Kernels of a chain are launched as programmatic dependents (launch_after): the next grid's CTAs are resident and waiting when the
+// last one finishes, which takes the launch and the ramp-up off the chain (1-2 us per kernel).  Every CTA of such a kernel calls
+// grid_dep_wait() before it reads or writes global memory and before it may return: when a grid has completed, so have all before.
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// (a failed launch is left to the check_launch() behind it, as with <<< >>>)
+template <typename... P, typename... A>
+inline void launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t cs, const A&... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = cs;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 __device__ __forceinline__ ChunkRec chunk_rec(const nha_chunk_desc& d, int cg) {
   const int ncb = (int)((d.Ttot + kChunk - 1) / kChunk + d.N);
-  const int4 r = __ldg(reinterpret_cast<const int4*>(d.plan + plan_rec_offset(d.N, ncb, d.H)) + cg);
+  // an ordinary load, which stays behind grid_dep_wait(); what a CTA reads through it depends on the record
+  const int4 r = *(reinterpret_cast<const int4*>(d.plan + plan_rec_offset(d.N, ncb, d.H)) + cg);
   ChunkRec c;
   c.n = r.x; c.ci = r.y; c.t0 = r.z; c.len = r.w;
   return c;

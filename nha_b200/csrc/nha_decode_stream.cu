@@ -132,8 +132,6 @@ __device__ __forceinline__ float2 ld_cluster_f2(uint32_t addr) {
 
 // programmatic dependent launch: wait until the grids this one depends on have completed and their writes are
 // visible; let the grid behind this one on the stream be scheduled
-__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // start of a 16-byte aligned range into L2
 __device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
