@@ -1,5 +1,6 @@
 // Backward of the window branch, key side, for head dim 64: dk_swa and the window part of dv, 64-row products with every lane at
-// work (nha_frag64.cuh).  What it computes is in nha_chunk_bwd_wcols_umma.cu, which it replaces at this head dim.
+// work (nha_frag64.cuh).  For every query row that can see a key, with the row's joint log-sum-exp L and delta = <do, o>:
+//     p = exp(scale q_swa k - L),  dz = scale p (do v - delta),  dv += p do,  dk_swa += dz q_swa.
 //
 // One CTA = the 64 keys of one (chunk, kv head), two CTAs per SM.  It walks the blocks of 64 query rows that can see a key (query
 // chunk x head of the group), one round of products per block:
@@ -182,11 +183,20 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_wcols64_kernel(const nha_
   if (failed) atomicExch(err, 1);
 }
 
-int bwd_wcols64_launch(const nha_chunk_desc* d, const BwdWs& w, int* err, cudaStream_t cs) {
+static int bwd_wcols64_launch(const nha_chunk_desc* d, const BwdWs& w, int* err, cudaStream_t cs) {
   cudaError_t e = set_max_smem((const void*)nha_bwd_wcols64_kernel, wc64::total);
   if (e != cudaSuccess) return record_cuda_error(e);
   launch_after(nha_bwd_wcols64_kernel, dim3((unsigned)(nha_chunk_count_bound(d->Ttot, d->N) * d->H)), kThreads, wc64::total, cs, *d, w, err);
   return check_launch();
+}
+
+bool bwd_wcols_umma_supported(const nha_chunk_desc* d) { return d->K == d->V && (d->K == 64 || d->K == 128); }
+
+int bwd_wcols128_launch(const nha_chunk_desc* d, const BwdWs& w, int* err, cudaStream_t cs);
+
+// The caller has checked bwd_wcols_umma_supported().
+int bwd_wcols_umma_launch(const nha_chunk_desc* d, const BwdWs& w, int* err, cudaStream_t cs) {
+  return d->K == 64 ? bwd_wcols64_launch(d, w, err, cs) : bwd_wcols128_launch(d, w, err, cs);
 }
 
 }  // namespace nha
