@@ -16,8 +16,12 @@
 //     S1       v'        p a, p e^G     keys of even tiles
 //     S2       Hv        Hk             values
 //     Q        q         q              q_swa
-// Gate terms are summed over the heads in registers, the local state-gradient terms by the thread that wrote them: one writer
-// per element, repeatable bits for any group size.
+// Gate terms are summed over the heads in registers, the local state-gradient terms in memory by the thread that wrote them: one
+// writer per element, repeatable bits for any group size.
+//
+// What bounds it: the chain of rounds of a CTA (HBM at 22 % of its rate, issue slots at 27 %).  Measured, 2 x 1999 tokens, 32 heads
+// on 8, window 127: 270 us with two heads to a 128-row tile and one CTA per SM, 204 us so, 187 us once the sums over the heads
+// are reductions in memory instead of loads, additions and stores.
 //
 // Replaces, with the other backward kernels, ChunkNativeHybridAttentionFunction.backward (nha_fla/ops/nha/chunk.py:491-564).
 #include "nha_bwd_common.cuh"
@@ -281,9 +285,8 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows128_kernel(const nha_
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         float2* p = reinterpret_cast<float2*>(base + (size_t)(r0 + 8 * i) * ld + 32 * half + 8 * j + 2 * tq);
-        float2 x = make_float2(v[4 * j + 2 * i], v[4 * j + 2 * i + 1]);
-        if (add) { const float2 y = *p; x.x += y.x; x.y += y.y; }
-        *p = x;
+        if (add) red_add2(reinterpret_cast<float*>(p), v[4 * j + 2 * i], v[4 * j + 2 * i + 1]);
+        else *p = make_float2(v[4 * j + 2 * i], v[4 * j + 2 * i + 1]);
       }
   };
   float* dkc = w.dkc + ((size_t)cg * H + h) * D * M;            // [D][M]

@@ -15,6 +15,8 @@
 // What bounds it: the chain of rounds of a CTA (HBM at 40 % of its rate).  Measured against the version with one row per lane,
 // the gate scan in shared memory and eleven rounds instead of seven: B16 T2048 H16 W64 627 -> 421 us; 32768 packed tokens,
 // windows 32-512, 740 -> 500 us; 16 query heads on 4, 4 x 2000 tokens, W 64, 164 -> 108 us (two heads to a tile before).
+// One head a kv head as a variant of its own 398 -> 388 us (first shape), sums over the heads as reductions in memory 112 -> 102 us
+// (last shape).
 //
 // Replaces, with the other backward kernels, ChunkNativeHybridAttentionFunction.backward (nha_fla/ops/nha/chunk.py:491-564).
 #include "nha_bwd_common.cuh"
@@ -37,11 +39,13 @@ constexpr int cLK = cAv, cLV = cY, cDQ = cQH, cS = cA, cDP = cAv, cDQS = cY;
 static_assert(total <= 113 * 1024, "two CTAs per SM");
 }  // namespace rw64
 
+// ONE: one query head per kv head (no loop over heads, nothing added up in memory)
+template <bool ONE>
 __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows64_kernel(const nha_chunk_desc d, const BwdWs w, int* __restrict__ err) {
   grid_dep_wait();
   grid_dep_launch();
   using namespace rw64;
-  const int H = d.H, HQ = d.HQ, M = d.M, NG = HQ / H;
+  const int H = d.H, HQ = d.HQ, M = d.M, NG = ONE ? 1 : HQ / H;
   const int cg = blockIdx.x / H, h = blockIdx.x - cg * H;
   const ChunkRec rc = chunk_rec(d, cg);
   if (rc.n < 0) return;
@@ -247,7 +251,7 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows64_kernel(const nha_c
 
   for (int ht = 0; ht < NG; ++ht) {
     const int hq = h * NG + ht;
-    if (ht > 0) {
+    if (!ONE && ht > 0) {
       load_head(hq);
       row_request(hq);
       row_stats(hq);
@@ -338,9 +342,8 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows64_kernel(const nha_c
           const int m = 32 * half + 8 * j + 2 * tq;
           if (m < M) {
             float2* p = reinterpret_cast<float2*>(dk + (size_t)(r0 + 8 * i) * M + m);
-            float2 x = make_float2(v[4 * j + 2 * i], v[4 * j + 2 * i + 1]);
-            if (ht > 0) { const float2 y = *p; x.x += y.x; x.y += y.y; }
-            *p = x;
+            if (!ONE && ht > 0) red_add2(reinterpret_cast<float*>(p), v[4 * j + 2 * i], v[4 * j + 2 * i + 1]);
+            else *p = make_float2(v[4 * j + 2 * i], v[4 * j + 2 * i + 1]);
           }
         }
       frag_ld(tl + cLV, v);
@@ -351,9 +354,8 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows64_kernel(const nha_c
         for (int i = 0; i < 2; ++i)
           if (r0 + 8 * i < M) {
             float2* p = reinterpret_cast<float2*>(dv + (r0 + 8 * i) * 64 + 32 * half + 8 * j + 2 * tq);
-            float2 x = make_float2(v[4 * j + 2 * i], v[4 * j + 2 * i + 1]);
-            if (ht > 0) { const float2 y = *p; x.x += y.x; x.y += y.y; }
-            *p = x;
+            if (!ONE && ht > 0) red_add2(reinterpret_cast<float*>(p), v[4 * j + 2 * i], v[4 * j + 2 * i + 1]);
+            else *p = make_float2(v[4 * j + 2 * i], v[4 * j + 2 * i + 1]);
           }
     }
     hand_over();
@@ -432,9 +434,11 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows64_kernel(const nha_c
 bool bwd64_supported(const nha_chunk_desc* d) { return d->K == 64 && d->V == 64 && d->M <= 64 && d->scale > 0.f; }
 
 int bwd_rows64_launch(const nha_chunk_desc* d, const BwdWs& w, int* err, cudaStream_t cs) {
-  cudaError_t e = set_max_smem((const void*)nha_bwd_rows64_kernel, rw64::total);
+  const bool one = d->HQ == d->H;
+  const auto kernel = one ? nha_bwd_rows64_kernel<true> : nha_bwd_rows64_kernel<false>;
+  cudaError_t e = set_max_smem((const void*)kernel, rw64::total);
   if (e != cudaSuccess) return record_cuda_error(e);
-  launch_after(nha_bwd_rows64_kernel, dim3((unsigned)(nha_chunk_count_bound(d->Ttot, d->N) * d->H)), kThreads, rw64::total, cs, *d, w, err);
+  launch_after(kernel, dim3((unsigned)(nha_chunk_count_bound(d->Ttot, d->N) * d->H)), kThreads, rw64::total, cs, *d, w, err);
   return check_launch();
 }
 

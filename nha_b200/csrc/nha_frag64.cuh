@@ -96,6 +96,11 @@ __device__ __forceinline__ void mma64(uint32_t d, uint64_t a, uint64_t b, uint32
 }
 __device__ __forceinline__ uint32_t idesc64(int amn, int bmn, int n = 64) { return make_idesc(64, n, bmn) | ((uint32_t)amn << 15); }
 
+// adds to two fp32 words of memory without reading them into the thread (their only writer is this thread, which wrote them before)
+__device__ __forceinline__ void red_add2(float* p, float x, float y) {
+  asm volatile("red.relaxed.gpu.global.add.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(x), "f"(y) : "memory");
+}
+
 // rows r and r + 32 of a [64][64] tile, piece c (r = tid / 8, c = tid % 8); off = sw_off(r, c)
 __device__ __forceinline__ void tile_in(unsigned char* tile, uint32_t off, const bf16* p0, bool ok0, const bf16* p1, bool ok1) {
   cp16(tile + off, p0, ok0);
