@@ -1,6 +1,6 @@
 // Backward of the chunked NHA operator on the sm_100a tensor-core path (tcgen05.mma, accumulators in
-// tensor memory, one thread per row for the element-wise work).  Two chunk-parallel kernels bracket the
-// state-gradient march of nha_chunk_bwd.cu:
+// tensor memory).  Two chunk-parallel passes bracket the state-gradient scan of nha_chunk_bwd.cu: the rows pass
+// (nha_chunk_bwd_rows64.cu, nha_chunk_bwd_rows128.cu) and the columns pass (nha_chunk_bwd_cols64.cu; head dim 128: here).
 //
 //   rows pass  (per chunk, kv head; query-row side)
 //       ok, p_slot recomputed as in the forward;  dp_slot = exp(G) .* (do Hv^T) + a .* (tril(do v'^T) SB)
@@ -168,9 +168,9 @@ __global__ void __launch_bounds__(kCarryThreads) nha_bwd_gate_carry_kernel(const
     }                                                                                            \
   } while (0)
 
-template <int D, int R>
+template <int R>
 struct ColsLayout {
-  static constexpr int KT = D / 64;
+  static constexpr int D = 128, KT = D / 64;
   static constexpr int kATile = R * 128;
   // per-head tiles and the tril buffers first: together they are dead once the head loop is over and
   // then hold the staged epilogue inputs (gate terms, window dv, s') and the dg scan
@@ -195,22 +195,18 @@ struct ColsLayout {
   static constexpr int eV = eG + 64 * kLdG * 4;         // [64][D+4] fp32 window part of dv
   static constexpr int eS = eV + 64 * kLdV * 4;         // [64][72] bf16 s'
   static_assert(eS + 64 * kLdS * 2 <= tK, "the staged epilogue inputs must fit in the per-head tiles");
-  // D == 64 with one query head per kv head: 256 columns, so two CTAs share an SM; the intra-chunk ds'
-  // accumulator then borrows the dk' columns for one MMA group and waits in registers
-  static constexpr bool kDsInRegs = D == 64 && R == 64;
-  static constexpr int kTmemCols = kDsInRegs ? 256 : 512;
-  static constexpr int cA = 0, cAv = 64, cDK = 128, cDV = 128 + D, cDS = kDsInRegs ? cDK : 128 + 2 * D, cDS2 = cA;
+  static constexpr int kTmemCols = 512;
+  static constexpr int cA = 0, cAv = 64, cDK = 128, cDV = 128 + D, cDS = 128 + 2 * D, cDS2 = cA;
 };
 
 // Two threads per row, as in the rows pass: the warps w and w + 4 share a TMEM lane quarter and take
 // alternate 32-column halves of every 64-column accumulator.
-template <int D, int R>
-__global__ void __launch_bounds__(kColsThreads, (D == 64 && R == 64) ? 2 : 1)
-    nha_bwd_cols_umma_kernel(const nha_chunk_desc d, const BwdWs w, int* __restrict__ err) {
+template <int R>
+__global__ void __launch_bounds__(kColsThreads, 1) nha_bwd_cols_umma_kernel(const nha_chunk_desc d, const BwdWs w, int* __restrict__ err) {
   grid_dep_wait();
   grid_dep_launch();
-  typedef ColsLayout<D, R> L;
-  constexpr int KT = L::KT, TH = R / 64, M = 64, NT = kColsThreads;
+  typedef ColsLayout<R> L;
+  constexpr int D = L::D, KT = L::KT, TH = R / 64, M = 64, NT = kColsThreads;
   const int H = d.H, HQ = d.HQ, NG = HQ / H, N = d.N;
   const int cg = blockIdx.x, h = blockIdx.y;
   const ChunkRec rc = chunk_rec(d, cg);
@@ -352,7 +348,6 @@ __global__ void __launch_bounds__(kColsThreads, (D == 64 && R == 64) ? 2 : 1)
   const uint32_t aPA = smem_u32(sm + L::tPA), aK = smem_u32(sm + L::tK), aV = smem_u32(sm + L::tV);
   const uint32_t aSB = smem_u32(sm + L::tSB), aDK = smem_u32(sm + L::tDK);
   const uint32_t aDV = smem_u32(sm + L::tDV), aA = smem_u32(sm + L::bufA), aB = smem_u32(sm + L::bufB);
-  float dsk[L::kDsInRegs ? 32 : 1];                   // this thread's half of the intra-chunk ds' accumulator
 
   for (int ht = 0; ht < NG / TH; ++ht) {
     if (ht > 0) NHA_LOAD_HEAD_TILE(ht);
@@ -374,7 +369,6 @@ __global__ void __launch_bounds__(kColsThreads, (D == 64 && R == 64) ? 2 : 1)
       mma_tile(tbase + L::cAv, aPA, L::kATile, aSB, 0, R, 64, 4, 0, false);               // Bv = pa SB^T
     }
     NHA_MMA_WAIT();
-    if constexpr (L::kDsInRegs) tmem_ld32(tlane + L::cDS + 32 * half, dsk);
     NHA_TRIL_TO_SMEM(L::cA, L::bufA);
     NHA_TRIL_TO_SMEM(L::cAv, L::bufB);
     NHA_SMEM_TO_MMA();
@@ -451,12 +445,7 @@ __global__ void __launch_bounds__(kColsThreads, (D == 64 && R == 64) ? 2 : 1)
   // ---- epilogue: two threads per key row, each its half of the columns ----------------------------------------------
   {
     float dsi[32], ds2[32];
-    if constexpr (L::kDsInRegs) {
-#pragma unroll
-      for (int e = 0; e < 32; ++e) dsi[e] = dsk[e];
-    } else {
-      tmem_ld32(tlane + L::cDS + 32 * half, dsi);
-    }
+    tmem_ld32(tlane + L::cDS + 32 * half, dsi);
     tmem_ld32(tlane + L::cDS2 + 32 * half, ds2);
     if (kactive) {
 #pragma unroll
@@ -542,16 +531,16 @@ __global__ void __launch_bounds__(kColsThreads, (D == 64 && R == 64) ? 2 : 1)
 #undef NHA_SMEM_TO_MMA
 #undef NHA_TRIL_TO_SMEM
 
-template <int D, int R>
+template <int R>
 static int launch_cols(const nha_chunk_desc* d, const BwdWs& w, int* err, cudaStream_t cs) {
-  typedef ColsLayout<D, R> L;
-  cudaError_t e = set_max_smem((const void*)nha_bwd_cols_umma_kernel<D, R>, L::total);
+  typedef ColsLayout<R> L;
+  cudaError_t e = set_max_smem((const void*)nha_bwd_cols_umma_kernel<R>, L::total);
   if (e != cudaSuccess) return record_cuda_error(e);
   const int NCB = (int)nha_chunk_count_bound(d->Ttot, d->N);
   launch_after(nha_bwd_gate_carry_kernel, dim3(NCB, d->H), kCarryThreads, 0, cs, *d, w);
   int st = check_launch();
   if (st != NHA_OK) return st;
-  launch_after(nha_bwd_cols_umma_kernel<D, R>, dim3(NCB, d->H), kColsThreads, L::total, cs, *d, w, err);
+  launch_after(nha_bwd_cols_umma_kernel<R>, dim3(NCB, d->H), kColsThreads, L::total, cs, *d, w, err);
   return check_launch();
 }
 
@@ -561,21 +550,17 @@ int bwd_cols64_launch(const nha_chunk_desc* d, const BwdWs& w, int* err, cudaStr
 int bwd_rows128_launch(const nha_chunk_desc* d, const BwdWs& w, int* err, cudaStream_t cs);
 
 bool bwd_umma_supported(const nha_chunk_desc* d) {
-  const int NG = d->HQ / d->H;
   if (d->K == 64) return bwd64_supported(d);
-  return d->K == d->V && d->M == 64 && d->K == 128 && (NG == 1 || NG % 2 == 0);
+  return d->K == 128 && d->V == 128 && d->M == 64 && d->scale > 0.f;
 }
 
 // which: 0 = rows pass, 1 = columns pass.  The caller has checked bwd_umma_supported().
 int bwd_umma_launch(const nha_chunk_desc* d, const BwdWs& w, int which, int* err, cudaStream_t cs) {
-  const int NG = d->HQ / d->H;
-  const bool one = NG == 1;
-  if (d->K == 64) {
-    if (which == 0) return bwd_rows64_launch(d, w, err, cs);
-    return bwd_cols64_launch(d, w, err, cs);
-  }
+  if (d->K == 64) return which == 0 ? bwd_rows64_launch(d, w, err, cs) : bwd_cols64_launch(d, w, err, cs);
   if (which == 0) return bwd_rows128_launch(d, w, err, cs);
-  return one ? launch_cols<128, 64>(d, w, err, cs) : launch_cols<128, 128>(d, w, err, cs);
+  // two heads to a 128-row tile where the group is even, one head to a 64-row tile where it is odd (2 x 1999 tokens, seven heads
+  // a group, whole training pass: 440 us, 1774 us with the general kernels)
+  return (d->HQ / d->H) % 2 ? launch_cols<64>(d, w, err, cs) : launch_cols<128>(d, w, err, cs);
 }
 
 }  // namespace nha

@@ -686,7 +686,7 @@ int chunk_output_pass_umma(const nha_chunk_desc* d, int* flags, int* err, cudaSt
     if (st != NHA_ERR_UNSUPPORTED) return st;
   }
   if (d->K == 128 && NG == 1) return launch_umma<128, 64>(d, flags, err, cs);
-  if (d->K == 128) return launch_umma<128, 128>(d, flags, err, cs);
+  if (d->K == 128 && NG % 2 == 0) return launch_umma<128, 128>(d, flags, err, cs);
   return NHA_ERR_UNSUPPORTED;
 }
 
