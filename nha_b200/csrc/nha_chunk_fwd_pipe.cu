@@ -38,7 +38,7 @@
 // too fast for one reference per chunk, and the general kernel that takes those: as in nha_chunk_fwd_umma.cu.
 //
 // What bounds it: the exchange of a window step - score product, tensor-memory load, exponentials, store, value product - whose
-// latencies two CTAs an SM cover to half (tensor pipe 44 %, exponential unit 35 %, issue slots 48 % busy).  Against one thread a
+// latencies two CTAs an SM cover in part (issue slots 48 % busy, DRAM 28 %).  Against one thread a
 // row, the gates scanned in shared memory, and the tiles of a chunk far apart in the grid: 131072 tokens, 32 heads on 8, W 512,
 // 2714 -> 2600-2640 us; 2 x 1999 tokens, 32 heads on 8, W 127, 76 -> 71 us.  An L2 prefetch of a later CTA's tiles: 1 % better in
 // the first, 4 % worse in the second.
