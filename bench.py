@@ -765,9 +765,9 @@ def main():
             dist.all_reduce(t_n, op=dist.ReduceOp.MAX)
             n = int(t_n.item())
         return timed(fn, n) / n
-    # plan, state pass (2), output pass (2), backward: rows (2), window columns (1), slot (1), state-gradient terms +
-    # scan + columns + general inter-chunk kernel (4); the general kernels run gated on the chunk flags
-    launches_per_step = 13
+    # plan, state pass (2), output pass (2), backward: rows and the flagged chunks' general kernel (2), window columns (1),
+    # state-gradient scan + columns + general inter-chunk kernel (3); the general kernels run gated on the chunk flags
+    launches_per_step = 11
 
     # ---- per-kernel timing: every kernel of a step on its own, CUDA events on the launching stream ----
     kernels = {}
@@ -788,7 +788,6 @@ def main():
         'output_pass': lambda: lib.nha_chunk_output_pass(ctypes.byref(desc), stream),
         'bwd_rows': lambda: lib.nha_chunk_bwd_stage(ctypes.byref(desc), 0, stream),
         'bwd_window_cols': lambda: lib.nha_chunk_bwd_stage(ctypes.byref(desc), 1, stream),
-        'bwd_slot_general': lambda: lib.nha_chunk_bwd_stage(ctypes.byref(desc), 2, stream),
         'bwd_state_scan': lambda: lib.nha_chunk_bwd_stage(ctypes.byref(desc), 3, stream),
         'bwd_cols': lambda: lib.nha_chunk_bwd_stage(ctypes.byref(desc), 4, stream),
     }
@@ -807,7 +806,6 @@ def main():
         # k_swa, v, q_swa, do, joint LSE, delta in; dk_swa and the fp32 window part of dv out
         'bwd_window_cols': H * (4 * D * e + 2 * f + D * e + D * f),
         # general kernel of the slot branch: runs only on chunks flagged by the forward (none here)
-        'bwd_slot_general': H * ((4 * D + 2 * M) * e + st * e + 4 * f + D * e + (2 * D + 2 * M) * f + 2 * M * e),
         # in-place scan of the chunks' fp32 state-gradient terms
         'bwd_state_scan': H * (st * 2 * f),
         # gate carry (fp32 state gradients and next states in, bf16 copies out), columns pass (q_gsa, do, k_gsa, v,

@@ -345,7 +345,8 @@ int nha_chunk_state_pass_static(const nha_chunk_desc* d, void* stream);
 /* one stage of nha_chunk_bwd on its own, so a harness can time each part with events on the
    launching stream: 0 = query-row side (delta, joint LSE, dq_gsa, dq_swa, gate terms, bf16 copies of
    dz and p, the chunks' own state-gradient terms), 1 = key side of the window (dk_swa, window part
-   of dv), 2 = general slot kernel (chunks flagged by the forward only), 3 = scan of the state
+   of dv), 2 = general slot kernel (shapes without a tensor-core query-row side; with one, the chunks
+   that the forward flagged are part of stage 0 and this stage launches nothing), 3 = scan of the state
    gradients over the chunks (dhk0/dhv0), 4 = gate carry and key-row side of the slot branch
    (dk_gsa, dv, ds, dg).  The stages of one backward must run in this order; running all five
    equals nha_chunk_bwd.  No counterpart in the reference (it has no timing hooks). */

@@ -20,6 +20,8 @@
 #include <stdlib.h>
 
 #include "nha_common.cuh"
+#include <algorithm>
+
 #include "nha_bwd_common.cuh"
 
 namespace nha {
@@ -735,6 +737,34 @@ __global__ void __launch_bounds__(kBwThreads) nha_bwd_local_terms_kernel(const n
   }
 }
 
+// The three above in one launch for the chunks that the tensor-core passes leave: each step reads what the one before wrote
+// for the same (chunk, kv head), and with nothing flagged a launch is all that they cost (two launches of 3 us of host time less).
+__global__ void __launch_bounds__(kBwThreads) nha_bwd_flagged_kernel(const nha_chunk_desc d, const BwdWs w, const int cpc) {
+  grid_dep_wait();
+  grid_dep_launch();
+  const int ncb = (int)((d.Ttot + kChunk - 1) / kChunk + d.N);
+  // which of my chunks have work: one flag load per chunk, all at once (cpc <= 32)
+  __shared__ unsigned todo;
+  if (threadIdx.x < 32) {
+    const int cgl = blockIdx.x * cpc + threadIdx.x;
+    const bool mine = (int)threadIdx.x < cpc && cgl < ncb && chunk_gate(w, cgl, blockIdx.y, d.H);
+    const unsigned m = __ballot_sync(0xffffffffu, mine);
+    if (threadIdx.x == 0) todo = m;
+  }
+  __syncthreads();
+  unsigned left = todo;
+  while (left) {
+    const int i = __ffs(left) - 1;
+    left &= left - 1;
+    nha_bwd_window_rows_kernel_body(d, w, blockIdx.x * cpc + i);
+    __syncthreads();
+    nha_bwd_slot_kernel_body(d, w, blockIdx.x * cpc + i);
+    __syncthreads();
+    nha_bwd_local_terms_kernel_body(d, w, blockIdx.x * cpc + i);
+    __syncthreads();
+  }
+}
+
 // In-place reverse scan over the chunks of one (sequence, kv head): on entry dkc/dvc hold L_c, on exit
 // the gradient at the END of chunk c; the value carried past chunk 0 is the initial state's gradient.
 // One thread owns four consecutive state elements and fetches kScanBatch chunks ahead of the serial
@@ -1089,6 +1119,9 @@ static int bwd_run(const nha_chunk_desc* d, int stage_mask, void* stream) {
   if (L5.total > kMaxSmem) return NHA_ERR_SMEM;
   e = set_max_smem((const void*)nha_bwd_local_terms_kernel, L5.total);
   if (e != cudaSuccess) return record_cuda_error(e);
+  const size_t flagged_smem = std::max(L1.total, std::max(L3.total, L5.total));
+  e = set_max_smem((const void*)nha_bwd_flagged_kernel, (int)flagged_smem);
+  if (e != cudaSuccess) return record_cuda_error(e);
   const int NCB = (int)nha_chunk_count_bound(d->Ttot, d->N);
   dim3 grid(NCB, d->H), block(kBwThreads);
   // gated launches (only the chunks the forward flagged do work): sixteen chunks per CTA
@@ -1110,7 +1143,7 @@ static int bwd_run(const nha_chunk_desc* d, int stage_mask, void* stream) {
       st = bwd_umma_launch(d, wu, 0, err, cs);
       if (st != NHA_OK) return st;
     }
-    if (umma) launch_after(nha_bwd_window_rows_kernel, ggrid, block, L1.total, cs, *d, wg, cpc);
+    if (umma) launch_after(nha_bwd_flagged_kernel, ggrid, block, flagged_smem, cs, *d, wg, cpc);
     else launch_after(nha_bwd_window_rows_kernel, grid, block, L1.total, cs, *d, wg, 1);
     st = check_launch();
     if (st != NHA_OK) return st;
@@ -1126,17 +1159,17 @@ static int bwd_run(const nha_chunk_desc* d, int stage_mask, void* stream) {
     }
     if (st != NHA_OK) return st;
   }
-  if (stage_mask & 4) {
-    if (umma) launch_after(nha_bwd_slot_kernel, ggrid, block, L3.total, cs, *d, wg, cpc);
-    else launch_after(nha_bwd_slot_kernel, grid, block, L3.total, cs, *d, wg, 1);
+  if ((stage_mask & 4) && !umma) {
+    launch_after(nha_bwd_slot_kernel, grid, block, L3.total, cs, *d, wg, 1);
     st = check_launch();
     if (st != NHA_OK) return st;
   }
   if (stage_mask & 8) {
-    if (umma) launch_after(nha_bwd_local_terms_kernel, ggrid, block, L5.total, cs, *d, wg, cpc);
-    else launch_after(nha_bwd_local_terms_kernel, grid, block, L5.total, cs, *d, wg, 1);
-    st = check_launch();
-    if (st != NHA_OK) return st;
+    if (!umma) {
+      launch_after(nha_bwd_local_terms_kernel, grid, block, L5.total, cs, *d, wg, 1);
+      st = check_launch();
+      if (st != NHA_OK) return st;
+    }
     const int SD = d->K * d->M + d->M * d->V;
     launch_after(nha_bwd_state_scan_kernel, dim3(d->N * d->H, (SD / 4 + 255) / 256), 256, 0, cs, *d, w);
     st = check_launch();
