@@ -45,6 +45,14 @@ inline void check(int status, const char* what) {
   raise(library_error, m);
 }
 
+// Every kernel reads raw pointers of one device: a tensor of another device (or of the host) is refused here, before a launch.
+inline void same_device(const Tensor& like, std::initializer_list<const Tensor*> rest, const char* what) {
+  if (C10_UNLIKELY(!like.is_cuda())) raise(PyExc_AssertionError, std::string(what) + " runs on the CUDA library only (there is no CPU path)");
+  for (const Tensor* t : rest)
+    if (C10_UNLIKELY(t->defined() && t->device() != like.device()))
+      raise(PyExc_AssertionError, std::string(what) + ": the tensors must be on one device, got " + like.device().str() + " and " + t->device().str());
+}
+
 // NHA_B200_CHECK=1: the operators read the kernels' device error word after every call (not under stream capture)
 inline bool check_device_words() {
   const char* e = getenv("NHA_B200_CHECK");

@@ -28,7 +28,13 @@ static void check_device(const Tensor& ws, int B, int H, void* stream, const cha
                              " (a bounded wait in the decode kernel ran out; the outputs of this call are invalid)");
 }
 
-// The slot memory of a step: the caller's own buffers when they can be updated in place, else copies (or, with no initial
+static void check_state(const Tensor& hk0, const Tensor& hv0, int64_t B, int64_t H, int64_t K, int64_t V, int64_t M) {
+  if (hk0.defined() && (hk0.sizes() != at::IntArrayRef({B, H, K, M}) || hv0.sizes() != at::IntArrayRef({B, H, M, V})))
+    raise(PyExc_AssertionError, "initial_state must be ([B,H,K,M], [B,H,M,V]) at the kv-head count " + std::to_string(H) + ", got " +
+                                    c10::str(hk0.sizes()) + " / " + c10::str(hv0.sizes()));
+}
+
+// The slot memory of a step (its shapes have been checked): the caller's own buffers when they can be updated in place, else copies (or, with no initial
 // state, fresh buffers that the kernel takes as zero).
 struct State {
   Tensor hk, hv;
@@ -41,9 +47,6 @@ struct State {
       zero = 1;
       return;
     }
-    if (hk0.sizes() != at::IntArrayRef({B, H, K, M}) || hv0.sizes() != at::IntArrayRef({B, H, M, V}))
-      raise(PyExc_AssertionError, "initial_state must be ([B,H,K,M], [B,H,M,V]) at the kv-head count " + std::to_string(H) +
-                                      ", got " + c10::str(hk0.sizes()) + " / " + c10::str(hv0.sizes()));
     if (keep && hk0.scalar_type() == dt && hv0.scalar_type() == dt && hk0.is_contiguous() && hv0.is_contiguous()) {
       hk = hk0;
       hv = hv0;
@@ -82,6 +85,12 @@ NHA_METHOD(decode) {
   if (k.size(2) != H || v.size(2) != H || g.size(2) != H)
     raise(PyExc_AssertionError, "popped-entry head count must match the kv-head count (" + std::to_string(H) + ") of the window tensors");
   require(sw_v.size(1) == W && sw_v.size(2) == H, "sw_k and sw_v must hold the same keys and heads");
+  // the kernel takes raw pointers: what it reads must be there
+  require(k.numel() == B * H * K && v.numel() == B * H * V && g.numel() == B * H * M,
+          "k, v and g must hold one token per sequence, with the head dim of q in k");
+  if (sw_k.size(0) != B || sw_k.size(3) != K || sw_v.size(0) != B || sw_v.size(3) != V)
+    raise(PyExc_AssertionError, "sw_k and sw_v must be " + c10::str(at::IntArrayRef({B, W, H, K})) + " and " +
+                                    c10::str(at::IntArrayRef({B, W, H, V})) + ", got " + c10::str(sw_k.sizes()) + " / " + c10::str(sw_v.sizes()));
   require(H > 0 && HQ % H == 0, "HQ must be a multiple of H");
   require(K >= 16 && V >= 16, "K and V must be at least 16");
   const bool rotary = cos.defined();
@@ -105,6 +114,8 @@ NHA_METHOD(decode) {
     require(sq.defined() && sq.sizes() == q.sizes(), "sq must have the shape of q");
   }
   if (s.defined()) require(s.sizes() == g.sizes(), "s must have the shape of g");
+  check_state(hk0, hv0, B, H, K, V, M);
+  same_device(q, {&k, &v, &g, &sw_k, &sw_v, &sq, &s, &cos, &sin, &hk0, &hv0}, "fused_recurrent_nha_decode");
 
   Tensor o, hk, hv;
   {
@@ -164,6 +175,8 @@ NHA_METHOD(decode_logits) {
   const double scale = args[6] == Py_None ? 1.0 / sqrt((double)k.size(-1)) : real(args[6]);
   require(k.numel() == B * H * K && v.numel() == B * H * V && s.numel() == B * H * M && g.numel() == B * H * M && win.numel() == B * HQ * W,
           "q, k, v, s, g and sliding_window must hold one token per sequence");
+  check_state(hk0, hv0, B, H, K, V, M);
+  same_device(q, {&k, &v, &win, &s, &g, &hk0, &hv0}, "fused_recurrent_nha");
   Tensor o, prob, hk, hv;
   {
     pybind11::gil_scoped_release no_gil;
@@ -187,6 +200,19 @@ NHA_METHOD(decode_logits) {
   NHA_END
 }
 
+// The rings of a layer: W rows per sequence, whatever way the heads and dims of a row are written; one index of the oldest entry per
+// sequence, or per (sequence, kv head) when the step also appends its token.
+static void check_rings(const Tensor& ring_k, const Tensor& ring_v, const Tensor& ring_g, const Tensor& head, int64_t B, int64_t W, int64_t H,
+                        int64_t K, int64_t V, int64_t M, bool fused) {
+  auto ring = [&](const Tensor& t, int64_t dim) {
+    return t.dim() >= 2 && t.size(0) == B && t.size(1) == W && t.numel() == B * W * H * dim && t.scalar_type() == at::kBFloat16 &&
+           t.is_contiguous();
+  };
+  require(ring(ring_k, K) && ring(ring_v, V) && ring(ring_g, M), "the rings must be contiguous bf16 [B, W, H, K|V|M] with the batch and heads of the step");
+  require(head.scalar_type() == at::kInt && head.is_contiguous() && head.numel() == (fused ? B * H : B),
+          "the ring index must be contiguous int32, one per sequence (with the token appended in the step: per kv head)");
+}
+
 // decode_ring(q, k, v, g, ring_k, ring_v, ring_g, head, cos, sin, hk, hv, fill, fused, scale) -> o
 NHA_METHOD(decode_ring) {
   NHA_BEGIN(15)
@@ -204,10 +230,21 @@ NHA_METHOD(decode_ring) {
   const Tensor& hv = tensor(args[11], "hv");
   const long fill = integer(args[12]);
   const bool fused = truth(args[13]);
+  require(q.dim() == 4 && k.dim() == 4 && v.dim() == 4 && g.dim() == 4 && ring_k.dim() >= 2, "q, k, v and g must have four dimensions");
   const int64_t B = q.size(0), HQ = q.size(2), K = q.size(3), H = k.size(2), V = v.size(3), M = g.size(3), W = ring_k.size(1);
   const double scale = args[14] == Py_None ? 1.0 / sqrt((double)K) : real(args[14]);
   const int64_t wlen = fill >= W ? W : fill + 1;
-  require(cos.size(-2) == wlen && cos.size(-1) == K, "cos/sin must cover the window positions");
+  require(cos.dim() >= 2 && cos.size(-2) == wlen && cos.size(-1) == K, "cos/sin must cover the window positions");
+  require(sin.sizes() == cos.sizes() && (cos.dim() == 2 || (cos.dim() == 3 && (cos.size(0) == 1 || cos.size(0) == B))),
+          "cos/sin must be [W, K] or [1|B, W, K]");
+  // the kernel takes raw pointers: what it reads and writes must be there
+  require(H > 0 && k.numel() == B * H * K && v.numel() == B * H * V && g.numel() == B * H * M,
+          "k, v and g must hold one token per sequence, with the head dim of q in k");
+  check_rings(ring_k, ring_v, ring_g, head, B, W, H, K, V, M, fused);
+  require(hk.scalar_type() == at::kFloat && hv.scalar_type() == at::kFloat && hk.is_contiguous() && hv.is_contiguous() &&
+              hk.numel() == B * H * K * M && hv.numel() == B * H * M * V,
+          "the slot memory must be contiguous fp32 [B,H,K,M] and [B,H,M,V]");
+  same_device(q, {&k, &v, &g, &ring_k, &ring_v, &ring_g, &head, &cos, &sin, &hk, &hv}, "fused_recurrent_nha_decode_ring");
   Tensor o;
   {
     pybind11::gil_scoped_release no_gil;

@@ -165,8 +165,20 @@ def _decode_ring_rot(q, k, v, g, layer: RingLayer, cos, sin, scale) -> torch.Ten
     lib = _lib.load()
     B, _, HQ, K = q.shape
     H, V, M, W = k.shape[2], v.shape[3], g.shape[3], layer.window
-    assert cos.shape[-1] == K and cos.shape == sin.shape
+    assert cos.shape[-1] == K and cos.shape == sin.shape and cos.dim() == 3 and cos.shape[0] in (1, B)
+    # the kernels take raw pointers: what they read and write must be there
+    assert k.numel() == B * H * K and v.numel() == B * H * V and g.numel() == B * H * M, \
+        'k, v and g must hold one token per sequence, with the head dim of q in k'
+    for x, n in ((layer.ring_k, H * K), (layer.ring_kr, H * K), (layer.ring_v, H * V), (layer.ring_g, H * M)):
+        assert x.shape[0] == B and x.numel() == B * W * n and x.dtype == _BF16 and x.is_contiguous(), \
+            'the rings must be contiguous bf16 [B, W, H, K|V|M] with the batch and heads of the step'
+    for x, n in ((layer.hk, K * M), (layer.hv, M * V)):
+        assert x.numel() == B * H * n and x.dtype == torch.float32 and x.is_contiguous(), \
+            'the slot memory must be contiguous fp32 [B,H,K,M] and [B,H,M,V]'
+    assert layer.head.numel() == B and layer.head.dtype == torch.int32
     dev = q.device
+    assert all(x.device == dev for x in (k, v, g, cos, sin, layer.ring_k, layer.ring_kr, layer.ring_v, layer.ring_g, layer.hk,
+                                         layer.hv, layer.head)), 'the tensors must be on one device'
     qc, kc, vc, gc = (x.to(_BF16).contiguous() for x in (q, k, v, g))
     cosq, sinq = cos[:, -1].to(_BF16).contiguous(), sin[:, -1].to(_BF16).contiguous()        # [1|B, K]
     cs_batch = cosq.stride(0) if cosq.shape[0] > 1 else 0
