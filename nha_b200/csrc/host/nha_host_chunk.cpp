@@ -315,9 +315,15 @@ NHA_METHOD(chunk_nha) {
   variable_list out;
   {
     pybind11::gil_scoped_release no_gil;
-    bool grad = hk0.defined() && (hk0.requires_grad() || hv0.requires_grad());
-    for (int i = 0; i < NIN; ++i) grad = grad || raw[i].requires_grad();
-    grad = grad && at::GradMode::is_enabled();
+    auto needs = [](const Tensor& t) { return t.defined() && t.requires_grad(); };
+    auto tangent = [](const Tensor& t) { return t.defined() && t._fw_grad(0).defined(); };
+    bool grad = needs(hk0) || needs(hv0), dual = tangent(hk0) || tangent(hv0);
+    for (int i = 0; i < NIN; ++i) {
+      grad = grad || needs(raw[i]);
+      dual = dual || tangent(raw[i]);
+    }
+    // an input with a forward-mode tangent goes to the autograd node too, which refuses it: nothing may drop it silently
+    grad = (grad && at::GradMode::is_enabled()) || dual;
     {
       at::AutoGradMode off(false);
       set_up(c, raw, cu, max_seqlen, scale, hk0, hv0);

@@ -252,3 +252,20 @@ def test_many_tiny_sequences_in_one_packing():
         want = orc.nha_varlen(sl['q_gsa'], sl['q_swa'], sl['k_gsa'], sl['k_swa'], sl['v'], sl['s'], sl['g'], [0, b - a],
                               K ** -0.5, 1, 1, None, None)
         assert_close(o[0, a:b], want[0], TOL_OUT, f'o of sequence {n}')
+
+
+def test_forward_mode_derivatives_are_refused():
+    """The operator has no forward-mode rule: a tangent on an input raises, whether or not a gradient is asked for as well."""
+    import torch.autograd.forward_ad as fw
+    from nha_b200 import chunk_nha
+    d = gen.layer_inputs(5, 1, 130, 2, 2, 64, 64, 64)
+    names = ('q_swa', 'k_swa', 'q_gsa', 'k_gsa', 'v', 's', 'g')
+    state = torch.zeros(1, 2, 64, 64, device='cuda')
+    for which in (*names, 'state'):
+        for grad in (False, True):
+            x = [d[n].cuda().requires_grad_(grad) for n in names]
+            with fw.dual_level():
+                x = [fw.make_dual(t, torch.ones_like(t)) if n == which else t for n, t in zip(names, x)]
+                hk = fw.make_dual(state, torch.ones_like(state)) if which == 'state' else state
+                with pytest.raises(RuntimeError, match='jvp'):
+                    chunk_nha(*x, window_size_left=64, window_size_right=0, initial_state=(hk, state))
