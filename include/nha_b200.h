@@ -67,6 +67,8 @@ int nha_abi_version(void);
  *   o        [B, HQ, V] bf16   output (slot readout + window readout; slot readout only in
  *            win_logits mode)
  *   win_prob [B, HQ, W] fp32   window probabilities of the joint softmax, or NULL
+ * q, sq, k, v, sw_k, sw_v, cos, sin, hk, hv and o must start on 16 bytes, cs_batch and cs_row be multiples of 8
+ * (NHA_ERR_BAD_ARG otherwise; the same holds for the ring entry points below and their rings).
  *   workspace  scratch of nha_decode_workspace_bytes(B, HQ, H, V, W) bytes, needed when W > 64
  *            (a (sequence, kv head) is then split over several CTAs whose partial softmaxes are
  *            merged by the last one to finish).  Its first B*H int32 are arrival counters, the next
@@ -86,7 +88,7 @@ int nha_decode_step(const void* q, const void* sq, const void* k, const void* v,
                     float* win_prob, void* workspace, int64_t workspace_bytes, int B, int HQ, int H, int K, int V,
                     int M, int W, float scale, void* stream);
 
-/* nha_decode_step with the slot memory kept in bf16 (hk [B,H,K,M], hv [B,H,M,V] bf16, 16-byte aligned, updated in
+/* nha_decode_step with the slot memory kept in bf16 (hk [B,H,K,M], hv [B,H,M,V] bf16, updated in
  * place): half the state bytes per step.  Arithmetic stays fp32 in registers; the state is rounded once per step when
  * it is stored, and the step's own readout uses the rounded values, so a step sees exactly what the next one reads.
  * An extension: the reference keeps fp32 states (nha_fla/ops/nha/fused_recurrent.py:536-545), so results follow it

@@ -77,6 +77,9 @@ inline Tensor typed(const Tensor& x, at::ScalarType dt) {
   if (C10_LIKELY(x.scalar_type() == dt && x.is_contiguous())) return x;
   return x.to(dt).contiguous();
 }
+// The kernels load and copy 16 bytes at a time: a contiguous view that starts elsewhere is copied.
+inline bool on_16_bytes(const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0; }
+inline Tensor on_16(Tensor t) { return C10_LIKELY(on_16_bytes(t)) ? t : t.clone(); }
 inline void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 
 inline const Tensor& tensor(PyObject* o, const char* name) {

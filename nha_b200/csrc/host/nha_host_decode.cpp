@@ -35,9 +35,10 @@ static void check_state(const Tensor& hk0, const Tensor& hv0, int64_t B, int64_t
 }
 
 // The slot memory of a step (its shapes have been checked): the caller's own buffers when they can be updated in place, else copies (or, with no initial
-// state, fresh buffers that the kernel takes as zero).
+// state, fresh buffers that the kernel takes as zero).  A caller's buffer that does not start on 16 bytes is updated through a copy.
 struct State {
   Tensor hk, hv;
+  Tensor back_k, back_v;                         // where the copies go after the step
   int zero = 0;
   State(Tensor hk0, Tensor hv0, int64_t B, int64_t H, int64_t K, int64_t V, int64_t M, bool keep, at::ScalarType dt,
         const Tensor& like) {
@@ -48,12 +49,21 @@ struct State {
       return;
     }
     if (keep && hk0.scalar_type() == dt && hv0.scalar_type() == dt && hk0.is_contiguous() && hv0.is_contiguous()) {
-      hk = hk0;
-      hv = hv0;
+      hk = on_16(hk0);
+      hv = on_16(hv0);
+      if (C10_UNLIKELY(!hk.is_same(hk0))) back_k = hk0;
+      if (C10_UNLIKELY(!hv.is_same(hv0))) back_v = hv0;
     } else {
       hk = hk0.to(dt).contiguous().clone();
       hv = hv0.to(dt).contiguous().clone();
     }
+  }
+  // after the launch: the updated buffers, the caller's own where it gave some
+  void done(Tensor& k, Tensor& v) {
+    if (C10_UNLIKELY(back_k.defined())) hk = back_k.copy_(hk);
+    if (C10_UNLIKELY(back_v.defined())) hv = back_v.copy_(hv);
+    k = std::move(hk);
+    v = std::move(hv);
   }
 };
 
@@ -104,8 +114,8 @@ NHA_METHOD(decode) {
     require(K % 2 == 0, "in-kernel rotate-half requires an even head dim");
     skip = cos.size(1) - W;                                   // the last W rows are the window positions
     if (!(table_ok(cos, skip) && table_ok(sin, skip) && cos.strides() == sin.strides())) {
-      cos = cos.narrow(1, skip, W).to(at::kBFloat16).contiguous();
-      sin = sin.narrow(1, skip, W).to(at::kBFloat16).contiguous();
+      cos = on_16(cos.narrow(1, skip, W).to(at::kBFloat16).contiguous());
+      sin = on_16(sin.narrow(1, skip, W).to(at::kBFloat16).contiguous());
       skip = 0;
     }
     cs_batch = cos.size(0) == B && B > 1 ? cos.stride(0) : 0;
@@ -121,8 +131,8 @@ NHA_METHOD(decode) {
   {
     pybind11::gil_scoped_release no_gil;
     const c10::cuda::OptionalCUDAGuard guard(q.device());
-    const Tensor qf = bf16c(q), sqf = sq.defined() ? bf16c(sq) : sq, kf = bf16c(k), vf = bf16c(v), gf = bf16c(g);
-    const Tensor sf = s.defined() ? bf16c(s) : s, wk = bf16c(sw_k), wv = bf16c(sw_v);
+    const Tensor qf = on_16(bf16c(q)), sqf = sq.defined() ? on_16(bf16c(sq)) : sq, kf = on_16(bf16c(k)), vf = on_16(bf16c(v));
+    const Tensor gf = bf16c(g), sf = s.defined() ? bf16c(s) : s, wk = on_16(bf16c(sw_k)), wv = on_16(bf16c(sw_v));
     State st(hk0, hv0, B, H, K, V, M, keep, bf16_state ? at::kBFloat16 : at::kFloat, q);
     o = empty({B, 1, HQ, V}, at::kBFloat16, q);
     Tensor ws;
@@ -143,8 +153,7 @@ NHA_METHOD(decode) {
             "nha_decode_step");
     check_device(ws, B, H, stream, "nha_decode_step");
     if (q.scalar_type() != at::kBFloat16) o = o.to(q.scalar_type());
-    hk = std::move(st.hk);
-    hv = std::move(st.hv);
+    st.done(hk, hv);
   }
   // buffers that were updated in place go back as the objects they came in
   PyObject* states;
@@ -181,7 +190,7 @@ NHA_METHOD(decode_logits) {
   {
     pybind11::gil_scoped_release no_gil;
     const c10::cuda::OptionalCUDAGuard guard(q.device());
-    const Tensor qf = bf16c(q), kf = bf16c(k), vf = bf16c(v), sf = bf16c(s), gf = bf16c(g), wf = bf16c(win);
+    const Tensor qf = on_16(bf16c(q)), kf = on_16(bf16c(k)), vf = on_16(bf16c(v)), sf = bf16c(s), gf = bf16c(g), wf = bf16c(win);
     State st(hk0, hv0, B, H, K, V, M, keep, at::kFloat, q);
     o = empty({B, 1, HQ, V}, at::kBFloat16, q);
     prob = empty({B, 1, HQ, W}, at::kFloat, q);
@@ -190,8 +199,7 @@ NHA_METHOD(decode_logits) {
                           (float*)prob.data_ptr(), nullptr, 0, B, HQ, H, K, V, M, W, (float)scale, stream_of(q)),
           "nha_decode_step");
     if (v.scalar_type() != at::kBFloat16) o = o.to(v.scalar_type());
-    hk = std::move(st.hk);
-    hv = std::move(st.hv);
+    st.done(hk, hv);
   }
   PyObject* states = PyList_New(2);
   PyList_SET_ITEM(states, 0, keep ? wrap(hk) : none());
@@ -249,7 +257,8 @@ NHA_METHOD(decode_ring) {
   {
     pybind11::gil_scoped_release no_gil;
     const c10::cuda::OptionalCUDAGuard guard(q.device());        // split count and launches follow the tensors' device
-    const Tensor qc = bf16c(q), kc = bf16c(k), vc = bf16c(v), gc = bf16c(g), cc = bf16c(cos), sc = bf16c(sin);
+    const Tensor qc = on_16(bf16c(q)), kc = on_16(bf16c(k)), vc = on_16(bf16c(v)), gc = on_16(bf16c(g));
+    const Tensor cc = on_16(bf16c(cos)), sc = on_16(bf16c(sin));
     const int64_t cs_batch = cc.dim() == 3 && cc.size(0) > 1 ? cc.stride(0) : 0, cs_row = cc.stride(-2);
     o = empty({B, 1, HQ, V}, at::kBFloat16, q);
     const Tensor ws = decode_workspace(q, B, HQ, H, V, W);

@@ -15,6 +15,8 @@
 // Replaces the two Triton launches of fused_recurrent_nha_decode
 // (nha_fla/ops/nha/fused_recurrent.py:229-353 k-kernel, :356-428 v-kernel) and, with caller-supplied
 // window logits, the kernels of fused_recurrent_nha (:48-147).
+#include <initializer_list>
+
 #include "nha_common.cuh"
 #include "nha_decode_args.cuh"
 
@@ -455,6 +457,13 @@ int decode_stream_try(const void* q, const void* sq, const void* k, const void* 
                       cudaStream_t st, const int* head, const void* ring_g, int ring_rows, int nopop,
                       const void* ring_kraw, const void* g_new, int state_bf16);
 
+// what the kernels load, copy or store 16 bytes at a time
+static bool aligned16(std::initializer_list<const void*> p) {
+  uintptr_t all = 0;
+  for (const void* x : p) all |= (uintptr_t)x;
+  return (all & 15) == 0;
+}
+
 bool decode_logits_supported(const DecodeArgs& a);
 int decode_logits_launch(const DecodeArgs& a, cudaStream_t cs);
 
@@ -507,6 +516,7 @@ static int decode_step_impl(const void* q, const void* sq, const void* k, const 
     if ((cosp == nullptr) != (sinp == nullptr)) return NHA_ERR_BAD_ARG;
     if (!cosp && !sq) return NHA_ERR_BAD_ARG;
   }
+  if (!aligned16({q, sq, k, v, sw_k, sw_v, cosp, sinp, hk, hv, o}) || cs_row % 8 || cs_batch % 8) return NHA_ERR_BAD_ARG;
   const int NG = HQ / H;
   if (K % 16 || V % 16 || K < 16 || V < 16 || K > 256 || V > 256 || M % 4 || M < 4 || M > 256 || NG > 16)
     return NHA_ERR_UNSUPPORTED;
@@ -583,7 +593,6 @@ extern "C" int nha_decode_step_bf16_state(const void* q, const void* sq, const v
                                           const void* sinp, int64_t cs_batch, int64_t cs_row, void* hk, void* hv,
                                           int zero_state, void* o, void* workspace, int64_t workspace_bytes, int B, int HQ,
                                           int H, int K, int V, int M, int W, float scale, void* stream) {
-  if (((uintptr_t)hk & 15) || ((uintptr_t)hv & 15)) return NHA_ERR_BAD_ARG;
   return decode_step_impl(q, sq, k, v, g, s, sw_k, sw_v, cosp, sinp, cs_batch, cs_row, nullptr, (float*)hk, (float*)hv, 1,
                           zero_state, o, nullptr, workspace, workspace_bytes, B, HQ, H, K, V, M, W, scale, stream);
 }
@@ -619,6 +628,7 @@ extern "C" int nha_decode_step_ring(const void* q, const void* k_new, const void
                                     int W, int fill, float scale, void* stream) {
   if (!q || !k_new || !v_new || !ring_k || !ring_v || !ring_g || !head || !cosp || !sinp || !hk || !hv || !o)
     return NHA_ERR_BAD_ARG;
+  if (!aligned16({q, k_new, v_new, ring_k, ring_v, cosp, sinp, hk, hv, o}) || cs_row % 8 || cs_batch % 8) return NHA_ERR_BAD_ARG;
   if (B <= 0 || H <= 0 || HQ <= 0 || HQ % H != 0 || W < 1 || fill < 0 || fill > W) return NHA_ERR_BAD_ARG;
   const int NG = HQ / H;
   // a full ring: W window entries (the oldest leaves); a filling ring: its `fill` rows and the new token
@@ -643,6 +653,7 @@ extern "C" int nha_decode_step_ring_fused(const void* q, const void* k_new, cons
                                           float scale, void* stream) {
   if (!q || !k_new || !v_new || !g_new || !ring_k || !ring_v || !ring_g || !head || !cosp || !sinp || !hk || !hv || !o)
     return NHA_ERR_BAD_ARG;
+  if (!aligned16({q, k_new, v_new, g_new, ring_k, ring_v, ring_g, cosp, sinp, hk, hv, o}) || cs_row % 8 || cs_batch % 8) return NHA_ERR_BAD_ARG;
   if (B <= 0 || H <= 0 || HQ <= 0 || HQ % H != 0 || W < 1 || fill < 0 || fill > W) return NHA_ERR_BAD_ARG;
   const int NG = HQ / H;
   const int nopop = fill < W, Weff = nopop ? fill + 1 : W;
@@ -663,6 +674,7 @@ extern "C" int nha_ring_append(void* ring_k, void* ring_v, void* ring_g, const v
                                const void* g_new, int32_t* head, int B, int H, int K, int V, int M, int W, int fill,
                                void* stream) {
   if (!ring_k || !ring_v || !ring_g || !k_new || !v_new || !g_new || !head) return NHA_ERR_BAD_ARG;
+  if (!aligned16({ring_k, ring_v, ring_g, k_new, v_new, g_new})) return NHA_ERR_BAD_ARG;
   if (B <= 0 || H <= 0 || W < 1 || fill < 0 || fill > W || (H * K) % 8 || (H * V) % 8 || (H * M) % 8) return NHA_ERR_BAD_ARG;
   nha_ring_append_kernel<<<B, 128, 0, (cudaStream_t)stream>>>((bf16*)ring_k, (bf16*)ring_v, (bf16*)ring_g, (const bf16*)k_new,
                                                               (const bf16*)v_new, (const bf16*)g_new, head, H, K, V, M, W, fill);
@@ -740,6 +752,7 @@ __global__ void nha_ring_append_rot_kernel(bf16* ring_k, bf16* ring_kr, bf16* ri
 extern "C" int nha_ring_rotate_rows(const void* ring_k, void* ring_kr, const void* cosp, const void* sinp, int64_t cs_batch,
                                     int64_t cs_row, int B, int H, int K, int W, int rows, void* stream) {
   if (!ring_k || !ring_kr || !cosp || !sinp) return NHA_ERR_BAD_ARG;
+  if (!aligned16({ring_k, ring_kr, cosp, sinp})) return NHA_ERR_BAD_ARG;
   if (B <= 0 || H <= 0 || W < 1 || rows < 0 || rows > W) return NHA_ERR_BAD_ARG;
   if (K <= 0 || K % 16 || cs_row % 8 || cs_batch % 8) return NHA_ERR_UNSUPPORTED;
   if (rows == 0) return NHA_OK;
@@ -756,6 +769,7 @@ extern "C" int nha_decode_step_ring_rot(const void* q, const void* k_new, const 
                                         int W, int fill, float scale, void* stream) {
   if (!q || !k_new || !v_new || !ring_k || !ring_kr || !ring_v || !ring_g || !head || !cos_q || !sin_q || !hk || !hv || !o)
     return NHA_ERR_BAD_ARG;
+  if (!aligned16({q, k_new, v_new, ring_k, ring_kr, ring_v, cos_q, sin_q, hk, hv, o}) || cs_batch % 8) return NHA_ERR_BAD_ARG;
   if (B <= 0 || H <= 0 || HQ <= 0 || HQ % H != 0 || W < 1 || fill < 0 || fill > W) return NHA_ERR_BAD_ARG;
   const int NG = HQ / H;
   const int nopop = fill < W, Weff = nopop ? fill + 1 : W;
@@ -780,6 +794,7 @@ extern "C" int nha_ring_append_rot(void* ring_k, void* ring_kr, void* ring_v, vo
                                    void* stream) {
   if (!ring_k || !ring_kr || !ring_v || !ring_g || !k_new || !v_new || !g_new || !cos_q || !sin_q || !head)
     return NHA_ERR_BAD_ARG;
+  if (!aligned16({ring_k, ring_kr, ring_v, ring_g, k_new, v_new, g_new, cos_q, sin_q})) return NHA_ERR_BAD_ARG;
   if (B <= 0 || H <= 0 || W < 1 || fill < 0 || fill > W || K % 16 || (H * V) % 8 || (H * M) % 8 || cs_batch % 8)
     return NHA_ERR_BAD_ARG;
   nha_ring_append_rot_kernel<<<B, 128, 0, (cudaStream_t)stream>>>((bf16*)ring_k, (bf16*)ring_kr, (bf16*)ring_v, (bf16*)ring_g,

@@ -304,3 +304,38 @@ def test_dependent_launch_modes_agree_on_a_stack_of_layers(B, pdl_mode):
         for part in range(4):
             for a, b in zip(results[0][part], results[mode][part]):
                 assert torch.equal(a, b), f'mode {mode} differs from plain launches'
+
+
+def _off_16(t):
+    """The same values in a contiguous view that starts one element past a 16-byte boundary."""
+    buf = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)
+    view = buf[1:].view(t.shape)
+    view.copy_(t)
+    assert view.data_ptr() % 16 and view.is_contiguous()
+    return view
+
+
+@pytest.mark.parametrize('K,W', [(64, 64), (128, 300), (32, 40)])              # streaming kernel, split and not; general kernel
+def test_tensors_that_do_not_start_on_16_bytes(K, W):
+    from nha_b200 import fused_recurrent_nha, fused_recurrent_nha_decode
+    from nha_b200.ring_cache import RingLayer, fused_recurrent_nha_decode_ring
+    c = {n: x.cuda() if torch.is_tensor(x) else x for n, x in gen.decode_inputs(77 + K, 2, 2, 2, K, K, 64 if K >= 64 else 32, W).items()}
+    move = lambda t, off: _off_16(t) if off else t.clone()  # noqa: E731
+
+    def step(off):
+        hk, hv = move(c['hk0'], off), move(c['hv0'], off)
+        x = {n: move(c[n], off) for n in ('q', 'k', 'v', 'g', 'cos', 'sin')}
+        o, (nk, nv) = fused_recurrent_nha_decode(sw_k=move(c['sw_k_raw'], off), sw_v=move(c['vw'], off), initial_state=(hk, hv), output_final_state=True, **x)
+        assert nk.data_ptr() == hk.data_ptr() and nv.data_ptr() == hv.data_ptr()        # updated in place all the same
+        win = torch.linspace(-1, 1, 2 * 4 * W, device='cuda').bfloat16().view(2, 1, 4, W)
+        s = (1 - c['g'].float().exp()).bfloat16()              # (s and g elsewhere take another kernel: other bits)
+        return [o, nk, nv, *fused_recurrent_nha(x['q'], x['k'], x['v'], move(win, off), s, c['g'], initial_state=(nk.clone(), nv.clone()))[:2]]
+
+    def ring(off):
+        y = RingLayer(c['sw_k_raw'], c['vw'], c['g'].expand(-1, W, -1, -1), c['hk0'], c['hv0'])
+        x = [move(c[n], off) for n in ('q', 'k', 'v', 'g')]
+        return [fused_recurrent_nha_decode_ring(*x, y, move(c['cos'][:, -W:], off), move(c['sin'][:, -W:], off)), y.hk, y.hv, y.ring_k]
+
+    for run in [step] + ([ring] if K >= 64 else []):
+        for a, b in zip(run(False), run(True)):
+            assert torch.equal(a, b)
