@@ -29,9 +29,9 @@ void cast_all(const Tensor* src, Tensor* dst, const at::ScalarType* to, int n) {
     const Tensor x = held[i] = src[i].contiguous();
     const int sa = type_code(x.scalar_type()), sb = type_code(to[i]);
     if (sa == sb && sa >= 0) {
-      dst[i] = x;
+      dst[i] = on_16(x);
     } else if (sa < 0 || sb < 0 || (count && (sa != a || sb != b))) {
-      dst[i] = x.to(to[i]);
+      dst[i] = on_16(x.to(to[i]));
     } else {
       dst[i] = empty(x.sizes(), to[i], x);
       a = sa;
@@ -146,14 +146,16 @@ void set_up(Call& c, const Tensor* raw, const Tensor& cu, int64_t max_seqlen, do
   }
   d.scale = (float)scale;
   if (hk0.defined()) {
-    c.hk0 = typed(hk0, at::kFloat);
-    c.hv0 = typed(hv0, at::kFloat);
+    require(hk0.numel() == (int64_t)d.N * d.H * d.K * d.M && hv0.numel() == (int64_t)d.N * d.H * d.M * d.V,
+            "initial_state must be ([N,H,K,M], [N,H,M,V]) at the kv-head count");
+    c.hk0 = on_16(typed(hk0, at::kFloat));
+    c.hv0 = on_16(typed(hv0, at::kFloat));
   }
   at::ScalarType to[NIN];
   bool all = true;
   for (int i = 0; i < NIN; ++i) {
     to[i] = at::kBFloat16;
-    all = all && raw[i].scalar_type() == at::kBFloat16 && raw[i].is_contiguous();
+    all = all && raw[i].scalar_type() == at::kBFloat16 && raw[i].is_contiguous() && on_16_bytes(raw[i]);
   }
   if (all) {
     for (int i = 0; i < NIN; ++i) c.in[i] = raw[i];
@@ -221,7 +223,7 @@ struct ChunkFunction : torch::autograd::Function<ChunkFunction> {
       cast_all(&d_o, &x, &to, 1);
       d_o = x;
     }
-    d_o = d_o.contiguous();
+    d_o = on_16(d_o.contiguous());
     Tensor d_lse, d_hkt, d_hvt;
     if (grads[2].defined()) d_lse = typed(grads[2], at::kFloat);
     if (grads.size() > 3 && (grads[3].defined() || grads[4].defined())) {
@@ -293,6 +295,9 @@ NHA_METHOD(chunk_nha) {
   const long right = integer(args[11]);
   require(right == 0 || right == -1, "the window branch is causal: window_size_right must be 0 or -1");
   const double scale = args[9] == Py_None ? 1.0 / sqrt((double)raw[QS].size(3)) : real(args[9]);
+  Tensor hk0, hv0;
+  state_pair(args[13], hk0, hv0);
+  same_device(raw[QS], {&raw[KS], &raw[QG], &raw[KG], &raw[VV], &raw[SS], &raw[GG], &hk0, &hv0}, "chunk_nha");
   const c10::cuda::OptionalCUDAGuard guard(raw[QS].device());
   Tensor cu;
   int64_t max_seqlen = 0;
@@ -304,8 +309,6 @@ NHA_METHOD(chunk_nha) {
     else
       max_seqlen = (cu.narrow(0, 1, cu.numel() - 1) - cu.narrow(0, 0, cu.numel() - 1)).max().item().toLong();
   }
-  Tensor hk0, hv0;
-  state_pair(args[13], hk0, hv0);
   const bool want = truth(args[14]);
   Call c;
   const int64_t N = cu.defined() ? cu.numel() - 1 : raw[QS].size(0);
@@ -371,6 +374,7 @@ NHA_METHOD(prefill) {
   if (hk0.defined() && (hk0.sizes() != at::IntArrayRef({B, H, K, M}) || hv0.sizes() != at::IntArrayRef({B, H, M, V})))
     raise(PyExc_AssertionError, "initial_state must be at the kv-head count [B, " + std::to_string(H) + ", ...], got " + c10::str(hk0.sizes()) +
                                     " / " + c10::str(hv0.sizes()));
+  same_device(q, {&k, &v, &rq, &rk, &s, &g, &hk0, &hv0}, "fused_chunk_nha_prefill");
   Call c;
   Tensor o;
   {

@@ -116,6 +116,8 @@ NHA_METHOD(rotary_pair) {
   } else {
     require(offset + T <= cos.size(0), "cos/sin tables do not cover the positions");
   }
+  same_device(q, {&k, &cos, &sin}, "rotary_pair");
+  if (cu) same_device(q, {&*cu}, "rotary_pair");
   variable_list out;
   {
     pybind11::gil_scoped_release no_gil;
@@ -199,6 +201,7 @@ NHA_METHOD(feature_maps) {
   const Tensor& v = tensor(args[2], "v");
   const long mode = integer(args[3]);
   require(q.is_cuda() && k.is_cuda() && v.is_cuda(), "feature_maps runs on the CUDA library only (there is no CPU path)");
+  if (mode != 2) same_device(v, {&q, &k}, "feature_maps");
   variable_list out;
   {
     pybind11::gil_scoped_release no_gil;
@@ -254,6 +257,10 @@ NHA_METHOD(silu_rms_norm) {
   if (args[2] != Py_None) b = tensor(args[2], "bias");
   const double eps = real(args[3]);
   require(o.is_cuda(), "silu_rms_norm runs on the CUDA library only (there is no CPU path)");
+  same_device(o, {&w}, "silu_rms_norm");
+  if (b) same_device(o, {&*b}, "silu_rms_norm");
+  // the kernel reads one weight (and bias) per column through their pointers
+  require(o.dim() >= 1 && w.numel() >= o.size(-1) && (!b || b->numel() >= o.size(-1)), "the weight and bias must hold one value per column");
   variable_list out;
   {
     pybind11::gil_scoped_release no_gil;
@@ -307,6 +314,7 @@ NHA_METHOD(gsa_aux_loss) {
   const Tensor& lg = tensor(args[1], "lse_gsa");
   const double target = real(args[2]);
   require(ls.is_cuda() && lg.is_cuda(), "gsa_aux_loss runs on the CUDA library only (there is no CPU path)");
+  same_device(ls, {&lg}, "gsa_aux_loss");
   require(ls.sizes() == lg.sizes() && ls.numel() > 0, "lse_swa and lse_gsa must have the same, non-empty shape");
   variable_list out;
   {

@@ -1,4 +1,4 @@
-"""CPU: the single-token operators refuse, on the host and before anything is launched, tensors that do not hold what the kernel would
+"""CPU: the operators refuse, on the host and before anything is launched, tensors that do not hold what the kernel would
 read through their pointers.  The tensors are host tensors: right shapes get as far as the device check behind the shape checks."""
 import pytest
 import torch
@@ -79,3 +79,13 @@ def test_recurrent():
         with pytest.raises(AssertionError) as e:
             call(**change)
         assert 'CUDA' not in str(e.value), (change, str(e.value))
+
+
+def test_chunk_operators_take_tensors_of_the_gpu():
+    T = 5
+    x = {n: torch.zeros(B, T, HQ if n[0] == 'q' else H, {'s': M, 'g': M, 'v': V}.get(n, K), dtype=torch.bfloat16)
+         for n in ('q_swa', 'k_swa', 'q_gsa', 'k_gsa', 'v', 's', 'g')}
+    with pytest.raises(AssertionError, match='CUDA library only'):
+        nha_b200.chunk_nha(**x, window_size_left=4, window_size_right=0)
+    with pytest.raises(AssertionError, match='CUDA library only'):
+        nha_b200.fused_chunk_nha_prefill(x['q_gsa'], x['k_gsa'], x['v'], x['q_swa'], x['k_swa'], x['s'], x['g'], 4)

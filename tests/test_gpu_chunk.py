@@ -269,3 +269,22 @@ def test_forward_mode_derivatives_are_refused():
                 hk = fw.make_dual(state, torch.ones_like(state)) if which == 'state' else state
                 with pytest.raises(RuntimeError, match='jvp'):
                     chunk_nha(*x, window_size_left=64, window_size_right=0, initial_state=(hk, state))
+
+
+@pytest.mark.parametrize('D', [64, 128, 32])
+def test_tensors_that_do_not_start_on_16_bytes_and_states_of_the_wrong_size(D):
+    from nha_b200 import chunk_nha
+    from tests.test_gpu_decode import _off_16
+    d = gen.layer_inputs(6, 1, 130, 2, 2, D, D, 64)
+    names = ('q_swa', 'k_swa', 'q_gsa', 'k_gsa', 'v', 's', 'g')
+    hk, hv = 0.1 * torch.randn(1, 2, D, 64, device='cuda'), 0.1 * torch.randn(1, 2, 64, D, device='cuda')
+    runs = []
+    for move in (lambda t: t.clone(), _off_16):
+        x = [move(d[n].cuda()).requires_grad_(True) for n in names]
+        o, _, _, state = chunk_nha(*x, window_size_left=64, window_size_right=0, initial_state=(move(hk), move(hv)), output_final_state=True)
+        runs.append([o, *state, *torch.autograd.grad(o, x, move(d['do'].cuda()))])
+    for a, b in zip(*runs):
+        assert torch.equal(a, b)
+    for bad in ((hk[:, :1], hv), (hk, hv[..., :16]), (hk[:0], hv[:0])):
+        with pytest.raises(AssertionError):
+            chunk_nha(*x, window_size_left=64, window_size_right=0, initial_state=bad)
