@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(kThreads, 2) nha_fwd64_kernel(const nha_chunk_
 #pragma unroll
       for (int k = 0; k < 16; ++k) {
         const int i = (k >> 1) & 1;
-        const float p = s[b][k] > -INFINITY ? exp2f(s[b][k] - mw[i]) : 0.f;
+        const float p = s[b][k] == -INFINITY ? 0.f : exp2f(s[b][k] - mw[i]);     // a NaN stays one
         ls[i] += p;
         s[b][k] = p * cw[i];
       }

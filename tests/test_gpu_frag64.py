@@ -61,3 +61,20 @@ def test_backward_128_repeatable():
     for other in runs[1:]:
         for a, b, n in zip(runs[0], other, NAMES):
             assert torch.equal(a, b), n
+
+
+@pytest.mark.parametrize('D', [64, 128])
+@pytest.mark.parametrize('wl', [20, 150])
+@pytest.mark.parametrize('which', ['q_swa', 'k_swa'])
+def test_a_nan_in_the_window_shows_in_every_row_that_sees_it(D, wl, which):
+    from nha_b200 import chunk_nha
+    T, at = 330, 70
+    d = gen.layer_inputs(92, 1, T, 2, 2, D, D, 64)
+    run = lambda: chunk_nha(*(d[n].cuda() for n in NAMES), window_size_left=wl, window_size_right=0)[:2]  # noqa: E731
+    o0, lse0 = run()
+    d[which][0, at, 1, 3] = float('nan')
+    o, lse = run()
+    sees = torch.zeros(T, dtype=torch.bool, device='cuda')
+    sees[at:at + (wl + 1 if which == 'k_swa' else 1)] = True
+    assert torch.isnan(o[0, sees, 1]).all() and torch.isnan(lse[0, sees, 1]).all()
+    assert torch.equal(o[0, ~sees], o0[0, ~sees]) and torch.equal(o[0, :, 0], o0[0, :, 0]) and torch.equal(lse[0, ~sees], lse0[0, ~sees])
