@@ -78,3 +78,13 @@ def test_a_nan_in_the_window_shows_in_every_row_that_sees_it(D, wl, which):
     sees[at:at + (wl + 1 if which == 'k_swa' else 1)] = True
     assert torch.isnan(o[0, sees, 1]).all() and torch.isnan(lse[0, sees, 1]).all()
     assert torch.equal(o[0, ~sees], o0[0, ~sees]) and torch.equal(o[0, :, 0], o0[0, :, 0]) and torch.equal(lse[0, ~sees], lse0[0, ~sees])
+
+
+def test_a_single_window_key_gives_its_logit_exactly():
+    # whole numbers: the product is exact, the scale 1/8 too, and the log-sum-exp over one key is its logit
+    from nha_b200 import chunk_nha
+    d = gen.layer_inputs(93, 1, 200, 2, 2, 64, 64, 64)
+    q, k = (torch.randint(-8, 9, d[n].shape, generator=torch.Generator().manual_seed(i)) for i, n in enumerate(('q_swa', 'k_swa')))
+    d['q_swa'], d['k_swa'] = q.bfloat16(), k.bfloat16()
+    lse = chunk_nha(*(d[n].cuda() for n in NAMES), window_size_left=0, window_size_right=0)[1]
+    assert torch.equal(lse.cpu(), (q * k).sum(-1).float() / 8)
