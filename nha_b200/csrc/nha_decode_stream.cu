@@ -565,14 +565,16 @@ __global__ void __launch_bounds__(kStrThreads, NT == 1 ? 2 : 1) nha_decode_strea
     const int ms = kGroup * warp;
     load_state();
     {
+      // h <- h e^g + k s with the small product rounded: the large one is the fused one, as the error of the state is made of it
+      // (against 64 bits 8.3e-8 a step; 8.7e-8 with the other one fused)
       const float4 e4 = *reinterpret_cast<const float4*>(eg + ms + hs), s4 = *reinterpret_cast<const float4*>(sv + ms + hs);
 #pragma unroll
       for (int i = 0; i < kHk; ++i) {
         const float kk = kpop[16 * i + hr];
-        hreg[i].x = hreg[i].x * e4.x + kk * s4.x;
-        hreg[i].y = hreg[i].y * e4.y + kk * s4.y;
-        hreg[i].z = hreg[i].z * e4.z + kk * s4.z;
-        hreg[i].w = hreg[i].w * e4.w + kk * s4.w;
+        hreg[i].x = fmaf(hreg[i].x, e4.x, __fmul_rn(kk, s4.x));
+        hreg[i].y = fmaf(hreg[i].y, e4.y, __fmul_rn(kk, s4.y));
+        hreg[i].z = fmaf(hreg[i].z, e4.z, __fmul_rn(kk, s4.z));
+        hreg[i].w = fmaf(hreg[i].w, e4.w, __fmul_rn(kk, s4.w));
         if (ms + hs < nslots) st_state4<SB16>(a.hk, ((size_t)bh * K + 16 * i + hr) * M + m0 + ms + hs, hreg[i]);
       }
     }
@@ -634,10 +636,10 @@ __global__ void __launch_bounds__(kStrThreads, NT == 1 ? 2 : 1) nha_decode_strea
       const int m = ms + kRowsI * u + vsub;
       if (m < nslots) {
         const float e = eg[m], sm = sv[m];
-        vreg[u].x = vreg[u].x * e + sm * vp.x;
-        vreg[u].y = vreg[u].y * e + sm * vp.y;
-        vreg[u].z = vreg[u].z * e + sm * vp.z;
-        vreg[u].w = vreg[u].w * e + sm * vp.w;
+        vreg[u].x = fmaf(vreg[u].x, e, __fmul_rn(sm, vp.x));
+        vreg[u].y = fmaf(vreg[u].y, e, __fmul_rn(sm, vp.y));
+        vreg[u].z = fmaf(vreg[u].z, e, __fmul_rn(sm, vp.z));
+        vreg[u].w = fmaf(vreg[u].w, e, __fmul_rn(sm, vp.w));
         st_state4<SB16>(a.hv, ((size_t)bh * M + m0 + m) * V + vcol, vreg[u]);
       }
 #pragma unroll

@@ -339,3 +339,15 @@ def test_tensors_that_do_not_start_on_16_bytes(K, W):
     for run in [step] + ([ring] if K >= 64 else []):
         for a, b in zip(run(False), run(True)):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize('K,H,NG,W', [(128, 4, 8, 512), (64, 16, 1, 64)])
+def test_the_state_update_fuses_the_large_product(K, H, NG, W):
+    # h e^g + k s: k s is rounded, h e^g is not.  Seen where e^g is 1, as the sum of h and the rounded product to the last bit.
+    from nha_b200 import fused_recurrent_nha_decode
+    d = {n: x.cuda() if torch.is_tensor(x) else x for n, x in gen.decode_inputs(5, 2, H, NG, K, K, 64, W).items()}
+    k, v, s = (d[n][:, 0].float() for n in ('k', 'v', 's'))
+    hk, hv = d['hk0'] + k[..., None] * s[:, :, None], d['hv0'] + s[..., None] * v[:, :, None]
+    _, got = fused_recurrent_nha_decode(*(d[n] for n in ('q', 'k', 'v')), torch.zeros_like(d['g']), d['sw_k_raw'], d['vw'], s=d['s'],
+                                        cos=d['cos'], sin=d['sin'], initial_state=(d['hk0'], d['hv0']), output_final_state=True)
+    assert torch.equal(got[0], hk) and torch.equal(got[1], hv)
