@@ -507,7 +507,8 @@ __global__ void __launch_bounds__(kStrThreads, NT == 1 ? 2 : 1) nha_decode_strea
             oacc[t][j][u][2] *= f0; oacc[t][j][u][3] *= f1;
           }
       }
-      const float p0 = exp2f(x0 - m_run[t]), p1 = exp2f(x1 - m_run[t]);
+      const float ref = m_run[t] > -INFINITY ? m_run[t] : 0.f;     // every logit so far minus infinity: weights zero (a NaN stays one)
+      const float p0 = exp2f(x0 - ref), p1 = exp2f(x1 - ref);
       l_run[t] += p0 + p1;
       const __nv_bfloat162 pk = __floats2bfloat162_rn(p0, p1);
       pb[t] = *reinterpret_cast<const uint32_t*>(&pk);
@@ -613,7 +614,8 @@ __global__ void __launch_bounds__(kStrThreads, NT == 1 ? 2 : 1) nha_decode_strea
       float mx = fmaxf(x0, x1);
       mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
       mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-      const float p0 = exp2f(x0 - mx), p1 = exp2f(x1 - mx);
+      const float ref = mx > -INFINITY ? mx : 0.f;                 // eight logits of minus infinity: weights zero (a NaN stays one)
+      const float p0 = exp2f(x0 - ref), p1 = exp2f(x1 - ref);
       pS[sl * NH + qh] = p0;
       pS[(sl + 1) * NH + qh] = p1;
       float sum = p0 + p1;
@@ -667,7 +669,7 @@ __global__ void __launch_bounds__(kStrThreads, NT == 1 ? 2 : 1) nha_decode_strea
         }
         if (qh < NG && (kRowsI == 1 || lane < 16)) {
           const float m1 = myml[4 * qh], m2 = myml[4 * qh + 2], mx = fmaxf(m1, m2);
-          const float f1 = exp2f(m1 - mx), f2 = exp2f(m2 - mx);    // the slots' maximum is finite
+          const float f1 = m1 > -INFINITY ? exp2f(m1 - mx) : 0.f, f2 = m2 > -INFINITY ? exp2f(m2 - mx) : 0.f;
           float4* o4 = reinterpret_cast<float4*>(osm + warp * kOut + qh * ldo + vcol);
           const float4 w4 = *o4;
           *o4 = make_float4(f1 * x.x + f2 * w4.x, f1 * x.y + f2 * w4.y, f1 * x.z + f2 * w4.z, f1 * x.w + f2 * w4.w);

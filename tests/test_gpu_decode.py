@@ -343,11 +343,38 @@ def test_tensors_that_do_not_start_on_16_bytes(K, W):
 
 @pytest.mark.parametrize('K,H,NG,W', [(128, 4, 8, 512), (64, 16, 1, 64)])
 def test_the_state_update_fuses_the_large_product(K, H, NG, W):
-    # h e^g + k s: k s is rounded, h e^g is not.  Seen where e^g is 1, as the sum of h and the rounded product to the last bit.
+    # h e^g + k s to the last bit: k s is rounded, h e^g is not (its 48 bits are exact in fp64)
     from nha_b200 import fused_recurrent_nha_decode
     d = {n: x.cuda() if torch.is_tensor(x) else x for n, x in gen.decode_inputs(5, 2, H, NG, K, K, 64, W).items()}
     k, v, s = (d[n][:, 0].float() for n in ('k', 'v', 's'))
-    hk, hv = d['hk0'] + k[..., None] * s[:, :, None], d['hv0'] + s[..., None] * v[:, :, None]
-    _, got = fused_recurrent_nha_decode(*(d[n] for n in ('q', 'k', 'v')), torch.zeros_like(d['g']), d['sw_k_raw'], d['vw'], s=d['s'],
-                                        cos=d['cos'], sin=d['sin'], initial_state=(d['hk0'], d['hv0']), output_final_state=True)
-    assert torch.equal(got[0], hk) and torch.equal(got[1], hv)
+
+    def step(k_, v_, hk, hv):
+        return fused_recurrent_nha_decode(d['q'], k_, v_, d['g'], d['sw_k_raw'], d['vw'], s=d['s'], cos=d['cos'], sin=d['sin'],
+                                          initial_state=(hk.clone(), hv.clone()), output_final_state=True)[1]
+    ek, ev = step(0 * d['k'], 0 * d['v'], torch.ones_like(d['hk0']), torch.ones_like(d['hv0']))       # e^g as the kernel has it
+    got = step(d['k'], d['v'], d['hk0'], d['hv0'])
+    for x, h, e, p in ((got[0], d['hk0'], ek, k[..., None] * s[:, :, None]), (got[1], d['hv0'], ev, s[..., None] * v[:, :, None])):
+        assert torch.equal(x, (h.double() * e.double() + p.double()).float())
+
+
+@pytest.mark.parametrize('K,H,NG,W', [(128, 2, 4, 512), (64, 4, 1, 64), (64, 2, 2, 300)])
+def test_logits_of_minus_infinity_and_nan(K, H, NG, W):
+    # whole groups of eight keys and of eight slots (what a warp takes at once) at minus infinity have weight zero; a NaN shows
+    from nha_b200 import fused_recurrent_nha_decode
+    d = gen.decode_inputs(9, 2, H, NG, K, K, 64, W)
+    d['q'][..., 3] = 1.0
+    d['sw_k_raw'][:, :W // 2, :, 3] = float('-inf')
+    d['hk0'][:, :, 3, 8:32] = float('-inf')
+    names = ('q', 'k', 'v', 'g', 'sw_k_raw', 'vw')
+
+    def step():
+        c = {n: x.cuda() if torch.is_tensor(x) else x for n, x in d.items()}
+        return fused_recurrent_nha_decode(*(c[n] for n in names), sq=c['q'], initial_state=(c['hk0'], c['hv0']), output_final_state=True)[0].cpu()
+    want = orc.decode_step(*(d[n] for n in names), d['scale'], sq=d['q'], hk0=d['hk0'], hv0=d['hv0'])[0]
+    assert torch.isfinite(want).all()
+    assert_close(step(), want, TOL_OUT, 'o')
+    d['sw_k_raw'][0, W - 1, 0, 5] = float('nan')
+    d['hk0'][1, 1, 5, 40] = float('nan')
+    o = step()
+    assert torch.isnan(o[0, 0, :NG]).all() and torch.isnan(o[1, 0, NG:2 * NG]).all()
+    assert torch.isfinite(o[0, 0, NG:]).all() and torch.isfinite(o[1, 0, :NG]).all()
