@@ -79,7 +79,10 @@ inline Tensor typed(const Tensor& x, at::ScalarType dt) {
 }
 // The kernels load and copy 16 bytes at a time: a contiguous view that starts elsewhere is copied.
 inline bool on_16_bytes(const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0; }
-inline Tensor on_16(Tensor t) { return C10_LIKELY(on_16_bytes(t)) ? t : t.clone(); }
+inline Tensor on_16(Tensor t) {
+  if (C10_LIKELY(on_16_bytes(t))) return t;
+  return t.clone();
+}
 inline void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 
 inline const Tensor& tensor(PyObject* o, const char* name) {

@@ -413,8 +413,10 @@ __global__ void __launch_bounds__(kStrThreads, NT == 1 ? 2 : 1) nha_decode_strea
   }
   __syncthreads();
   const float sc2 = a.scale * kLog2e;
-  constexpr float kRaise = 8.f;
-
+  // A warp raises its reference (and rescales its output) when a key exceeds it by this much (log2): the weights are rounded to bf16
+  // for the product with the values, and the key a reference was taken from has the weight 1, which is exact.  Error of the output
+  // against 64 bits, 32 heads on 4, D 128, W 512: 3.42e-3 with 8, 3.31e-3 with 1, 3.27e-3 with 0; 17.1, 17.15 and 17.3 us a layer.
+  constexpr float kRaise = 1.f;
 
   // ---- the window, eight keys at a time --------------------------------------------------------------------------------
   const int gq = lane >> 2, tq = lane & 3;                         // fragment coordinates of the lane
@@ -493,7 +495,7 @@ __global__ void __launch_bounds__(kStrThreads, NT == 1 ? 2 : 1) nha_decode_strea
       float mx = fmaxf(x0, x1);
       mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
       mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-      const bool raise = mx > m_run[t] + kRaise;                   // weights stay below 2^8, exact enough in fp32 sums
+      const bool raise = mx > m_run[t] + kRaise;
       if (__any_sync(0xffffffffu, raise)) {
         const float f = raise ? exp2f(m_run[t] - mx) : 1.f;        // 0 when nothing came before
         if (raise) m_run[t] = mx;
