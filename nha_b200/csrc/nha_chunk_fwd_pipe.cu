@@ -34,7 +34,10 @@
 // ONE softmax over the slot logits and all window logits, in a single sweep: the running reference m of a row starts
 // as its slot maximum and is only raised when a window logit exceeds it by more than 8 ln 2 (probabilities then stay
 // below 256, exact in the fp32 accumulator); raising it rescales the row of O in tensor memory (tcgen05.ld / st by the
-// row's thread, after the products in flight on O have completed).  Decay factorisation, flags for chunks that decay
+// row's thread, after the products in flight on O have completed).  With one head per kv head the reference follows the
+// maximum itself: those calls came from a kernel with exact maxima, whose largest probability, rounded to bf16 for the value
+// product, is exactly 1 (error of o against 64 bits, W 512: 2.14e-3, with the lagging reference 2.34e-3; the rescaling that it
+// costs would be 7 % of the document prefill of a grouped model, which never had it).  Decay factorisation, flags for chunks that decay
 // too fast for one reference per chunk, and the general kernel that takes those: as in nha_chunk_fwd_umma.cu.
 //
 // What bounds it: the exchange of a window step - score product, tensor-memory load, exponentials, store, value product - whose
@@ -475,6 +478,7 @@ __global__ void __launch_bounds__(pipe::kThreads, 2)
     const int klo = in_seq ? (wl < 0 ? 0 : max(0, pos - wl)) : (1 << 30);
     const unsigned kspan = in_seq ? (unsigned)(pos - klo) : 0u;
     const float sc2 = d.scale * kLog2e;
+    const float lag = NG == 1 ? 0.f : kRaise;                      // how far a window logit may exceed the reference of its row
     uint32_t gph = 0u;
     // one lane of a warp polls a barrier, the others wait at the warp barrier: far fewer shared-memory polls
 #define NHA_WAIT_WARP(idx_, par_)                        \
@@ -613,10 +617,10 @@ __global__ void __launch_bounds__(pipe::kThreads, 2)
           m1 = max3(m1, s[e + 2], s[e + 3]);
         }
         float mc = d.scale * fmaxf(m0, m1);
-        if (pair_any(mc > mref + kRaise)) {
+        if (pair_any(mc > mref + lag)) {
           mc = fmaxf(mc, partner(mc));
           float f = 1.f;
-          if (mc > mref + kRaise) {
+          if (mc > mref + lag) {
             f = __expf(mref - mc);
             mref = mc;
           }
@@ -718,7 +722,7 @@ __global__ void __launch_bounds__(pipe::kThreads, 2)
 
 // Any number of query heads per kv head: an odd group's last tile is half empty, and so is every tile of a group of one,
 // where two 64-row CTAs of nha_fwd_umma_kernel would do the same work - slower all the same (B4 T2048 H16 W64, whole
-// prefill: 215 us here, 298 us there; seven heads a group, B4 T500: 77 us here, 341 us with the general kernel).
+// prefill: 195 us here, 301 us there; seven heads a group, B2 T2048 W512: 110 us here, 1570 us with the general kernel).
 bool fwd_pipe_supported(const nha_chunk_desc* d) {
   if (d->K != 128 || d->V != 128 || d->M != 64 || !(d->scale > 0.f)) return false;
   const char* off = getenv("NHA_B200_NO_PIPE");

@@ -119,10 +119,11 @@ def test_strong_gates_stay_finite_and_exact():
     assert_close(hk, ref_hk, TOL_OUT, 'hkt')
 
 
-@pytest.mark.parametrize('K,H,NG,W,M,bound', [(64, 4, 1, 512, 64, 2.2e-3), (64, 2, 4, 300, 64, 2.22e-3)])
+@pytest.mark.parametrize('K,H,NG,W,M,bound', [(64, 4, 1, 512, 64, 2.2e-3), (64, 2, 4, 300, 64, 2.22e-3), (128, 4, 1, 512, 64, 2.2e-3),
+                                              (128, 4, 1, 64, 64, 2.2e-3)])
 def test_the_rounding_of_the_window_weights(K, H, NG, W, M, bound):
     # error of o against 64 bits where the reference of the weights is the running maximum: 2.16e-3 and 2.19e-3; where it may lag by
-    # 2^8, 2.24e-3 and 2.26e-3
+    # 2^8, 2.24e-3 and 2.26e-3 (head dim 128: 2.14e-3 and 2.18e-3 against 2.34e-3 and 2.35e-3)
     from nha_b200 import fused_chunk_nha_prefill
     d = gen.prefill_inputs(31, 1, H, NG, K, K, M, W, 900, False)
     names = ('q', 'k', 'v', 'rotary_q', 'rotary_k', 's', 'g')
