@@ -38,6 +38,12 @@ cudaError_t set_max_smem(const void* func, int bytes) {
   return e;
 }
 
+int sm_count() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms > 0 ? sms : 148;
+}
+
 // One CTA waits, with a poll limit, on an mbarrier phase that nobody completes: the wait must come back as "ran out"
 // and the kernel reports it in the error word, exactly as the tensor-core kernels report a completion that never came.
 __global__ void nha_selftest_wait_kernel(int* err, int limit) {

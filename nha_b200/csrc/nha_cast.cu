@@ -68,7 +68,7 @@ extern "C" int nha_cast_many(const void* const* src, void* const* dst, const int
   }
   const int64_t total = a.first[count];
   if (total == 0) return NHA_OK;
-  const int64_t want = (total + 255) / 256, most = 148 * 8;
+  const int64_t want = (total + 255) / 256, most = (int64_t)sm_count() * 8;     // whole waves of eight 256-thread CTAs per SM
   const dim3 grid((unsigned)(want < most ? want : most));
   cudaStream_t cs = (cudaStream_t)stream;
 #define NHA_CAST(s_, d_, S_, D_) if (src_type == s_ && dst_type == d_) { nha_cast_kernel<S_, D_><<<grid, 256, 0, cs>>>(a); return check_launch(); }

@@ -28,10 +28,6 @@ constexpr int oTot = oPart + 9 * 64 * 4;                      // fp32 [4 quarter
 constexpr int oBar = oTot + 4 * 64 * 4;
 constexpr int total = oBar + 64 + 1024;
 static_assert(total <= 113 * 1024, "two CTAs per SM");
-// The pass waits for its loads: two CTAs an SM keep too few bytes in flight, so each prefetches the inputs of a later CTA into L2.
-// B16 T2048 H16 W64: 386 us with TMA tiles alone (392 before them), 325-330 with the prefetch 148 CTAs ahead, 341 with 296, 374
-// with 444.
-constexpr int kAhead = 148;                                   // CTAs by which the prefetch runs ahead: one per SM
 }  // namespace cl64
 
 // Tensor maps of the call's tensors (this GPU's own memory).  A tile whose 64 rows lie inside its sequence comes by TMA; the
@@ -45,7 +41,7 @@ struct ColsMaps {
 // ONE: one query head per kv head.  Several heads accumulate in columns of their own (512 columns, one CTA per SM).
 template <bool ONE>
 __global__ void __launch_bounds__(kThreads, ONE ? 2 : 1) nha_bwd_cols64_kernel(const nha_chunk_desc d, const BwdWs w, int* __restrict__ err,
-                                                                                 const __grid_constant__ ColsMaps maps) {
+                                                                                 const __grid_constant__ ColsMaps maps, const unsigned ahead) {
   grid_dep_wait();
   grid_dep_launch();
   using namespace cl64;
@@ -75,7 +71,7 @@ __global__ void __launch_bounds__(kThreads, ONE ? 2 : 1) nha_bwd_cols64_kernel(c
   const uint32_t loff = sw_off(lr, lc);
   const int64_t rq = (int64_t)HQ * 64, rp = (int64_t)H * 64, rm = (int64_t)H * M, rz = (int64_t)HQ * M;
   // load barriers: each phase is closed by one arrival of thread 0 behind its last TMA; bits of lph: their parities
-  uint64_t* bl = mbar + 2;
+  uint64_t* bl = mbar + 2;                                     // [0] gates and write weights, [1] the rest
   uint32_t lph = 0;
   auto loads_done = [&](int bar) {
     cp_commit();
@@ -105,7 +101,6 @@ __global__ void __launch_bounds__(kThreads, ONE ? 2 : 1) nha_bwd_cols64_kernel(c
     mbar_init(mbar, 1);
     mbar_init(&bl[0], 1);
     mbar_init(&bl[1], 1);
-    mbar_init(&bl[2], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_async_smem();
   }
@@ -148,10 +143,11 @@ __global__ void __launch_bounds__(kThreads, ONE ? 2 : 1) nha_bwd_cols64_kernel(c
       if (!last) nv[u] = *reinterpret_cast<const uint4*>((const bf16*)d.hv_chunks + ((size_t)(cg + 1) * H + h) * M * 64 + r * 64 + 8 * lc);
     }
   }
-  // What the CTA that follows on this SM will read goes into L2 now: the loads are what the pass waits for (B16 T2048 H16: 386 us
-  // without, 325 us with it; two or three CTAs ahead 341 and 374 us).
-  if (maps.use && tid == 64 && blockIdx.x + kAhead < gridDim.x) {
-    const int ncg = (blockIdx.x + kAhead) / H, nhd = blockIdx.x + kAhead - ncg * H;
+  // The pass waits for its loads: two CTAs an SM keep too few bytes in flight, so each prefetches the inputs of the CTA `ahead`
+  // places on into L2, one per SM.  16 x 2048 tokens, 16 heads, W 64: 386 us without it, 325-330 so, 341 and 374 two and three
+  // places per SM ahead.
+  if (maps.use && tid == 64 && blockIdx.x + ahead < gridDim.x) {
+    const int ncg = (blockIdx.x + ahead) / H, nhd = blockIdx.x + ahead - ncg * H;
     const ChunkRec nr = chunk_rec(d, ncg);
     if (nr.n >= 0) {
       const int row = nr.t0 + nr.ci * kChunk;
@@ -469,8 +465,9 @@ int bwd_cols64_launch(const nha_chunk_desc* d, const BwdWs& w, int* err, cudaStr
              make_map_rows_heads(&maps.s, d->s, d->Ttot, d->H, 64) && make_map_rows_heads(&maps.dout, d->d_o, d->Ttot, d->HQ, 64) &&
              make_map_rows_heads(&maps.za, w.dza, d->Ttot, d->HQ, 64) && make_map_rows_heads(&maps.pa, w.paq, d->Ttot, d->HQ, 64);
   const dim3 grid((unsigned)(nha_chunk_count_bound(d->Ttot, d->N) * d->H));
-  if (d->HQ == d->H) launch_after(nha_bwd_cols64_kernel<true>, grid, kThreads, cl64::total, cs, *d, w, err, maps);
-  else launch_after(nha_bwd_cols64_kernel<false>, grid, kThreads, cl64::total, cs, *d, w, err, maps);
+  const unsigned ahead = (unsigned)sm_count();
+  if (d->HQ == d->H) launch_after(nha_bwd_cols64_kernel<true>, grid, kThreads, cl64::total, cs, *d, w, err, maps, ahead);
+  else launch_after(nha_bwd_cols64_kernel<false>, grid, kThreads, cl64::total, cs, *d, w, err, maps, ahead);
   return check_launch();
 }
 

@@ -859,8 +859,7 @@ static int stream_layout(DecodeStreamArgs& a, int D) {
 // Splits of a (sequence, kv head) for the streaming kernel: as many as keep the whole grid in one wave of two
 // CTAs per SM, each split keeping at least kMinKeys keys and 4 slots.
 int decode_stream_splits(int B, int H, int W, int M) {
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
   int spl = M > 64 && M <= 128 ? 2 : 1;            // a split has at most 64 slots: eight a warp
   while (spl < 16 && (int64_t)B * H * spl * 2 <= 2 * (int64_t)sms && W / (spl * 2) >= kMinKeys && M / (spl * 2) >= 4 &&
          M % (spl * 2 * 4) == 0)

@@ -79,10 +79,8 @@ __global__ void __launch_bounds__(kActThreads) nha_act3_kernel(const __grid_cons
 }
 
 static int wave_grid(int64_t work_items, int64_t per_cta, int ctas_per_sm) {
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int64_t want = (work_items + per_cta - 1) / per_cta;
-  const int64_t cap = (int64_t)sms * ctas_per_sm;
+  const int64_t cap = (int64_t)sm_count() * ctas_per_sm;
   return (int)(want < 1 ? 1 : (want < cap ? want : cap));
 }
 static bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }

@@ -93,11 +93,9 @@ extern "C" int nha_rope_pair(const void* q, const void* k, void* q_out, void* k_
   a.cosp = (const bf16*)cos; a.sinp = (const bf16*)sin; a.cs_row = cs_row;
   a.cu = cu_seqlens; a.N = N; a.T = T; a.Ttot = Ttot; a.K = K; a.offset = offset; a.table_rows = table_rows;
   a.sin_sign = inverse ? -1.0f : 1.0f;
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int64_t units = Ttot * (a.heads[0] + a.heads[1]) * (K >> 4);
   const int64_t want = (units + kRopeThreads - 1) / kRopeThreads;
-  const int64_t cap = (int64_t)sms * 8 * 4;                   // four trips of eight CTAs per SM at most
+  const int64_t cap = (int64_t)sm_count() * 8 * 4;                   // four trips of eight CTAs per SM at most
   nha_rope_kernel<<<(int)(want < cap ? want : cap), kRopeThreads, 0, (cudaStream_t)stream>>>(a);
   return check_launch();
 }
