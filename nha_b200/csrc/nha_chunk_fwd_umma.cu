@@ -1,11 +1,10 @@
-// Output pass of the chunked NHA forward for head dim 128 where the pipelined kernel (nha_chunk_fwd_pipe.cu) is not available: tcgen05.mma with operands in
-// 128-byte-swizzled shared memory, accumulators in tensor memory (TMEM), two (D = 64) or four (D = 128)
-// threads per query row for the softmax: tcgen05.ld hands a thread 32 or 16 columns of its row, the warps
-// that share a TMEM lane quarter (w, w + 4, ...) take alternate parts of the columns and combine row maxima
-// and sums through shared memory.  Eight or sixteen warps per CTA keep the element-wise phases, which are bound by
-// instruction issue, from stalling on their own dependencies.  One CTA per (chunk, kv head); an MMA tile is 64 tokens x 1 head (R = 64, for
-// HQ == H) or 64 tokens x 2 heads of the group (R = 128), and the CTA walks the heads of the group
-// reusing the chunk's k', v', gates and chunk-start states.
+// Output pass of the chunked NHA forward for head dim 128 where the pipelined kernel (nha_chunk_fwd_pipe.cu) is switched off or its
+// tensor maps cannot be made: tcgen05.mma with operands in 128-byte-swizzled shared memory, accumulators in tensor memory (TMEM),
+// four threads per query row for the softmax: tcgen05.ld hands a thread 16 columns of its row, the warps that share a TMEM lane
+// quarter (w, w + 4, ...) take alternate parts of the columns and combine row maxima and sums through shared memory.  Sixteen warps
+// per CTA keep the element-wise phases, which are bound by instruction issue, from stalling on their own dependencies.  One CTA
+// per (chunk, kv head); an MMA tile is 64 tokens x 1 head (R = 64, for HQ == H) or 64 tokens x 2 heads of the group (R = 128), and
+// the CTA walks the heads of the group reusing the chunk's k', v', gates and chunk-start states.
 //
 // Per tile:   A  = q k'^T,  QH = q Hk,  S = q_swa k_swa^T (newest window step)           MMA group 1
 //             X  = tril(A) (s' .* b)                                                      MMA group 2
@@ -19,8 +18,7 @@
 // untouched and flagged, and the general kernel (16-row block references, nha_chunk_fwd.cu) computes it
 // instead, so the result never depends on the bound.  Probabilities are formed unnormalised against the
 // joint row maximum (p~ = exp(x - max)), accumulated in one TMEM accumulator and divided by the row sum
-// at the end, so every logit is exponentiated once.  A window step is two 64-key tiles for D = 64 and
-// one for D = 128; a window of up to one step (W <= 64 at D = 64) needs no loop at all.
+// at the end, so every logit is exponentiated once.  A window step is one 64-key tile.
 //
 // Replaces chunk_nha_fused_o_kernel (nha_fla/ops/nha/chunk_fused.py:117-283) and, for chunk_nha, the
 // flash-attn varlen forward + fla chunk_gsa forward + log-sum-exp merge (nha_fla/ops/nha/chunk.py:423-470).
@@ -44,16 +42,14 @@ struct WindowMaps {
   int use;                                            // 0: no tensor maps (copies go through cp.async)
 };
 
-template <int D, int R>
+template <int R>
 struct UmmaLayout {
-  static constexpr int KT = D / 64;
-  static constexpr int TP = D == 64 ? 2 : 1;          // 64-key tiles per window step
-  static constexpr int NS = D == 64 ? 2 : 4;          // threads per row (D = 128 runs one CTA per SM: more warps)
+  static constexpr int D = 128, KT = D / 64;
+  static constexpr int NS = 4;                        // threads per row (one CTA per SM: many warps)
   static constexpr int kThreads = 128 * NS;
   static constexpr int kATile = R * 128;              // one 64-wide k tile of an R-row A operand
-  static constexpr int kWTile = TP * 8192;            // one 64-wide k tile of a window-step operand (64 TP rows)
+  static constexpr int kWTile = 8192;                 // one 64-wide k tile of a window-step operand
   static constexpr bool kAlias = R == 64;             // one head per CTA: k' and Hk are dead after MMA group 1
-  static constexpr bool kPOverW = R <= D;             // P~ fits over the window keys it was computed from
   static constexpr int tQ = 0;                        // q_gsa; later p~ .* a
   static constexpr int tQS = tQ + KT * kATile;        // q_swa
   static constexpr int tK = tQS + KT * kATile;        // k'
@@ -61,44 +57,38 @@ struct UmmaLayout {
   static constexpr int tHk = tV + KT * 8192;          // Hk [D][64]
   static constexpr int tHv = tHk + D * 128;           // Hv [64][D]
   static constexpr int tSB = tHv + KT * 8192;         // s' .* b [64][64]
-  static constexpr int tW = tSB + 8192;               // window keys of one step [64 TP][D]
-  static constexpr int tWV = tW + KT * kWTile;        // window values of one step [64 TP][D]
+  static constexpr int tW = tSB + 8192;               // window keys of one step [64][D]; then P~ [R][64] over them
+  static constexpr int tWV = tW + KT * kWTile;        // window values of one step [64][D]
   static constexpr int end0 = tWV + KT * kWTile;
-  static constexpr int tP = kPOverW ? tW : end0;      // P~ [R][64 TP]
-  static constexpr int end1 = kPOverW ? end0 : end0 + TP * kATile;
-  static constexpr int tAB = kAlias ? tHk : end1;     // tril(A) / tril(Bv)  [R][64]
-  static constexpr int tPG = kAlias ? tK : end1 + kATile;   // p~ .* a .* e^R   [R][64]
-  static constexpr int end2 = kAlias ? end1 : end1 + 2 * kATile;
-  // D = 128 runs one CTA per SM, so the window loops are pipelined inside the CTA: a second set of window
-  // buffers (behind k' and Hk, which are dead after MMA group 1 and fetched again for the next head tile; with one
-  // head per CTA those tiles hold p~ and tril(A), so the set gets room of its own) and a second S accumulator.
-  static constexpr bool kPipe = D == 128;
-  static constexpr int end3 = (kPipe && kAlias) ? end2 + 2 * KT * kWTile : end2;
-  static constexpr int tW2 = !kPipe ? tW : (kAlias ? end2 : tK);
-  static constexpr int tWV2 = !kPipe ? tWV : (kAlias ? end2 + KT * kWTile : tHk);
-  static constexpr int oA = end3;                     // fp32 [64][65]: cumulative gates, then a = exp(G - R)
+  static constexpr int tAB = kAlias ? tHk : end0;     // tril(A) / tril(Bv)  [R][64]
+  static constexpr int tPG = kAlias ? tK : end0 + kATile;   // p~ .* a .* e^R   [R][64]
+  static constexpr int end1 = kAlias ? end0 : end0 + 2 * kATile;
+  // One CTA per SM, so the window loops are pipelined inside the CTA: a second set of window buffers (behind k' and Hk, which are
+  // dead after MMA group 1 and fetched again for the next head tile; with one head per CTA those tiles hold p~ and tril(A), so the
+  // set gets room of its own) and a second S accumulator.
+  static constexpr int end2 = kAlias ? end1 + 2 * KT * kWTile : end1;
+  static constexpr int tW2 = kAlias ? end1 : tK;
+  static constexpr int tWV2 = kAlias ? end1 + KT * kWTile : tHk;
+  static constexpr int oA = end2;                     // fp32 [64][65]: cumulative gates, then a = exp(G - R)
   static constexpr int oR = oA + 64 * 65 * 4;         // fp32 [64] exp(R)
   static constexpr int oX = oR + 256;                 // fp32 [4][NS][128] row statistics swapped between the column parts
-  static constexpr int oBar = oX + 4 * NS * 128 * 4;  // mbarriers (MMA groups; loads, S and PV of the pipelined loops) + TMEM slot              // mbarrier + TMEM slot
+  static constexpr int oBar = oX + 4 * NS * 128 * 4;  // mbarriers (MMA groups; loads, S and PV of the window loops) + TMEM slot
   static constexpr int total = oBar + 128 + 1024;     // + slack for the 1024-byte alignment of the base
-  static constexpr int kTmemCols = D == 64 ? 256 : 512;
-  // O reuses QH's columns at D = 64 (QH has been read by then)
-  static constexpr int cA = 0, cQH = 64, cS = 128, cO = D == 64 ? 64 : 256;
-  static constexpr int cS2 = kPipe ? 192 : cS;        // second S accumulator of the pipelined loops
+  static constexpr int kTmemCols = 512;
+  static constexpr int cA = 0, cQH = 64, cS = 128, cS2 = 192, cO = 256;     // cS, cS2: the two S accumulators
   static_assert(total <= 227 * 1024, "shared memory of the output pass");
 };
 
-template <int D, int R>
-__global__ void __launch_bounds__(UmmaLayout<D, R>::kThreads, (D == 64 && R == 64) ? 2 : 1) nha_fwd_umma_kernel(const nha_chunk_desc d, int* __restrict__ flags,
-                                                                  int* __restrict__ err,
-                                                                  const __grid_constant__ WindowMaps maps) {
-  typedef UmmaLayout<D, R> L;
-  constexpr int KT = L::KT, TH = R / 64, M = 64, TP = L::TP, WK = 64 * TP;
+template <int R>
+__global__ void __launch_bounds__(UmmaLayout<R>::kThreads, 1) nha_fwd_umma_kernel(const nha_chunk_desc d, int* __restrict__ flags,
+                                                                                  int* __restrict__ err,
+                                                                                  const __grid_constant__ WindowMaps maps) {
+  typedef UmmaLayout<R> L;
+  constexpr int D = L::D, KT = L::KT, TH = R / 64, M = 64, WK = 64;
   constexpr int NS = L::NS, kUThreads = L::kThreads;
   constexpr int CW = 64 / NS;                       // columns of a 64-column accumulator per thread
   constexpr int KW = WK / NS;                       // keys of a window step per thread
-  constexpr int LW = KW < 32 ? KW : 32;             // columns per tensor-memory load of the window logits
-  const int H = d.H, HQ = d.HQ, NG = HQ / H, N = d.N;
+  const int H = d.H, HQ = d.HQ, NG = HQ / H;
   const int cg = blockIdx.x, h = blockIdx.y;
   const ChunkRec rc = chunk_rec(d, cg);
   const int n = rc.n;
@@ -124,8 +114,8 @@ __global__ void __launch_bounds__(UmmaLayout<D, R>::kThreads, (D == 64 && R == 6
   // window steps, newest first: step p covers the keys [kbase(p), kbase(p) + WK)
   const int jt_hi = ci;
   const int jt_lo = wl < 0 ? 0 : max(0, c0 - wl) / kChunk;
-  const int nsteps = (jt_hi - jt_lo + TP) / TP;
-#define NHA_KBASE(p_) ((jt_hi + 1 - TP * ((p_) + 1)) * kChunk)
+  const int nsteps = jt_hi - jt_lo + 1;
+#define NHA_KBASE(p_) ((jt_hi - (p_)) * kChunk)
   const bf16* ksw = (const bf16*)d.k_swa + ((size_t)t0 * H + h) * D;
   const bf16* vsw = (const bf16*)d.v + ((size_t)t0 * H + h) * D;
 
@@ -151,18 +141,16 @@ __global__ void __launch_bounds__(UmmaLayout<D, R>::kThreads, (D == 64 && R == 6
   load_sw<D, kUThreads>(sm + L::tV, 8192, (const bf16*)d.v + ((size_t)t0 * H + h) * D, (int64_t)H * D, c0 - shift, lo, hi, 64, 0, tid);
   load_sw<64, kUThreads>(sm + L::tHk, 0, (const bf16*)d.hk_chunks + ((size_t)cg * H + h) * D * M, M, 0, 0, D, D, 0, tid);
   load_sw<D, kUThreads>(sm + L::tHv, 8192, (const bf16*)d.hv_chunks + ((size_t)cg * H + h) * M * D, D, 0, 0, M, M, 0, tid);
-// an odd group's last 128-row tile holds one head: its other 64 rows are zeros and never stored
-#define NHA_HEAD_ROWS(hq_) (R == 64 || (hq_) < (h + 1) * NG ? len : 0)
 #define NHA_LOAD_HEAD_TILE(ht_)                                                                                       \
   do {                                                                                                                \
     const int hq0_ = h * NG + (ht_) * TH;                                                                             \
     _Pragma("unroll") for (int t2 = 0; t2 < TH; ++t2) {                                                               \
       load_sw<D, kUThreads>(sm + L::tQ, L::kATile, (const bf16*)d.q_gsa + ((size_t)t0 * HQ + hq0_ + t2) * D, (int64_t)HQ * D,    \
-                 c0, 0, NHA_HEAD_ROWS(hq0_ + t2), 64, 64 * t2, tid);                                                  \
+                 c0, 0, len, 64, 64 * t2, tid);                                                  \
       load_sw<D, kUThreads>(sm + L::tQS, L::kATile, (const bf16*)d.q_swa + ((size_t)t0 * HQ + hq0_ + t2) * D, (int64_t)HQ * D,   \
-                 c0, 0, NHA_HEAD_ROWS(hq0_ + t2), 64, 64 * t2, tid);                                                  \
+                 c0, 0, len, 64, 64 * t2, tid);                                                  \
     }                                                                                                                 \
-    if (L::kPipe && !L::kAlias && (ht_) > 0) {     /* the second window buffer set has overwritten k' and Hk */       \
+    if (!L::kAlias && (ht_) > 0) {                 /* the second window buffer set has overwritten k' and Hk */       \
       load_sw<D, kUThreads>(sm + L::tK, 8192, (const bf16*)d.k_gsa + ((size_t)t0 * H + h) * D, (int64_t)H * D,          \
                             c0 - shift, lo, hi, 64, 0, tid);                                                            \
       load_sw<64, kUThreads>(sm + L::tHk, 0, (const bf16*)d.hk_chunks + ((size_t)cg * H + h) * D * M, M, 0, 0, D, D,    \
@@ -265,7 +253,7 @@ __global__ void __launch_bounds__(UmmaLayout<D, R>::kThreads, (D == 64 && R == 6
   const uint32_t aQ = smem_u32(sm + L::tQ), aQS = smem_u32(sm + L::tQS), aK = smem_u32(sm + L::tK);
   const uint32_t aV = smem_u32(sm + L::tV), aHk = smem_u32(sm + L::tHk), aHv = smem_u32(sm + L::tHv);
   const uint32_t aSB = smem_u32(sm + L::tSB), aW = smem_u32(sm + L::tW), aWV = smem_u32(sm + L::tWV);
-  const uint32_t aAB = smem_u32(sm + L::tAB), aPG = smem_u32(sm + L::tPG), aPA = aQ, aP = smem_u32(sm + L::tP);
+  const uint32_t aAB = smem_u32(sm + L::tAB), aPG = smem_u32(sm + L::tPG), aPA = aQ;
 
 #define NHA_MMA_WAIT()                                   \
   do {                                                   \
@@ -304,51 +292,41 @@ __global__ void __launch_bounds__(UmmaLayout<D, R>::kThreads, (D == 64 && R == 6
 #define NHA_STEP_MAX(kb_) NHA_STEP_MAX_AT(kb_, L::cS)
 #define NHA_STEP_MAX_AT(kb_, cs_)                                                                \
   do {                                                                                           \
-    float sv_[LW];                                                                               \
-    _Pragma("unroll") for (int pp = 0; pp < KW / LW; ++pp) {                                     \
-      const int key0 = KW * cpart + LW * pp;                                                     \
-      tmem_ldw<LW>(tlane + (cs_) + key0, sv_);                                                   \
-      const int off_ = (kb_) + key0 - klo;                                                       \
-      float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};                                \
-      _Pragma("unroll") for (int e = 0; e < LW; ++e)                                             \
-        m4[e & 3] = fmaxf(m4[e & 3], (unsigned)(off_ + e) <= kspan ? sv_[e] : -INFINITY);        \
-      ms = fmaxf(ms, d.scale * fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])));                 \
-    }                                                                                            \
+    float sv_[KW];                                                                               \
+    tmem_ldw<KW>(tlane + (cs_) + KW * cpart, sv_);                                               \
+    const int off_ = (kb_) + KW * cpart - klo;                                                   \
+    float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};                                  \
+    _Pragma("unroll") for (int e = 0; e < KW; ++e)                                               \
+      m4[e & 3] = fmaxf(m4[e & 3], (unsigned)(off_ + e) <= kspan ? sv_[e] : -INFINITY);          \
+    ms = fmaxf(ms, d.scale * fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])));                   \
   } while (0)
 // P~ = exp(scale S - ms) cw of this thread's keys of a step, into the swizzled tile; row sum into ls
-#define NHA_STEP_PROB(kb_) NHA_STEP_PROB_AT(kb_, L::cS, L::tP)
 #define NHA_STEP_PROB_AT(kb_, cs_, tp_)                                                          \
   do {                                                                                           \
-    float sv_[LW];                                                                               \
+    float sv_[KW];                                                                               \
     const float nms_ = -ms * kLog2e;                                                             \
-    _Pragma("unroll") for (int pp = 0; pp < KW / LW; ++pp) {                                     \
-      const int key0 = KW * cpart + LW * pp;                                                     \
-      tmem_ldw<LW>(tlane + (cs_) + key0, sv_);                                                   \
-      const int off_ = (kb_) + key0 - klo;                                                       \
-      if (active) {                                                                              \
-        float l4[4] = {0.f, 0.f, 0.f, 0.f};                                                      \
-        _Pragma("unroll") for (int c8 = 0; c8 < LW / 8; ++c8) {                                  \
-          float o8[8];                                                                           \
-          _Pragma("unroll") for (int e = 0; e < 8; ++e) {                                        \
-            const float pe = (unsigned)(off_ + 8 * c8 + e) <= kspan                              \
-                                 ? exp2f(fmaf(sv_[8 * c8 + e], sc2, nms_)) : 0.f;                \
-            l4[e & 3] += pe;                                                                     \
-            o8[e] = pe * cw;                                                                     \
-          }                                                                                      \
-          const int kk_ = key0 + 8 * c8;                                                         \
-          *reinterpret_cast<uint4*>(sm + (tp_) + (kk_ >> 6) * L::kATile +                        \
-                                    sw_off(row, (kk_ & 63) >> 3)) = pack8(o8);                   \
+    tmem_ldw<KW>(tlane + (cs_) + KW * cpart, sv_);                                               \
+    const int off_ = (kb_) + KW * cpart - klo;                                                   \
+    if (active) {                                                                                \
+      float l4[4] = {0.f, 0.f, 0.f, 0.f};                                                        \
+      _Pragma("unroll") for (int c8 = 0; c8 < KW / 8; ++c8) {                                    \
+        float o8[8];                                                                             \
+        _Pragma("unroll") for (int e = 0; e < 8; ++e) {                                          \
+          const float pe = (unsigned)(off_ + 8 * c8 + e) <= kspan                                \
+                               ? exp2f(fmaf(sv_[8 * c8 + e], sc2, nms_)) : 0.f;                  \
+          l4[e & 3] += pe;                                                                       \
+          o8[e] = pe * cw;                                                                       \
         }                                                                                        \
-        ls += (l4[0] + l4[1]) + (l4[2] + l4[3]);                                                 \
+        *reinterpret_cast<uint4*>(sm + (tp_) + sw_off(row, (KW / 8) * cpart + c8)) = pack8(o8);  \
       }                                                                                          \
+      ls += (l4[0] + l4[1]) + (l4[2] + l4[3]);                                                   \
     }                                                                                            \
   } while (0)
 // O += P~ (window values of one step)
-#define NHA_ISSUE_PV() NHA_ISSUE_PV_AT(aP, aWV)
 #define NHA_ISSUE_PV_AT(ap_, awv_)                                                               \
   do {                                                                                           \
     _Pragma("unroll") for (int ct = 0; ct < KT; ++ct)                                            \
-      mma_tile(tbase + L::cO + 64 * ct, (ap_), L::kATile, (awv_) + ct * L::kWTile, 0, R, 64, 4 * TP, 1, true); \
+      mma_tile(tbase + L::cO + 64 * ct, (ap_), L::kATile, (awv_) + ct * L::kWTile, 0, R, 64, 4, 1, true); \
   } while (0)
 // combine a row statistic over the NS threads of the row (slot_: exchange point 0..3; OP_: fmaxf or addf);
 // the barrier inside is reached by every thread of the CTA
@@ -362,7 +340,7 @@ __global__ void __launch_bounds__(UmmaLayout<D, R>::kThreads, (D == 64 && R == 6
   } while (0)
   auto addf = [](float x, float y) { return x + y; };
 
-// pipelined loops (D = 128): window step p_ into buffer set set_ (its keys, with wv_ also its values).  A step whose
+// window loops: window step p_ into buffer set set_ (its keys, with wv_ also its values).  A step whose
 // 64 keys lie inside the sequence comes by TMA (one thread, two or four boxes, bytes counted on the set's mbarrier);
 // a step that sticks out of the sequence is copied with zero fill by every thread and then arrives on the same
 // barrier.  Every thread of the CTA runs the macro.  Issue work is spread over three threads of three warps so that
@@ -400,10 +378,10 @@ __global__ void __launch_bounds__(UmmaLayout<D, R>::kThreads, (D == 64 && R == 6
   } while (0)
   uint32_t phases = 0u;                               // parities: bits 0-1 loads, 2-3 S products, 4 P~ V product
 
-  for (int ht = 0; ht < (NG + TH - 1) / TH; ++ht) {
+  for (int ht = 0; ht < NG / TH; ++ht) {
     const int hq0 = h * NG + ht * TH;
     const int hq = hq0 + th;
-    const bool in_seq = pos < NHA_HEAD_ROWS(hq);
+    const bool in_seq = pos < len;
     // visible keys of this row: klo <= key <= pos, tested as (unsigned)(key - klo) <= kspan; a row past the
     // sequence end sees nothing
     const int klo = in_seq ? (wl < 0 ? 0 : max(0, pos - wl)) : (1 << 30);
@@ -446,7 +424,6 @@ __global__ void __launch_bounds__(UmmaLayout<D, R>::kThreads, (D == 64 && R == 6
     float lg = 0.f;
     {
       float l4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
       const float nmg = -mg * kLog2e;
 #pragma unroll
       for (int e = 0; e < CW; ++e) {
@@ -457,7 +434,7 @@ __global__ void __launch_bounds__(UmmaLayout<D, R>::kThreads, (D == 64 && R == 6
     }
     // ---- maxima of the newer window steps (the newest one last: its S stays in TMEM) -----------------------------
     int rset = 0;                                      // buffer set / accumulator that hold the newest step afterwards
-    if constexpr (L::kPipe) {
+    {
       // step index i counts from the oldest step (i = 0: loaded with the head tile, S formed in MMA group 1); step i uses
       // buffer set and accumulator i & 1.  The load of step i + 1 and the maximum of step i - 1 overlap S of step i.
       if (nsteps > 1) NHA_LOAD_STEP(1, nsteps - 2, nsteps - 2 == 0);
@@ -487,19 +464,6 @@ __global__ void __launch_bounds__(UmmaLayout<D, R>::kThreads, (D == 64 && R == 6
         tc_fence_before();
         __syncthreads();
         if (rset) NHA_LOAD_STEP(0, 1, true); else NHA_LOAD_STEP(1, 1, true);
-      }
-    } else {
-      for (int p = nsteps - 2; p >= 0; --p) {
-        tc_fence_before();
-        __syncthreads();
-        load_sw<D, kUThreads>(sm + L::tW, L::kWTile, ksw, (int64_t)H * D, NHA_KBASE(p), 0, len, WK, 0, tid);
-        if (p == 0) load_sw<D, kUThreads>(sm + L::tWV, L::kWTile, vsw, (int64_t)H * D, NHA_KBASE(0), 0, len, WK, 0, tid);
-        cp_commit();
-        cp_wait_all();
-        NHA_SMEM_TO_MMA();
-        if (tid == 0) NHA_ISSUE_S();
-        NHA_MMA_WAIT();
-        NHA_STEP_MAX(NHA_KBASE(p));
       }
     }
     // ---- joint maximum; unnormalised slot probabilities as bf16 A operands -----------------------------------------
@@ -533,7 +497,7 @@ __global__ void __launch_bounds__(UmmaLayout<D, R>::kThreads, (D == 64 && R == 6
       mma_tile(tbase + L::cA, aPA, L::kATile, aSB, 0, R, 64, 4, 0, false);
     }
     float ls = 0.f;
-    if (rset) NHA_STEP_PROB_AT(NHA_KBASE(0), L::cS2, L::tW2); else NHA_STEP_PROB(NHA_KBASE(0));
+    if (rset) NHA_STEP_PROB_AT(NHA_KBASE(0), L::cS2, L::tW2); else NHA_STEP_PROB_AT(NHA_KBASE(0), L::cS, L::tW);
     NHA_MMA_WAIT();
     NHA_TRIL_TO_SMEM(L::cA, L::tAB);
     NHA_SMEM_TO_MMA();
@@ -542,11 +506,11 @@ __global__ void __launch_bounds__(UmmaLayout<D, R>::kThreads, (D == 64 && R == 6
 #pragma unroll
       for (int ct = 0; ct < KT; ++ct)
         mma_tile(tbase + L::cO + 64 * ct, aAB, L::kATile, aV + ct * 8192, 0, R, 64, 4, 1, true);
-      if (rset) NHA_ISSUE_PV_AT(smem_u32(sm + L::tW2), smem_u32(sm + L::tWV2)); else NHA_ISSUE_PV();
+      if (rset) NHA_ISSUE_PV_AT(smem_u32(sm + L::tW2), smem_u32(sm + L::tWV2)); else NHA_ISSUE_PV_AT(aW, aWV);
     }
     NHA_MMA_WAIT();
     // ---- older window steps ------------------------------------------------------------------------------------------------
-    if constexpr (L::kPipe) {
+    {
       // step j (j = 1: the first older one) uses buffer set and accumulator (rset + j) & 1; its load was issued one
       // step ahead, P~ V of step j runs while step j + 1 is prepared
       for (int j = 1; j < nsteps; ++j) {
@@ -573,22 +537,6 @@ __global__ void __launch_bounds__(UmmaLayout<D, R>::kThreads, (D == 64 && R == 6
         }
       }
       if (nsteps > 1) NHA_WAIT_BAR(bpv, 4);
-    } else {
-      for (int p = 1; p < nsteps; ++p) {
-        tc_fence_before();
-        __syncthreads();
-        load_sw<D, kUThreads>(sm + L::tW, L::kWTile, ksw, (int64_t)H * D, NHA_KBASE(p), 0, len, WK, 0, tid);
-        load_sw<D, kUThreads>(sm + L::tWV, L::kWTile, vsw, (int64_t)H * D, NHA_KBASE(p), 0, len, WK, 0, tid);
-        cp_commit();
-        cp_wait_all();
-        NHA_SMEM_TO_MMA();
-        if (tid == 0) NHA_ISSUE_S();
-        NHA_MMA_WAIT();
-        NHA_STEP_PROB(NHA_KBASE(p));
-        NHA_SMEM_TO_MMA();
-        if (tid == 0) NHA_ISSUE_PV();
-        NHA_MMA_WAIT();
-      }
     }
     // ---- row sums of all column parts, normalise and store ----------------------------------------------------------------
     {
@@ -637,11 +585,8 @@ __global__ void __launch_bounds__(UmmaLayout<D, R>::kThreads, (D == 64 && R == 6
 #undef NHA_LOAD_STEP
 #undef NHA_WAIT_BAR
 #undef NHA_STEP_MAX
-#undef NHA_STEP_PROB
-#undef NHA_ISSUE_PV
 #undef NHA_XCHG
 #undef NHA_LOAD_HEAD_TILE
-#undef NHA_HEAD_ROWS
 #undef NHA_KBASE
   if (failed) atomicExch(err, 1);
   cp_wait_all();
@@ -650,24 +595,22 @@ __global__ void __launch_bounds__(UmmaLayout<D, R>::kThreads, (D == 64 && R == 6
   if (warp == 0) tmem_dealloc(tbase, L::kTmemCols);
 }
 
-template <int D, int R>
+template <int R>
 static int launch_umma(const nha_chunk_desc* d, int* flags, int* err, cudaStream_t cs) {
-  typedef UmmaLayout<D, R> L;
-  cudaError_t e = set_max_smem((const void*)nha_fwd_umma_kernel<D, R>, L::total);
+  typedef UmmaLayout<R> L;
+  cudaError_t e = set_max_smem((const void*)nha_fwd_umma_kernel<R>, L::total);
   if (e != cudaSuccess) return record_cuda_error(e);
   WindowMaps maps;
   memset(&maps, 0, sizeof(maps));
-  if (L::kPipe) {
-    const char* off = getenv("NHA_B200_NO_TMA");
-    maps.use = !(off && off[0] == '1') && make_map_rows_heads(&maps.k, d->k_swa, d->Ttot, d->H, D) &&
-               make_map_rows_heads(&maps.v, d->v, d->Ttot, d->H, D);
-  }
+  const char* off = getenv("NHA_B200_NO_TMA");
+  maps.use = !(off && off[0] == '1') && make_map_rows_heads(&maps.k, d->k_swa, d->Ttot, d->H, L::D) &&
+             make_map_rows_heads(&maps.v, d->v, d->Ttot, d->H, L::D);
   const int NCB = (int)nha_chunk_count_bound(d->Ttot, d->N);
-  nha_fwd_umma_kernel<D, R><<<dim3(NCB, d->H), L::kThreads, L::total, cs>>>(*d, flags, err, maps);
+  nha_fwd_umma_kernel<R><<<dim3(NCB, d->H), L::kThreads, L::total, cs>>>(*d, flags, err, maps);
   return check_launch();
 }
 
-// Runs the tensor-memory output pass when the shape has one (K == V in {64, 128}, M == 64, positive
+// Runs the tensor-memory output pass when the shape has one (K == V == 64 and M <= 64, or K == V == 128 and M == 64; positive
 // scale).  Returns NHA_ERR_UNSUPPORTED otherwise.
 bool fwd64_supported(const nha_chunk_desc* d);
 int fwd64_launch(const nha_chunk_desc* d, int* flags, int* err, cudaStream_t cs);
@@ -685,8 +628,8 @@ int chunk_output_pass_umma(const nha_chunk_desc* d, int* flags, int* err, cudaSt
     const int st = fwd_pipe_launch(d, flags, err, cs);
     if (st != NHA_ERR_UNSUPPORTED) return st;
   }
-  if (d->K == 128 && NG == 1) return launch_umma<128, 64>(d, flags, err, cs);
-  if (d->K == 128 && NG % 2 == 0) return launch_umma<128, 128>(d, flags, err, cs);
+  if (d->K == 128 && NG == 1) return launch_umma<64>(d, flags, err, cs);
+  if (d->K == 128 && NG % 2 == 0) return launch_umma<128>(d, flags, err, cs);
   return NHA_ERR_UNSUPPORTED;
 }
 
