@@ -149,28 +149,10 @@ __device__ __forceinline__ void nha_bwd_window_rows_kernel_body(const nha_chunk_
   }
 }
 
-// One CTA walks `cpc` consecutive chunks (1 when the kernel handles every chunk; more when it is launched gated
-// on the chunk flags and most chunks return at once, so that an all-clear launch costs few CTAs).
-__global__ void __launch_bounds__(kBwThreads) nha_bwd_window_rows_kernel(const nha_chunk_desc d, const BwdWs w, const int cpc) {
+__global__ void __launch_bounds__(kBwThreads) nha_bwd_window_rows_kernel(const nha_chunk_desc d, const BwdWs w) {
   grid_dep_wait();
   grid_dep_launch();
-  const int ncb = (int)((d.Ttot + kChunk - 1) / kChunk + d.N);
-  // which of my chunks have work: one flag load per chunk, all at once (cpc <= 32)
-  __shared__ unsigned todo;
-  if (threadIdx.x < 32) {
-    const int cgl = blockIdx.x * cpc + threadIdx.x;
-    const bool mine = (int)threadIdx.x < cpc && cgl < ncb && chunk_gate(w, cgl, blockIdx.y, d.H);
-    const unsigned m = __ballot_sync(0xffffffffu, mine);
-    if (threadIdx.x == 0) todo = m;
-  }
-  __syncthreads();
-  unsigned left = todo;
-  while (left) {
-    const int i = __ffs(left) - 1;
-    left &= left - 1;
-    nha_bwd_window_rows_kernel_body(d, w, blockIdx.x * cpc + i);
-    __syncthreads();
-  }
+  nha_bwd_window_rows_kernel_body(d, w, blockIdx.x);
 }
 
 // ================================================================================================
@@ -616,28 +598,10 @@ __device__ __forceinline__ void nha_bwd_slot_kernel_body(const nha_chunk_desc d,
   }
 }
 
-// One CTA walks `cpc` consecutive chunks (1 when the kernel handles every chunk; more when it is launched gated
-// on the chunk flags and most chunks return at once, so that an all-clear launch costs few CTAs).
-__global__ void __launch_bounds__(kBwThreads) nha_bwd_slot_kernel(const nha_chunk_desc d, const BwdWs w, const int cpc) {
+__global__ void __launch_bounds__(kBwThreads) nha_bwd_slot_kernel(const nha_chunk_desc d, const BwdWs w) {
   grid_dep_wait();
   grid_dep_launch();
-  const int ncb = (int)((d.Ttot + kChunk - 1) / kChunk + d.N);
-  // which of my chunks have work: one flag load per chunk, all at once (cpc <= 32)
-  __shared__ unsigned todo;
-  if (threadIdx.x < 32) {
-    const int cgl = blockIdx.x * cpc + threadIdx.x;
-    const bool mine = (int)threadIdx.x < cpc && cgl < ncb && chunk_gate(w, cgl, blockIdx.y, d.H);
-    const unsigned m = __ballot_sync(0xffffffffu, mine);
-    if (threadIdx.x == 0) todo = m;
-  }
-  __syncthreads();
-  unsigned left = todo;
-  while (left) {
-    const int i = __ffs(left) - 1;
-    left &= left - 1;
-    nha_bwd_slot_kernel_body(d, w, blockIdx.x * cpc + i);
-    __syncthreads();
-  }
+  nha_bwd_slot_kernel_body(d, w, blockIdx.x);
 }
 
 // ================================================================================================
@@ -713,32 +677,15 @@ __device__ __forceinline__ void nha_bwd_local_terms_kernel_body(const nha_chunk_
   for (int i = tid; i < M * V; i += kBwThreads) dv[i] = OV[(i / V) * ldov + (i % V)];
 }
 
-// One CTA walks `cpc` consecutive chunks (1 when the kernel handles every chunk; more when it is launched gated
-// on the chunk flags and most chunks return at once, so that an all-clear launch costs few CTAs).
-__global__ void __launch_bounds__(kBwThreads) nha_bwd_local_terms_kernel(const nha_chunk_desc d, const BwdWs w, const int cpc) {
+__global__ void __launch_bounds__(kBwThreads) nha_bwd_local_terms_kernel(const nha_chunk_desc d, const BwdWs w) {
   grid_dep_wait();
   grid_dep_launch();
-  const int ncb = (int)((d.Ttot + kChunk - 1) / kChunk + d.N);
-  // which of my chunks have work: one flag load per chunk, all at once (cpc <= 32)
-  __shared__ unsigned todo;
-  if (threadIdx.x < 32) {
-    const int cgl = blockIdx.x * cpc + threadIdx.x;
-    const bool mine = (int)threadIdx.x < cpc && cgl < ncb && chunk_gate(w, cgl, blockIdx.y, d.H);
-    const unsigned m = __ballot_sync(0xffffffffu, mine);
-    if (threadIdx.x == 0) todo = m;
-  }
-  __syncthreads();
-  unsigned left = todo;
-  while (left) {
-    const int i = __ffs(left) - 1;
-    left &= left - 1;
-    nha_bwd_local_terms_kernel_body(d, w, blockIdx.x * cpc + i);
-    __syncthreads();
-  }
+  nha_bwd_local_terms_kernel_body(d, w, blockIdx.x);
 }
 
 // The three above in one launch for the chunks that the tensor-core passes leave: each step reads what the one before wrote
 // for the same (chunk, kv head), and with nothing flagged a launch is all that they cost (two launches of 3 us of host time less).
+// One CTA walks `cpc` consecutive chunks, so that an all-clear launch costs few CTAs.
 __global__ void __launch_bounds__(kBwThreads) nha_bwd_flagged_kernel(const nha_chunk_desc d, const BwdWs w, const int cpc) {
   grid_dep_wait();
   grid_dep_launch();
@@ -1144,7 +1091,7 @@ static int bwd_run(const nha_chunk_desc* d, int stage_mask, void* stream) {
       if (st != NHA_OK) return st;
     }
     if (umma) launch_after(nha_bwd_flagged_kernel, ggrid, block, flagged_smem, cs, *d, wg, cpc);
-    else launch_after(nha_bwd_window_rows_kernel, grid, block, L1.total, cs, *d, wg, 1);
+    else launch_after(nha_bwd_window_rows_kernel, grid, block, L1.total, cs, *d, wg);
     st = check_launch();
     if (st != NHA_OK) return st;
   }
@@ -1160,13 +1107,13 @@ static int bwd_run(const nha_chunk_desc* d, int stage_mask, void* stream) {
     if (st != NHA_OK) return st;
   }
   if ((stage_mask & 4) && !umma) {
-    launch_after(nha_bwd_slot_kernel, grid, block, L3.total, cs, *d, wg, 1);
+    launch_after(nha_bwd_slot_kernel, grid, block, L3.total, cs, *d, wg);
     st = check_launch();
     if (st != NHA_OK) return st;
   }
   if (stage_mask & 8) {
     if (!umma) {
-      launch_after(nha_bwd_local_terms_kernel, grid, block, L5.total, cs, *d, wg, 1);
+      launch_after(nha_bwd_local_terms_kernel, grid, block, L5.total, cs, *d, wg);
       st = check_launch();
       if (st != NHA_OK) return st;
     }
