@@ -72,14 +72,14 @@ int nha_abi_version(void);
  *   workspace  scratch of nha_decode_workspace_bytes(B, HQ, H, V, W) bytes, needed when W > 64
  *            (a (sequence, kv head) is then split over several CTAs whose partial softmaxes are
  *            merged by the last one to finish).  Its first B*H int32 are arrival counters, the next
- *            int32 is a device error word (nha_decode_device_error): they must be zero before the
- *            first call and every call leaves the counters zero, so one zero-initialised buffer can
+ *            int32 is the word of nha_decode_device_error: they must be zero before the
+ *            first call and every call leaves them zero, so one zero-initialised buffer can
  *            be reused by all calls with the same B*H that do not overlap on the GPU.  May be NULL
  *            for W <= 64 (M > 64 then takes the general kernel).
- * K == V in {64, 128} with window keys takes a streaming kernel (ring of asynchronous copies, whole
+ * K == V in {64, 128} with window keys takes a streaming kernel (rings of asynchronous copies, whole
  * grid resident in one wave; 2, 4 or 8 splits run as a thread-block cluster and merge through shared
- * memory without touching the workspace, which must be passed all the same); other shapes and the
- * win_logits mode take the general kernel.
+ * memory without touching the workspace, which must be passed all the same); the win_logits mode with 64 slots
+ * and K == V in {64, 128} takes a kernel that holds the state in registers; other shapes take the general kernel.
  */
 int64_t nha_decode_workspace_bytes(int B, int HQ, int H, int V, int W);
 int nha_decode_step(const void* q, const void* sq, const void* k, const void* v, const void* g, const void* s,
@@ -104,15 +104,15 @@ int nha_decode_step_bf16_state(const void* q, const void* sq, const void* k, con
  *   0  plain launches.
  *   1  (default; NHA_PDL unset or "1") the kernel may be scheduled while the kernel in front of it on the stream is
  *      still draining and waits for that kernel before its first global read: always safe, hides the launch gap.
- *   2  as 1, and the slot memory (hk, hv) and the window (sw_k / sw_v, or the rings and head) of the call are
- *      requested BEFORE the wait; q, the popped or new token and the gates are read after it.  Only for callers who
+ *   2  as 1, and the first loads of the window (sw_k / sw_v, or the rings and head) of the call go out BEFORE the
+ *      wait; everything else is read after it.  Only for callers who
  *      know that the kernel immediately in front on the stream writes neither this call's slot memory nor its window
  *      (a stack of layers with one cache per layer: the kernel in front works on another layer, or is a projection).
  * The mode is process-wide; NHA_PDL ("0", "1", "2") gives the initial value. */
 int nha_decode_set_pdl(int mode);
 int nha_decode_get_pdl(void);
-/* reads the workspace's device error word (synchronises the stream): non-zero when a bounded wait
-   inside the streaming decode kernel ran out.  No counterpart in the reference. */
+/* reads the workspace's device error word (synchronises the stream).  Always 0: the decode kernels have no wait that
+   could run out.  Kept for callers that ask.  No counterpart in the reference. */
 int nha_decode_device_error(const void* workspace, int B, int H, void* stream);
 
 /* Decode on a device-resident ring buffer (the rolling window of the reference's NHACache,

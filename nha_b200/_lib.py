@@ -181,14 +181,6 @@ def check_chunk_device(lib, desc, stream, what: str):
                                   f'the outputs of this call are invalid)')
 
 
-def check_decode_device(lib, ws, B, H, stream, what: str):
-    if ws is not None and check_device_words():
-        e = lib.nha_decode_device_error(ws.data_ptr(), B, H, stream)
-        if e != 0:
-            raise NHALibraryError(f'{what}: device error word {e} (a bounded wait in the decode kernel ran out; '
-                                  f'the outputs of this call are invalid)')
-
-
 def ptr(t):
     """Device pointer of a tensor (or NULL for None)."""
     return None if t is None else t.data_ptr()

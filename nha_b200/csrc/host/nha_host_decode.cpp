@@ -20,14 +20,6 @@ Tensor decode_workspace(const Tensor& like, int B, int HQ, int H, int V, int W) 
   return ws;
 }
 
-static void check_device(const Tensor& ws, int B, int H, void* stream, const char* what) {
-  if (!ws.defined() || !check_device_words()) return;
-  const int e = nha_decode_device_error(ws.data_ptr(), B, H, stream);
-  if (e != 0)
-    raise(library_error, std::string(what) + ": device error word " + std::to_string(e) +
-                             " (a bounded wait in the decode kernel ran out; the outputs of this call are invalid)");
-}
-
 static void check_state(const Tensor& hk0, const Tensor& hv0, int64_t B, int64_t H, int64_t K, int64_t V, int64_t M) {
   if (hk0.defined() && (hk0.sizes() != at::IntArrayRef({B, H, K, M}) || hv0.sizes() != at::IntArrayRef({B, H, M, V})))
     raise(PyExc_AssertionError, "initial_state must be ([B,H,K,M], [B,H,M,V]) at the kv-head count " + std::to_string(H) + ", got " +
@@ -151,7 +143,6 @@ NHA_METHOD(decode) {
                             cp, sp, cs_batch, cs_row, nullptr, (float*)st.hk.data_ptr(), (float*)st.hv.data_ptr(), st.zero, o.data_ptr(),
                             nullptr, ptr(ws), wsb, B, HQ, H, K, V, M, W, (float)scale, stream),
             "nha_decode_step");
-    check_device(ws, B, H, stream, "nha_decode_step");
     if (q.scalar_type() != at::kBFloat16) o = o.to(q.scalar_type());
     st.done(hk, hv);
   }
@@ -279,7 +270,6 @@ NHA_METHOD(decode_ring) {
                             (int32_t*)head.data_ptr(), B, H, K, V, M, W, fill, stream),
             "nha_ring_append");
     }
-    check_device(ws, B, H, stream, "nha_decode_step_ring");
   }
   return wrap(o);
   NHA_END

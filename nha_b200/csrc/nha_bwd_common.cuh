@@ -14,15 +14,15 @@ struct BwdWs {
   float* dvp;     // [Ttot, H, V]    intra-chunk part of dv'
   float* dsp;     // [Ttot, H, M]    intra-chunk part of ds'
   float* dga;     // [Ttot, H, M]    ok .* dz + p .* dp summed over the group
-  bf16* dzg;      // [Ttot, HQ, M]   scale * dz_slot .* exp(G)   (general kernels; the tensor-memory rows pass keeps it on chip)
-  bf16* pgq;      // [Ttot, HQ, M]   p_slot .* exp(G)            (general kernels, and the two-heads-per-tile rows pass)
+  bf16* dzg;      // [Ttot, HQ, M]   scale * dz_slot .* exp(G)   (general kernels; the tensor-core rows passes keep both on chip)
+  bf16* pgq;      // [Ttot, HQ, M]   p_slot .* exp(G)
   float* dkc;     // [NC, H, K, M]   first the chunk's own term q^T (scale dz exp G), then (after the scan)
                   //                 the gradient of hk at the END of the chunk
   float* dvc;     // [NC, H, M, V]   likewise (p exp G)^T do, then the gradient of hv at the chunk end
   float* gend;    // [NC, H, M]      total shifted log gate of each chunk
-  bf16* dza;      // [Ttot, HQ, M]   scale * dz_slot .* a   (tensor-memory path only)
-  bf16* paq;      // [Ttot, HQ, M]   p_slot .* a            (tensor-memory path only)
-  bf16* dkb;      // [NC, H, K, M]   bf16 copy of the scanned dkc (tensor-memory path only)
+  bf16* dza;      // [Ttot, HQ, M]   scale * dz_slot .* a   (tensor-core path only)
+  bf16* paq;      // [Ttot, HQ, M]   p_slot .* a            (tensor-core path only)
+  bf16* dkb;      // [NC, H, K, M]   bf16 copy of the scanned dkc (tensor-core path at head dim 128 only, like the next two)
   bf16* dvb;      // [NC, H, M, V]   bf16 copy of the scanned dvc
   float* gcarry;  // [NC, H, M]      gate-gradient carry of all later chunks
   const int* flags;   // [NC, H] chunks the tensor-memory forward left to the general kernels, or NULL

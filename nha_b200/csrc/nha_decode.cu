@@ -452,7 +452,7 @@ void decode_set_pdl_mode(int m);
 bool decode_stream_supported(int K, int V, int M, int W, int NG, bool logits_mode);
 int decode_stream_try(const void* q, const void* sq, const void* k, const void* v, const void* g, const void* s,
                       const void* sw_k, const void* sw_v, const void* cosp, const void* sinp, int64_t cs_batch,
-                      int64_t cs_row, float* hk, float* hv, int zero_state, void* o, int* tickets, int* err,
+                      int64_t cs_row, float* hk, float* hv, int zero_state, void* o, int* tickets,
                       float* part_ml, float* part_o, int splits, int B, int HQ, int H, int D, int M, int W, float scale,
                       cudaStream_t st, const int* head, const void* ring_g, int ring_rows, int nopop,
                       const void* ring_kraw, const void* g_new, int state_bf16);
@@ -467,8 +467,8 @@ static bool aligned16(std::initializer_list<const void*> p) {
 bool decode_logits_supported(const DecodeArgs& a);
 int decode_logits_launch(const DecodeArgs& a, cudaStream_t cs);
 
-// Workspace: [B*H tickets | error word] (ints, zero between calls), then the (max, sum) and the partial outputs of
-// every split.  Sized for whichever kernel cuts a (sequence, kv head) into more splits.
+// Workspace: [B*H tickets | one word that stays zero] (ints, zero between calls), then the (max, sum) and the partial
+// outputs of every split.  Sized for whichever kernel cuts a (sequence, kv head) into more splits.
 static int decode_max_splits(int B, int H, int W) {
   const int a = decode_splits(W, false), b = decode_stream_splits(B, H, W, 1 << 20);
   const int c = a > b ? a : b;
@@ -527,7 +527,7 @@ static int decode_step_impl(const void* q, const void* sq, const void* k, const 
   a.hk = hk; a.hv = hv; a.o = (bf16*)o; a.win_prob = win_prob;
   a.cs_batch = cs_batch; a.cs_row = cs_row;
   a.B = B; a.HQ = HQ; a.H = H; a.K = K; a.V = V; a.M = M; a.W = W; a.NG = NG;
-  // common shapes take the streaming kernel (ring of bulk copies, whole grid resident in one wave)
+  // common shapes take the streaming kernel (warps with rings of their own, whole grid resident in one wave)
   const char* force_general = getenv("NHA_B200_DECODE_GENERAL");
   const bool stream_ok = decode_stream_supported(K, V, M, W, NG, logits_mode) && !(force_general && force_general[0] == '1') &&
                          (M <= 64 || workspace);                  // more than 64 slots are split, and splits may merge through it
@@ -544,13 +544,11 @@ static int decode_step_impl(const void* q, const void* sq, const void* k, const 
   a.MQ = align_up((M + a.SPLITS - 1) / a.SPLITS, 4);
   a.zero_state = zero_state; a.scale = scale;
   a.part_o = nullptr; a.part_ml = nullptr; a.tickets = nullptr;
-  int* errw = nullptr;
   if (a.SPLITS > 1 || stream_ok) {
     if (a.SPLITS > 1 && (!workspace || workspace_bytes < nha_decode_workspace_bytes(B, HQ, H, V, W))) return NHA_ERR_WORKSPACE;
     if (workspace && workspace_bytes >= nha_decode_workspace_bytes(B, HQ, H, V, W)) {
-      // tickets and the error word first (they must stay zero between calls), then the partials
+      // tickets first (they must stay zero between calls), then the partials
       a.tickets = (int*)workspace;
-      errw = a.tickets + (size_t)B * H;
       char* base = (char*)workspace + align_up((B * H + 1) * 4, 256);
       a.part_ml = (float*)base;
       a.part_o = (float*)(base + align_up(B * H * a.SPLITS * NG * 2 * 4, 256));
@@ -558,7 +556,7 @@ static int decode_step_impl(const void* q, const void* sq, const void* k, const 
   }
   if (stream_ok)
     return decode_stream_try(q, sq, k, v, g, s, sw_k, sw_v, cosp, sinp, cs_batch, cs_row, hk, hv, zero_state, o, a.tickets,
-                             errw, a.part_ml, a.part_o, a.SPLITS, B, HQ, H, K, M, W, scale, (cudaStream_t)stream, nullptr,
+                             a.part_ml, a.part_o, a.SPLITS, B, HQ, H, K, M, W, scale, (cudaStream_t)stream, nullptr,
                              nullptr, W, 0, nullptr, nullptr, state_bf16);
   if (decode_logits_supported(a) && !(force_general && force_general[0] == '1')) return decode_logits_launch(a, (cudaStream_t)stream);
   const int smem = decode_layout(a);
@@ -637,12 +635,11 @@ extern "C" int nha_decode_step_ring(const void* q, const void* k_new, const void
   const int splits = decode_stream_splits(B, H, Weff, M);
   if (!workspace || workspace_bytes < nha_decode_workspace_bytes(B, HQ, H, V, W)) return NHA_ERR_WORKSPACE;
   int* tickets = (int*)workspace;
-  int* errw = tickets + (size_t)B * H;
   char* base = (char*)workspace + align_up((B * H + 1) * 4, 256);
   float* part_ml = (float*)base;
   float* part_o = (float*)(base + align_up(B * H * splits * NG * 2 * 4, 256));
   return decode_stream_try(q, nullptr, k_new, v_new, nullptr, nullptr, ring_k, ring_v, cosp, sinp, cs_batch, cs_row, hk, hv, 0,
-                           o, tickets, errw, part_ml, part_o, splits, B, HQ, H, K, M, Weff, scale, (cudaStream_t)stream, head,
+                           o, tickets, part_ml, part_o, splits, B, HQ, H, K, M, Weff, scale, (cudaStream_t)stream, head,
                            ring_g, W, nopop, nullptr, nullptr, 0);
 }
 
@@ -661,12 +658,11 @@ extern "C" int nha_decode_step_ring_fused(const void* q, const void* k_new, cons
   const int splits = decode_stream_splits(B, H, Weff, M);
   if (!workspace || workspace_bytes < nha_decode_workspace_bytes(B, HQ, H, V, W)) return NHA_ERR_WORKSPACE;
   int* tickets = (int*)workspace;
-  int* errw = tickets + (size_t)B * H;
   char* base = (char*)workspace + align_up((B * H + 1) * 4, 256);
   float* part_ml = (float*)base;
   float* part_o = (float*)(base + align_up(B * H * splits * NG * 2 * 4, 256));
   return decode_stream_try(q, nullptr, k_new, v_new, nullptr, nullptr, ring_k, ring_v, cosp, sinp, cs_batch, cs_row, hk, hv, 0,
-                           o, tickets, errw, part_ml, part_o, splits, B, HQ, H, K, M, Weff, scale, (cudaStream_t)stream, head,
+                           o, tickets, part_ml, part_o, splits, B, HQ, H, K, M, Weff, scale, (cudaStream_t)stream, head,
                            ring_g, W, nopop, nullptr, g_new, 0);
 }
 
@@ -777,14 +773,13 @@ extern "C" int nha_decode_step_ring_rot(const void* q, const void* k_new, const 
   const int splits = decode_stream_splits(B, H, Weff, M);
   if (!workspace || workspace_bytes < nha_decode_workspace_bytes(B, HQ, H, V, W)) return NHA_ERR_WORKSPACE;
   int* tickets = (int*)workspace;
-  int* errw = tickets + (size_t)B * H;
   char* base = (char*)workspace + align_up((B * H + 1) * (int)sizeof(int), 256);
   float* part_ml = (float*)base;
   float* part_o = (float*)(base + align_up(B * H * splits * NG * 2 * 4, 256));
   // a table row stride of 0: every window position reads the query's row; the kernel rotates only the query and the
   // token of this step
   return decode_stream_try(q, nullptr, k_new, v_new, nullptr, nullptr, ring_kr, ring_v, cos_q, sin_q, cs_batch, 0, hk, hv, 0,
-                           o, tickets, errw, part_ml, part_o, splits, B, HQ, H, K, M, Weff, scale, (cudaStream_t)stream, head,
+                           o, tickets, part_ml, part_o, splits, B, HQ, H, K, M, Weff, scale, (cudaStream_t)stream, head,
                            ring_g, W, nopop, ring_k, nullptr, 0);
 }
 

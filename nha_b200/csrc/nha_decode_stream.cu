@@ -55,7 +55,6 @@ struct DecodeStreamArgs {
   float* part_o;      // [B*H, SPLITS, NG, V] unnormalised partial outputs
   float* part_ml;     // [B*H, SPLITS, NG, 2] maximum and sum of each split
   int* tickets;       // [B*H] arrival counters, zero between calls
-  int* err;           // device error word (a bounded wait ran out)
   // ring mode (head != NULL): sw_k / sw_v are rings of W physical rows per sequence whose oldest entry sits at
   // row head[b]; that entry is the token that leaves the window and enters the slot memory in this step (its
   // gate row comes from ring_g, the popped k / v from the rings), the token of this step (k, v: not yet in the
@@ -80,8 +79,9 @@ struct DecodeStreamArgs {
   int B, HQ, H, M, W, NG, SPLITS, KSPL, MQ, zero_state;
   int cluster;        // 1: the SPLITS CTAs of a (sequence, kv head) form a thread-block cluster and merge through shared memory
   // programmatic dependent launch: 0 = plain launch; 1 = the grid may be scheduled before the kernel in front of it on
-  // the stream has finished and waits for it before its first global read; 2 = as 1, but the slot memory and the
-  // window of this call are requested BEFORE that wait (the caller asserts that the kernel in front writes neither)
+  // the stream has finished and waits for it before its first global read (it only prefetches into L2 before that); 2 = as 1,
+  // but the first window loads of this call go out BEFORE that wait (the caller asserts that the kernel in front writes
+  // neither the window nor the slot memory)
   int pdl;
   float scale;
   int off_ring, off_q, off_sqA, off_p, off_eg, off_sv, off_kpop, off_vpop, off_wml, off_ml, off_out;
@@ -129,9 +129,6 @@ __device__ __forceinline__ float2 ld_cluster_f2(uint32_t addr) {
   asm volatile("ld.shared::cluster.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
   return v;
 }
-
-// programmatic dependent launch: wait until the grids this one depends on have completed and their writes are
-// visible; let the grid behind this one on the stream be scheduled
 
 // start of a 16-byte aligned range into L2
 __device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
@@ -289,7 +286,7 @@ __global__ void __launch_bounds__(kStrThreads, NT == 1 ? 2 : 1) nha_decode_strea
     __syncwarp();                                                  // every lane's copies have landed
   };
 
-  // ---- requests: the small inputs, the first task's slot memory into registers, the first window loads ------------------
+  // ---- requests: the small inputs and the first window loads (the slot memory comes last, behind the window) -------------
   // hk of a task: lane -> slots 4 (lane & 1) .. + 3 of the eight, rows 16 i + lane / 2; hv: rows (slots) kRowsI u + lane / V4
   constexpr int kHk = K / 16, kHv = kGroup / kRowsI;
   const int hs = 4 * (lane & 1), hr = lane >> 1;
@@ -306,8 +303,8 @@ __global__ void __launch_bounds__(kStrThreads, NT == 1 ? 2 : 1) nha_decode_strea
       vreg[u] = !a.zero_state && ms + kRowsI * u + vsub < nslots
                     ? ld_state4<SB16>(a.hv, ((size_t)bh * M + m0 + ms + kRowsI * u + vsub) * V + vcol) : make_float4(0.f, 0.f, 0.f, 0.f);
   };
-  // Dependent launch with early requests (pdl == 2): the state and the window of this call do not depend on the
-  // kernel in front, so they go in flight before the wait.  In ring mode the newest window entry is the token of
+  // Dependent launch with early requests (pdl == 2): the window of this call does not depend on the kernel in front, so its
+  // first loads go out before the wait.  In ring mode the newest window entry is the token of
   // this step (a.k / a.v, written by the caller's projections): the loads from the first one that holds it on
   // are issued after the wait, in the same order as always.
   int npre = 0;                                                    // groups requested before the wait
@@ -942,7 +939,7 @@ int decode_stream_launch(const DecodeStreamArgs& in, int D, cudaStream_t st) {
 // Runs the streaming kernel when the shape has one; *used tells the caller whether it did.
 int decode_stream_try(const void* q, const void* sq, const void* k, const void* v, const void* g, const void* s,
                       const void* sw_k, const void* sw_v, const void* cosp, const void* sinp, int64_t cs_batch,
-                      int64_t cs_row, float* hk, float* hv, int zero_state, void* o, int* tickets, int* err,
+                      int64_t cs_row, float* hk, float* hv, int zero_state, void* o, int* tickets,
                       float* part_ml, float* part_o, int splits, int B, int HQ, int H, int D, int M, int W, float scale,
                       cudaStream_t st, const int* head, const void* ring_g, int ring_rows, int nopop,
                       const void* ring_kraw, const void* g_new, int state_bf16) {
@@ -951,7 +948,7 @@ int decode_stream_try(const void* q, const void* sq, const void* k, const void* 
   a.s = (const bf16*)s; a.sw_k = (const bf16*)sw_k; a.sw_v = (const bf16*)sw_v; a.cosp = (const bf16*)cosp;
   a.sinp = (const bf16*)sinp;
   a.hk = hk; a.hv = hv; a.o = (bf16*)o;
-  a.part_o = part_o; a.part_ml = part_ml; a.tickets = tickets; a.err = err;
+  a.part_o = part_o; a.part_ml = part_ml; a.tickets = tickets;
   a.head = head; a.ring_g = (const bf16*)ring_g;
   a.WR = head ? ring_rows : W; a.nopop = head ? nopop : 0;
   a.ring_kraw = head ? (const bf16*)ring_kraw : nullptr;

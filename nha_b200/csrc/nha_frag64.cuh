@@ -1,4 +1,5 @@
-// Building blocks of the chunk kernels for head dim 64 and one query head per kv head: 64-row products.
+// Building blocks of the chunk kernels with 64-row products: all of them at head dim 64, the query-row and window-key passes of the
+// backward at head dim 128.
 //
 // The accumulator of a product with M = 64 fills only the first 16 lanes of each tensor-memory quarter, so a warp that reads
 // it with one row per lane leaves half of its lanes without work.  These kernels read it with tcgen05.ld.16x256b, which spreads

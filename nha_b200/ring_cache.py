@@ -198,7 +198,6 @@ def _decode_ring_rot(q, k, v, g, layer: RingLayer, cos, sin, scale) -> torch.Ten
                                            layer.ring_g.data_ptr(), kc.data_ptr(), vc.data_ptr(), gc.data_ptr(),
                                            cosq.data_ptr(), sinq.data_ptr(), cs_batch, layer.head.data_ptr(), B, H, K, V,
                                            M, W, fill, st), 'nha_ring_append_rot')
-        _lib.check_decode_device(lib, ws, B, H, st, 'nha_decode_step_ring_rot')
     layer.fill = min(fill + 1, W)
     return o
 

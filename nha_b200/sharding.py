@@ -173,7 +173,8 @@ class CudaEngine:
         K, V, M = k_e.shape[-1], v_e.shape[-1], s_e.shape[-1]
         NG = q.shape[2] // k_e.shape[2]
         self.dims = (k_e.shape[2], K, M, V)
-        # the three-step path needs the pipelined output pass (it alone knows late-starting queries)
+        # the three-step path needs the pipelined output pass (it alone knows late-starting queries); that pass takes any
+        # group, but the path has been run on even groups only, and odd ones keep the older route
         self.steps = None
         if B == 1 and K == 128 and V == 128 and M == 64 and NG % 2 == 0 and q_offset % 64 == 0:
             f = lambda x: x[0].to(_BF16).contiguous()
