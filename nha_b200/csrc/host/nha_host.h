@@ -147,7 +147,7 @@ NHA_METHOD(silu_rms_norm);
 NHA_METHOD(gsa_aux_loss);
 
 // Zero-initialised scratch of the split decode kernels, one per (device, stream, B * H): the kernels leave their counters
-// at zero, so later calls on the same stream use it again (the layout depends on B * H).
+// at zero, so later calls on the same stream use it again (the layout depends on B * H).  A bounded number is kept.
 Tensor decode_workspace(const Tensor& like, int B, int HQ, int H, int V, int W);
 
 }  // namespace nha_host

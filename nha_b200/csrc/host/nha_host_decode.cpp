@@ -10,13 +10,36 @@
 namespace nha_host {
 
 Tensor decode_workspace(const Tensor& like, int B, int HQ, int H, int V, int W) {
+  struct Entry {
+    Tensor t;
+    unsigned long long capture = 0, used = 0;                  // the capture it was made in (0: none); when it was last asked for
+  };
+  constexpr size_t kMost = 64;                                 // buffers kept; a server's batch sizes come and go
   static std::mutex mu;
-  static std::map<std::tuple<int, void*, int64_t>, Tensor>& pool = *new std::map<std::tuple<int, void*, int64_t>, Tensor>();
+  static std::map<std::tuple<int, void*, int64_t>, Entry>& pool = *new std::map<std::tuple<int, void*, int64_t>, Entry>();
+  static unsigned long long now = 0;
   const int64_t need = nha_decode_workspace_bytes(B, HQ, H, V, W);
-  const auto key = std::make_tuple((int)like.device().index(), stream_of(like), (int64_t)B * H);
+  void* stream = stream_of(like);
+  // A graph keeps the address that it was captured with, so a capture has a buffer of its own: it lies in the graph's memory, which
+  // stays with the graph when the buffer leaves this pool, and each replay zeroes it.
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamGetCaptureInfo((cudaStream_t)stream, &status, &id) != cudaSuccess) (void)cudaGetLastError();
+  if (status != cudaStreamCaptureStatusActive) id = 0;
   std::lock_guard<std::mutex> lock(mu);
-  Tensor& ws = pool[key];
-  if (!ws.defined() || ws.numel() < need) ws = zeros({need}, at::kByte, like);
+  Entry& e = pool[std::make_tuple((int)like.device().index(), stream, (int64_t)B * H)];
+  if (!e.t.defined() || e.t.numel() < need || e.capture != id) {
+    e.t = zeros({need}, at::kByte, like);
+    e.capture = id;
+  }
+  e.used = ++now;
+  const Tensor ws = e.t;
+  if (pool.size() > kMost) {                                   // memory goes back in the order of its stream
+    auto oldest = pool.begin();
+    for (auto it = pool.begin(); it != pool.end(); ++it)
+      if (it->second.used < oldest->second.used) oldest = it;
+    pool.erase(oldest);
+  }
   return ws;
 }
 

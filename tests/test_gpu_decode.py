@@ -391,3 +391,44 @@ def test_the_rounding_of_the_window_weights(K, H, NG, W, bound):
     o, _ = fused_recurrent_nha_decode(*(d[n].cuda() for n in names), cos=d['cos'].cuda(), sin=d['sin'].cuda(),
                                       initial_state=(d['hk0'].cuda(), d['hv0'].cuda()))
     assert orc.rel_l2(o.cpu(), want) < bound
+
+
+def _steps(seed, B, HQ, H, K, W):
+    d = {n: x.cuda() if torch.is_tensor(x) else x for n, x in gen.decode_inputs(seed, B, H, HQ // H, K, K, 16, W).items()}
+    names = ('q', 'k', 'v', 'g', 'sw_k_raw', 'vw')
+    from nha_b200 import fused_recurrent_nha_decode
+    return lambda: fused_recurrent_nha_decode(*(d[n] for n in names), cos=d['cos'], sin=d['sin'], initial_state=(d['hk0'], d['hv0']))[0]
+
+
+def test_a_captured_step_keeps_its_workspace():
+    # several splits that merge through the workspace; after the capture the same stream needs a larger one for the same B * H, and what
+    # the first one would have freed is written over
+    small, large = _steps(1, 2, 4, 2, 32, 300), _steps(2, 2, 8, 2, 96, 1000)
+    want = small()
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        small()
+        g = torch.cuda.CUDAGraph()
+        g.capture_begin()
+        o = small()
+        g.capture_end()
+        large()
+        junk = [torch.full((n,), 0x7f7f7f7f, dtype=torch.int32, device='cuda') for n in (64, 256, 1024, 4096, 16384) for _ in range(8)]
+        for _ in range(3):
+            o.zero_()
+            g.replay()
+            assert torch.equal(o, want)
+        assert all(bool((t == 0x7f7f7f7f).all()) for t in junk)
+        small()
+    torch.cuda.synchronize()
+
+
+def test_workspaces_do_not_pile_up():
+    used = []
+    for B in range(1, 161):
+        _steps(3, B, 1, 1, 32, 80)()
+        if B in (80, 160):
+            torch.cuda.synchronize()
+            used.append(torch.cuda.memory_allocated())
+    # a workspace of two splits is 276 B + 1 KB bytes: the 80 added last would be 2.7 MB, the 64 kept are 1.4 MB more than the 64 before
+    assert used[1] - used[0] < 2_100_000
