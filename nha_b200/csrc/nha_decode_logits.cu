@@ -150,8 +150,11 @@ __global__ void __launch_bounds__(kLogThreads, D == 64 ? 3 : 2) nha_decode_logit
 
 static int logits_smem(int D, int NG, int W) { return (kLogWarps * (D > 64 ? D : 64) + 64 + NG * (64 + W)) * 4; }
 
-// Faster than the general kernel wherever measured, up to eight heads a group; larger groups, whose heads each cost two block
-// barriers here, are left to it.  Vectors of eight bytes are loaded from v, s and g.
+// Up to eight heads a group, whose heads each cost two block barriers here; larger groups have not been measured and stay with the
+// general kernel.  A CTA per (sequence, kv head) pays from the smallest grid on, kernel time against the general kernel's, windows of
+// 32 and 512 logits: one head of 64, 1 sequence 2.8 / 6.4 and 3.6 / 7.1 us; 16 heads of 64, 4 sequences 3.2 / 6.7 and 3.7 / 7.4, 64
+// sequences 10.5 / 26.9 and 12.6 / 30.2; 32 heads of 128 on 4, 1 sequence 6.8 / 18.4 and 7.5 / 20.9, 64 sequences 9.6 / 29.1 and
+// 10.6 / 41.1.  Vectors of eight bytes are loaded from v, s and g.
 bool decode_logits_supported(const DecodeArgs& a) {
   const uintptr_t al8 = (uintptr_t)a.v | (uintptr_t)a.s | (uintptr_t)a.g, al16 = (uintptr_t)a.hk | (uintptr_t)a.hv;
   return a.win_logits && a.K == a.V && (a.K == 64 || a.K == 128) && a.M == 64 && a.NG <= 8 && logits_smem(a.K, a.NG, a.W) <= 48 * 1024 &&

@@ -88,3 +88,20 @@ def test_a_single_window_key_gives_its_logit_exactly():
     d['q_swa'], d['k_swa'] = q.bfloat16(), k.bfloat16()
     lse = chunk_nha(*(d[n].cuda() for n in NAMES), window_size_left=0, window_size_right=0)[1]
     assert torch.equal(lse.cpu(), (q * k).sum(-1).float() / 8)
+
+
+@pytest.mark.parametrize('M', [32, 64])
+@pytest.mark.parametrize('D,wl,shift', [(64, 64, 0), (64, 63, 64), (128, 127, 128)])
+def test_gradients_at_the_gates_of_training(M, D, wl, shift):
+    # gate logits ~ N(0, 1) undivided.  The gradient of the gates is a difference of large terms: 1.9e-2 to 2.1e-2 from 64 bits on the
+    # tensor-core and on the general kernels alike (16 inputs each); the others stay below 6e-3
+    from nha_b200 import chunk_nha
+    d = gen.layer_inputs(94 + M, 1, 300, 4, 4, D, D, M, gate_div=1.0)
+    xs = [d[n].double()[0].requires_grad_(True) for n in NAMES]
+    y = dict(zip(NAMES, xs))
+    o = orc.nha_sequence(y['q_gsa'], y['q_swa'], y['k_gsa'], y['k_swa'], y['v'], y['s'], y['g'], D ** -0.5, wl, shift)[0]
+    want = torch.autograd.grad(o, xs, d['do'].double()[0])
+    x = [d[n].cuda().requires_grad_(True) for n in NAMES]
+    got = torch.autograd.grad(chunk_nha(*x, window_size_left=wl, window_size_right=0, gsa_kv_shift=shift)[0], x, d['do'].cuda())
+    for n, a, b in zip(NAMES, got, want):
+        assert_close(a[0], b, 2.6e-2 if n == 'g' else 8e-3, n)
