@@ -796,8 +796,8 @@ def main():
     e, f = 2, 4
     st = 2 * D * M / 64
     per_tok = {
-        # k', v, s, g in; per-chunk terms out (fp32) and back in; chunk-start states out (bf16)
-        'state_pass': H * ((2 * D + 2 * M) * e + st * (2 * f + e)),
+        # k', v, s, g in; per-chunk terms out and back in; chunk-start states out (all bf16)
+        'state_pass': H * ((2 * D + 2 * M) * e + st * 3 * e),
         # q_gsa, q_swa, k_gsa, k_swa, v, s, g, states in; o and both log-sum-exps out
         'output_pass': H * ((5 * D + 2 * M) * e + st * e + D * e + 2 * f),
         # q_gsa, q_swa, do, o, k_gsa, k_swa, v, s, g, states, log-sum-exps in; dq_gsa, dq_swa, delta, joint LSE,
@@ -808,9 +808,9 @@ def main():
         # general kernel of the slot branch: runs only on chunks flagged by the forward (none here)
         # in-place scan of the chunks' fp32 state-gradient terms
         'bwd_state_scan': H * (st * 2 * f),
-        # gate carry (fp32 state gradients and next states in, bf16 copies out), columns pass (q_gsa, do, k_gsa, v,
-        # s, g, dz / p copies, bf16 state gradients, gate terms, window dv in; dk_gsa, dv, ds, dg out)
-        'bwd_cols': H * (st * (f + 2 * e) + (4 * D + 4 * M) * e + st * e + M * f + D * f + (2 * D + 2 * M) * e),
+        # fp32 state gradients, next states, q_gsa, do, k_gsa, v, s, g, dz / p copies, gate terms, window dv in;
+        # dk_gsa, dv, ds, dg out
+        'bwd_cols': H * (st * (f + e) + (4 * D + 4 * M) * e + M * f + D * f + (2 * D + 2 * M) * e),
     }
     for name, fn in calls.items():
         for _ in range(3):
