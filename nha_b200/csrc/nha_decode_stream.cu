@@ -575,8 +575,11 @@ __global__ void __launch_bounds__(kStrThreads, NT == 1 ? 2 : 1) nha_decode_strea
         hreg[i].y = fmaf(hreg[i].y, e4.y, __fmul_rn(kk, s4.y));
         hreg[i].z = fmaf(hreg[i].z, e4.z, __fmul_rn(kk, s4.z));
         hreg[i].w = fmaf(hreg[i].w, e4.w, __fmul_rn(kk, s4.w));
-        if (ms + hs < nslots) st_state4<SB16>(a.hk, ((size_t)bh * K + 16 * i + hr) * M + m0 + ms + hs, hreg[i]);
       }
+      // (stores behind the updates: between them, 4 sequences, 32 heads on 8, W 128 take 9.2 us a layer and not 8.6)
+#pragma unroll
+      for (int i = 0; i < kHk; ++i)
+        if (ms + hs < nslots) st_state4<SB16>(a.hk, ((size_t)bh * K + 16 * i + hr) * M + m0 + ms + hs, hreg[i]);
     }
 #pragma unroll
     for (int t = 0; t < NT; ++t) {
