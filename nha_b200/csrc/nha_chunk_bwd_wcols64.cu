@@ -2,14 +2,15 @@
 // work (nha_frag64.cuh).  For every query row that can see a key, with the row's joint log-sum-exp L and delta = <do, o>:
 //     p = exp(scale q_swa k - L),  dz = scale p (do v - delta),  dv += p do,  dk_swa += dz q_swa.
 //
-// One CTA = the 64 keys of one (chunk, kv head), two CTAs per SM.  It walks the blocks of 64 query rows that can see a key (query
+// One CTA = the 64 keys of one (chunk, kv head), three CTAs per SM: the four accumulators lie two and two in the lane halves of
+// 128 tensor-memory columns, and eight operand tiles are 67 KB.  It walks the blocks of 64 query rows that can see a key (query
 // chunk x head of the group), one round of products per block:
 //     dv += P^T do,  dk += dZ^T q_swa  of block i   together with   S = q_swa k^T,  dP = do v^T  of block i + 1
 // with the rows of block i + 2 on their way.  The window part does not depend on the gates, so flagged chunks are done here too.
 //
-// What bounds it: the chain of rounds of a CTA; fetching the rows of later CTAs into L2 does not help (181 us without, 186 with
-// it).  Measured against two blocks of 64 rows to a product with two rounds per pair, one row per lane: B16 T2048 H16 W64
-// 210 -> 181 us; 32768 packed tokens, windows 32-512, 336 -> 288 us.
+// What bounds it: the chain of rounds of a CTA, so that a third CTA of an SM is nearly as good as the first two: against two CTAs
+// with 256 columns each B16 T2048 H16 W64 181 -> 153 us (48 % of the copy rate); 32768 packed tokens, windows 32-512, 288 -> 233 us.
+// Fetching the rows of later CTAs into L2 does not help (with two CTAs: 181 us without, 186 with it).
 //
 // Replaces the third-party flash-attn varlen backward's dk / dv (call site nha_fla/ops/nha/chunk.py:333-344).
 #include "nha_bwd_common.cuh"
@@ -23,10 +24,12 @@ namespace wc64 {
 constexpr int tK = 0, tV = 1, tQ = 2, tDO = 3, kSet = 2, tP = 6, tZ = 7, kTiles = 8;       // tQ, tDO: two sets
 constexpr int oBar = kTiles * kTile;
 constexpr int total = oBar + 64 + 1024;
-constexpr int cS = 0, cDP = 64, cDV = 128, cDK = 192, kTmemCols = 256;
+// an accumulator of 64 rows takes half of the lanes of its columns, and the next one the other half
+constexpr uint32_t cS = 0, cDP = kOtherLanes, cDV = 64, cDK = 64 + kOtherLanes;
+constexpr int kTmemCols = 128;
 }  // namespace wc64
 
-__global__ void __launch_bounds__(kThreads, 2) nha_bwd_wcols64_kernel(const nha_chunk_desc d, const BwdWs w, int* __restrict__ err) {
+__global__ void __launch_bounds__(kThreads, 3) nha_bwd_wcols64_kernel(const nha_chunk_desc d, const BwdWs w, int* __restrict__ err) {
   grid_dep_wait();
   grid_dep_launch();
   using namespace wc64;

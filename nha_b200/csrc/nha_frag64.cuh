@@ -25,6 +25,7 @@ using namespace umma;
 constexpr int kThreads = 256;
 constexpr int kTile = 8192;                        // [64][64] bf16 operand tile
 constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
+constexpr uint32_t kOtherLanes = 16u << 16;        // tensor-memory address of lanes 16-31 of each quarter, where a second such accumulator fits
 
 // 32 columns of the warp's 16 rows: v[4 j + e] = (row gq + 8 (e >> 1), column 8 j + 2 tq + (e & 1))
 __device__ __forceinline__ void frag_ld_nowait(uint32_t taddr, float (&v)[16]) {
