@@ -1,6 +1,7 @@
 // Status plumbing and size helpers of the C ABI.
 #include <string.h>
 
+#include <atomic>
 #include <map>
 #include <mutex>
 #include <utility>
@@ -39,9 +40,14 @@ cudaError_t set_max_smem(const void* func, int bytes) {
 }
 
 int sm_count() {
+  static std::atomic<int> known[64];                 // of each device, once asked
   int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms > 0 ? sms : 148;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 148;
+  if (dev < 64 && (sms = known[dev].load(std::memory_order_relaxed)) > 0) return sms;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (sms <= 0) return 148;
+  if (dev < 64) known[dev].store(sms, std::memory_order_relaxed);
+  return sms;
 }
 
 // One CTA waits, with a poll limit, on an mbarrier phase that nobody completes: the wait must come back as "ran out"

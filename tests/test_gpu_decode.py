@@ -341,6 +341,25 @@ def test_tensors_that_do_not_start_on_16_bytes(K, W):
             assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize('B,H,NG,W', [(1, 2, 8, 64), (3, 4, 2, 300), (2, 1, 16, 513)])
+def test_table_rows_that_do_not_start_on_32_bytes(B, H, NG, W):
+    """Rows of the rotary tables are read 32 bytes at a time where they start there, else 16: the same values, the same bits."""
+    from nha_b200 import fused_recurrent_nha_decode
+    c = cuda(gen.decode_inputs(77, B, H, NG, 128, 128, 64, W))
+
+    def shifted(t):
+        room = torch.empty(t.numel() + 8, dtype=t.dtype, device=t.device)
+        room[8:] = t.reshape(-1)
+        return room[8:].view(t.shape)
+
+    def step(cos, sin):
+        return fused_recurrent_nha_decode(q=c['q'], k=c['k'], v=c['v'], g=c['g'], sw_k=c['sw_k_raw'], sw_v=c['vw'], cos=cos, sin=sin,
+                                          initial_state=(c['hk0'].clone(), c['hv0'].clone()), output_final_state=True)[0]
+    assert c['cos'].data_ptr() % 32 == 0 and shifted(c['cos']).data_ptr() % 32 == 16
+    o = step(c['cos'], c['sin'])
+    assert torch.equal(step(shifted(c['cos']), c['sin']), o) and torch.equal(step(shifted(c['cos']), shifted(c['sin'])), o)
+
+
 @pytest.mark.parametrize('K,H,NG,W', [(128, 4, 8, 512), (64, 16, 1, 64)])
 def test_the_state_update_fuses_the_large_product(K, H, NG, W):
     # h e^g + k s to the last bit: k s is rounded, h e^g is not (its 48 bits are exact in fp64)
