@@ -22,9 +22,7 @@
 #include <cstdlib>
 #include <cstring>
 
-#include "nha_common.cuh"
-#include "nha_tma.cuh"
-#include "nha_umma.cuh"
+#include "nha_frag64.cuh"
 
 namespace nha {
 
@@ -33,7 +31,9 @@ using namespace umma;
 namespace stu {
 constexpr int kThreads = 128;
 constexpr int kTile = 8192;        // one [64][64] bf16 operand tile
-constexpr int kTmemCols = 128;     // E then L_k in columns 0-63, a 64-column half of L_v in columns 64-127
+// E, then L_k in columns 0-63; 64 columns of L_v are an accumulator of 64 rows, which takes half of the lanes: D = 64 in the lanes
+// that L_k leaves of columns 0-63, D = 128 both halves side by side in columns 64-127
+template <int D> constexpr int kCols = D == 64 ? 64 : 128;
 constexpr int kPoll = 1 << 12;     // polls of at most kWaitHintNs each before a wait gives up
 }  // namespace stu
 
@@ -49,6 +49,7 @@ __global__ void __launch_bounds__(stu::kThreads) nha_state_local_umma_kernel(con
   grid_dep_launch();
   using namespace stu;
   constexpr int DT = D / 64;                      // 64-column tiles of k' and v'
+  constexpr int kTmemCols = kCols<D>;
   constexpr int M = 64;
   const int cg = chunk_lo + blockIdx.x, h = blockIdx.y;
   const ChunkRec rc = chunk_rec(d, cg);
@@ -140,82 +141,99 @@ __global__ void __launch_bounds__(stu::kThreads) nha_state_local_umma_kernel(con
   }
   if (!failed && !mbar_wait_limit(&bar[1], 0, kPoll)) failed = true;
   tc_fence_after();
-  // E is an M = 64 accumulator: row 16 w + l sits in lane l < 16 of warp w's lane quarter
+  // E is an M = 64 accumulator, read in fragments (nha_frag64.cuh): this warp has the rows 16 warp + gq (+ 8), 32 columns at a time
+  const int gq = lane >> 2, tq = lane & 3;
   const uint32_t tl = tbase + ((uint32_t)(warp * 32) << 16);
-  const int r = 16 * warp + lane;
-  {
-    float e[64];
-    tmem_ld64(tl, e);
-    if (lane < 16 && !failed) {
-      if (r == 0) {
-        float* ge = w.gend + ((size_t)cg * H + h) * M;
+  float e0[16], e1[16];
+  f64::frag_ld_nowait(tl, e0);
+  f64::frag_ld_nowait(tl + 32, e1);
+  tmem_ld_wait();
+  if (warp == 0 && gq == 0 && !failed) {          // row 0: Gend = E + g'
+    float* ge = w.gend + ((size_t)cg * H + h) * M + 2 * tq;
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          float g0[8];
-          unpack8(*reinterpret_cast<const uint4*>(sG + sw_off(0, c)), g0);
-          *reinterpret_cast<float4*>(ge + 8 * c) = make_float4(e[8 * c] + g0[0], e[8 * c + 1] + g0[1], e[8 * c + 2] + g0[2],
-                                                                e[8 * c + 3] + g0[3]);
-          *reinterpret_cast<float4*>(ge + 8 * c + 4) = make_float4(e[8 * c + 4] + g0[4], e[8 * c + 5] + g0[5],
-                                                                    e[8 * c + 6] + g0[6], e[8 * c + 7] + g0[7]);
-        }
-      }
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        uint4* cell = reinterpret_cast<uint4*>(sS + sw_off(r, c));
-        float sv[8];
-        unpack8(*cell, sv);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) sv[i] *= __expf(e[8 * c + i]);
-        *cell = pack8(sv);
-      }
+    for (int c = 0; c < 8; ++c) {
+      const float2 g0 = f64::pair_f32(*reinterpret_cast<const uint32_t*>(sG + sw_off(0, c) + 4 * tq));
+      const float *e = c < 4 ? e0 + 4 * c : e1 + 4 * (c - 4);
+      *reinterpret_cast<float2*>(ge + 8 * c) = make_float2(e[0] + g0.x, e[1] + g0.y);
     }
   }
+  uint32_t fo[2][2];                              // this lane's rows of the blocks that one stmatrix / ldmatrix moves
+#pragma unroll
+  for (int x = 0; x < 4; ++x) fo[x >> 1][x & 1] = f64::frag_off(warp, x >> 1, lane, x & 1);
+#pragma unroll
+  for (int half = 0; half < 2; ++half)
+#pragma unroll
+    for (int jp = 0; jp < 2; ++jp) {
+      uint32_t sv[4];
+      const uint32_t at = smem_u32(sS) + fo[half][jp];
+      f64::ldm4(at, sv);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        // matrix q of the pair: rows gq (+ 8 for odd q), columns of block 2 jp + q / 2
+        const float* e = (half ? e1 : e0) + 4 * (2 * jp + (q >> 1)) + 2 * (q & 1);
+        const float2 x = f64::pair_f32(sv[q]);
+        sv[q] = f64::pair_bf16(x.x * __expf(e[0]), x.y * __expf(e[1]));
+      }
+      f64::stm4(at, sv[0], sv[1], sv[2], sv[3]);
+    }
   fence_async_smem();
   tc_fence_before();
   __syncthreads();
+  const uint32_t cV = D == 64 ? f64::kOtherLanes : 64u;
   if (tid == 0 && !failed) {
     tc_fence_after();
     // L_k [D x 64] = k'^T sb: both operands MN-major, 16 tokens per k step; with D = 128 the A operand spans two
-    // 64-column tiles, kTile bytes apart (LBO)
+    // 64-column tiles, kTile bytes apart (LBO).  L_v [64 x D] = sb^T v', 64 columns to an accumulator.
     const uint32_t idk = make_idesc(D, 64, 1) | (1u << 15);
     const uint32_t idv = make_idesc(64, 64, 1) | (1u << 15);
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks) {
       mma_f16(tbase, make_desc_lbo(smem_u32(sK) + ks * 2048, kTile), make_desc(smem_u32(sS) + ks * 2048), idk, ks > 0);
-      // L_v [64 x 64] (columns 0-63 of V) = sb^T v'
-      mma_f16(tbase + 64, make_desc(smem_u32(sS) + ks * 2048), make_desc(smem_u32(sV) + ks * 2048), idv, ks > 0);
+#pragma unroll
+      for (int t = 0; t < DT; ++t)
+        mma_f16(tbase + cV + t * f64::kOtherLanes, make_desc(smem_u32(sS) + ks * 2048), make_desc(smem_u32(sV) + t * kTile + ks * 2048), idv,
+                ks > 0);
     }
     commit(&bar[1]);
   }
   if (!failed && !mbar_wait_limit(&bar[1], 1, kPoll)) failed = true;
   tc_fence_after();
+  // The terms leave through the tiles that the products have read, in whole rows of 128 bytes: stored straight from the accumulators'
+  // lanes every 16 bytes would be a line of their own.
   bf16* Lk = w.local + ((size_t)cg * H + h) * ((size_t)D * M + (size_t)M * D);
   bf16* Lv = Lk + (size_t)D * M;
-  auto store_row = [&](uint32_t taddr, bf16* dst, bool active) {
-    float x[64];
-    tmem_ld64(taddr, x);
-    if (active && !failed) {
+  const int sr = lane >> 3, sc = lane & 7;
+  auto stage = [&](unsigned char* tile, uint32_t taddr) {       // an accumulator of 64 rows: this warp's sixteen
+    float x[16];
 #pragma unroll
-      for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(dst + 8 * c) = pack8(x + 8 * c);
+    for (int half = 0; half < 2; ++half) {
+      f64::frag_ld(taddr + 32 * half, x);
+      f64::frag_to_tile(smem_u32(tile) + fo[half][0], smem_u32(tile) + fo[half][1], x);
     }
   };
-  if (D == 128) store_row(tl, Lk + (size_t)tid * M, true);                 // M = 128 accumulator: row = lane
-  else store_row(tl, Lk + (size_t)r * M, lane < 16);
-  store_row(tl + 64, Lv + (size_t)r * D, lane < 16);
-  if (DT == 2) {
-    tc_fence_before();
-    __syncthreads();
-    if (tid == 0 && !failed) {
-      tc_fence_after();
-      const uint32_t idv = make_idesc(64, 64, 1) | (1u << 15);
+  auto store = [&](bf16* dst, int pitch, const unsigned char* tile, int r0, auto rows) {
 #pragma unroll
-      for (int ks = 0; ks < 4; ++ks)
-        mma_f16(tbase, make_desc(smem_u32(sS) + ks * 2048), make_desc(smem_u32(sV) + kTile + ks * 2048), idv, ks > 0);
-      commit(&bar[1]);
+    for (int u = 0; u < decltype(rows)::value / 4; ++u) {
+      const int r = r0 + 4 * u + sr;
+      *reinterpret_cast<uint4*>(dst + (size_t)r * pitch + 8 * sc) = *reinterpret_cast<const uint4*>(tile + sw_off(r, sc));
     }
-    if (!failed && !mbar_wait_limit(&bar[1], 0, kPoll)) failed = true;
-    tc_fence_after();
-    store_row(tl, Lv + (size_t)r * D + 64, lane < 16);
+  };
+  if (D == 128) {                                               // M = 128 accumulator: row = lane
+    float x[64];
+    tmem_ld64(tl, x);
+#pragma unroll
+    for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(sK + sw_off(tid, c)) = pack8(x + 8 * c);
+  } else {
+    stage(sK, tl);
+  }
+#pragma unroll
+  for (int t = 0; t < DT; ++t) stage(sV + t * kTile, tl + cV + t * f64::kOtherLanes);
+  __syncwarp();
+  if (!failed) {
+    if (D == 128) store(Lk, M, sK, 32 * warp, std::integral_constant<int, 32>{});
+    else store(Lk, M, sK, 16 * warp, std::integral_constant<int, 16>{});
+#pragma unroll
+    for (int t = 0; t < DT; ++t) store(Lv + 64 * t, D, sV + t * kTile, 16 * warp, std::integral_constant<int, 16>{});
   }
   if (failed) atomicExch(err, 1);
   tc_fence_before();
