@@ -406,7 +406,7 @@ __global__ void __launch_bounds__(kFwdThreads) nha_chunk_fwd_kernel(const nha_ch
 
 int64_t state_workspace_bytes(const nha_chunk_desc* d);
 int check_chunk_desc(const nha_chunk_desc* d);
-int chunk_output_pass_umma(const nha_chunk_desc* d, int* flags, int* err, cudaStream_t cs);
+int chunk_output_pass_umma(const nha_chunk_desc* d, int* flags, int* err, cudaStream_t cs, bool early);
 bool fwd_pipe_supported(const nha_chunk_desc* d);
 
 }  // namespace nha
@@ -418,7 +418,8 @@ extern "C" int64_t nha_chunk_fwd_workspace_bytes(const nha_chunk_desc* d) {
   return state_workspace_bytes(d);
 }
 
-extern "C" int nha_chunk_output_pass(const nha_chunk_desc* d, void* stream) {
+// `early`: the launch in front on this stream is the scan of this call's state pass
+static int output_pass(const nha_chunk_desc* d, void* stream, bool early) {
   int st = check_chunk_desc(d);
   if (st != NHA_OK) return st;
   if (!d->o || !d->lse_swa || !d->lse_gsa || !d->hk_chunks || !d->hv_chunks) return NHA_ERR_BAD_ARG;
@@ -434,7 +435,7 @@ extern "C" int nha_chunk_output_pass(const nha_chunk_desc* d, void* stream) {
   const char* off = getenv("NHA_B200_NO_UMMA");
   bool umma_done = false;
   if (!(off && off[0] == '1')) {
-    st = chunk_output_pass_umma(d, flags, err, cs);
+    st = chunk_output_pass_umma(d, flags, err, cs, early);
     if (st == NHA_OK) umma_done = true;
     else if (st != NHA_ERR_UNSUPPORTED) return st;
   }
@@ -458,6 +459,8 @@ extern "C" int nha_chunk_output_pass(const nha_chunk_desc* d, void* stream) {
   return check_launch();
 }
 
+extern "C" int nha_chunk_output_pass(const nha_chunk_desc* d, void* stream) { return output_pass(d, stream, false); }
+
 // Device-side error word of the last tensor-memory output pass that used this descriptor's plan
 // (non-zero: a bounded wait on an MMA completion barrier ran out).  Synchronises the stream.
 extern "C" int nha_chunk_device_error(const nha_chunk_desc* d, void* stream) {
@@ -475,7 +478,7 @@ static int fwd_after_plan(const nha_chunk_desc* d, int st, void* stream) {
   if (st != NHA_OK) return st;
   st = nha_chunk_state_pass(d, stream);
   if (st != NHA_OK) return st;
-  return nha_chunk_output_pass(d, stream);
+  return output_pass(d, stream, true);
 }
 
 extern "C" int nha_chunk_fwd(const nha_chunk_desc* d, void* stream) { return fwd_after_plan(d, nha_chunk_plan(d, stream), stream); }

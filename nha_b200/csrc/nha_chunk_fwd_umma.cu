@@ -615,9 +615,9 @@ static int launch_umma(const nha_chunk_desc* d, int* flags, int* err, cudaStream
 bool fwd64_supported(const nha_chunk_desc* d);
 int fwd64_launch(const nha_chunk_desc* d, int* flags, int* err, cudaStream_t cs);
 bool fwd_pipe_supported(const nha_chunk_desc* d);
-int fwd_pipe_launch(const nha_chunk_desc* d, int* flags, int* err, cudaStream_t cs);
+int fwd_pipe_launch(const nha_chunk_desc* d, int* flags, int* err, cudaStream_t cs, bool early);
 
-int chunk_output_pass_umma(const nha_chunk_desc* d, int* flags, int* err, cudaStream_t cs) {
+int chunk_output_pass_umma(const nha_chunk_desc* d, int* flags, int* err, cudaStream_t cs, bool early) {
   const int NG = d->HQ / d->H;
   // head dim 64: 64-row products with full lanes, whatever the group (nha_chunk_fwd64.cu)
   if (fwd64_supported(d)) return fwd64_launch(d, flags, err, cs);
@@ -625,7 +625,7 @@ int chunk_output_pass_umma(const nha_chunk_desc* d, int* flags, int* err, cudaSt
   if (!(d->scale > 0.f)) return NHA_ERR_UNSUPPORTED;     // row maxima are taken before scaling
   // head dim 128: the warp-specialised pipeline (nha_chunk_fwd_pipe.cu)
   if (fwd_pipe_supported(d)) {
-    const int st = fwd_pipe_launch(d, flags, err, cs);
+    const int st = fwd_pipe_launch(d, flags, err, cs, early);
     if (st != NHA_ERR_UNSUPPORTED) return st;
   }
   if (d->K == 128 && NG == 1) return launch_umma<64>(d, flags, err, cs);

@@ -150,12 +150,26 @@ inline void launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t sme
   cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
-__device__ __forceinline__ ChunkRec chunk_rec(const nha_chunk_desc& d, int cg) {
+// Loads from L2, in program order with the waits: what a CTA may read in front of grid_dep_wait() (nha_fwd_pipe_kernel).
+__device__ __forceinline__ int ld_l2(const int* p) {
+  int v;
+  asm volatile("ld.global.cg.s32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint4 ld_l2(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.global.cg.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+
+// (`early`: in front of grid_dep_wait(), from L2; otherwise an ordinary load, which stays behind it)
+__device__ __forceinline__ ChunkRec chunk_rec(const nha_chunk_desc& d, int cg, bool early = false) {
   const int ncb = (int)((d.Ttot + kChunk - 1) / kChunk + d.N);
-  // an ordinary load, which stays behind grid_dep_wait(); what a CTA reads through it depends on the record
-  const int4 r = *(reinterpret_cast<const int4*>(d.plan + plan_rec_offset(d.N, ncb, d.H)) + cg);
+  // what a CTA reads through it depends on the record
+  const uint4* at = reinterpret_cast<const uint4*>(d.plan + plan_rec_offset(d.N, ncb, d.H)) + cg;
+  const uint4 r = early ? ld_l2(at) : *at;
   ChunkRec c;
-  c.n = r.x; c.ci = r.y; c.t0 = r.z; c.len = r.w;
+  c.n = (int)r.x; c.ci = (int)r.y; c.t0 = (int)r.z; c.len = (int)r.w;
   return c;
 }
 
@@ -168,11 +182,11 @@ struct StateWs {
   float* gtot;
 };
 
-__device__ __forceinline__ int seq_window(const nha_chunk_desc& d, int n) {
-  return d.window_left ? d.window_left[n] : d.window_left_all;
+__device__ __forceinline__ int seq_window(const nha_chunk_desc& d, int n, bool early = false) {
+  return !d.window_left ? d.window_left_all : early ? ld_l2(d.window_left + n) : d.window_left[n];
 }
-__device__ __forceinline__ int seq_shift(const nha_chunk_desc& d, int n) {
-  int s = d.shift ? d.shift[n] : d.shift_all;
+__device__ __forceinline__ int seq_shift(const nha_chunk_desc& d, int n, bool early = false) {
+  const int s = !d.shift ? d.shift_all : early ? ld_l2(d.shift + n) : d.shift[n];
   return s < 0 ? 0 : s;
 }
 

@@ -101,3 +101,32 @@ def test_strong_gates_are_left_to_the_general_kernel(monkeypatch):
     d['s'] = (1 - d['g'].float().exp()).to(torch.bfloat16)
     x = {n: d[n][0] for n in NAMES}
     _check(x, [0, T], K ** -0.5, 63, 64, None, None, monkeypatch)
+
+
+@pytest.mark.parametrize('B,T,HQ,H,state', [(1, 777, 32, 4, False), (2, 130, 4, 4, True), (4, 500, 28, 4, True)])
+def test_calls_in_a_row_on_the_same_buffers(B, T, HQ, H, state):
+    """A grid of one wave (the first two) starts while the state pass still runs and reads its inputs before it waits: calls in a row on
+    buffers that change in between, ragged chunks among them, give the bits of calls on their own."""
+    from nha_b200 import fused_chunk_nha_prefill
+    D, M = 128, 64
+    keys = ('q', 'rotary_q', 'k', 'rotary_k', 'v', 's', 'g')
+    want, sets = [], []
+    for seed in range(6):
+        p = gen.prefill_inputs(300 + seed, B, H, HQ // H, D, D, M, 100, T, state)
+        x = {n: p[n].cuda() for n in keys}
+        st = (p['hk0'].cuda(), p['hv0'].cuda()) if state else None
+        sets.append((x, st))
+        torch.cuda.synchronize()
+        o, (hk, hv) = fused_chunk_nha_prefill(**x, window_size=100, initial_state=st, output_final_state=True)
+        torch.cuda.synchronize()
+        want.append((o, hk, hv))
+    buf = {n: torch.empty_like(t) for n, t in sets[0][0].items()}
+    got = []
+    for i in range(18):
+        x, st = sets[i % 6]
+        for n in keys:
+            buf[n].copy_(x[n])
+        o, (hk, hv) = fused_chunk_nha_prefill(**buf, window_size=100, initial_state=st, output_final_state=True)
+        got.append((o, hk, hv))
+    for i, three in enumerate(got):
+        assert all(torch.equal(a, b) for a, b in zip(three, want[i % 6])), i
