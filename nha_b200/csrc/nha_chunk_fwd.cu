@@ -408,6 +408,7 @@ int64_t state_workspace_bytes(const nha_chunk_desc* d);
 int check_chunk_desc(const nha_chunk_desc* d);
 int chunk_output_pass_umma(const nha_chunk_desc* d, int* flags, int* err, cudaStream_t cs, bool early);
 bool fwd_pipe_supported(const nha_chunk_desc* d);
+int state_pass(const nha_chunk_desc* d, void* stream, int dense_T);
 
 }  // namespace nha
 
@@ -474,14 +475,14 @@ extern "C" int nha_chunk_device_error(const nha_chunk_desc* d, void* stream) {
   return v;
 }
 
-static int fwd_after_plan(const nha_chunk_desc* d, int st, void* stream) {
+static int fwd_after_plan(const nha_chunk_desc* d, int st, void* stream, int dense_T) {
   if (st != NHA_OK) return st;
-  st = nha_chunk_state_pass(d, stream);
+  st = state_pass(d, stream, dense_T);
   if (st != NHA_OK) return st;
   return output_pass(d, stream, true);
 }
 
-extern "C" int nha_chunk_fwd(const nha_chunk_desc* d, void* stream) { return fwd_after_plan(d, nha_chunk_plan(d, stream), stream); }
+extern "C" int nha_chunk_fwd(const nha_chunk_desc* d, void* stream) { return fwd_after_plan(d, nha_chunk_plan(d, stream), stream, 0); }
 extern "C" int nha_chunk_fwd_dense(const nha_chunk_desc* d, int T, void* stream) {
-  return fwd_after_plan(d, nha_chunk_plan_dense(d, T, stream), stream);
+  return fwd_after_plan(d, nha_chunk_plan_dense(d, T, stream), stream, T);
 }

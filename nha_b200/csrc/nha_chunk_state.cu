@@ -25,7 +25,7 @@
 namespace nha {
 
 bool state_local_umma_supported(const nha_chunk_desc* d);
-int state_local_umma_launch(const nha_chunk_desc* d, const StateWs& w, int* err, int chunk_lo, int chunk_n, cudaStream_t cs);
+int state_local_umma_launch(const nha_chunk_desc* d, const StateWs& w, int* err, int chunk_lo, int chunk_n, cudaStream_t cs, int dense_T);
 
 constexpr int kStThreads = 256;
 constexpr int kStWarps = kStThreads / 32;
@@ -447,8 +447,8 @@ static void state_ws_layout(const nha_chunk_desc* d, void* scratch, StateWs* w) 
 }
 
 // Per-chunk terms of the chunks [chunk_lo, chunk_lo + chunk_n) on `scratch`: the tensor-core kernel where it has the
-// shape, else the wmma kernel.
-static int state_terms_on(const nha_chunk_desc* d, void* scratch, int chunk_lo, int chunk_n, cudaStream_t cs) {
+// shape, else the wmma kernel.  dense_T: tokens of each sequence where the launch in front is the plan of such a batch, else 0.
+static int state_terms_on(const nha_chunk_desc* d, void* scratch, int chunk_lo, int chunk_n, cudaStream_t cs, int dense_T) {
   const int NCB = (int)nha_chunk_count_bound(d->Ttot, d->N);
   if (chunk_lo < 0 || chunk_n < 0 || chunk_lo + chunk_n > NCB) return NHA_ERR_BAD_ARG;
   if (chunk_n == 0) return NHA_OK;
@@ -457,7 +457,7 @@ static int state_terms_on(const nha_chunk_desc* d, void* scratch, int chunk_lo, 
   int st = NHA_ERR_UNSUPPORTED;
   if (state_local_umma_supported(d)) {
     int* err = d->plan + d->N + 1 + NCB + (size_t)NCB * d->H;
-    st = state_local_umma_launch(d, w, err, chunk_lo, chunk_n, cs);
+    st = state_local_umma_launch(d, w, err, chunk_lo, chunk_n, cs, dense_T);
     if (st != NHA_OK && st != NHA_ERR_UNSUPPORTED) return st;
   }
   if (st == NHA_ERR_UNSUPPORTED) {
@@ -504,8 +504,8 @@ static int state_scan_on(const nha_chunk_desc* d, void* scratch, cudaStream_t cs
 }
 
 // Both parts of the state pass.
-static int state_pass_on(const nha_chunk_desc* d, void* scratch, cudaStream_t cs) {
-  const int st = state_terms_on(d, scratch, 0, (int)nha_chunk_count_bound(d->Ttot, d->N), cs);
+static int state_pass_on(const nha_chunk_desc* d, void* scratch, cudaStream_t cs, int dense_T) {
+  const int st = state_terms_on(d, scratch, 0, (int)nha_chunk_count_bound(d->Ttot, d->N), cs, dense_T);
   return st != NHA_OK ? st : state_scan_on(d, scratch, cs);
 }
 
@@ -639,21 +639,25 @@ extern "C" int nha_chunk_plan_dense(const nha_chunk_desc* d, int T, void* stream
   return plan_launch(d, T, stream);
 }
 
-extern "C" int nha_chunk_state_pass(const nha_chunk_desc* d, void* stream) {
+namespace nha {
+// The state pass; dense_T as in state_terms_on.
+int state_pass(const nha_chunk_desc* d, void* stream, int dense_T) {
   int st = check_chunk_desc(d);
   if (st != NHA_OK) return st;
   if (!d->hk_chunks || !d->hv_chunks) return NHA_ERR_BAD_ARG;
   const int64_t need = state_workspace_bytes(d);
   if (!d->workspace || (int64_t)d->workspace_bytes < need) return NHA_ERR_WORKSPACE;
-  return state_pass_on(d, d->workspace, (cudaStream_t)stream);
+  return state_pass_on(d, d->workspace, (cudaStream_t)stream, dense_T);
 }
+}  // namespace nha
+extern "C" int nha_chunk_state_pass(const nha_chunk_desc* d, void* stream) { return nha::state_pass(d, stream, 0); }
 
 extern "C" int nha_chunk_state_terms(const nha_chunk_desc* d, int chunk_lo, int chunk_n, void* stream) {
   int st = check_chunk_desc(d);
   if (st != NHA_OK) return st;
   const int64_t need = state_workspace_bytes(d);
   if (!d->workspace || (int64_t)d->workspace_bytes < need) return NHA_ERR_WORKSPACE;
-  return state_terms_on(d, d->workspace, chunk_lo, chunk_n, (cudaStream_t)stream);
+  return state_terms_on(d, d->workspace, chunk_lo, chunk_n, (cudaStream_t)stream, 0);
 }
 
 extern "C" int nha_chunk_state_scan(const nha_chunk_desc* d, void* stream) {
@@ -752,5 +756,5 @@ extern "C" int nha_chunk_state_pass_static(const nha_chunk_desc* d, void* stream
   if (st != NHA_OK) return st;
   // every element of the scratch that is read is written earlier in this same call, so the contents
   // left by the previous call never matter and nothing has to be cleared
-  return state_pass_on(d, scratch, (cudaStream_t)stream);
+  return state_pass_on(d, scratch, (cudaStream_t)stream, 0);
 }
