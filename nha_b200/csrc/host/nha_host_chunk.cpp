@@ -44,6 +44,13 @@ void cast_all(const Tensor* src, Tensor* dst, const at::ScalarType* to, int n) {
   if (count) check(nha_cast_many(from, into, len, count, a, b, stream_of(src[0].defined() ? src[0] : src[n - 1])), "nha_cast_many");
 }
 
+// one tensor in another type, by the same kernel
+Tensor in_type(const Tensor& x, at::ScalarType to) {
+  Tensor y;
+  cast_all(&x, &y, &to, 1);
+  return y;
+}
+
 struct Call {
   nha_chunk_desc d;
   int dense_T = -1;                            // tokens per sequence of an unpacked batch
@@ -185,7 +192,7 @@ struct ChunkFunction : torch::autograd::Function<ChunkFunction> {
     Call& c = *p.c;
     nha_host::forward(c, p.want_state);
     const bool converted = c.out_type != at::kBFloat16;
-    const Tensor out = converted ? c.o.to(c.out_type) : c.o;
+    const Tensor out = converted ? in_type(c.o, c.out_type) : c.o;
     auto meta = c10::make_intrusive<Meta>();
     const Tensor* raw[NIN] = {&q_swa, &k_swa, &q_gsa, &k_gsa, &v, &s, &g};
     for (int i = 0; i < NIN; ++i) meta->types[i] = raw[i]->scalar_type();
@@ -218,10 +225,7 @@ struct ChunkFunction : torch::autograd::Function<ChunkFunction> {
     Tensor d_o = grads[0];
     if (!d_o.defined()) d_o = zeros({c.B, c.T, d.HQ, d.V}, at::kBFloat16, like);
     if (d_o.scalar_type() != at::kBFloat16) {
-      const at::ScalarType to = at::kBFloat16;
-      Tensor x;
-      cast_all(&d_o, &x, &to, 1);
-      d_o = x;
+      d_o = in_type(d_o, at::kBFloat16);
     }
     d_o = on_16(d_o.contiguous());
     Tensor d_lse, d_hkt, d_hvt;
@@ -341,7 +345,7 @@ NHA_METHOD(chunk_nha) {
     } else {
       at::AutoGradMode off(false);
       forward(c, want);
-      out = {c.out_type != at::kBFloat16 ? c.o.to(c.out_type) : c.o, c.lse_swa, c.lse_gsa};
+      out = {c.out_type != at::kBFloat16 ? in_type(c.o, c.out_type) : c.o, c.lse_swa, c.lse_gsa};
       if (want) { out.push_back(c.hkt); out.push_back(c.hvt); }
     }
   }
@@ -386,7 +390,7 @@ NHA_METHOD(prefill) {
     c.d.window_left_all = (int32_t)W - 1;
     c.d.shift_all = (int32_t)W;
     forward(c, want);
-    o = q.scalar_type() != at::kBFloat16 ? c.o.to(q.scalar_type()) : c.o;
+    o = q.scalar_type() != at::kBFloat16 ? in_type(c.o, q.scalar_type()) : c.o;
   }
   return tuple({wrap(o), want ? tuple({wrap(c.hkt), wrap(c.hvt)}) : tuple({none(), none()})});
   NHA_END
