@@ -121,7 +121,8 @@ __global__ void __launch_bounds__(pipe::kThreads, 2)
   // Only Hk and Hv come from the kernel in front.  Behind the scan of the state pass (`early`), whose CTAs let this grid start when they
   // have themselves waited for all that came before, everything else is in memory: the loads, the decay factors and A = q k'^T go
   // ahead, and the load warp alone waits, in front of Hk.  (What threads read before that they read from L2.)  777 tokens, 32 heads
-  // on 4, W 512: 44.2 -> 39.0 us for the whole prefill.
+  // on 4, W 512: 41.9 -> 37.3 us for the whole prefill; where the grid is several waves, the first of them gains: 1500 tokens, 32 heads
+  // on 8, W 64: 47.1 -> 46.4; 8000 tokens, W 512: 211.7 -> 210.4.
   if (!early) grid_dep_wait();
   grid_dep_launch();
   using namespace pipe;
@@ -769,11 +770,7 @@ int fwd_pipe_launch(const nha_chunk_desc* d, int* flags, int* err, cudaStream_t 
   if (!ok) return NHA_ERR_UNSUPPORTED;
   cudaError_t e = set_max_smem((const void*)nha_fwd_pipe_kernel, total);
   if (e != cudaSuccess) return record_cuda_error(e);
-  // A grid of one wave is resident while the scan still runs, and its first products are done when the states are there; of a larger grid
-  // only the first of several waves could gain (4 x 500 tokens, 28 heads on 4; 2 x 3000: not faster).
-  const int64_t ctas = (int64_t)NCB * d->H * ((d->HQ / d->H + 1) / 2);
-  early = early && ctas <= 2 * sm_count();
-  launch_after(nha_fwd_pipe_kernel, dim3((unsigned)ctas), kThreads, total, cs, *d, flags, err, maps, early ? 1 : 0);
+  launch_after(nha_fwd_pipe_kernel, dim3((unsigned)(NCB * d->H * ((d->HQ / d->H + 1) / 2))), kThreads, total, cs, *d, flags, err, maps, early ? 1 : 0);
   return check_launch();
 }
 

@@ -10,7 +10,9 @@
 // fp32 are exact up to the order of the additions.  All four inputs arrive by TMA into 128-byte-swizzled tiles that
 // the products read in place (k', v', g', sb as MN-major operands: the token index is the contraction dimension of
 // every product).  The wmma version of this kernel (nha_state_local_kernel) was bound by shared-memory bandwidth
-// (fragment loads); this one touches shared memory from threads only for the 8 KB weight tile.
+// (fragment loads); this one touches shared memory from threads for the 8 KB weight tile and for the terms on their way out: stored
+// straight from the accumulators' lanes, 16 bytes to a line, they took 94 us instead of 73 (16 x 2048 tokens, 16 heads of 64; 85 % of
+// the copy rate) and 306 instead of 244 (131072 tokens, 8 heads of 128).  What bounds it: memory, then the chain of two rounds.
 //
 // Chunks whose rows are not all inside their sequence (the first chunks of a shifted sequence, a ragged last chunk,
 // a sequence start inside a packed buffer) are filled by the threads with zero fill instead of TMA, so that no row of
@@ -46,10 +48,9 @@ __global__ void __launch_bounds__(stu::kThreads) nha_state_local_umma_kernel(con
                                                                              int* __restrict__ err, const int chunk_lo,
                                                                              const __grid_constant__ StateMaps maps, const int dense_T) {
   // Behind the plan of a batch of equal lengths (dense_T tokens each; that kernel lets this one start when it has itself waited for all
-  // that came before) a CTA forms its chunk's record itself, reads the inputs from L2 and waits when its products are done.
-  // With the zero-filling
-  // loads of ragged chunks as asynchronous copies, all in flight: 777 tokens, 32 heads on 4, W 512: 39.0 -> 37.3 us for the
-  // whole prefill; 4 x 500, 28 heads on 4: 56.0 -> 51.0 us.
+  // that came before) a CTA forms its chunk's record itself, reads the inputs from L2 and waits when its products are done.  With the
+  // zero-filling loads of ragged chunks as asynchronous copies, all in flight: 777 tokens, 32 heads on 4, W 512: 39.0 -> 37.3 us for
+  // the whole prefill; 4 x 500, 28 heads on 4: 56.0 -> 51.0 us.
   if (dense_T == 0) grid_dep_wait();
   grid_dep_launch();
   using namespace stu;

@@ -130,7 +130,10 @@ __host__ __device__ __forceinline__ int64_t plan_rec_offset(int64_t N, int64_t N
 struct ChunkRec { int n, ci, t0, len; };
 // Kernels of a chain are launched as programmatic dependents (launch_after): the next grid's CTAs are resident and waiting when the
 // last one finishes, which takes the launch and the ramp-up off the chain (1-2 us per kernel).  Every CTA of such a kernel calls
-// grid_dep_wait() before it reads or writes global memory and before it may return: when a grid has completed, so have all before.
+// grid_dep_wait() before it reads or writes what the grid in front has to do with, and before it may return: when a grid has completed,
+// so have all before.  A grid calls grid_dep_launch() behind its own wait, so that what lies before it is in memory when the next one
+// starts; nha_fwd_pipe_kernel and nha_state_local_umma_kernel use that to begin before they wait.  (The latter lets the scan start
+// before its own wait; the scan waits for it first of all.)
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

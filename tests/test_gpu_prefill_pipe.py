@@ -105,8 +105,9 @@ def test_strong_gates_are_left_to_the_general_kernel(monkeypatch):
 
 @pytest.mark.parametrize('B,T,HQ,H,state', [(1, 777, 32, 4, False), (2, 130, 4, 4, True), (4, 500, 28, 4, True)])
 def test_calls_in_a_row_on_the_same_buffers(B, T, HQ, H, state):
-    """A grid of one wave (the first two) starts while the state pass still runs and reads its inputs before it waits: calls in a row on
-    buffers that change in between, ragged chunks among them, give the bits of calls on their own."""
+    """The output pass (one wave of CTAs and two) starts while the state pass still runs, the state terms beside the plan, and both read their
+    inputs before they wait: calls in a row on buffers that change in between, ragged chunks among them, give the bits of calls on their
+    own."""
     from nha_b200 import fused_chunk_nha_prefill
     D, M = 128, 64
     keys = ('q', 'rotary_q', 'k', 'rotary_k', 'v', 's', 'g')
