@@ -193,6 +193,7 @@ __global__ void __launch_bounds__(pipe::kThreads, 2)
   const uint32_t tbase = *tslot;
   if (s_abort) {
     if (warp == 0) tmem_dealloc(tbase, kTmemCols);
+    grid_dep_wait();
     return;
   }
   bool failed = false;

@@ -61,17 +61,17 @@ __global__ void __launch_bounds__(stu::kThreads) nha_state_local_umma_kernel(con
   ChunkRec rc;
   if (dense_T == 0) {
     rc = chunk_rec(d, cg);
-    if (rc.n < 0) return;
   } else {
     const int per = (dense_T + kChunk - 1) / kChunk;
     rc.n = cg / per;
     rc.ci = cg - rc.n * per;
     rc.t0 = rc.n * dense_T;
     rc.len = dense_T;
-    if (rc.n >= d.N) {
-      grid_dep_wait();
-      return;
-    }
+    if (rc.n >= d.N) rc.n = -1;
+  }
+  if (rc.n < 0) {
+    grid_dep_wait();
+    return;
   }
   const int H = d.H;
   const int t0 = rc.t0, len = rc.len, p0 = rc.ci * kChunk;
@@ -139,6 +139,7 @@ __global__ void __launch_bounds__(stu::kThreads) nha_state_local_umma_kernel(con
   const uint32_t tbase = *tslot;
   if (s_abort) {
     if (warp == 0) tmem_dealloc(tbase, kTmemCols);
+    grid_dep_wait();
     return;
   }
   bool failed = false;

@@ -130,10 +130,12 @@ __host__ __device__ __forceinline__ int64_t plan_rec_offset(int64_t N, int64_t N
 struct ChunkRec { int n, ci, t0, len; };
 // Kernels of a chain are launched as programmatic dependents (launch_after): the next grid's CTAs are resident and waiting when the
 // last one finishes, which takes the launch and the ramp-up off the chain (1-2 us per kernel).  Every CTA of such a kernel calls
-// grid_dep_wait() before it reads or writes what the grid in front has to do with, and before it may return: when a grid has completed,
-// so have all before.  A grid calls grid_dep_launch() behind its own wait, so that what lies before it is in memory when the next one
-// starts; nha_fwd_pipe_kernel and nha_state_local_umma_kernel use that to begin before they wait.  (The latter lets the scan start
-// before its own wait; the scan waits for it first of all.)
+// grid_dep_wait() before it reads or writes what the grid in front has to do with, and before it may return, on every way out
+// (tests/test_dependent_launch.py): when a grid has completed, so have all before.  A grid calls grid_dep_launch() behind its own wait,
+// so that what lies before it is in memory when the next one starts.  Two kernels let the next one start before they have waited
+// themselves, which is sound because that one waits first of all: nha_state_local_umma_kernel (the scan behind it) and
+// nha_fwd_pipe_kernel (the general kernel behind it).  Those two may do so because the grids in front of them, the plan and the
+// scan, launch behind their own waits.
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
