@@ -37,6 +37,7 @@ constexpr int kTile = 8192;        // one [64][64] bf16 operand tile
 // that L_k leaves of columns 0-63, D = 128 both halves side by side in columns 64-127
 template <int D> constexpr int kCols = D == 64 ? 64 : 128;
 constexpr int kPoll = 1 << 12;     // polls of at most kWaitHintNs each before a wait gives up
+constexpr int kSmem = 228 * 1024;  // shared memory of an SM, of which every CTA takes 1 KB more than it asks for
 }  // namespace stu
 
 struct StateMaps {
@@ -46,12 +47,16 @@ struct StateMaps {
 template <int D>
 __global__ void __launch_bounds__(stu::kThreads) nha_state_local_umma_kernel(const nha_chunk_desc d, const StateWs w,
                                                                              int* __restrict__ err, const int chunk_lo,
-                                                                             const __grid_constant__ StateMaps maps, const int dense_T) {
+                                                                             const __grid_constant__ StateMaps maps, const int dense_T,
+                                                                             const int first_wave) {
   // Behind the plan of a batch of equal lengths (dense_T tokens each; that kernel lets this one start when it has itself waited for all
   // that came before) a CTA forms its chunk's record itself, reads the inputs from L2 and waits when its products are done.  With the
   // zero-filling loads of ragged chunks as asynchronous copies, all in flight: 777 tokens, 32 heads on 4, W 512: 39.0 -> 37.3 us for
   // the whole prefill; 4 x 500, 28 heads on 4: 56.0 -> 51.0 us.
-  if (dense_T == 0) grid_dep_wait();
+  // So does the first wave alone, which may run beside the plan and cannot tell whether the error word is set already or still what the
+  // memory held before.  A later CTA finds the plan done: its wait costs nothing, and it does not start where one before it gave up.
+  const bool beside = dense_T != 0 && (int)(blockIdx.y * gridDim.x + blockIdx.x) < first_wave;
+  if (!beside) grid_dep_wait();
   grid_dep_launch();
   using namespace stu;
   constexpr int DT = D / 64;                      // 64-column tiles of k' and v'
@@ -75,7 +80,7 @@ __global__ void __launch_bounds__(stu::kThreads) nha_state_local_umma_kernel(con
   }
   const int H = d.H;
   const int t0 = rc.t0, len = rc.len, p0 = rc.ci * kChunk;
-  const int shift = seq_shift(d, rc.n, dense_T != 0);
+  const int shift = seq_shift(d, rc.n, beside);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   extern __shared__ unsigned char smem_raw[];
@@ -94,7 +99,7 @@ __global__ void __launch_bounds__(stu::kThreads) nha_state_local_umma_kernel(con
     mbar_init(&bar[0], 1);
     mbar_init(&bar[1], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    s_abort = dense_T == 0 ? *(volatile int*)err : 0;   // an earlier CTA of this launch gave up on a wait: do not start
+    s_abort = beside ? 0 : *(volatile int*)err;         // an earlier CTA of this launch gave up on a wait: do not start
   }
   if (tid < 64) {
     // row r of U: ones right of the diagonal
@@ -287,8 +292,10 @@ int state_local_umma_launch(const nha_chunk_desc* d, const StateWs& w, int* err,
   const void* fn = DT == 2 ? (const void*)nha_state_local_umma_kernel<128> : (const void*)nha_state_local_umma_kernel<64>;
   cudaError_t e = set_max_smem(fn, total);
   if (e != cudaSuccess) return record_cuda_error(e);
-  if (DT == 2) launch_after(nha_state_local_umma_kernel<128>, dim3(chunk_n, d->H), kThreads, total, cs, *d, w, err, chunk_lo, maps, dense_T);
-  else launch_after(nha_state_local_umma_kernel<64>, dim3(chunk_n, d->H), kThreads, total, cs, *d, w, err, chunk_lo, maps, dense_T);
+  // shared memory is what limits the CTAs of an SM: five at head dim 64, three at 128
+  const int first_wave = sm_count() * (kSmem / (total + 1024));
+  if (DT == 2) launch_after(nha_state_local_umma_kernel<128>, dim3(chunk_n, d->H), kThreads, total, cs, *d, w, err, chunk_lo, maps, dense_T, first_wave);
+  else launch_after(nha_state_local_umma_kernel<64>, dim3(chunk_n, d->H), kThreads, total, cs, *d, w, err, chunk_lo, maps, dense_T, first_wave);
   return check_launch();
 }
 

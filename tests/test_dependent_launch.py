@@ -84,3 +84,23 @@ def test_the_check_sees_a_missing_wait():
     assert ways_out_without_wait(ok.replace('x) { grid_dep_wait();', 'x) {')) == ['return in if (x)']
     assert ways_out_without_wait(ok.replace('warp == 8', 'z')) == ['if (y) return in the kernel', 'end of the kernel']
     assert ways_out_without_wait('{ auto f = [&](int i) { if (i) return; g(); }; grid_dep_wait(); }') == []
+
+
+def _stops():
+    return [(f, m.group(1)) for f, t in SOURCES.items() for m in re.finditer(r'\bs_abort = ([^;]+);', t)]
+
+
+@pytest.mark.parametrize('name,value', _stops())
+def test_a_set_error_word_stops_the_ctas_that_start_later(name, value):
+    """A CTA reads the error word before its first wait, so that one wait that has run out does not cost every CTA its limit.  A CTA that
+    may run beside the kernel that clears the word cannot read it: that is a matter of its place in the grid, never of the launch."""
+    m = re.fullmatch(r'(?:(\w+) \? 0 : )?\*\(volatile int\*\)err', value)
+    assert m, f'{name}: s_abort = {value}'
+    if m.group(1):
+        rule = re.search(r'const bool ' + m.group(1) + r' = ([^;]+);', SOURCES[name]).group(1)
+        assert 'blockIdx' in rule, f'{name}: {m.group(1)} = {rule}'
+        assert f'if (!{m.group(1)}) grid_dep_wait();' in SOURCES[name]
+
+
+def test_the_stop_is_looked_for_where_it_is():
+    assert {f for f, _ in _stops()} >= {'nha_chunk_state_umma.cu', 'nha_chunk_fwd_pipe.cu'}

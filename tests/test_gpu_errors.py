@@ -81,3 +81,41 @@ def test_the_fold_of_the_peer_exchange_gives_up_on_a_summary_that_never_arrives(
     torch.cuda.synchronize()
     assert int(err.item()) == 0
     assert torch.equal(sk, torch.full_like(sk, 2.0)) and torch.equal(sv, torch.full_like(sv, 2.0))
+
+
+@pytest.mark.parametrize('D', [64, 128])
+def test_a_set_error_word_stops_the_kernels_that_look_at_it(D):
+    """State terms, and at head dim 128 the pipelined output pass, behind an error word that is set by hand: every CTA leaves and nothing
+    is written; with the word cleared the same launches give the bits of before."""
+    from nha_b200 import _lib
+    from nha_b200.chunk import SegmentForward
+    lib = _lib.load()
+    T, HQ, H, M = 330, 4, 2, 64
+    x = {n: t[0].cuda() for n, t in gen.layer_inputs(77, 1, T, HQ, H, D, D, M, gate_div=8.0).items()}
+    seg = SegmentForward(x['q_gsa'], x['q_swa'], x['k_gsa'], x['k_swa'], x['v'], x['s'], x['g'], D ** -0.5, 100, 0)
+    stream = torch.cuda.current_stream().cuda_stream
+    seg.start()
+    seg.summary()
+    o, ls, lg = (t.clone() for t in seg.output_pass()[:3])          # also leaves every chunk's flag clear
+    scratch, geo = seg.t['workspace'], seg.geo
+    word = geo.N + 1 + geo.ncb + geo.ncb * geo.H
+    terms = lambda: _lib.check(lib.nha_chunk_state_terms(seg.desc, 0, geo.ncb, stream), 'nha_chunk_state_terms')
+    terms()
+    want = scratch.clone()
+    geo.plan[word] = 1
+    scratch.fill_(0x77)
+    terms()
+    assert bool((scratch == 0x77).all())
+    if D == 128:
+        for n in ('o', 'lse_swa', 'lse_gsa'):
+            seg.t[n].fill_(7.0)
+        with pytest.raises(_lib.NHALibraryError):
+            seg.output_pass()
+        assert all(bool((seg.t[n] == 7.0).all()) for n in ('o', 'lse_swa', 'lse_gsa'))
+    geo.plan[word] = 0
+    terms()
+    SD = 2 * D * M
+    used = (T + 63) // 64 * geo.H                                   # (chunks that hold tokens; the bound has one more)
+    assert torch.equal(scratch[:used * SD * 2], want[:used * SD * 2])
+    got = seg.output_pass()[:3]
+    assert all(torch.equal(a, b) for a, b in zip(got, (o, ls, lg)))
