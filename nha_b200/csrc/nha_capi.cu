@@ -39,15 +39,23 @@ cudaError_t set_max_smem(const void* func, int bytes) {
   return e;
 }
 
+// An attribute of the current device, asked for once per device; `usual` where it cannot be had.
+static int device_attribute(std::atomic<int> (&known)[64], cudaDeviceAttr what, int usual) {
+  int dev = 0, v = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return usual;
+  if (dev < 64 && (v = known[dev].load(std::memory_order_relaxed)) > 0) return v;
+  cudaDeviceGetAttribute(&v, what, dev);
+  if (v <= 0) return usual;
+  if (dev < 64) known[dev].store(v, std::memory_order_relaxed);
+  return v;
+}
 int sm_count() {
-  static std::atomic<int> known[64];                 // of each device, once asked
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return 148;
-  if (dev < 64 && (sms = known[dev].load(std::memory_order_relaxed)) > 0) return sms;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (sms <= 0) return 148;
-  if (dev < 64) known[dev].store(sms, std::memory_order_relaxed);
-  return sms;
+  static std::atomic<int> known[64];
+  return device_attribute(known, cudaDevAttrMultiProcessorCount, 148);
+}
+int l2_bytes() {
+  static std::atomic<int> known[64];
+  return device_attribute(known, cudaDevAttrL2CacheSize, 126 << 20);
 }
 
 // One CTA waits, with a poll limit, on an mbarrier phase that nobody completes: the wait must come back as "ran out"

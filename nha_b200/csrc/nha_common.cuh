@@ -23,7 +23,8 @@ int check_launch();                     // cudaGetLastError() -> status
 // raises a kernel's dynamic shared-memory limit; remembered per (device, kernel), so the runtime is asked only
 // the first time or when more is needed
 cudaError_t set_max_smem(const void* func, int bytes);
-int sm_count();                         // of the current device
+int sm_count();                         // of the current device, as the next
+int l2_bytes();
 
 // ---- small device utilities ------------------------------------------------------------------
 __device__ __forceinline__ float bf2f(bf16 x) { return __bfloat162float(x); }

@@ -50,7 +50,6 @@ constexpr int kStrThreads = 256;
 constexpr int kStrWarps = kStrThreads / 32;
 constexpr int kGroup = 8;                // keys of one step of a warp, slots of one task of a warp
 constexpr int kAhead = 4;                // loads a warp keeps in flight: keys and values of two steps
-constexpr int64_t kAheadMost = 60 << 20; // bytes of a call whose window goes into L2 ahead of its use
 template <int D> constexpr int kLdq = D == 128 ? D + 8 : D + 32;   // row pitch of the rotated query
 constexpr int kMinKeys = 128;            // a split holds at least this many window keys: a CTA costs about 4 us whatever it holds
 constexpr int kSlotCost = 4;             // eight slots cost a warp about as much as this many groups of eight keys
@@ -916,6 +915,20 @@ int decode_stream_splits(int B, int H, int W, int M) {
   return spl;
 }
 
+// Whether a call's window goes into L2 ahead of its use, as its state always does.  The resident CTAs of this call prefetch while those of
+// the call in front still use what they have prefetched; L2 serves both as long as one wave takes up to a third of it.  Us a layer in a
+// stack, HQ 32, D 128 (132.6 MB of L2), without and with the prefetch of the window, by what a wave holds:
+//   W 512, decode: 31 MB 16.20 | 15.03, 42 MB 16.62 | 16.61, 47 MB 16.90 | 17.57, 52 MB 22.6 | 24.5, 63 MB 23.7 | 24.8, 84 MB 25.2 | 25.2;
+//   on rings: 42 MB 18.28 | 18.67, 52 MB 25.8 | 27.2, 84 MB 26.5 | 28.2;  W 1200: 33 MB 15.57 | 14.67, 44 MB 16.01 | 16.51;
+// grids of several waves, H 4, HQ 16, W 128: 39 of 59 MB 29.26 | 27.75; 16 heads of 64, W 128: 19 of 84 MB 42.9 | 41.3.
+// The line lies behind 42 MB, where the window tensors of a 48-layer stack gain 0.5 % and rings lose 2 %, and in front of 44.
+// state_bytes: of an element of the slot memory, 0 where none is read.
+bool decode_window_ahead(int B, int H, int D, int M, int rows, int splits, int state_bytes, int ctas_per_sm, int sms, int64_t l2) {
+  const int64_t each = ((int64_t)D * (4 * (int64_t)rows + 2 * (int64_t)state_bytes * M)) / splits;
+  const int64_t ctas = std::min((int64_t)B * H * splits, (int64_t)ctas_per_sm * sms);
+  return ctas * each <= l2 / 100 * 32;
+}
+
 // Mode of the programmatic dependent launch of the streaming kernel (see DecodeStreamArgs::pdl): set by
 // nha_decode_set_pdl(), else taken once from the environment variable NHA_PDL (the reference's switch of the same
 // name, nha_fla/ops/nha/fused_recurrent.py:32-34: "0" turns it off), default 1.
@@ -982,10 +995,7 @@ int decode_stream_launch(const DecodeStreamArgs& in, int D, cudaStream_t st) {
     }
   };
   attributes();
-  // The window and the state of this call go into L2 while the call in front still uses its own there: past about half of L2 the window
-  // would push that out.  32 sequences, HQ 32, H 8, D 128, W 512 (84 MB), on rings: 222 us for 8 layers with the window, 211 without;
-  // 48 sequences, H 4 (63 MB): 24.8 and 24.5 us a layer; 32 of them (42 MB): 16.4 and 16.8.
-  a.ahead = (int64_t)a.B * a.H * D * (4 * (int64_t)a.WR + (a.state_bf16 ? 4 : 8) * (int64_t)a.M) <= kAheadMost;
+  a.ahead = decode_window_ahead(a.B, a.H, D, a.M, a.WR, a.SPLITS, a.zero_state ? 0 : a.state_bf16 ? 2 : 4, a.NG > 8 ? 1 : 2, sm_count(), l2_bytes());
   a.tab32 = ((uintptr_t)a.cosp | (uintptr_t)a.sinp | (uintptr_t)(2 * a.cs_row) | (uintptr_t)(2 * a.cs_batch)) % 32 == 0;
   void* args[1] = {(void*)&a};
   e = cudaLaunchKernelExC(&cfg, fn, args);

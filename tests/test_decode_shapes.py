@@ -89,3 +89,16 @@ def test_chunk_operators_take_tensors_of_the_gpu():
         nha_b200.chunk_nha(**x, window_size_left=4, window_size_right=0)
     with pytest.raises(AssertionError, match='CUDA library only'):
         nha_b200.fused_chunk_nha_prefill(x['q_gsa'], x['k_gsa'], x['v'], x['q_swa'], x['k_swa'], x['s'], x['g'], 4)
+
+
+@pytest.mark.parametrize('want,B,H,D,W,splits', [
+    # us a layer without and with the prefetch differ by more than 2 % at each of these (64 slots, fp32 state)
+    (True, 24, 4, 128, 512, 2), (True, 12, 4, 128, 1200, 4), (True, 64, 4, 128, 128, 1), (True, 112, 4, 128, 128, 1), (True, 80, 16, 64, 128, 1),
+    (False, 36, 4, 128, 512, 2), (False, 40, 4, 128, 512, 1), (False, 48, 4, 128, 512, 1), (False, 56, 4, 128, 512, 1), (False, 20, 8, 128, 512, 1),
+    (False, 28, 8, 128, 512, 1), (False, 16, 4, 128, 1200, 4), (False, 24, 4, 128, 1200, 2)])
+def test_the_window_is_prefetched_where_that_measured_faster(want, B, H, D, W, splits):
+    import ctypes
+    from nha_b200 import _lib
+    rule = _lib.load()['_ZN3nha19decode_window_aheadEiiiiiiiiil']         # nha::decode_window_ahead, not part of the C ABI
+    rule.restype, rule.argtypes = ctypes.c_bool, [ctypes.c_int] * 9 + [ctypes.c_int64]
+    assert rule(B, H, D, 64, W, splits, 4, 2, 148, 132644864) is want
