@@ -54,7 +54,6 @@ template <int D> constexpr int kLdq = D == 128 ? D + 8 : D + 32;   // row pitch 
 constexpr int kMinKeys = 128;            // a split holds at least this many window keys: a CTA costs about 4 us whatever it holds
 constexpr int kSlotCost = 4;             // eight slots cost a warp about as much as this many groups of eight keys
 
-// (288 bytes.  The host's part of a launch varies with the size in no evident order: 5.5 us a call with 288, 5.9 with 256 and with 296.)
 struct DecodeStreamArgs {
   const bf16* q; const bf16* sq; const bf16* k; const bf16* v; const bf16* g; const bf16* s;
   const bf16* sw_k; const bf16* sw_v; const bf16* cosp; const bf16* sinp;
@@ -67,10 +66,6 @@ struct DecodeStreamArgs {
   // gate row comes from ring_g, the popped k / v from the rings), the token of this step (k, v: not yet in the
   // ring) is the newest window entry
   const int* head; const bf16* ring_g;
-  // WR: rows of a ring (W outside ring mode).  nopop != 0: the rings are still filling - they hold the W - 1 oldest
-  // window entries in rows 0 .. W - 2, nothing leaves the window and the slot memory keeps its value
-  int WR;
-  int8_t nopop;
   // ring_kraw != NULL (ring mode only): sw_k is a ring of keys that were rotated when they entered it (rotary by
   // absolute position does not change while the window slides), so only the token of this step is rotated here;
   // the raw key that enters the slot memory comes from ring_kraw
@@ -81,22 +76,29 @@ struct DecodeStreamArgs {
   // (sequence, kv head) is finished by exactly one CTA, after all its splits have read the rings, so no other CTA
   // reads the index or the row that is overwritten.
   const bf16* g_new;
-  // state_bf16 != 0: hk and hv point to bf16 tensors (half the state bytes; arithmetic stays fp32 in registers)
-  int8_t state_bf16;
   int64_t cs_batch, cs_row;
-  int8_t zero_state;
-  int8_t ahead;        // 1: the window goes into L2 ahead of its use
-  int8_t tab32;        // 1: rows of the rotary tables start on 32 bytes
-  int8_t cluster;        // 1: the SPLITS CTAs of a (sequence, kv head) form a thread-block cluster and merge through shared memory
+  int WR;             // rows of a ring (W outside ring mode)
+  // the rings are still filling - they hold the W - 1 oldest window entries in rows 0 .. W - 2, nothing leaves the window and the
+  // slot memory keeps its value
+  int nopop;
+  int state_bf16;     // hk and hv point to bf16 tensors (half the state bytes; arithmetic stays fp32 in registers)
+  int zero_state;
+  bool ahead;         // the window goes into L2 ahead of its use
+  bool tab32;         // rows of the rotary tables start on 32 bytes
+  int cluster;        // the SPLITS CTAs of a (sequence, kv head) form a thread-block cluster and merge through shared memory
   // programmatic dependent launch: 0 = plain launch; 1 = the grid may be scheduled before the kernel in front of it on
   // the stream has finished and waits for it before its first global read (it only prefetches into L2 before that); 2 = as 1,
   // but the first window loads of this call go out BEFORE that wait (the caller asserts that the kernel in front writes
   // neither the window nor the slot memory)
-  int8_t pdl;
+  int pdl;
   int B, HQ, H, M, W, NG, SPLITS, KSPL, MQ;
   float scale;
   int off_ring, off_q, off_sqA, off_p, off_eg, off_sv, off_kpop, off_vpop, off_wml, off_ml, off_out;
 };
+// The host's part of a dependent launch depends on the size of the argument block.  Us a launch of an empty kernel, median of 41 rounds
+// with the sizes in random order, spread 0.06: 240 to 272 bytes 1.95-2.00, 280 to 288 1.64, 292 to 336 1.94-2.02 (driver 580.159).  A step
+// of 24 layers for one sequence, which the host bounds: 132.7 us with 288 bytes, 137.3 with 296.  Hence `bool` twice.
+static_assert(sizeof(DecodeStreamArgs) >= 280 && sizeof(DecodeStreamArgs) <= 288, "another size costs 0.3 us a launch: measure it");
 
 // four elements of the slot memory, fp32 or bf16 storage
 template <bool SB16>
