@@ -94,12 +94,26 @@ __global__ void __launch_bounds__(stu::kThreads) nha_state_local_umma_kernel(con
   uint32_t* tslot = (uint32_t*)(bar + 2);
   __shared__ int s_abort;
 
+  // rows of the chunk hold shifted positions p = p0 + r, token p - shift; valid while shift <= p < len
+  const bool full = p0 >= shift && p0 + kChunk <= len;
+  const int64_t row0 = (int64_t)t0 + p0 - shift;  // packed row of the chunk's first row
   if (warp == 0) tmem_alloc(tslot, kTmemCols);
   if (tid == 32) {
     mbar_init(&bar[0], 1);
     mbar_init(&bar[1], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     s_abort = beside ? 0 : *(volatile int*)err;         // an earlier CTA of this launch gave up on a wait: do not start
+    if (full && !s_abort) {                             // (the tiles are on their way while the others reach the barrier)
+      fence_async_smem();
+      mbar_expect_tx(&bar[0], (2 + 2 * DT) * kTile);
+      tma_load_3d(sG, &maps.g, 0, h, (int)row0, &bar[0]);
+      tma_load_3d(sS, &maps.s, 0, h, (int)row0, &bar[0]);
+#pragma unroll
+      for (int kt = 0; kt < DT; ++kt) {
+        tma_load_3d(sK + kt * kTile, &maps.k, 64 * kt, h, (int)row0, &bar[0]);
+        tma_load_3d(sV + kt * kTile, &maps.v, 64 * kt, h, (int)row0, &bar[0]);
+      }
+    }
   }
   if (tid < 64) {
     // row r of U: ones right of the diagonal
@@ -114,9 +128,6 @@ __global__ void __launch_bounds__(stu::kThreads) nha_state_local_umma_kernel(con
       *reinterpret_cast<uint4*>(sU + sw_off(tid, c)) = make_uint4(pr[0], pr[1], pr[2], pr[3]);
     }
   }
-  // rows of the chunk hold shifted positions p = p0 + r, token p - shift; valid while shift <= p < len
-  const bool full = p0 >= shift && p0 + kChunk <= len;
-  const int64_t row0 = (int64_t)t0 + p0 - shift;  // packed row of the chunk's first row
   if (!full) {
     // zero-filling copies by the threads: 16-byte pieces into the swizzled tiles
     auto fill = [&](unsigned char* dst, const bf16* base, int width, int col0) {
@@ -148,16 +159,6 @@ __global__ void __launch_bounds__(stu::kThreads) nha_state_local_umma_kernel(con
     return;
   }
   bool failed = false;
-  if (full && tid == 0) {
-    mbar_expect_tx(&bar[0], (2 + 2 * DT) * kTile);
-    tma_load_3d(sG, &maps.g, 0, h, (int)row0, &bar[0]);
-    tma_load_3d(sS, &maps.s, 0, h, (int)row0, &bar[0]);
-#pragma unroll
-    for (int kt = 0; kt < DT; ++kt) {
-      tma_load_3d(sK + kt * kTile, &maps.k, 64 * kt, h, (int)row0, &bar[0]);
-      tma_load_3d(sV + kt * kTile, &maps.v, 64 * kt, h, (int)row0, &bar[0]);
-    }
-  }
   // every thread observes the arrival of the tiles itself (it reads the weight tile with ordinary loads later)
   if (full && !mbar_wait_limit(&bar[0], 0, kPoll)) failed = true;
   if (tid == 0 && !failed) {
