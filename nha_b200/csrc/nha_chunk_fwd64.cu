@@ -12,6 +12,8 @@
 //     largest of them, rounded to bf16 for the product, is exactly 1: error of o against 64 bits at 16 heads, W 512, 2.17e-3, and
 //     2.25e-3 with a reference that may lag by 2^8; no difference in time (32768 packed tokens, windows 32-512: 1.685 ms a step).
 // What bounds it: the chain of rounds (two CTAs of eight warps per SM; about 13 k cycles per CTA, HBM at half its rate).
+// It waits for the scan as its first instruction, although it needs only Hk and Hv from it: the early start of nha_fwd_pipe_kernel has not
+// been tried here.
 // Measured against the version with one row per lane and the gate scan in shared memory: B16 T2048 H16 W64 373 -> 230 us;
 // 32768 packed tokens, windows 32-512, 555 -> 328 us; 8 query heads on 2, 4 x 3000 tokens, W 512, 136 -> 90 us; 32 slots
 // (general kernel before), 4 x 2000 tokens, 194 -> 33 us.

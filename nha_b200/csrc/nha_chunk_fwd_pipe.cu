@@ -40,8 +40,10 @@
 // costs would be 7 % of the document prefill of a grouped model, which never had it).  Decay factorisation, flags for chunks that decay
 // too fast for one reference per chunk, and the general kernel that takes those: as in nha_chunk_fwd_umma.cu.
 //
-// What bounds it: the exchange of a window step - score product, tensor-memory load, exponentials, store, value product - whose
-// latencies two CTAs an SM cover in part (issue slots 48 % busy, DRAM 28 %).  Against one thread a
+// What bounds it: latencies that two CTAs an SM cover in part (issue slots 48 % busy, DRAM 28 %).  Clocks of a tile at W 512, two CTAs
+// an SM: 8 k to the decay factors, 13 k for the slot rounds, 2.2-2.6 k for each of nine window steps (score product, tensor-memory load,
+// exponentials, store, value product), 3 k to the end: nearly half lies in front of the window steps, and all of that but the products
+// with q is the same for every pair of heads of a kv head.  Against one thread a
 // row, the gates scanned in shared memory, and the tiles of a chunk far apart in the grid: 131072 tokens, 32 heads on 8, W 512,
 // 2714 -> 2600-2640 us; 2 x 1999 tokens, 32 heads on 8, W 127, 76 -> 71 us.  An L2 prefetch of a later CTA's tiles: 1 % better in
 // the first, 4 % worse in the second.
@@ -120,9 +122,10 @@ __global__ void __launch_bounds__(pipe::kThreads, 2)
                         const __grid_constant__ PipeMaps maps, const int early) {
   // Only Hk and Hv come from the kernel in front.  Behind the scan of the state pass (`early`), whose CTAs let this grid start when they
   // have themselves waited for all that came before, everything else is in memory: the loads, the decay factors and A = q k'^T go
-  // ahead, and the load warp alone waits, in front of Hk.  (What threads read before that they read from L2.)  777 tokens, 32 heads
-  // on 4, W 512: 41.9 -> 37.3 us for the whole prefill; where the grid is several waves, the first of them gains: 1500 tokens, 32 heads
-  // on 8, W 64: 47.1 -> 46.4; 8000 tokens, W 512: 211.7 -> 210.4.
+  // ahead, and the load warp alone waits, in front of Hk.  (What threads read before that they read from L2.)  Whole prefill without
+  // and with it, nothing else changed: 777 tokens, 32 heads on 4, W 512: 42.1 -> 36.9 us; where the grid is several waves, the first of
+  // them gains: 4 x 500 tokens, 28 heads on 4, W 64: 50.9 -> 50.4; 1500 tokens, 32 heads on 8, W 64: 47.1 -> 46.5; 8000 tokens, W 512:
+  // 211.6 -> 210.3; 32768 tokens: no difference.
   if (!early) grid_dep_wait();
   grid_dep_launch();
   using namespace pipe;

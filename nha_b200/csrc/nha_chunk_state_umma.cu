@@ -50,9 +50,9 @@ __global__ void __launch_bounds__(stu::kThreads) nha_state_local_umma_kernel(con
                                                                              const __grid_constant__ StateMaps maps, const int dense_T,
                                                                              const int first_wave) {
   // Behind the plan of a batch of equal lengths (dense_T tokens each; that kernel lets this one start when it has itself waited for all
-  // that came before) a CTA forms its chunk's record itself, reads the inputs from L2 and waits when its products are done.  With the
-  // zero-filling loads of ragged chunks as asynchronous copies, all in flight: 777 tokens, 32 heads on 4, W 512: 39.0 -> 37.3 us for
-  // the whole prefill; 4 x 500, 28 heads on 4: 56.0 -> 51.0 us.
+  // that came before) a CTA forms its chunk's record itself, reads the inputs from L2 and waits when its products are done.  Whole
+  // prefill without and with it, nothing else changed: 777 tokens, 32 heads on 4, W 512: 38.0 -> 36.9 us; 4 x 500, 28 heads on 4, W 64:
+  // 51.3 -> 50.4; 777 tokens, 16 heads of 64: 27.3 -> 26.5; training steps: no difference.
   // So does the first wave alone, which may run beside the plan and cannot tell whether the error word is set already or still what the
   // memory held before.  A later CTA finds the plan done: its wait costs nothing, and it does not start where one before it gave up.
   const bool beside = dense_T != 0 && (int)(blockIdx.y * gridDim.x + blockIdx.x) < first_wave;

@@ -26,7 +26,7 @@
 //
 // What bounds it: the chain of a CTA, about 4 us whatever it holds, and the requests to the first-level cache (table rows, window,
 // state), not the instructions: a version with half of them, sixteen keys a step, was slower.  32 sequences, HQ 32, H 4, D 128, W 512:
-// 17.3 -> 16.4 us a layer with 32-byte table loads and the small inputs fetched ahead (47 % of the copy rate).  Without the table loads
+// 17.3 -> 16.3 us a layer with 32-byte table loads and the small inputs fetched ahead (48 % of the copy rate).  Without the table loads
 // 2.2 us less, without the slot memory 3.8, without the window 5.2.  Measured per layer in a stack, against
 // a version that formed all logits of a CTA first and requested the values only when the keys had been used: 32 sequences,
 // HQ 32, H 4, D 128, W 512: 18.8 -> 17.3 us; H 8: 41.8 -> 25.9 us (3.9 TB/s); the same on rings 47.1 -> 28.7 us; 64 sequences,
