@@ -327,6 +327,9 @@ int nha_chunk_fwd_dense(const nha_chunk_desc* d, int T, void* stream);
 /* backward: needs the forward's o, lse_swa, lse_gsa, hk_chunks, hv_chunks, plan (and hkt/hvt
    when d_hkt/d_hvt are given); writes dq_*, dk_*, dv, ds, dg (+ dhk0/dhv0 when non-NULL) */
 int nha_chunk_bwd(const nha_chunk_desc* d, void* stream);
+/* the same for a batch of N sequences of T tokens each (the forward was nha_chunk_fwd_dense, or cu_seqlens says the same);
+   a backward that knows it on the host can give whole sequences to a CTA */
+int nha_chunk_bwd_dense(const nha_chunk_desc* d, int T, void* stream);
 
 /* State pass for callers that cannot allocate device memory (a plugin host that passes only
    input and output buffers, a serving loop that forbids allocation after start-up).  Same
@@ -350,7 +353,9 @@ int nha_chunk_state_pass_static(const nha_chunk_desc* d, void* stream);
    of dv), 2 = general slot kernel (shapes without a tensor-core query-row side; with one, the chunks
    that the forward flagged are part of stage 0 and this stage launches nothing), 3 = scan of the state
    gradients over the chunks (dhk0/dhv0), 4 = gate carry and key-row side of the slot branch
-   (dk_gsa, dv, ds, dg).  The stages of one backward must run in this order; running all five
+   (dk_gsa, dv, ds, dg).  Head dim 64 with up to 64 slots: 0 = the slot branch (delta, joint LSE, dq_gsa,
+   dk_gsa, ds, dg, the slot part of dv in fp32, dhk0/dhv0), 1 = the window branch (dq_swa, dk_swa) and dv, the
+   others launch nothing.  The stages of one backward must run in this order; running all five
    equals nha_chunk_bwd.  No counterpart in the reference (it has no timing hooks). */
 int nha_chunk_bwd_stage(const nha_chunk_desc* d, int stage, void* stream);
 

@@ -85,6 +85,7 @@ SYMBOLS = {
     'nha_sp_halo_ack': (C.c_int, [c_void_p, c_void_p, c_void_p]),
     'nha_chunk_fwd': (C.c_int, [C.POINTER(ChunkDesc), c_void_p]),
     'nha_chunk_bwd': (C.c_int, [C.POINTER(ChunkDesc), c_void_p]),
+    'nha_chunk_bwd_dense': (C.c_int, [C.POINTER(ChunkDesc), C.c_int, c_void_p]),
     'nha_chunk_state_pass_static_max_bytes': (C.c_int64, []),
     'nha_chunk_state_pass_static': (C.c_int, [C.POINTER(ChunkDesc), c_void_p]),
     'nha_chunk_bwd_stage': (C.c_int, [C.POINTER(ChunkDesc), C.c_int, c_void_p]),

@@ -253,7 +253,7 @@ struct ChunkFunction : torch::autograd::Function<ChunkFunction> {
     d.workspace = ws.data_ptr();
     d.workspace_bytes = nbytes;
     void* stream = stream_of(like);
-    check(nha_chunk_bwd(&d, stream), "nha_chunk_bwd");
+    check(c.dense_T > 0 ? nha_chunk_bwd_dense(&d, c.dense_T, stream) : nha_chunk_bwd(&d, stream), "nha_chunk_bwd");
     check_device(&d, stream, "nha_chunk_bwd");
     bool same = true;
     for (int i = 0; i < NIN; ++i) same = same && meta->types[i] == at::kBFloat16;

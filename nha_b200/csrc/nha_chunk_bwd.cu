@@ -717,7 +717,8 @@ __global__ void __launch_bounds__(kBwThreads) nha_bwd_flagged_kernel(const nha_c
 // One thread owns four consecutive state elements and fetches kScanBatch chunks ahead of the serial
 // recurrence so that enough loads are in flight to cover the memory latency.
 constexpr int kScanBatch = 8;
-__global__ void __launch_bounds__(256) nha_bwd_state_scan_kernel(const nha_chunk_desc d, const BwdWs w) {
+// win: the sums are stored at the last chunk of every `win` and where no sequence ends (1: everywhere): what the walk over runs of chunks starts from.
+__global__ void __launch_bounds__(256) nha_bwd_state_scan_kernel(const nha_chunk_desc d, const BwdWs w, const int win) {
   grid_dep_wait();
   grid_dep_launch();
   const int K = d.K, V = d.V, M = d.M, H = d.H;
@@ -754,14 +755,14 @@ __global__ void __launch_bounds__(256) nha_bwd_state_scan_kernel(const nha_chunk
       const int ci = hi - u;
       if (ci >= 0) {
         const size_t cgi = (size_t)(chunk0 + ci) * H + h;
-        __stcs((float4*)(buf + cgi * per + e), run);
+        if (win == 1 || ((chunk0 + ci) % win == win - 1 && ci + 1 < nchunks)) __stcs((float4*)(buf + cgi * per + e), run);
         float4 a;
         if (is_k) a = make_float4(__expf(decay[u].x), __expf(decay[u].y), __expf(decay[u].z), __expf(decay[u].w));
         else { const float x = __expf(decay[u].x); a = make_float4(x, x, x, x); }
-        run.x = run.x * a.x + local[u].x;
-        run.y = run.y * a.y + local[u].y;
-        run.z = run.z * a.z + local[u].z;
-        run.w = run.w * a.w + local[u].w;
+        run.x = fmaf(run.x, a.x, local[u].x);
+        run.y = fmaf(run.y, a.y, local[u].y);
+        run.z = fmaf(run.z, a.z, local[u].z);
+        run.w = fmaf(run.w, a.w, local[u].w);
       }
     }
   }
@@ -1018,7 +1019,15 @@ __global__ void __launch_bounds__(kBwThreads) nha_bwd_inter_kernel(const nha_chu
 }
 
 
+void bwd_state_scan_launch(const nha_chunk_desc* d, const BwdWs& w, int win, cudaStream_t cs) {
+  const int SD = d->K * d->M + d->M * d->V;
+  launch_after(nha_bwd_state_scan_kernel, dim3(d->N * d->H, (SD / 4 + 255) / 256), 256, 0, cs, *d, w, win);
+}
+
 int check_chunk_desc(const nha_chunk_desc* d);
+bool bwd64_supported(const nha_chunk_desc* d);
+int bwd_slot64_launch(const nha_chunk_desc* d, const BwdWs& w, int dense_T, int* err, cudaStream_t cs);
+int bwd_win64_launch(const nha_chunk_desc* d, const BwdWs& w, int* err, cudaStream_t cs);
 bool bwd_umma_supported(const nha_chunk_desc* d);
 int bwd_umma_launch(const nha_chunk_desc* d, const BwdWs& w, int which, int* err, cudaStream_t cs);
 bool bwd_wcols_umma_supported(const nha_chunk_desc* d);
@@ -1033,7 +1042,7 @@ extern "C" int64_t nha_chunk_bwd_workspace_bytes(const nha_chunk_desc* d) {
   return bwd_ws_layout(d, nullptr, nullptr);
 }
 
-static int bwd_run(const nha_chunk_desc* d, int stage_mask, void* stream) {
+static int bwd_run(const nha_chunk_desc* d, int dense_T, int stage_mask, void* stream) {
   int st = check_chunk_desc(d);
   if (st != NHA_OK) return st;
   if (!d->o || !d->lse_swa || !d->lse_gsa || !d->hk_chunks || !d->hv_chunks || !d->d_o || !d->dq_gsa || !d->dq_swa ||
@@ -1053,6 +1062,20 @@ static int bwd_run(const nha_chunk_desc* d, int stage_mask, void* stream) {
   const MarchLayout L4 = march_layout(d->K, d->V, d->M);
   if (L1.total > kMaxSmem || L2.total > kMaxSmem || L3.total > kMaxSmem || L4.total > kMaxSmem) return NHA_ERR_SMEM;
   cudaStream_t cs = (cudaStream_t)stream;
+  const char* off = getenv("NHA_B200_NO_UMMA");
+  const bool tensor_cores = !(off && off[0] == '1');
+  const int NCB = (int)nha_chunk_count_bound(d->Ttot, d->N);
+  int* flags = d->plan + d->N + 1 + NCB;
+  int* err = flags + (size_t)NCB * d->H;
+  // Head dim 64: the slot branch as a walk that takes the flagged chunks too, then the window branch.
+  if (tensor_cores && bwd64_supported(d)) {
+    w.flags = flags;
+    if (stage_mask & 1) {
+      st = bwd_slot64_launch(d, w, dense_T, err, cs);
+      if (st != NHA_OK) return st;
+    }
+    return stage_mask & 2 ? bwd_win64_launch(d, w, err, cs) : st;
+  }
   cudaError_t e;
   e = set_max_smem((const void*)nha_bwd_window_rows_kernel, L1.total);
   if (e != cudaSuccess) return record_cuda_error(e);
@@ -1069,17 +1092,13 @@ static int bwd_run(const nha_chunk_desc* d, int stage_mask, void* stream) {
   const size_t flagged_smem = std::max(L1.total, std::max(L3.total, L5.total));
   e = set_max_smem((const void*)nha_bwd_flagged_kernel, (int)flagged_smem);
   if (e != cudaSuccess) return record_cuda_error(e);
-  const int NCB = (int)nha_chunk_count_bound(d->Ttot, d->N);
   dim3 grid(NCB, d->H), block(kBwThreads);
   // gated launches (only the chunks the forward flagged do work): sixteen chunks per CTA
   const int cpc = 16;
   dim3 ggrid((NCB + cpc - 1) / cpc, d->H);
   // Shapes with tensor-memory kernels: those handle every chunk the forward did not flag, the general
   // kernels below are launched gated on the flags and pick up the rest.
-  const char* off = getenv("NHA_B200_NO_UMMA");
-  const bool umma = bwd_umma_supported(d) && !(off && off[0] == '1');
-  int* flags = d->plan + d->N + 1 + NCB;
-  int* err = flags + (size_t)NCB * d->H;
+  const bool umma = bwd_umma_supported(d) && tensor_cores;
   BwdWs wu = w, wg = w;                 // tensor-memory kernels: unflagged chunks; general kernels: flagged ones
   if (umma) {
     wu.flags = flags; wu.gate = 2;
@@ -1098,7 +1117,7 @@ static int bwd_run(const nha_chunk_desc* d, int stage_mask, void* stream) {
   if (stage_mask & 2) {
     // the window part does not depend on the gates: every chunk takes the tensor-memory kernel when the
     // shape has one
-    if (bwd_wcols_umma_supported(d) && !(off && off[0] == '1')) {
+    if (bwd_wcols_umma_supported(d) && tensor_cores) {
       st = bwd_wcols_umma_launch(d, w, err, cs);
     } else {
       launch_after(nha_bwd_window_cols_kernel, grid, block, L2.total, cs, *d, w);
@@ -1117,8 +1136,7 @@ static int bwd_run(const nha_chunk_desc* d, int stage_mask, void* stream) {
       st = check_launch();
       if (st != NHA_OK) return st;
     }
-    const int SD = d->K * d->M + d->M * d->V;
-    launch_after(nha_bwd_state_scan_kernel, dim3(d->N * d->H, (SD / 4 + 255) / 256), 256, 0, cs, *d, w);
+    bwd_state_scan_launch(d, w, 1, cs);
     st = check_launch();
     if (st != NHA_OK) return st;
   }
@@ -1134,9 +1152,14 @@ static int bwd_run(const nha_chunk_desc* d, int stage_mask, void* stream) {
   return st;
 }
 
-extern "C" int nha_chunk_bwd(const nha_chunk_desc* d, void* stream) { return bwd_run(d, 31, stream); }
+extern "C" int nha_chunk_bwd(const nha_chunk_desc* d, void* stream) { return bwd_run(d, 0, 31, stream); }
+
+extern "C" int nha_chunk_bwd_dense(const nha_chunk_desc* d, int T, void* stream) {
+  if (!d || T <= 0 || (int64_t)T * d->N != d->Ttot) return NHA_ERR_BAD_ARG;
+  return bwd_run(d, T, 31, stream);
+}
 
 extern "C" int nha_chunk_bwd_stage(const nha_chunk_desc* d, int stage, void* stream) {
   if (stage < 0 || stage > 4) return NHA_ERR_BAD_ARG;
-  return bwd_run(d, 1 << stage, stream);
+  return bwd_run(d, 0, 1 << stage, stream);
 }

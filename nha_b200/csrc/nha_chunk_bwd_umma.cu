@@ -544,19 +544,14 @@ static int launch_cols(const nha_chunk_desc* d, const BwdWs& w, int* err, cudaSt
   return check_launch();
 }
 
-bool bwd64_supported(const nha_chunk_desc* d);
-int bwd_rows64_launch(const nha_chunk_desc* d, const BwdWs& w, int* err, cudaStream_t cs);
-int bwd_cols64_launch(const nha_chunk_desc* d, const BwdWs& w, int* err, cudaStream_t cs);
 int bwd_rows128_launch(const nha_chunk_desc* d, const BwdWs& w, int* err, cudaStream_t cs);
 
 bool bwd_umma_supported(const nha_chunk_desc* d) {
-  if (d->K == 64) return bwd64_supported(d);
   return d->K == 128 && d->V == 128 && d->M == 64 && d->scale > 0.f;
 }
 
 // which: 0 = rows pass, 1 = columns pass.  The caller has checked bwd_umma_supported().
 int bwd_umma_launch(const nha_chunk_desc* d, const BwdWs& w, int which, int* err, cudaStream_t cs) {
-  if (d->K == 64) return which == 0 ? bwd_rows64_launch(d, w, err, cs) : bwd_cols64_launch(d, w, err, cs);
   if (which == 0) return bwd_rows128_launch(d, w, err, cs);
   // two heads to a 128-row tile where the group is even, one head to a 64-row tile where it is odd (2 x 1999 tokens, seven heads
   // a group, whole training pass: 440 us, 1774 us with the general kernels)

@@ -55,6 +55,19 @@ __device__ __forceinline__ uint32_t make_idesc(int M, int N, int b_mn_major) {
 // byte offset of 16-byte chunk c of row r inside a swizzled [rows][64 bf16] tile
 __device__ __forceinline__ int sw_off(int r, int c) { return (r >> 3) * 1024 + (r & 7) * 128 + ((c ^ (r & 7)) << 4); }
 
+// Products are issued by one elected lane of a warp that the compiler can see to be whole there, from addresses that it can see to be
+// the same in all lanes (uniform(), close to the use so that the descriptors are not kept in registers): a 64 x 64 x 16 product
+// then issues in the 32 cycles that it takes to run.  Behind `if (tid == 0)` every descriptor goes through a register-to-uniform move
+// and the same product takes 57 cycles to issue (32 of them in a row, one CTA per SM; two CTAs: 62 against 72).
+// true in one lane of a warp (all lanes must be here)
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
+  return one != 0;
+}
+// a value that is the same in all lanes, in a form the compiler can tell
+__device__ __forceinline__ uint32_t uniform(uint32_t x) { return __shfl_sync(0xffffffffu, x, 0); }
+
 __device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, bool accumulate) {
   const uint32_t acc = accumulate ? 1u : 0u;
   asm volatile(
