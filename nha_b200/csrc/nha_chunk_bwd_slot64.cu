@@ -33,11 +33,12 @@ namespace nha {
 
 using namespace f64;
 
-// Tensor maps of the call's tensors (this GPU's own memory).  A tile whose 64 rows lie inside its sequence comes by TMA; the
-// others (ragged ends, rows in front of a sequence) are copied piece by piece with zero fill.  use == 0: all tiles are copied
-// (fewer than 64 slots, or no tensor maps).
+// Tensor maps of the call's tensors (this GPU's own memory).  A chunk whose 64 rows lie inside its sequence, shifted or not, is moved by
+// TMA: warp i asks for tile i of `in` and for `out` i - 1.  Others (ragged ends, rows in front of a sequence) are copied piece by piece with
+// zero fill.  use == 0: all chunks are (fewer than 64 slots, or no tensor maps).
+enum { kInQ, kInDO, kInK, kInS, kInG, kInV, kInHk, kInHv, kIns };
 struct SlotMaps {
-  CUtensorMap qg, kg, v, g, s, dout, hk, hv, o, dq, dk, ds, dg;
+  CUtensorMap in[kIns], out[4], o;
   int use;
 };
 
@@ -53,7 +54,8 @@ struct SlotSm {
   static constexpr int oTot = oRow + 4 * 256;                   // fp32 [64][4 quarters] totals of the gate terms
   static constexpr int oPart = oTot + (TERMS ? 0 : 4 * 256);                  // fp32 [2][64][4 quarters, 2 halves, -] dot products of the carry
   static constexpr int oBar = oPart + (TERMS ? 0 : 16 * 256);
-  static constexpr int total = oBar + 64 + 1024;
+  static constexpr int oRec = oBar + 64;
+  static constexpr int total = oRec + 128 + 1024;
   static constexpr int kCtas = TERMS && ONE ? 3 : 2;
   // accumulators: four of a head, the chunk's terms, and the state gradient (one head) or dk', dv' (summed over the heads)
   static constexpr uint32_t cA = 0, cB = kOtherLanes, cC = 64, cD = 64 + kOtherLanes;
@@ -82,7 +84,7 @@ __device__ __forceinline__ float tile_at(const unsigned char* t, int r, int c) {
 }
 // log decays up to row r and behind it, columns m and m + 1: {G, G, Gend - G, Gend - G} (sums of their own, so that a gate of minus
 // infinity leaves no difference of infinities)
-__device__ __noinline__ float4 steep_sums(const SteepCtx& c, int r, int m) {
+__device__ float4 steep_sums(const SteepCtx& c, int r, int m) {
   float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int i = 0; i < kChunk && m < c.M; ++i) {
     const bf16* gr = steep_row(c, c.g, i);
@@ -91,46 +93,63 @@ __device__ __noinline__ float4 steep_sums(const SteepCtx& c, int r, int m) {
   }
   return x;
 }
-// X[t,m] = sum_{i<=t} A[t,i] s_i[m] exp(G_t - G_i), the same for Av: fp32 rows of 64 in scratch (row = position)
-__device__ __noinline__ void steep_x(const SteepCtx& c, const unsigned char* A, const unsigned char* Av, float* x, float* x2, int64_t xpitch, int tid) {
+__device__ __forceinline__ float2 steep_pair(const bf16* row, int m) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(row + m)); }
+// tile <- tile .* exp(G) (behind: exp(Gend - G)); from: the values of g's row layout instead of the tile's own (s'), or NULL
+__device__ __noinline__ void steep_decay(const SteepCtx& c, unsigned char* t, const bf16* from, bool behind, int tid) {
   const int r = tid >> 2, m0 = 16 * (tid & 3);
-  if (m0 >= c.M || c.c0 + r >= c.len) return;
-  for (int mm = m0; mm < m0 + 16; mm += 2) {
+  const bf16* fr = from ? steep_row(c, from, r) : nullptr;
+  for (int m = m0; m < m0 + 16; m += 2) {
+    __nv_bfloat162* at = reinterpret_cast<__nv_bfloat162*>(t + sw_off(r, m >> 3) + 2 * (m & 7));
+    const float4 g = steep_sums(c, r, m);
+    const float2 v = from ? (fr && m < c.M ? steep_pair(fr, m) : make_float2(0.f, 0.f)) : __bfloat1622float2(*at);
+    *at = __floats2bfloat162_rn(v.x * __expf(behind ? g.z : g.x), v.y * __expf(behind ? g.w : g.y));
+  }
+}
+// The rows' products with the start states, in the accumulators at z and y, become what the whole chunk gives: times exp(G), plus
+// sum_{i<=t} A[t,i] s_i[m] exp(G_t - G_i) from A's tile, and Av's for y
+__device__ __noinline__ void steep_rows(const SteepCtx& c, const unsigned char* A, const unsigned char* Av, uint32_t z, uint32_t y, int r0, int cbase) {
+  float vz[16], vy[16];
+  frag_ld(z, vz);
+  frag_ld(y, vy);
+#pragma unroll
+  for (int k = 0; k < 16; k += 2) {
+    const int r = r0 + 4 * (k & 2), m = cbase + 2 * (k & 12);
     float w0 = 1.f, w1 = 1.f, a0 = 0.f, a1 = 0.f, b0 = 0.f, b1 = 0.f;
-    for (int i = r; i >= 0; --i) {
+#pragma unroll 1
+    for (int i = r; i >= 0 && m < c.M; --i) {
       const bf16* sr = steep_row(c, c.s, i);
-      if (!sr) break;                                          // rows in front of the sequence's first token
-      const float2 sv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sr + mm));
-      const float2 gv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(steep_row(c, c.g, i) + mm));
+      if (!sr) continue;
+      const float2 sv = steep_pair(sr, m), gv = steep_pair(steep_row(c, c.g, i), m);
       const float ai = tile_at(A, r, i), vi = tile_at(Av, r, i);
       a0 += ai * (sv.x * w0); a1 += ai * (sv.y * w1);
       b0 += vi * (sv.x * w0); b1 += vi * (sv.y * w1);
       w0 *= __expf(gv.x); w1 *= __expf(gv.y);
     }
-    *reinterpret_cast<float2*>(x + (int64_t)r * xpitch + mm) = make_float2(a0, a1);
-    *reinterpret_cast<float2*>(x2 + (int64_t)r * xpitch + mm) = make_float2(b0, b1);
+    const float4 g = steep_sums(c, r, m);
+    vz[k] = fmaf(vz[k], __expf(g.x), a0); vz[k + 1] = fmaf(vz[k + 1], __expf(g.y), a1);
+    vy[k] = fmaf(vy[k], __expf(g.x), b0); vy[k + 1] = fmaf(vy[k + 1], __expf(g.y), b1);
   }
+  frag_st(z, vz);
+  frag_st(y, vy);
 }
 // dS[i,m] (+)= sum_{t>=i} (A[t,i] dz_t[m] + Av[t,i] p_t[m]) exp(G_t - G_i) into scratch; then E[t,i] = sum_m dz_t[m] s_i[m]
-// exp(G_t - G_i) and Bv likewise, into A's and Av's tiles (zeros above the diagonal).  dz (times scale) and p: bf16 rows of positions.
-__device__ __noinline__ void steep_grads(const SteepCtx& c, unsigned char* A, unsigned char* Av, const bf16* dz, const bf16* p, int64_t zpitch,
-                                         float* ds, int64_t dpitch, bool add, int tid) {
+// exp(G_t - G_i) and Bv likewise, into A's and Av's tiles (zeros above the diagonal); then the tiles of dz and p are decayed
+__device__ __noinline__ void steep_grads(const SteepCtx& c, unsigned char* A, unsigned char* Av, unsigned char* dz, unsigned char* p, float* ds,
+                                         int64_t dpitch, bool add, int tid) {
   {
     const int r = tid >> 2, m0 = 16 * (tid & 3);
     if (m0 < c.M && c.c0 + r < c.len) {
       for (int mm = m0; mm < m0 + 16; mm += 2) {
         float w0 = 1.f, w1 = 1.f, a0 = 0.f, a1 = 0.f;
-        for (int t = r; t < kChunk && c.c0 + t < c.len; ++t) {
+        for (int t = r; t < kChunk; ++t) {
           if (t > r) {
             const bf16* gr = steep_row(c, c.g, t);
-            const float2 gv = gr ? __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(gr + mm)) : make_float2(0.f, 0.f);
+            const float2 gv = gr ? steep_pair(gr, mm) : make_float2(0.f, 0.f);
             w0 *= __expf(gv.x); w1 *= __expf(gv.y);
           }
-          const float2 zv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(dz + (int64_t)t * zpitch + mm));
-          const float2 pv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p + (int64_t)t * zpitch + mm));
           const float ai = tile_at(A, t, r), vi = tile_at(Av, t, r);
-          a0 += (ai * zv.x + vi * pv.x) * w0;
-          a1 += (ai * zv.y + vi * pv.y) * w1;
+          a0 += (ai * tile_at(dz, t, mm) + vi * tile_at(p, t, mm)) * w0;
+          a1 += (ai * tile_at(dz, t, mm + 1) + vi * tile_at(p, t, mm + 1)) * w1;
         }
         float2* o = reinterpret_cast<float2*>(ds + (int64_t)r * dpitch + mm);
         const float2 old = add ? *o : make_float2(0.f, 0.f);
@@ -141,19 +160,14 @@ __device__ __noinline__ void steep_grads(const SteepCtx& c, unsigned char* A, un
   __syncthreads();
   const int warp = tid >> 5, lane = tid & 31, m = 2 * lane;
   for (int t = warp; t < kChunk; t += kThreads / 32) {
-    float2 zv = make_float2(0.f, 0.f), pv = zv;
-    if (m < c.M && c.c0 + t < c.len) {
-      zv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(dz + (int64_t)t * zpitch + m));
-      pv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p + (int64_t)t * zpitch + m));
-    }
+    const float2 zv = make_float2(tile_at(dz, t, m), tile_at(dz, t, m + 1)), pv = make_float2(tile_at(p, t, m), tile_at(p, t, m + 1));
     float w0 = 1.f, w1 = 1.f;
     for (int i = kChunk - 1; i >= 0; --i) {
       float e = 0.f, b = 0.f;
       if (i <= t) {                                            // (the same for all lanes)
         const bf16* sr = steep_row(c, c.s, i);
         if (sr && m < c.M) {
-          const float2 sv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sr + m));
-          const float2 gv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(steep_row(c, c.g, i) + m));
+          const float2 sv = steep_pair(sr, m), gv = steep_pair(steep_row(c, c.g, i), m);
           e = zv.x * (sv.x * w0) + zv.y * (sv.y * w1);
           b = pv.x * (sv.x * w0) + pv.y * (sv.y * w1);
           w0 *= __expf(gv.x); w1 *= __expf(gv.y);
@@ -168,25 +182,86 @@ __device__ __noinline__ void steep_grads(const SteepCtx& c, unsigned char* A, un
       }
     }
   }
+  __syncthreads();
+  steep_decay(c, dz, nullptr, false, tid);
+  steep_decay(c, p, nullptr, false, tid);
+}
+// the products with the state gradient at the chunk's end, in the accumulator at v, become ds': times exp(Gend - G), plus dS
+__device__ __noinline__ void steep_ds(const SteepCtx& c, uint32_t v, const float* ds, int64_t dpitch, int r0, int cbase) {
+  float x[16];
+  frag_ld(v, x);
+#pragma unroll
+  for (int k = 0; k < 16; k += 2) {
+    const int r = r0 + 4 * (k & 2), m = cbase + 2 * (k & 12);
+    const float4 g = steep_sums(c, r, m);
+    const float2 f = m < c.M && c.c0 + r < c.len ? *reinterpret_cast<const float2*>(ds + (int64_t)r * dpitch + m) : make_float2(0.f, 0.f);
+    x[k] = fmaf(x[k], __expf(g.z), f.x);
+    x[k + 1] = fmaf(x[k + 1], __expf(g.w), f.y);
+  }
+  frag_st(v, x);
 }
 
-// Sum of v[c] over the eight lanes of equal lane % 4, for eight values c: lane (gq, tq) returns the sum of value gq (bits reversed in
-// the order of the halvings: 4 (gq >> 2) + ..., see the indexing below).  Seven exchanges instead of 24.
-__device__ __forceinline__ float lanes_sum8(const float (&v)[8], int lane) {
+// ---- rows that are not whole tiles ------------------------------------------------------------------------------------------
+// [64][64] tile <- rows row .. row + 63 of a sequence's tensor (p: the sequence's first row), zeros outside [0, hi) and behind `width` columns
+__device__ void rows_in(unsigned char* t, const bf16* p, int64_t pitch, int width, int row, int hi, int tid, int nt) {
+  const int c = tid & 7;
+  const bool cok = 8 * c < width;
+  for (int r = tid >> 3; r < kChunk; r += nt >> 3) {
+    const bool ok = cok && row + r >= 0 && row + r < hi;
+    cp16(t + sw_off(r, c), p + (ok ? (int64_t)(row + r) * pitch + 8 * c : 0), ok);
+  }
+}
+// rows [lo, hi) of a tile to `width` columns of a tensor
+__device__ void rows_out(const unsigned char* t, bf16* base, int64_t pitch, int width, int lo, int hi, int tid, int nt) {
+  const int c = tid & 7;
+  for (int r = tid >> 3; r < kChunk; r += nt >> 3)
+    if (8 * c < width && r >= lo && r < hi) *reinterpret_cast<uint4*>(base + (int64_t)r * pitch + 8 * c) = *reinterpret_cast<const uint4*>(t + sw_off(r, c));
+}
+// the tiles of a ragged chunk: which & 1: v', Hk, Hv; & 2: q, do of head hq; & 4: g', k', s'
+template <typename S>
+__device__ __noinline__ void ragged_in(const nha_chunk_desc& d, unsigned char* sm, const ChunkRec& r, int shift, int c, int h, int hq, int which, int tid) {
+  const int c0 = r.ci * kChunk, H = d.H, HQ = d.HQ, M = d.M, hi = r.len - shift;
+  const size_t ch = (size_t)c * H + h;
+  const int64_t rq = (int64_t)HQ * 64, rp = (int64_t)H * 64, rm = (int64_t)H * M, t0 = r.t0;
+  auto t = [&](int i) { return sm + i * kTile; };
+  if (which & 1) {
+    rows_in(t(S::tV), (const bf16*)d.v + t0 * rp + h * 64, rp, 64, c0 - shift, hi, tid, kThreads);
+    rows_in(t(S::tHk), (const bf16*)d.hk_chunks + ch * 64 * M, M, M, 0, kChunk, tid, kThreads);       // [64][M]
+    rows_in(t(S::tHv), (const bf16*)d.hv_chunks + ch * M * 64, 64, 64, 0, M, tid, kThreads);          // [M][64]
+  }
+  if (which & 2) {
+    rows_in(t(S::tQ), (const bf16*)d.q_gsa + t0 * rq + hq * 64, rq, 64, c0, r.len, tid, kThreads);
+    rows_in(t(S::tDO), (const bf16*)d.d_o + t0 * rq + hq * 64, rq, 64, c0, r.len, tid, kThreads);
+  }
+  if (which & 4) {
+    rows_in(t(S::tA), (const bf16*)d.g + t0 * rm + h * M, rm, M, c0 - shift, hi, tid, kThreads);
+    rows_in(t(S::tK), (const bf16*)d.k_gsa + t0 * rp + h * 64, rp, 64, c0 - shift, hi, tid, kThreads);
+    rows_in(t(S::tSB), (const bf16*)d.s + t0 * rm + h * M, rm, M, c0 - shift, hi, tid, kThreads);
+  }
+}
+// the results of a ragged chunk: dq of a head, and with the last one dk', ds', dg
+template <typename S>
+__device__ __noinline__ void ragged_out(const nha_chunk_desc& d, const unsigned char* sm, const ChunkRec& r, int shift, int h, int hq, bool keys, int tid) {
+  const int c0 = r.ci * kChunk, H = d.H, HQ = d.HQ, M = d.M, n = r.len - c0, lo = max(0, shift - c0);
+  auto t = [&](int i) { return sm + i * kTile; };
+  rows_out(t(S::tZA), (bf16*)d.dq_gsa + ((int64_t)(r.t0 + c0) * HQ + hq) * 64, (int64_t)HQ * 64, 64, 0, n, tid, kThreads);
+  if (keys) {
+    const int64_t row = ((int64_t)r.t0 + c0 - shift) * H + h;
+    rows_out(t(S::tPA), (bf16*)d.dk_gsa + row * 64, (int64_t)H * 64, 64, lo, n, tid, kThreads);
+    rows_out(t(S::tDK), (bf16*)d.ds + row * M, (int64_t)H * M, M, lo, n, tid, kThreads);
+    rows_out(t(S::tDV), (bf16*)d.dg + row * M, (int64_t)H * M, M, lo, n, tid, kThreads);
+  }
+}
+
+// Sums over the eight lanes of equal lane % 4 of eight values each, by halving: the lane returns the sum of value gq.
+__device__ __forceinline__ float lanes_sum(const float (&v)[8], int lane) {
   float u[4], t[2];
   const bool h2 = lane & 16, h1 = lane & 8, h0 = lane & 4;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const float mine = h2 ? v[k + 4] : v[k], other = h2 ? v[k] : v[k + 4];
-    u[k] = mine + __shfl_xor_sync(0xffffffffu, other, 16);
-  }
+  for (int k = 0; k < 4; ++k) u[k] = (h2 ? v[k + 4] : v[k]) + __shfl_xor_sync(0xffffffffu, h2 ? v[k] : v[k + 4], 16);
 #pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    const float mine = h1 ? u[k + 2] : u[k], other = h1 ? u[k] : u[k + 2];
-    t[k] = mine + __shfl_xor_sync(0xffffffffu, other, 8);
-  }
-  const float mine = h0 ? t[1] : t[0], other = h0 ? t[0] : t[1];
-  return mine + __shfl_xor_sync(0xffffffffu, other, 4);          // value 4 h2 + 2 h1 + h0 = gq
+  for (int k = 0; k < 2; ++k) t[k] = (h1 ? u[k + 2] : u[k]) + __shfl_xor_sync(0xffffffffu, h1 ? u[k] : u[k + 2], 8);
+  return (h0 ? t[1] : t[0]) + __shfl_xor_sync(0xffffffffu, h0 ? t[0] : t[1], 4);
 }
 
 // k step ks of a product of 64-deep operands (mma64).  The steps of one product wait for one another; those of several products,
@@ -197,21 +272,13 @@ __device__ __forceinline__ void mma_step(uint32_t d, uint64_t a, uint64_t b, uin
 }
 
 // win: chunks per CTA (TERMS: one).  have_stats: delta and the joint log-sum-exp are in memory already (the terms kernel ran).
-template <bool ONE, bool TERMS>
-__global__ void __launch_bounds__(kThreads, SlotSm<ONE, TERMS>::kCtas)
-nha_bwd_slot64_kernel(const nha_chunk_desc d, const BwdWs w, int* __restrict__ err, const __grid_constant__ SlotMaps maps, const int win,
-                      const int have_stats) {
-  grid_dep_wait();
-  grid_dep_launch();
+// STEEP: some chunk of the run may be steep; DL: a gradient arrives on lse_gsa.  (Bodies of their own, so that the usual one is small.)
+template <bool ONE, bool TERMS, bool STEEP, bool DL, bool M64>
+__device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs& w, int* __restrict__ err, const SlotMaps& maps, const int have_stats,
+                                           const int h, const int lo, const int top) {
   typedef SlotSm<ONE, TERMS> S;
-  const int H = d.H, HQ = d.HQ, M = d.M, NG = ONE ? 1 : HQ / H;
-  const int ncb = (int)((d.Ttot + kChunk - 1) / kChunk + d.N);
-  const int wi = blockIdx.x / H, h = blockIdx.x - wi * H, lo = wi * win;
-  int cg = min(ncb, lo + win) - 1;
-  ChunkRec rc = chunk_rec(d, cg);
-  while (rc.n < 0 && --cg >= lo) rc = chunk_rec(d, cg);         // chunks that the plan does not use are the last ones
-  if (rc.n < 0) return;
-  const int top = cg;
+  const int H = d.H, HQ = d.HQ, M = M64 ? 64 : d.M, NG = ONE ? 1 : HQ / H;
+  int cg = top;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int quarter = warp & 3, half = warp >> 2, gq = lane >> 2, tq = lane & 3;
   const int uwarp = (int)uniform(threadIdx.x >> 5);
@@ -224,123 +291,90 @@ nha_bwd_slot64_kernel(const nha_chunk_desc d, const BwdWs w, int* __restrict__ e
   float* tot = (float*)(sm + S::oTot);
   uint64_t* mb = (uint64_t*)(sm + S::oBar);                    // [0..4] products, [5] loads
   uint32_t* tslot = (uint32_t*)(mb + 6);
+  // records of the chunk behind, this one and the next (chunk % 4): {sequence, chunk, first token, length, shift, flag}
+  int4* recs = (int4*)(sm + S::oRec);
+  auto rec_put = [&](int c, const ChunkRec& r) {
+    recs[2 * (c & 3)] = make_int4(r.n, r.ci, r.t0, r.len);
+    recs[2 * (c & 3) + 1] = make_int4(seq_shift(d, r.n), w.flags[(size_t)c * H + h], 0, 0);
+  };
+  auto rec_get = [&](int c) {
+    const int4 r = recs[2 * (c & 3)];
+    return ChunkRec{r.x, r.y, r.z, r.w};
+  };
+  auto rec_shift = [&](int c) { return recs[2 * (c & 3) + 1].x; };
   auto tile = [&](int i) { return sm + i * kTile; };
   const uint32_t sbase = smem_u32(sm);
   auto at = [&](int t, uint32_t off) { return sbase + (uint32_t)(t * kTile) + off; };
 
   bool failed = false;
   uint32_t lph = 0, ph = 0;
-  const int lr = tid >> 3, lc = tid & 7;
-  const uint32_t loff = sw_off(lr, lc);
-  const bool mcol = 8 * lc < M;
-  const int64_t rq = (int64_t)HQ * 64, rp = (int64_t)H * 64, rm = (int64_t)H * M;
+  const int64_t rm = (int64_t)H * M;
 
-  // ---- loads: each warp's elected lane asks for one tile, so that no warp is held up by all of them -----------------------------
-  // the load barrier's phase takes one arrival of each warp, with the bytes of its tile where that comes by TMA
-  auto whole = [&](int row, int hi) { return maps.use && row >= 0 && row + kChunk <= hi; };
-  auto load_tokens = [&](int by, int t, const CUtensorMap& map, int head, const void* base, int64_t pitch, int width, int t0, int row, int hi) {
-    if (whole(row, hi)) {
-      if (uwarp == by && elect_one()) {
+  // ---- loads: warp i's elected lane asks for tile i of SlotMaps::in, so that no warp is held up by all of them ---------------------
+  // The load barrier's phase takes one arrival of each of these warps, with the bytes of its tile where that comes by TMA.
+  auto ask = [&](const ChunkRec& r, int shift, int c, int hq, int from, int to) {
+    const int c0 = r.ci * kChunk;
+    if (maps.use && c0 >= shift && c0 + kChunk <= r.len) {
+      if (uwarp >= from && uwarp <= to && elect_one()) {
+        constexpr uint32_t kIn = S::tQ | S::tDO << 4 | S::tK << 8 | S::tSB << 12 | S::tA << 16 | S::tV << 20 | S::tHk << 24 | S::tHv << 28;
+        const int y = uwarp < kInK ? hq : uwarp < kInHk ? h : 0, z = uwarp < kInK ? r.t0 + c0 : uwarp < kInHk ? r.t0 + c0 - shift : (c * H + h) * 64;
         mbar_expect_tx(&mb[5], kTile);
-        tma_load_3d(tile(t), &map, 0, head, t0 + row, &mb[5]);
+        tma_load_3d(tile((kIn >> (4 * uwarp)) & 15), &maps.in[uwarp], 0, y, z, &mb[5]);
       }
     } else {
-      const bf16* p = (const bf16*)base + (int64_t)t0 * pitch + head * width + 8 * lc;
-      const bool cok = 8 * lc < width;
-      const bool ok0 = cok && row + lr >= 0 && row + lr < hi, ok1 = cok && row + lr + 32 >= 0 && row + lr + 32 < hi;
-      tile_in(tile(t), loff, p + (ok0 ? row + lr : 0) * pitch, ok0, p + (ok1 ? row + lr + 32 : 0) * pitch, ok1);
-      if (uwarp == by && elect_one()) mbar_arrive(&mb[5]);
+      ragged_in<S>(d, sm, r, shift, c, h, hq, from >= kInV ? 1 : to <= kInDO ? 2 : 6, tid);
+      if (uwarp >= from && uwarp <= to && elect_one()) mbar_arrive(&mb[5]);
     }
-  };
-  auto load_states = [&](const ChunkRec& r, int c, int shift) {  // v', Hk, Hv
-    const int c0 = r.ci * kChunk;
-    const size_t ch = (size_t)c * H + h;
-    load_tokens(5, S::tV, maps.v, h, d.v, rp, 64, r.t0, c0 - shift, r.len - shift);
-    if (maps.use) {
-      if (uwarp >= 6 && elect_one()) {
-        mbar_expect_tx(&mb[5], kTile);
-        tma_load_2d(tile(uwarp == 6 ? S::tHk : S::tHv), uwarp == 6 ? &maps.hk : &maps.hv, 0, (int)(ch * 64), &mb[5]);
-      }
-    } else {
-      const bf16* hk = (const bf16*)d.hk_chunks + ch * 64 * M;      // [64][M]
-      const bf16* hv = (const bf16*)d.hv_chunks + ch * M * 64;      // [M][64]
-      const int o0 = lr * M + 8 * lc, o1 = o0 + 32 * M;
-      tile_in(tile(S::tHk), loff, hk + (mcol ? o0 : 0), mcol, hk + (mcol ? o1 : 0), mcol);
-      const bool v0 = lr < M, v1 = lr + 32 < M;
-      tile_in(tile(S::tHv), loff, hv + (v0 ? lr * 64 + 8 * lc : 0), v0, hv + (v1 ? (lr + 32) * 64 + 8 * lc : 0), v1);
-      if (uwarp >= 6 && elect_one()) mbar_arrive(&mb[5]);
-    }
-  };
-  auto load_head = [&](const ChunkRec& r, int hq) {
-    load_tokens(0, S::tQ, maps.qg, hq, d.q_gsa, rq, 64, r.t0, r.ci * kChunk, r.len);
-    load_tokens(1, S::tDO, maps.dout, hq, d.d_o, rq, 64, r.t0, r.ci * kChunk, r.len);
-  };
-  auto load_rows = [&](const ChunkRec& r, int shift) {           // the first head's rows, k', s', g'
-    const int c0 = r.ci * kChunk;
-    load_tokens(4, S::tA, maps.g, h, d.g, rm, M, r.t0, c0 - shift, r.len - shift);
-    load_head(r, h * NG);
-    load_tokens(2, S::tK, maps.kg, h, d.k_gsa, rp, 64, r.t0, c0 - shift, r.len - shift);
-    load_tokens(3, S::tSB, maps.s, h, d.s, rm, M, r.t0, c0 - shift, r.len - shift);
-    cp_commit();
   };
   auto loads_wait = [&]() {
     cp_wait_all();
     if (!failed && !mbar_wait(&mb[5], lph)) failed = true;
     lph ^= 1;
   };
-  // row statistics of a head: delta = <do, o> by four threads per row (do from its tile), the joint log-sum-exp by one
-  uint4 o0, o1;
-  float lsw, lgs, dl;
+  // row statistics of a head: delta = <do, o> by the threads of a row (do from its tile) and the joint log-sum-exp.  Rows past the end
+  // read the last one's.
+  struct RowIn { uint4 o[2]; float lsw, lgs, dl; };
   auto row_request = [&](const ChunkRec& r, int hq) {
-    const int row = tid >> 2, part = tid & 3, pos = r.ci * kChunk + row;
-    o0 = o1 = make_uint4(0u, 0u, 0u, 0u);
-    lsw = lgs = dl = 0.f;
-    if (pos < r.len) {
-      const size_t i = (size_t)(r.t0 + pos) * HQ + hq;
-      if (!have_stats) {
-        const uint4* o = reinterpret_cast<const uint4*>((const bf16*)d.o + i * 64 + 16 * part);
-        o0 = __ldg(o); o1 = __ldg(o + 1);
-      }
-      if (part == 0) {
-        lgs = d.lse_gsa[i];
-        dl = d.d_lse_gsa ? d.d_lse_gsa[i] : 0.f;
-        if (have_stats) {
-          lsw = w.lj[i];
-          o0.x = __float_as_uint(w.delta[i]);
-        } else {
-          lsw = d.lse_swa[i];
-        }
-      }
-    }
-  };
-  auto row_stats = [&](const ChunkRec& r, int hq) {
-    const int row = tid >> 2, part = tid & 3, pos = r.ci * kChunk + row;
-    float del, lj;
+    const int row = tid >> 2, part = tid & 3, pos = min(r.ci * kChunk + row, r.len - 1);
+    const size_t i = (size_t)(r.t0 + pos) * HQ + hq;
+    RowIn x;
+    x.lgs = d.lse_gsa[i];
+    x.dl = DL && d.d_lse_gsa ? d.d_lse_gsa[i] : 0.f;
+    x.lsw = have_stats ? w.lj[i] : d.lse_swa[i];
     if (have_stats) {
-      del = __uint_as_float(o0.x);
-      lj = lsw;
+      x.o[0].x = __float_as_uint(w.delta[i]);
     } else {
-      float x[8], y[8];
-      const unsigned char* t = tile(S::tDO);
-      unpack8(o0, x);
-      unpack8(*reinterpret_cast<const uint4*>(t + sw_off(row, 2 * part)), y);
+      const uint4* o = reinterpret_cast<const uint4*>((const bf16*)d.o + i * 64 + 16 * part);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) x.o[u] = __ldg(o + u);
+    }
+    return x;
+  };
+  auto row_stats = [&](const RowIn& in, const ChunkRec& r, int hq) {
+    const int row = tid >> 2, part = tid & 3, pos = r.ci * kChunk + row;
+    float del = __uint_as_float(in.o[0].x), lj = in.lsw;
+    if (!have_stats) {
       del = 0.f;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) del += x[e] * y[e];
-      unpack8(o1, x);
-      unpack8(*reinterpret_cast<const uint4*>(t + sw_off(row, 2 * part + 1)), y);
+      for (int u = 0; u < 2; ++u) {
+        float x[8], y[8];
+        unpack8(in.o[u], x);
+        unpack8(*reinterpret_cast<const uint4*>(tile(S::tDO) + sw_off(row, 2 * part + u)), y);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) del += x[e] * y[e];
-      del += __shfl_xor_sync(0xffffffffu, del, 1);
-      del += __shfl_xor_sync(0xffffffffu, del, 2);
-      const float mx = fmaxf(lsw, lgs);
-      lj = mx + __logf(__expf(lsw - mx) + __expf(lgs - mx));
+        for (int e = 0; e < 8; ++e) del += x[e] * y[e];
+      }
+#pragma unroll
+      for (int o = 1; o < 4; o <<= 1) del += __shfl_xor_sync(0xffffffffu, del, o);
+      const float mx = fmaxf(in.lsw, in.lgs);
+      lj = mx + __logf(__expf(in.lsw - mx) + __expf(in.lgs - mx));
     }
     if (part == 0) {
-      rowv[row] = del;
-      rowv[64 + row] = -lj * kLog2e;
-      rowv[128 + row] = -lgs * kLog2e;
-      rowv[192 + row] = dl;
+      rowv[row] = -del;
+      rowv[64 + row] = pos < r.len ? -lj * kLog2e : -INFINITY;  // a row past the end has no weights
+      if (DL) {
+        rowv[128 + row] = pos < r.len ? -in.lgs * kLog2e : -INFINITY;
+        rowv[192 + row] = in.dl;
+      }
       if (pos < r.len && !have_stats) {
         w.delta[(size_t)(r.t0 + pos) * HQ + hq] = del;
         w.lj[(size_t)(r.t0 + pos) * HQ + hq] = lj;
@@ -349,8 +383,9 @@ nha_bwd_slot64_kernel(const nha_chunk_desc d, const BwdWs w, int* __restrict__ e
   };
 
   if (tid == 0) {
+    rec_put(cg, chunk_rec(d, cg));
 #pragma unroll
-    for (int i = 0; i < 6; ++i) mbar_init(&mb[i], i == 5 ? kThreads / 32 : 1);
+    for (int i = 0; i < 6; ++i) mbar_init(&mb[i], i == 5 ? kIns : 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_async_smem();
   }
@@ -359,13 +394,11 @@ nha_bwd_slot64_kernel(const nha_chunk_desc d, const BwdWs w, int* __restrict__ e
   tc_fence_before();
   __syncthreads();                                             // the barriers are initialised
   tc_fence_after();
-  {
-    const int sh = seq_shift(d, rc.n);
-    load_states(rc, cg, sh);
-    load_rows(rc, sh);
-  }
+  ask(rec_get(cg), rec_shift(cg), cg, h * NG, kInV, kInHv);
+  ask(rec_get(cg), rec_shift(cg), cg, h * NG, kInQ, kInG);
+  cp_commit();
   const uint32_t tbase = *tslot;
-  const uint32_t tl = tbase + ((uint32_t)(quarter * 32) << 16) + 32 * half;       // this warp's columns of an accumulator at +0
+  const uint32_t tl = tbase + ((uint32_t)(quarter * 32) << 16) + 32 * half;  // this warp's columns of an accumulator at +0
   auto mma_wait = [&](int i) {
     if (!failed && !mbar_wait(&mb[i], ph)) failed = true;
     tc_fence_after();
@@ -377,201 +410,156 @@ nha_bwd_slot64_kernel(const nha_chunk_desc d, const BwdWs w, int* __restrict__ e
     tc_fence_after();
   };
   const uint32_t iKK = idesc64(0, 0), iKM = idesc64(0, 1), iMM = idesc64(1, 1);
-  const uint32_t fo0 = frag_off(quarter, half, lane, 0), fo1 = frag_off(quarter, half, lane, 1);
+  uint32_t fo[2];
+#pragma unroll
+  for (int jp = 0; jp < 2; ++jp) fo[jp] = frag_off(quarter, half, lane, jp);
   const int r0 = 16 * quarter + gq, cbase = 32 * half + 2 * tq;  // this lane's rows r0, r0 + 8; columns cbase + 8 j, + 1
-  const float sc2 = d.scale * kLog2e;
+  auto to_tile = [&](int t, const float (&v)[16]) {
+#pragma unroll
+    for (int jp = 0; jp < 2; ++jp)
+      stm4(at(t, fo[jp]), pair_bf16(v[8 * jp], v[8 * jp + 1]), pair_bf16(v[8 * jp + 2], v[8 * jp + 3]), pair_bf16(v[8 * jp + 4], v[8 * jp + 5]),
+           pair_bf16(v[8 * jp + 6], v[8 * jp + 7]));
+  };
   // tril of an accumulator -> bf16 tile (columns i <= row)
   auto tril_to = [&](uint32_t col, int t) {
     float v[16];
     frag_ld(tl + col, v);
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if (cbase + 8 * j + (e & 1) > r0 + 8 * (e >> 1)) v[4 * j + e] = 0.f;
-    frag_to_tile(at(t, fo0), at(t, fo1), v);
+    for (int k = 0; k < 16; ++k)
+      if (cbase + 8 * (k >> 2) + (k & 1) > r0 + 4 * (k & 2)) v[k] = 0.f;
+    to_tile(t, v);
   };
-  // fp32 rows of a [64][M] or [M][64] state, this thread's fragment
+  // fp32 rows of a [64][M] or [M][64] state: this thread's part
   auto state_k = [&](const float* p, float (&v)[16]) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int m = cbase + 8 * j;
-        const float2 x = p && m < M ? *reinterpret_cast<const float2*>(p + (r0 + 8 * i) * M + m) : make_float2(0.f, 0.f);
-        v[4 * j + 2 * i] = x.x;
-        v[4 * j + 2 * i + 1] = x.y;
-      }
+    for (int k = 0; k < 16; k += 2) {
+      const int m = cbase + 2 * (k & ~3);
+      const float2 x = p && m < M ? *reinterpret_cast<const float2*>(p + (r0 + 4 * (k & 2)) * M + m) : make_float2(0.f, 0.f);
+      v[k] = x.x;
+      v[k + 1] = x.y;
+    }
   };
   auto state_v = [&](const float* p, float (&v)[16]) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const float2 x = p && r0 + 8 * i < M ? *reinterpret_cast<const float2*>(p + (r0 + 8 * i) * 64 + cbase + 8 * j) : make_float2(0.f, 0.f);
-        v[4 * j + 2 * i] = x.x;
-        v[4 * j + 2 * i + 1] = x.y;
-      }
+    for (int k = 0; k < 16; k += 2) {
+      const int m = r0 + 4 * (k & 2);
+      const float2 x = p && m < M ? *reinterpret_cast<const float2*>(p + m * 64 + cbase + 2 * (k & ~3)) : make_float2(0.f, 0.f);
+      v[k] = x.x;
+      v[k + 1] = x.y;
+    }
   };
   auto put_k = [&](float* p, const float (&v)[16]) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int m = cbase + 8 * j;
-        if (m < M) *reinterpret_cast<float2*>(p + (r0 + 8 * i) * M + m) = make_float2(v[4 * j + 2 * i], v[4 * j + 2 * i + 1]);
-      }
+    for (int k = 0; k < 16; k += 2) {
+      const int m = cbase + 2 * (k & ~3);
+      if (m < M) *reinterpret_cast<float2*>(p + (r0 + 4 * (k & 2)) * M + m) = make_float2(v[k], v[k + 1]);
+    }
   };
   auto put_v = [&](float* p, const float (&v)[16]) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-        if (r0 + 8 * i < M) *reinterpret_cast<float2*>(p + (r0 + 8 * i) * 64 + cbase + 8 * j) = make_float2(v[4 * j + 2 * i], v[4 * j + 2 * i + 1]);
+    for (int k = 0; k < 16; k += 2) {
+      const int m = r0 + 4 * (k & 2);
+      if (m < M) *reinterpret_cast<float2*>(p + m * 64 + cbase + 2 * (k & ~3)) = make_float2(v[k], v[k + 1]);
+    }
   };
-  // dot products of the carry: columns m of DK . hk over the rows (one part per quarter), rows m of DV . hv (one part per half)
-  auto dots_k = [&](const float (&v)[16], const float (&x)[16], float* part, bool unscale) {
-    float c[8];
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) c[2 * j + e] = fmaf(v[4 * j + e], x[4 * j + e], v[4 * j + 2 + e] * x[4 * j + 2 + e]);
-    const float sum = lanes_sum8(c, lane);
+  // dot products of the carry from a thread's products: columns m of DK . hk over the rows (one part per quarter), rows m of DV . hv
+  // (one part per block of columns)
+  auto part_k = [&](const float (&c)[8], float* part, bool unscale) {
+    const float sum = lanes_sum(c, lane);
     const int m = cbase + 8 * (gq >> 1) + (gq & 1);             // value gq = 2 j + e
     part[8 * m + quarter] = unscale ? sum * tab[kTabIP + m] : sum;
   };
-  auto dots_v = [&](const float (&v)[16], const float (&x)[16], float* part, bool unscale) {
+  auto part_v = [&](float (&c)[2], float* part, bool unscale) {
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-      float c = 0.f;
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) c = fmaf(v[4 * j + 2 * i + e], x[4 * j + 2 * i + e], c);
-      c += __shfl_xor_sync(0xffffffffu, c, 1);
-      c += __shfl_xor_sync(0xffffffffu, c, 2);
+      c[i] += __shfl_xor_sync(0xffffffffu, c[i], 1);
+      c[i] += __shfl_xor_sync(0xffffffffu, c[i], 2);
       const int m = r0 + 8 * i;
-      if (tq == 0) part[8 * m + 4 + half] = unscale ? c * tab[kTabIP + m] : c;
-    }
-  };
-  auto tile_frag = [&](int t, float (&x)[16]) {
-#pragma unroll
-    for (int jp = 0; jp < 2; ++jp) {
-      uint32_t u[4];
-      ldm4(at(t, jp ? fo1 : fo0), u);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const float2 f = pair_f32(u[q]);
-        const int e = 4 * (2 * jp + (q >> 1)) + 2 * (q & 1);
-        x[e] = f.x;
-        x[e + 1] = f.y;
-      }
+      if (tq == 0) part[8 * m + 4 + half] = unscale ? c[i] * tab[kTabIP + m] : c[i];
     }
   };
   // Results wait in their tiles until the products of the next round have been issued: whole tiles leave by TMA (one elected lane
   // for each, which sees to it that the tile has been read before anything is written there again), others as rows.
-  struct { int tok, hq, n, lo, key; bool q, k; } out;           // first token, head, valid rows; first valid key row, first key token
-  out.q = out.k = false;
-  auto rows_out = [&](int t, bf16* base, int64_t pitch, int lo_, int hi_, bool cok) {
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int r = lr + 32 * u;
-      if (cok && r >= lo_ && r < hi_) *reinterpret_cast<uint4*>(base + (int64_t)r * pitch + 8 * lc) = *reinterpret_cast<const uint4*>(tile(t) + loff + 4096 * u);
-    }
-  };
+  int out_c = -1, out_h = 0;                                    // chunk and head of the waiting rows of dq; the chunk's last head: keys too
   auto flush = [&]() {
-    if (out.q) {
-      if (maps.use && out.n >= kChunk) {
-        if (uwarp == 1 && elect_one()) tma_store_3d(&maps.dq, tile(S::tZA), 0, out.hq, out.tok);
-      } else {
-        rows_out(S::tZA, (bf16*)d.dq_gsa + ((int64_t)out.tok * HQ + out.hq) * 64, rq, 0, out.n, true);
+    if (out_c < 0) return;
+    const ChunkRec r = rec_get(out_c);
+    const int sh = rec_shift(out_c), c0 = r.ci * kChunk;
+    const bool keys = ONE || out_h + 1 == (h + 1) * NG;
+    if (maps.use && c0 >= sh && c0 + kChunk <= r.len) {
+      if (uwarp >= 1 && uwarp <= (keys ? 4 : 1) && elect_one()) {
+        static_assert(TERMS || (S::tZA == 9 && S::tPA == 10 && S::tDK == 11 && S::tDV == 12), "order of SlotMaps::out");
+        tma_store_3d(&maps.out[uwarp - 1], tile(8 + uwarp), 0, uwarp == 1 ? out_h : h, r.t0 + c0 - (uwarp == 1 ? 0 : sh));
+        bulk_commit();
       }
+    } else {
+      ragged_out<S>(d, sm, r, sh, h, out_h, keys, tid);
     }
-    if (out.k) {
-      if (maps.use && out.n >= kChunk && out.lo == 0) {
-        if (uwarp == 2 && elect_one()) tma_store_3d(&maps.dk, tile(S::tPA), 0, h, out.key);
-        if (uwarp == 3 && elect_one()) tma_store_3d(&maps.ds, tile(S::tDK), 0, h, out.key);
-        if (uwarp == 4 && elect_one()) tma_store_3d(&maps.dg, tile(S::tDV), 0, h, out.key);
-      } else {
-        const int64_t row = (int64_t)out.key * H + h;
-        rows_out(S::tPA, (bf16*)d.dk_gsa + row * 64, rp, out.lo, out.n, true);
-        rows_out(S::tDK, (bf16*)d.ds + row * M, rm, out.lo, out.n, mcol);
-        rows_out(S::tDV, (bf16*)d.dg + row * M, rm, out.lo, out.n, mcol);
-      }
-    }
-    out.q = out.k = false;
-    if (uwarp >= 1 && uwarp <= 4 && elect_one()) bulk_commit();
+    out_c = -1;
   };
   auto flushed = [&]() {                                        // in front of the barrier behind which the tiles are written again
     if (uwarp >= 1 && uwarp <= 4 && elect_one()) bulk_wait_read();
   };
 
-  int par = 0, shift = seq_shift(d, rc.n), flag = w.flags[(size_t)cg * H + h];
-  row_request(rc, h * NG);
+  int par = 0;
   for (;; --cg) {
-    const int ci = rc.ci, t0 = rc.t0, len = rc.len, c0 = ci * kChunk;
+    const ChunkRec rc = rec_get(cg);
+    const int ci = rc.ci, t0 = rc.t0, len = rc.len, c0 = ci * kChunk, shift = rec_shift(cg);
     const size_t ch = (size_t)cg * H + h, nh = (size_t)rc.n * H + h;
-    const bool steep = flag != 0;
-    const bool more = cg > lo;
-    ChunkRec rn = rc;                                          // the next chunk's record, shift and flag
-    int shift_next = 0;
-    const int nchunks = (len + kChunk - 1) / kChunk;
-    const bool last = ci == nchunks - 1;
+    const bool steep = STEEP && recs[2 * (cg & 3) + 1].y != 0;
+    const bool more = cg > lo, last = c0 + kChunk >= len;
     float* part = (float*)(sm + S::oPart) + par * 512;
     float* part_next = (float*)(sm + S::oPart) + (par ^ 1) * 512;
     // the state gradient at this chunk's end where it does not come from the chunk behind
     const float* endk = last ? (d.d_hkt ? d.d_hkt + nh * 64 * M : nullptr) : w.dkc + ch * 64 * M;
     const float* endv = last ? (d.d_hvt ? d.d_hvt + nh * M * 64 : nullptr) : w.dvc + ch * M * 64;
     if (!TERMS && (last || cg == top)) {
-      float v[16], x[16];
+      float v[16], x[16], c[8], cv[2] = {0.f, 0.f};
+      auto next = [&](const bf16* p, bool ok) { return ok ? pair_f32(*reinterpret_cast<const uint32_t*>(p)) : make_float2(0.f, 0.f); };
       state_k(endk, v);
       if (ONE) frag_st(tl + S::cSK, v);
-      if (last) {
-        state_k(d.d_hkt ? d.hkt + nh * 64 * M : nullptr, x);
-      } else {
-        const bf16* p = (const bf16*)d.hk_chunks + (ch + H) * 64 * M;
+      if (last) state_k(d.d_hkt ? d.hkt + nh * 64 * M : nullptr, x);
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-          for (int i = 0; i < 2; ++i) {
-            const int m = cbase + 8 * j;
-            const float2 f = m < M ? pair_f32(*reinterpret_cast<const uint32_t*>(p + (r0 + 8 * i) * M + m)) : make_float2(0.f, 0.f);
-            x[4 * j + 2 * i] = f.x;
-            x[4 * j + 2 * i + 1] = f.y;
-          }
+      for (int k = 0; k < 16 && !last; k += 2) {
+        const int m = cbase + 2 * (k & ~3);
+        const float2 f = next((const bf16*)d.hk_chunks + (ch + H) * 64 * M + (r0 + 4 * (k & 2)) * M + m, m < M);
+        x[k] = f.x;
+        x[k + 1] = f.y;
       }
-      dots_k(v, x, part, false);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) c[2 * j + e] = fmaf(v[4 * j + e], x[4 * j + e], v[4 * j + 2 + e] * x[4 * j + 2 + e]);
+      part_k(c, part, false);
       state_v(endv, v);
       if (ONE) frag_st(tl + S::cSV, v);
-      if (last) {
-        state_v(d.d_hkt ? d.hvt + nh * M * 64 : nullptr, x);
-      } else {
-        const bf16* p = (const bf16*)d.hv_chunks + (ch + H) * M * 64;
+      if (last) state_v(d.d_hkt ? d.hvt + nh * M * 64 : nullptr, x);
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-          for (int i = 0; i < 2; ++i) {
-            const float2 f = r0 + 8 * i < M ? pair_f32(*reinterpret_cast<const uint32_t*>(p + (r0 + 8 * i) * 64 + cbase + 8 * j)) : make_float2(0.f, 0.f);
-            x[4 * j + 2 * i] = f.x;
-            x[4 * j + 2 * i + 1] = f.y;
-          }
+      for (int k = 0; k < 16; k += 2) {
+        const int m = r0 + 4 * (k & 2);
+        if (!last) {
+          const float2 f = next((const bf16*)d.hv_chunks + (ch + H) * M * 64 + m * 64 + cbase + 2 * (k & ~3), m < M);
+          x[k] = f.x;
+          x[k + 1] = f.y;
+        }
+        cv[(k >> 1) & 1] = fmaf(v[k + 1], x[k + 1], fmaf(v[k], x[k], cv[(k >> 1) & 1]));
       }
-      dots_v(v, x, part, false);
+      part_v(cv, part, false);
     }
     SteepCtx sx;
     if (steep) sx = SteepCtx{(const bf16*)d.g + (size_t)h * M, (const bf16*)d.s + (size_t)h * M, rm, t0, c0, len, shift, M};
     float a[16], ga[16], dsum[16];
-    uint32_t s[2][4];
+    uint32_t s[8];
 #pragma unroll
     for (int k = 0; k < 16; ++k) ga[k] = dsum[k] = 0.f;
     for (int ht = 0; ht < NG; ++ht) {
       const int hq = h * NG + ht;
       const bool first = ONE || ht == 0, fin = ONE || ht + 1 == NG;
+      const RowIn rows = row_request(rc, hq);
       if (!first) {
-        load_head(rc, hq);
+        ask(rc, shift, cg, hq, kInQ, kInDO);
         cp_commit();
-        if (uwarp >= 2 && elect_one()) mbar_arrive(&mb[5]);
-        row_request(rc, hq);
+        if (uwarp > kInDO && uwarp < kIns && elect_one()) mbar_arrive(&mb[5]);
       }
       loads_wait();
       hand_over();
@@ -589,7 +577,7 @@ nha_bwd_slot64_kernel(const nha_chunk_desc d, const BwdWs w, int* __restrict__ e
         }
       }
       if (!TERMS) flush();
-      row_stats(rc, hq);
+      row_stats(rows, rc, hq);
       mma_wait(0);
       if (first) {
         frag_ld(tl + S::cC, a);
@@ -619,58 +607,40 @@ nha_bwd_slot64_kernel(const nha_chunk_desc d, const BwdWs w, int* __restrict__ e
       tril_to(S::cB, S::tB);
       if (first) {
         __syncthreads();
-        // a = exp(G - R), SB = s' exp(R - G) (steep: R = 0, and s' exp(Gend - G)), and the states times exp(R)
-        ldm4(at(S::tSB, fo0), s[0]);
-        ldm4(at(S::tSB, fo1), s[1]);
-        uint32_t hk[2][4], hv[2][4], sb[2][4];
-        ldm4(at(S::tHk, fo0), hk[0]);
-        ldm4(at(S::tHk, fo1), hk[1]);
-        ldm4(at(S::tHv, fo0), hv[0]);
-        ldm4(at(S::tHv, fo1), hv[1]);
+        // a = exp(G - R), SB = s' exp(R - G), and the states times exp(R)
         const uint32_t pv0 = pair_bf16(tab[kTabP + r0], tab[kTabP + r0]), pv1 = pair_bf16(tab[kTabP + r0 + 8], tab[kTabP + r0 + 8]);
         auto times = [](uint32_t x, uint32_t y) {
           const __nv_bfloat162 z = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&x), *reinterpret_cast<const __nv_bfloat162*>(&y));
           return *reinterpret_cast<const uint32_t*>(&z);
         };
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 c2 = *reinterpret_cast<const float2*>(tab + kTabC + cbase + 8 * j);
-          const float2 p2 = *reinterpret_cast<const float2*>(tab + kTabP + cbase + 8 * j);
-          const uint32_t pk = pair_bf16(p2.x, p2.y);
+        for (int jp = 0; jp < 2; ++jp) {
+          uint32_t hk[4], hv[4], sv[4], sb[4];
+          ldm4(at(S::tSB, fo[jp]), sv);
+          ldm4(at(S::tHk, fo[jp]), hk);
+          ldm4(at(S::tHv, fo[jp]), hv);
 #pragma unroll
-          for (int i = 0; i < 2; ++i) {
-            const int e = 4 * j + 2 * i, q = 2 * (j & 1) + i, jp = j >> 1;
+          for (int q = 0; q < 4; ++q) {                        // rows gq (+ 8 for odd q), columns of block 2 jp + q / 2
+            const int e = 8 * jp + 2 * q, m = cbase + 16 * jp + 8 * (q >> 1);
+            const float2 c2 = *reinterpret_cast<const float2*>(tab + kTabC + m), p2 = *reinterpret_cast<const float2*>(tab + kTabP + m);
             const float x0 = fmaf(a[e], kLog2e, c2.x), x1 = fmaf(a[e + 1], kLog2e, c2.y);
-            const float2 sv = pair_f32(s[jp][q]);
-            sb[jp][q] = pair_bf16(sv.x * exp2f(-x0), sv.y * exp2f(-x1));
+            const float2 f = pair_f32(sv[q]);
+            sb[q] = pair_bf16(f.x * exp2f(-x0), f.y * exp2f(-x1));
             a[e] = exp2f(x0);
             a[e + 1] = exp2f(x1);
-            hk[jp][q] = times(hk[jp][q], pk);
-            hv[jp][q] = times(hv[jp][q], i ? pv1 : pv0);
+            hk[q] = times(hk[q], pair_bf16(p2.x, p2.y));
+            hv[q] = times(hv[q], (q & 1) ? pv1 : pv0);
+            s[4 * jp + q] = sv[q];
           }
+          stm4(at(S::tSB, fo[jp]), sb[0], sb[1], sb[2], sb[3]);
+          stm4(at(S::tHk, fo[jp]), hk[0], hk[1], hk[2], hk[3]);
+          stm4(at(S::tHv, fo[jp]), hv[0], hv[1], hv[2], hv[3]);
         }
-        if (steep) {
+        if (steep) {                                           // no factors on the rows: the steep_ functions put them in
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-              const int e = 4 * j + 2 * i, q = 2 * (j & 1) + i, jp = j >> 1, m = cbase + 8 * j, p = c0 + r0 + 8 * i;
-              const float4 g4 = steep_sums(sx, r0 + 8 * i, m);
-              const float b0 = __expf(g4.z), b1 = __expf(g4.w);
-              const float2 sv = pair_f32(s[jp][q]);
-              sb[jp][q] = pair_bf16(sv.x * b0, sv.y * b1);
-              a[e] = __expf(g4.x);
-              a[e + 1] = __expf(g4.y);
-              // the factor of ds, which is not 1 / a here
-              if (!TERMS && m < M && p < len) *reinterpret_cast<float2*>(w.dga + ((size_t)(t0 + p) * H + h) * M + m) = make_float2(b0, b1);
-            }
-        }
-#pragma unroll
-        for (int jp = 0; jp < 2; ++jp) {
-          const uint32_t fo = jp ? fo1 : fo0;
-          stm4(at(S::tSB, fo), sb[jp][0], sb[jp][1], sb[jp][2], sb[jp][3]);
-          stm4(at(S::tHk, fo), hk[jp][0], hk[jp][1], hk[jp][2], hk[jp][3]);
-          stm4(at(S::tHv, fo), hv[jp][0], hv[jp][1], hv[jp][2], hv[jp][3]);
+          for (int k = 0; k < 16; ++k) a[k] = 1.f;
+          __syncthreads();
+          steep_decay(sx, tile(S::tSB), sx.s, true, tid);
         }
       }
       if (!TERMS) flushed();
@@ -694,41 +664,35 @@ nha_bwd_slot64_kernel(const nha_chunk_desc d, const BwdWs w, int* __restrict__ e
           commit(&mb[1]);
         }
       }
-      if (steep) {
-        steep_x(sx, tile(S::tA), tile(S::tB), w.dkp + ((size_t)(t0 + c0) * H + h) * 64, w.dvp + ((size_t)(t0 + c0) * H + h) * 64, rp, tid);
-        __syncthreads();
-      }
       if (!TERMS && fin) {                                     // DK' and DV'
-        float v[16];
-        if (ONE) frag_ld(tl + S::cSK, v); else state_k(endk, v);
+        const float f0 = tab[kTabF + r0], f1 = tab[kTabF + r0 + 8];
+        float g[16], v[16];
+        if (ONE) {
+          frag_ld_nowait(tl + S::cSK, g);
+          frag_ld_nowait(tl + S::cSV, v);
+          tmem_ld_wait();
+        } else {
+          state_k(endk, g);
+          state_v(endv, v);
+        }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const float2 f = *reinterpret_cast<const float2*>(tab + kTabF + cbase + 8 * j);
-          v[4 * j] *= f.x; v[4 * j + 1] *= f.y; v[4 * j + 2] *= f.x; v[4 * j + 3] *= f.y;
-        }
-        frag_to_tile(at(S::tDK, fo0), at(S::tDK, fo1), v);
-        if (ONE) frag_ld(tl + S::cSV, v); else state_v(endv, v);
-        const float f0 = tab[kTabF + r0], f1 = tab[kTabF + r0 + 8];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          v[4 * j] *= f0; v[4 * j + 1] *= f0; v[4 * j + 2] *= f1; v[4 * j + 3] *= f1;
+          for (int k = 4 * j; k < 4 * j + 4; ++k) {
+            g[k] *= (k & 1) ? f.y : f.x;
+            v[k] *= (k & 2) ? f1 : f0;
+          }
         }
-        frag_to_tile(at(S::tDV, fo0), at(S::tDV, fo1), v);
+        to_tile(S::tDK, g);
+        to_tile(S::tDV, v);
       }
-      if (!TERMS && first && more) {
-        rn = chunk_rec(d, cg - 1);
-        flag = w.flags[ch - H];
-      }
-      float delta[2], nLj[2], nLg[2], dls[2];
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        delta[i] = rowv[r0 + 8 * i];
-        nLj[i] = rowv[64 + r0 + 8 * i];
-        nLg[i] = rowv[128 + r0 + 8 * i];
-        dls[i] = rowv[192 + r0 + 8 * i];
-      }
+      const float nd[2] = {rowv[r0], rowv[r0 + 8]}, nLj[2] = {rowv[64 + r0], rowv[64 + r0 + 8]};   // -delta, -Lj
+      const float sc2 = d.scale * kLog2e;
+      const uint64_t sc22 = pack2(sc2, sc2), scale2 = pack2(d.scale, d.scale);
       mma_wait(1);
-      // ---- slot part of dz (16 columns at a time), decayed bf16 operands, gate terms ---------------------------------------
+      if (steep) steep_rows(sx, tile(S::tA), tile(S::tB), tl + S::cC, tl + S::cD, r0, cbase);
+      // ---- slot part of dz, decayed bf16 operands, gate terms --------------------------------------------------------------
 #pragma unroll
       for (int jp = 0; jp < 2; ++jp) {
         float z[8], y[8];
@@ -736,50 +700,34 @@ nha_bwd_slot64_kernel(const nha_chunk_desc d, const BwdWs w, int* __restrict__ e
         frag_ld8_nowait(tl + S::cD + 16 * jp, y);
         tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const int m = cbase + 16 * jp + 8 * j;
-#pragma unroll
-          for (int i = 0; i < 2; ++i) {
-            const bool live = m < M && c0 + r0 + 8 * i < len;
-            float2 x = make_float2(0.f, 0.f), x2 = x, pr, zr;
-            if (steep && live) {
-              const size_t row = ((size_t)(t0 + c0 + r0 + 8 * i) * H + h) * 64 + m;
-              x = *reinterpret_cast<const float2*>(w.dkp + row);
-              x2 = *reinterpret_cast<const float2*>(w.dvp + row);
-            }
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              const int k = 4 * j + 2 * i + e;
-              const float aI = a[8 * jp + k];
-              float ok = aI * z[k], dps = aI * y[k];
-              if (steep) {
-                ok += e ? x.y : x.x;
-                dps += e ? x2.y : x2.x;
-              }
-              ok *= sc2;                                       // log2 units
-              float ps = 0.f, dz = 0.f;
-              if (live) {
-                ps = exp2f(ok + nLj[i]);
-                dz = ps * (dps - delta[i]);
-                if (d.d_lse_gsa) dz += dls[i] * exp2f(ok + nLg[i]);
-              }
-              if (!TERMS) ga[8 * jp + k] += ok * kLn2 * dz + ps * dps;
-              const float zs = d.scale * dz;
-              (e ? pr.y : pr.x) = ps;
-              (e ? zr.y : zr.x) = zs;
-              z[k] = zs * aI;                                  // scale dz a
-              y[k] = ps * aI;                                  // p a
-            }
-            if (!TERMS && steep && live) {
-              const size_t row = ((size_t)(t0 + c0 + r0 + 8 * i) * HQ + hq) * M + m;
-              *reinterpret_cast<uint32_t*>(w.dza + row) = pair_bf16(zr.x, zr.y);
-              *reinterpret_cast<uint32_t*>(w.paq + row) = pair_bf16(pr.x, pr.y);
-            }
+        for (int k = 0; k < 8; k += 2) {
+          const int i = (k >> 1) & 1, K = 8 * jp + k;
+          const bool mlive = M == 64 || cbase + 16 * jp + 2 * (k & 4) < M;
+          const float L = mlive ? nLj[i] : -INFINITY;
+          const uint64_t a2 = pack2(a[K], a[K + 1]), ok = fmul2(a2, pack2(z[k], z[k + 1])), dps = fmul2(a2, pack2(y[k], y[k + 1]));
+          float e0, e1;
+          unpack2(ffma2(ok, sc22, pack2(L, L)), e0, e1);
+          const uint64_t ps = pack2(exp2f(e0), exp2f(e1));
+          uint64_t dz = fmul2(ps, fadd2(dps, pack2(nd[i], nd[i])));
+          if (DL && d.d_lse_gsa) {
+            const float g = mlive ? rowv[128 + r0 + 8 * i] : -INFINITY, dl = rowv[192 + r0 + 8 * i];
+            unpack2(ffma2(ok, sc22, pack2(g, g)), e0, e1);
+            dz = ffma2(pack2(dl, dl), pack2(exp2f(e0), exp2f(e1)), dz);
           }
+          const uint64_t zs = fmul2(dz, scale2);
+          if (!TERMS) {
+            const uint64_t g = ffma2(ps, dps, ffma2(ok, zs, pack2(ga[K], ga[K + 1])));
+            unpack2(g, ga[K], ga[K + 1]);
+          }
+          unpack2(fmul2(zs, a2), z[k], z[k + 1]);              // scale dz a
+          unpack2(fmul2(ps, a2), y[k], y[k + 1]);              // p a
         }
-        const uint32_t fo = jp ? fo1 : fo0;
-        frag8_to_tile(at(S::tZA, fo), z);
-        frag8_to_tile(at(S::tPA, fo), y);
+        frag8_to_tile(at(S::tZA, fo[jp]), z);
+        frag8_to_tile(at(S::tPA, fo[jp]), y);
+      }
+      if (steep) {
+        __syncthreads();
+        steep_grads(sx, tile(S::tA), tile(S::tB), tile(S::tZA), tile(S::tPA), w.dsp + ((size_t)(t0 + c0) * H + h) * M, rm, !first, tid);
       }
       hand_over();
       if (issuer) {
@@ -814,27 +762,17 @@ nha_bwd_slot64_kernel(const nha_chunk_desc d, const BwdWs w, int* __restrict__ e
         ph ^= 1;
         continue;
       }
-      if (!TERMS && first && more) {                           // the next chunk's rows into L2
-        shift_next = seq_shift(d, rn.n);
+      if (first && more) {                                     // the next chunk's record, and its rows into L2
+        const ChunkRec rn = chunk_rec(d, cg - 1);
+        const int i = uwarp, row = rn.t0 + rn.ci * kChunk;
+        if (i == kInHv && lane == 0) rec_put(cg - 1, rn);
         if (maps.use && elect_one()) {
-          const int row = rn.t0 + rn.ci * kChunk;
-          if (uwarp == 0) prefetch_tile(maps.qg, 0, h * NG, row);
-          if (uwarp == 1) prefetch_tile(maps.dout, 0, h * NG, row);
-          if (uwarp == 2) prefetch_tile(maps.kg, 0, h, row);
-          if (uwarp == 3) prefetch_tile(maps.s, 0, h, row);
-          if (uwarp == 4) prefetch_tile(maps.g, 0, h, row);
-          if (uwarp == 5) prefetch_tile(maps.v, 0, h, row);
-          if (uwarp == 6) prefetch_bytes((const bf16*)d.hk_chunks + (ch - H) * 4096, kTile);
-          if (uwarp == 7) prefetch_bytes((const bf16*)d.hv_chunks + (ch - H) * 4096, kTile);
-          if (uwarp == 6 && !have_stats) prefetch_tile(maps.o, 0, h * NG, row);
+          prefetch_tile(maps.in[i], 0, i < kInK ? h * NG : i < kInHk ? h : 0, i < kInHk ? row : (int)((ch - H) * 64));
+          if (i == 1 && !have_stats) prefetch_tile(maps.o, 0, h * NG, row);
         }
       }
-      if (steep) {
-        steep_grads(sx, tile(S::tA), tile(S::tB), w.dza + ((size_t)(t0 + c0) * HQ + hq) * M, w.paq + ((size_t)(t0 + c0) * HQ + hq) * M,
-                    (int64_t)HQ * M, w.dsp + ((size_t)(t0 + c0) * H + h) * M, rm, !first, tid);
-        mma_wait(2);
-      } else {
-        mma_wait(2);
+      mma_wait(2);
+      if (!steep) {
         tril_to(S::cA, S::tA);
         tril_to(S::cB, S::tB);
       }
@@ -863,8 +801,8 @@ nha_bwd_slot64_kernel(const nha_chunk_desc d, const BwdWs w, int* __restrict__ e
       bool keep[2];
       uint32_t dsp[8];
       if (!fin) {
-        float v[16];
         if (!steep) {
+          float v[16];
           frag_ld(tl + S::cD, v);
 #pragma unroll
           for (int k = 0; k < 16; ++k) dsum[k] += v[k];
@@ -875,64 +813,62 @@ nha_bwd_slot64_kernel(const nha_chunk_desc d, const BwdWs w, int* __restrict__ e
           const int p = c0 + r0 + 8 * i;
           keep[i] = p >= shift && p < len;                     // rows of this lane that are a token's
         }
+        if (steep) steep_ds(sx, tl + S::cD, w.dsp + ((size_t)(t0 + c0) * H + h) * M, rm, r0, cbase);
         float v[16];
         frag_ld(tl + S::cD, v);
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-          for (int i = 0; i < 2; ++i) {
-            const int e = 4 * j + 2 * i, q = 2 * (j & 1) + i, jp = j >> 1, m = cbase + 8 * j;
-            float d0, d1;
-            if (steep) {
-              float2 f = make_float2(0.f, 0.f), add = f;
-              if (keep[i] && m < M) {
-                const size_t row = ((size_t)(t0 + c0 + r0 + 8 * i) * H + h) * M + m;
-                f = *reinterpret_cast<const float2*>(w.dga + row);
-                add = *reinterpret_cast<const float2*>(w.dsp + row);
-              }
-              d0 = fmaf(v[e], f.x, add.x);
-              d1 = fmaf(v[e + 1], f.y, add.y);
-            } else {
-              if (!ONE) { v[e] += dsum[e]; v[e + 1] += dsum[e + 1]; }
-              d0 = __fdividef(v[e], a[e]);
-              d1 = __fdividef(v[e + 1], a[e + 1]);
-            }
-            const float2 sv = pair_f32(s[jp][q]);
-            ga[e] = keep[i] ? ga[e] - sv.x * d0 : 0.f;
-            ga[e + 1] = keep[i] ? ga[e + 1] - sv.y * d1 : 0.f;
-            dsp[2 * j + i] = pair_bf16(d0, d1);
-          }
+        for (int k = 0; k < 16; k += 2) {
+          const int i = (k >> 1) & 1;
+          if (!ONE) { v[k] += dsum[k]; v[k + 1] += dsum[k + 1]; }
+          const float d0 = __fdividef(v[k], a[k]), d1 = __fdividef(v[k + 1], a[k + 1]);
+          const float2 sv = pair_f32(s[k >> 1]);
+          ga[k] = keep[i] ? ga[k] - sv.x * d0 : 0.f;
+          ga[k + 1] = keep[i] ? ga[k + 1] - sv.y * d1 : 0.f;
+          dsp[k >> 1] = pair_bf16(d0, d1);
+        }
         // the state gradient at the chunk's start, and its dot products with the chunk's start state: the next chunk's carry
         {
-          float g[16], x[16];
+          float g[16], c[8], cv[2] = {0.f, 0.f};
+          uint32_t x[4];
           if (ONE) frag_ld_nowait(tl + S::cSK, g); else state_k(endk, g);
           frag_ld(tl + S::cLK, v);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const float2 dec = *reinterpret_cast<const float2*>(tab + kTabD + cbase + 8 * j);
-            const float2 p2 = *reinterpret_cast<const float2*>(tab + kTabP + cbase + 8 * j);
+          for (int jp = 0; jp < 2; ++jp) {
+            ldm4(at(S::tHk, fo[jp]), x);
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
-              const int e = 4 * j + 2 * i;
-              g[e] = fmaf(g[e], dec.x, v[e] * p2.x);
-              g[e + 1] = fmaf(g[e + 1], dec.y, v[e + 1] * p2.y);
+            for (int j = 2 * jp; j < 2 * jp + 2; ++j) {
+              const int m = cbase + 8 * j;
+              const float2 dec = *reinterpret_cast<const float2*>(tab + kTabD + m), p2 = *reinterpret_cast<const float2*>(tab + kTabP + m);
+              const float2 h0 = pair_f32(x[2 * (j & 1)]), h1 = pair_f32(x[2 * (j & 1) + 1]);
+#pragma unroll
+              for (int k = 4 * j; k < 4 * j + 4; ++k) g[k] = fmaf(g[k], (k & 1) ? dec.y : dec.x, v[k] * ((k & 1) ? p2.y : p2.x));
+              c[2 * j] = fmaf(g[4 * j], h0.x, g[4 * j + 2] * h1.x);
+              c[2 * j + 1] = fmaf(g[4 * j + 1], h0.y, g[4 * j + 3] * h1.y);
             }
           }
           if (ONE) frag_st(tl + S::cSK, g);
           else if (more && ci > 0) put_k(w.dkc + (ch - H) * 64 * M, g);
           if (ci == 0 && d.dhk0) put_k(d.dhk0 + nh * 64 * M, g);
-          tile_frag(S::tHk, x);
-          dots_k(g, x, part_next, true);
+          part_k(c, part_next, true);
           if (ONE) frag_ld_nowait(tl + S::cSV, g); else state_v(endv, g);
           frag_ld(tl + S::cLV, v);
           const float d0 = tab[kTabD + r0], d1 = tab[kTabD + r0 + 8], p0 = tab[kTabP + r0], p1 = tab[kTabP + r0 + 8];
 #pragma unroll
-          for (int k = 0; k < 16; ++k) g[k] = fmaf(g[k], (k & 2) ? d1 : d0, v[k] * ((k & 2) ? p1 : p0));
+          for (int jp = 0; jp < 2; ++jp) {
+            ldm4(at(S::tHv, fo[jp]), x);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const int k = 8 * jp + 2 * q, i = q & 1;
+              const float2 hv = pair_f32(x[q]);
+              g[k] = fmaf(g[k], i ? d1 : d0, v[k] * (i ? p1 : p0));
+              g[k + 1] = fmaf(g[k + 1], i ? d1 : d0, v[k + 1] * (i ? p1 : p0));
+              cv[i] = fmaf(g[k + 1], hv.y, fmaf(g[k], hv.x, cv[i]));
+            }
+          }
           if (ONE) frag_st(tl + S::cSV, g);
           else if (more && ci > 0) put_v(w.dvc + (ch - H) * M * 64, g);
           if (ci == 0 && d.dhv0) put_v(d.dhv0 + nh * M * 64, g);
-          tile_frag(S::tHv, x);
-          dots_v(g, x, part_next, true);
+          part_v(cv, part_next, true);
         }
         // reverse running sum over the rows: inside the blocks of eight rows over the lanes, then the later block, then the later
         // quarters and the carry
@@ -952,7 +888,7 @@ nha_bwd_slot64_kernel(const nha_chunk_desc d, const BwdWs w, int* __restrict__ e
             if (gq == 0) tot[4 * (cbase + 8 * j + e) + quarter] = x;
           }
         hand_over();
-        if (more) load_states(rn, cg - 1, shift_next);
+        if (more) ask(rec_get(cg - 1), rec_shift(cg - 1), cg - 1, h * NG, kInV, kInHv);
 #pragma unroll
         for (int j = 0; j < 4; ++j)
 #pragma unroll
@@ -969,22 +905,20 @@ nha_bwd_slot64_kernel(const nha_chunk_desc d, const BwdWs w, int* __restrict__ e
       mma_wait(4);
       ph ^= 1;
       if (fin && more) {
-        load_rows(rn, shift_next);
-        row_request(rn, h * NG);
+        ask(rec_get(cg - 1), rec_shift(cg - 1), cg - 1, h * NG, kInQ, kInG);
+        cp_commit();
       }
       float v[16];
       frag_ld(tl + S::cC, v);
-      frag_to_tile(at(S::tZA, fo0), at(S::tZA, fo1), v);
-      out.q = true;
-      out.tok = t0 + c0;
-      out.hq = hq;
-      out.n = len - c0;
+      to_tile(S::tZA, v);
+      out_c = cg;
+      out_h = hq;
       if (fin) {
         frag_ld(tl + S::cOK, v);
-        frag_to_tile(at(S::tPA, fo0), at(S::tPA, fo1), v);
-        stm4(at(S::tDK, fo0), dsp[0], dsp[1], dsp[2], dsp[3]);
-        stm4(at(S::tDK, fo1), dsp[4], dsp[5], dsp[6], dsp[7]);
-        frag_to_tile(at(S::tDV, fo0), at(S::tDV, fo1), ga);
+        to_tile(S::tPA, v);
+#pragma unroll
+        for (int jp = 0; jp < 2; ++jp) stm4(at(S::tDK, fo[jp]), dsp[4 * jp], dsp[4 * jp + 1], dsp[4 * jp + 2], dsp[4 * jp + 3]);
+        to_tile(S::tDV, ga);
         frag_ld(tl + S::cOV, v);
 #pragma unroll
         for (int i = 0; i < 2; ++i)
@@ -993,31 +927,29 @@ nha_bwd_slot64_kernel(const nha_chunk_desc d, const BwdWs w, int* __restrict__ e
 #pragma unroll
             for (int j = 0; j < 4; ++j) *reinterpret_cast<float2*>(p + 8 * j) = make_float2(v[4 * j + 2 * i], v[4 * j + 2 * i + 1]);
           }
-        out.k = true;
-        out.lo = max(0, shift - c0);
-        out.key = t0 + c0 - shift;
         if (more) fill_half_signs(tile(S::tB), tid);
       }
     }
     if (TERMS) {
-      float v[16];
-      frag_ld(tl + S::cLK, v);
+      const float p0 = tab[kTabP + r0], p1 = tab[kTabP + r0 + 8];
+      float g[16], v[16];
+      frag_ld_nowait(tl + S::cLK, g);
+      frag_ld_nowait(tl + S::cLV, v);
+      tmem_ld_wait();
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const float2 p2 = *reinterpret_cast<const float2*>(tab + kTabP + cbase + 8 * j);
-        v[4 * j] *= p2.x; v[4 * j + 1] *= p2.y; v[4 * j + 2] *= p2.x; v[4 * j + 3] *= p2.y;
-      }
-      put_k(w.dkc + ch * 64 * M, v);
-      frag_ld(tl + S::cLV, v);
-      const float p0 = tab[kTabP + r0], p1 = tab[kTabP + r0 + 8];
 #pragma unroll
-      for (int k = 0; k < 16; ++k) v[k] *= (k & 2) ? p1 : p0;
+        for (int k = 4 * j; k < 4 * j + 4; ++k) {
+          g[k] *= (k & 1) ? p2.y : p2.x;
+          v[k] *= (k & 2) ? p1 : p0;
+        }
+      }
+      put_k(w.dkc + ch * 64 * M, g);
       put_v(w.dvc + ch * M * 64, v);
       break;
     }
     if (!more) break;
-    rc = rn;
-    shift = shift_next;
     par ^= 1;
   }
   if (failed) atomicExch(err, 1);
@@ -1030,6 +962,26 @@ nha_bwd_slot64_kernel(const nha_chunk_desc d, const BwdWs w, int* __restrict__ e
     if (uwarp >= 1 && uwarp <= 4 && elect_one()) bulk_wait_all();
   }
   if (warp == 0) tmem_dealloc(tbase, S::kTmemCols);
+}
+
+template <bool ONE, bool TERMS>
+__global__ void __launch_bounds__(kThreads, SlotSm<ONE, TERMS>::kCtas)
+nha_bwd_slot64_kernel(const __grid_constant__ nha_chunk_desc d, const __grid_constant__ BwdWs w, int* __restrict__ err,
+                      const __grid_constant__ SlotMaps maps, const int win,
+                      const int have_stats) {
+  grid_dep_wait();
+  grid_dep_launch();
+  const int ncb = (int)((d.Ttot + kChunk - 1) / kChunk + d.N);
+  const int wi = blockIdx.x / d.H, h = blockIdx.x - wi * d.H, lo = wi * win;
+  int top = min(ncb, lo + win) - 1;
+  while (top >= lo && d.plan[d.N + 1 + top] < 0) --top;         // chunks that the plan does not use are the last ones
+  if (top < lo) return;
+  int steep = 0;
+  for (int c = lo + threadIdx.x; c <= top; c += kThreads) steep |= w.flags[(size_t)c * d.H + h];
+  if (__syncthreads_or(steep)) slot64_run<ONE, TERMS, true, true, false>(d, w, err, maps, have_stats, h, lo, top);
+  else if (d.M != 64) slot64_run<ONE, TERMS, false, true, false>(d, w, err, maps, have_stats, h, lo, top);
+  else if (!ONE || d.d_lse_gsa) slot64_run<ONE, TERMS, false, true, true>(d, w, err, maps, have_stats, h, lo, top);
+  else slot64_run<ONE, TERMS, false, false, true>(d, w, err, maps, have_stats, h, lo, top);
 }
 
 bool bwd64_supported(const nha_chunk_desc* d) { return d->K == 64 && d->V == 64 && d->M <= 64 && d->scale > 0.f; }
@@ -1066,13 +1018,14 @@ int bwd_slot64_launch(const nha_chunk_desc* d, const BwdWs& w, int dense_T, int*
   SlotMaps maps;
   memset(&maps, 0, sizeof(maps));
   const int64_t rows = nha_chunk_count_bound(d->Ttot, d->N) * d->H * 64;
-  maps.use = d->M == 64 && rows < (int64_t)1 << 31 && make_map_rows_heads(&maps.qg, d->q_gsa, d->Ttot, d->HQ, 64) &&
-             make_map_rows_heads(&maps.kg, d->k_gsa, d->Ttot, d->H, 64) && make_map_rows_heads(&maps.v, d->v, d->Ttot, d->H, 64) &&
-             make_map_rows_heads(&maps.g, d->g, d->Ttot, d->H, 64) && make_map_rows_heads(&maps.s, d->s, d->Ttot, d->H, 64) &&
-             make_map_rows_heads(&maps.dout, d->d_o, d->Ttot, d->HQ, 64) && make_map_rows_heads(&maps.o, d->o, d->Ttot, d->HQ, 64) &&
-             make_map_matrix(&maps.hk, d->hk_chunks, rows, 64, 64) && make_map_matrix(&maps.hv, d->hv_chunks, rows, 64, 64) &&
-             make_map_rows_heads(&maps.dq, d->dq_gsa, d->Ttot, d->HQ, 64) && make_map_rows_heads(&maps.dk, d->dk_gsa, d->Ttot, d->H, 64) &&
-             make_map_rows_heads(&maps.ds, d->ds, d->Ttot, d->H, 64) && make_map_rows_heads(&maps.dg, d->dg, d->Ttot, d->H, 64);
+  CUtensorMap* in = maps.in;
+  maps.use = d->M == 64 && rows < (int64_t)1 << 31 && make_map_rows_heads(&in[kInQ], d->q_gsa, d->Ttot, d->HQ, 64) &&
+             make_map_rows_heads(&in[kInDO], d->d_o, d->Ttot, d->HQ, 64) && make_map_rows_heads(&in[kInK], d->k_gsa, d->Ttot, d->H, 64) &&
+             make_map_rows_heads(&in[kInS], d->s, d->Ttot, d->H, 64) && make_map_rows_heads(&in[kInG], d->g, d->Ttot, d->H, 64) &&
+             make_map_rows_heads(&in[kInV], d->v, d->Ttot, d->H, 64) && make_map_rows_heads(&in[kInHk], d->hk_chunks, rows, 1, 64) &&
+             make_map_rows_heads(&in[kInHv], d->hv_chunks, rows, 1, 64) && make_map_rows_heads(&maps.out[0], d->dq_gsa, d->Ttot, d->HQ, 64) &&
+             make_map_rows_heads(&maps.out[1], d->dk_gsa, d->Ttot, d->H, 64) && make_map_rows_heads(&maps.out[2], d->ds, d->Ttot, d->H, 64) &&
+             make_map_rows_heads(&maps.out[3], d->dg, d->Ttot, d->H, 64) && make_map_rows_heads(&maps.o, d->o, d->Ttot, d->HQ, 64);
   const SlotPlan p = slot64_plan(d, dense_T);
   const bool one = d->HQ == d->H;
   if (p.scan) {

@@ -49,6 +49,13 @@ __device__ __forceinline__ void frag_ld8_nowait(uint32_t taddr, float (&v)[8]) {
                : "r"(taddr)
                : "memory");
 }
+__device__ __forceinline__ void frag_st8(uint32_t taddr, const float (&v)[8]) {
+  const uint32_t* r = reinterpret_cast<const uint32_t*>(v);
+  asm volatile("tcgen05.st.sync.aligned.16x256b.x2.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]),
+               "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // the reverse (rescaling an accumulator in place)
 __device__ __forceinline__ void frag_st(uint32_t taddr, const float (&v)[16]) {
   const uint32_t* r = reinterpret_cast<const uint32_t*>(v);
