@@ -57,6 +57,7 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows128_kernel(const nha_
   const int wl = seq_window(d, rc.n), shift = seq_shift(d, rc.n);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int quarter = warp & 3, half = warp >> 2, gq = lane >> 2, tq = lane & 3;
+  const bool issuer = uniform(threadIdx.x >> 5) == 0;          // the warp whose elected lane issues the products
 
   extern __shared__ unsigned char smem_raw[];
   unsigned char* sm = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -174,7 +175,6 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows128_kernel(const nha_
   uint32_t phase = 0;
   bool failed = false;
   auto mma_wait = [&]() {
-    if (tid == 0) commit(mbar);
     if (!failed && !mbar_wait(mbar, phase)) failed = true;
     phase ^= 1;
     tc_fence_after();
@@ -187,18 +187,27 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows128_kernel(const nha_
   };
   const uint32_t sbase = smem_u32(sm);
   auto at = [&](int t, uint32_t off) { return sbase + (uint32_t)(t * kTile) + off; };
-  auto desc = [&](int t) { return make_desc(sbase + t * kTile); };
-  auto desc2 = [&](int t) { return make_desc_lbo(sbase + t * kTile, kTile); };    // MN-major operand of two 64-column tiles
+  // one round of products by the elected lane of warp 0, committed to the barrier of mma_wait(): f(descriptor of a tile, of an MN-major
+  // operand of two 64-column tiles, tensor memory)
+  auto round = [&](auto f) {
+    if (issuer) {
+      const uint32_t sb = uniform(sbase), tb = uniform(tbase);
+      if (elect_one()) {
+        f([&](int t) { return make_desc(sb + t * kTile); }, [&](int t) { return make_desc_lbo(sb + t * kTile, kTile); }, tb);
+        commit(mbar);
+      }
+    }
+  };
   const uint32_t iKK = idesc64(0, 0), iKM = idesc64(0, 1), iMM = idesc64(1, 1);
   const uint32_t iKK2 = idesc64(0, 0, 128), iKM2 = idesc64(0, 1, 128), iMM2 = idesc64(1, 1, 128);
   // a product over the head dim, both operands K-major
-  auto mma_dd = [&](int col, int ta, int tb) {
-    mma64<0, 0>(tbase + col, desc(ta), desc(tb), iKK, false);
-    mma64<0, 0>(tbase + col, desc(ta + 1), desc(tb + 1), iKK, true);
+  auto mma_dd = [&](auto desc, uint32_t d, int x, int y) {
+    mma64<0, 0>(d, desc(x), desc(y), iKK, false);
+    mma64<0, 0>(d, desc(x + 1), desc(y + 1), iKK, true);
   };
 
   // ---- x, then a and s' .* b ------------------------------------------------------------------------------------------
-  if (tid == 0) mma64<0, 1>(tbase + cA, desc(bufA), desc(bufB), iKM, false);
+  round([&](auto desc, auto desc2, uint32_t tb) { mma64<0, 1>(tb + cA, desc(bufA), desc(bufB), iKM, false); });
   mma_wait();
   const uint32_t fo0 = frag_off(quarter, half, lane, 0), fo1 = frag_off(quarter, half, lane, 1);
   const int r0 = 16 * quarter + gq;                            // this lane's rows: r0 and r0 + 8
@@ -299,11 +308,11 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows128_kernel(const nha_
     const int hq = h * NG + ht;
     cp_wait_all();
     hand_over();
-    if (tid == 0) {
-      mma_dd(cA, tQ, tS0);
-      mma_dd(cAv, tDO, tS1);
-      mma_dd(cY, tDO, tS2);
-    }
+    round([&](auto desc, auto desc2, uint32_t tb) {
+      mma_dd(desc, tb + cA, tQ, tS0);
+      mma_dd(desc, tb + cAv, tDO, tS1);
+      mma_dd(desc, tb + cY, tDO, tS2);
+    });
     row_stats(hq);
     mma_wait();
     load_hk();
@@ -312,12 +321,12 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows128_kernel(const nha_
     tril_to(cAv, bufB);
     cp_wait_all();
     hand_over();
-    if (tid == 0) {
-      mma64<0, 1>(tbase + cA, desc(bufA), desc(tSB), iKM, false);
-      mma64<0, 1>(tbase + cAv, desc(bufB), desc(tSB), iKM, false);
-      mma64<0, 1>(tbase + cQH, desc(tQ), desc(tS2), iKM, false);
-      mma64<0, 1>(tbase + cQH, desc(tQ + 1), desc(tS2 + 1), iKM, true);
-    }
+    round([&](auto desc, auto desc2, uint32_t tb) {
+      mma64<0, 1>(tb + cA, desc(bufA), desc(tSB), iKM, false);
+      mma64<0, 1>(tb + cAv, desc(bufB), desc(tSB), iKM, false);
+      mma64<0, 1>(tb + cQH, desc(tQ), desc(tS2), iKM, false);
+      mma64<0, 1>(tb + cQH, desc(tQ + 1), desc(tS2 + 1), iKM, true);
+    });
     float delta[2], nLj[2], nLg[2], dls[2];
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
@@ -365,11 +374,11 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows128_kernel(const nha_
       frag8_to_tile(at(tPG, fo), pg);
     }
     hand_over();
-    if (tid == 0) {
-      mma64<0, 0>(tbase + cA, desc(bufA), desc(tSB), iKK, false);       // E
-      mma64<1, 1>(tbase + cLK0, desc(tQ), desc(bufB), iMM, false);
-      mma64<1, 1>(tbase + cLV, desc(tPG), desc2(tDO), iMM2, false);
-    }
+    round([&](auto desc, auto desc2, uint32_t tb) {
+      mma64<0, 0>(tb + cA, desc(bufA), desc(tSB), iKK, false);       // E
+      mma64<1, 1>(tb + cLK0, desc(tQ), desc(bufB), iMM, false);
+      mma64<1, 1>(tb + cLV, desc(tPG), desc2(tDO), iMM2, false);
+    });
     // the two copies that the columns pass reads
     block_out(bufA, w.dza + (size_t)hq * M, (int64_t)HQ * M);
     block_out(tPA, w.paq + (size_t)hq * M, (int64_t)HQ * M);
@@ -379,11 +388,11 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows128_kernel(const nha_
     acc_add(cLV, dvc, D, ht > 0);
     acc_add(cLV + 64, dvc + 64, D, ht > 0);
     hand_over();
-    if (tid == 0) {
-      mma64<0, 0>(tbase + cDQ, desc(bufB), desc(tS2), iKK2, false);
-      mma64<0, 1>(tbase + cDQ, desc(bufA), desc2(tS0), iKM2, true);
-      mma64<1, 1>(tbase + cLK1, desc(tQ + 1), desc(bufB), iMM, false);
-    }
+    round([&](auto desc, auto desc2, uint32_t tb) {
+      mma64<0, 0>(tb + cDQ, desc(bufB), desc(tS2), iKK2, false);
+      mma64<0, 1>(tb + cDQ, desc(bufA), desc2(tS0), iKM2, true);
+      mma64<1, 1>(tb + cLK1, desc(tQ + 1), desc(bufB), iMM, false);
+    });
     load_wk(0);                                                 // p a and p e^G have been read
     mma_wait();
     load_q(d.q_swa, tQ, hq);
@@ -395,10 +404,10 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows128_kernel(const nha_
     acc_add(cLK1, dkc + 64 * M, M, ht > 0);
     cp_wait_but_one();
     hand_over();
-    if (tid == 0) {
-      mma_dd(cS, tQ, tS1);
-      mma_dd(cDP, tDO, tS2);
-    }
+    round([&](auto desc, auto desc2, uint32_t tb) {
+      mma_dd(desc, tb + cS, tQ, tS1);
+      mma_dd(desc, tb + cDP, tDO, tS2);
+    });
     mma_wait();
     // ---- window tiles: dz_win, dq_swa ----------------------------------------------------------------------------------
     const bool more = ht + 1 < NG;
@@ -429,13 +438,13 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows128_kernel(const nha_
       }
       if (!fin) cp_wait_all();
       hand_over();
-      if (tid == 0) {
-        mma64<0, 1>(tbase + cDQS, desc(bufA), desc2(i & 1 ? tS0 : tS1), iKM2, i > 0);
+      round([&](auto desc, auto desc2, uint32_t tb) {
+        mma64<0, 1>(tb + cDQS, desc(bufA), desc2(i & 1 ? tS0 : tS1), iKM2, i > 0);
         if (!fin) {
-          mma_dd(cS, tQ, i & 1 ? tS1 : tS0);
-          mma_dd(cDP, tDO, tS2);
+          mma_dd(desc, tb + cS, tQ, i & 1 ? tS1 : tS0);
+          mma_dd(desc, tb + cDP, tDO, tS2);
         }
-      }
+      });
       mma_wait();
       if (i + 2 < ntile) load_wk(i + 2);                        // this tile's keys have been read
       if (fin && more) {

@@ -139,7 +139,6 @@ __global__ void __launch_bounds__(kCarryThreads) nha_bwd_gate_carry_kernel(const
 // ================================================================================================
 #define NHA_MMA_WAIT()                                   \
   do {                                                   \
-    if (tid == 0) commit(mbar);                          \
     if (!failed && !mbar_wait(mbar, phase)) failed = true;          \
     phase ^= 1;                                          \
     tc_fence_after();                                    \
@@ -344,42 +343,49 @@ __global__ void __launch_bounds__(kColsThreads, 1) nha_bwd_cols_umma_kernel(cons
   const int tk = row & 63;
   const bool kactive = lane < 16;
   const int krow = quarter * 16 + (lane & 15);
-  const uint32_t aQ = smem_u32(sm + L::tQ), aDO = smem_u32(sm + L::tDO), aZA = smem_u32(sm + L::tZA);
-  const uint32_t aPA = smem_u32(sm + L::tPA), aK = smem_u32(sm + L::tK), aV = smem_u32(sm + L::tV);
-  const uint32_t aSB = smem_u32(sm + L::tSB), aDK = smem_u32(sm + L::tDK);
-  const uint32_t aDV = smem_u32(sm + L::tDV), aA = smem_u32(sm + L::bufA), aB = smem_u32(sm + L::bufB);
+  const bool issuer = uniform(threadIdx.x >> 5) == 0;
+  // one round of products by the elected lane of warp 0, committed to the barrier of NHA_MMA_WAIT: f(address of shared memory, tensor memory)
+  auto round = [&](auto f) {
+    if (issuer) {
+      const uint32_t sb = uniform(smem_u32(sm)), tb = uniform(tbase);
+      if (elect_one()) {
+        f(sb, tb);
+        commit(mbar);
+      }
+    }
+  };
 
   for (int ht = 0; ht < NG / TH; ++ht) {
     if (ht > 0) NHA_LOAD_HEAD_TILE(ht);
     cp_wait_all();
     NHA_SMEM_TO_MMA();
-    if (tid == 0) {
-      mma_tile(tbase + L::cA, aQ, L::kATile, aK, 8192, R, 64, D / 16, 0, false);         // A  = q k'^T
-      mma_tile(tbase + L::cAv, aDO, L::kATile, aV, 8192, R, 64, D / 16, 0, false);       // Av = do v'^T
-    }
+    round([&](uint32_t sb, uint32_t tb) {
+      mma_tile(tb + L::cA, sb + L::tQ, L::kATile, sb + L::tK, 8192, R, 64, D / 16, 0, false);         // A  = q k'^T
+      mma_tile(tb + L::cAv, sb + L::tDO, L::kATile, sb + L::tV, 8192, R, 64, D / 16, 0, false);       // Av = do v'^T
+    });
     NHA_MMA_WAIT();
     NHA_TRIL_TO_SMEM(L::cA, L::bufA);
     NHA_TRIL_TO_SMEM(L::cAv, L::bufB);
     NHA_SMEM_TO_MMA();
-    if (tid == 0) {
+    round([&](uint32_t sb, uint32_t tb) {
       // ds' (intra) += tril(A)^T dza + tril(Av)^T pa      (both operands MN-major, k = query row)
-      mma_tile_ex(tbase + L::cDS, aA, 0, 1, aZA, 0, 1, 64, 64, R / 16, ht > 0);
-      mma_tile_ex(tbase + L::cDS, aB, 0, 1, aPA, 0, 1, 64, 64, R / 16, true);
-      mma_tile(tbase + L::cA, aZA, L::kATile, aSB, 0, R, 64, 4, 0, false);                // E  = dza SB^T
-      mma_tile(tbase + L::cAv, aPA, L::kATile, aSB, 0, R, 64, 4, 0, false);               // Bv = pa SB^T
-    }
+      mma_tile_ex(tb + L::cDS, sb + L::bufA, 0, 1, sb + L::tZA, 0, 1, 64, 64, R / 16, ht > 0);
+      mma_tile_ex(tb + L::cDS, sb + L::bufB, 0, 1, sb + L::tPA, 0, 1, 64, 64, R / 16, true);
+      mma_tile(tb + L::cA, sb + L::tZA, L::kATile, sb + L::tSB, 0, R, 64, 4, 0, false);                // E  = dza SB^T
+      mma_tile(tb + L::cAv, sb + L::tPA, L::kATile, sb + L::tSB, 0, R, 64, 4, 0, false);               // Bv = pa SB^T
+    });
     NHA_MMA_WAIT();
     NHA_TRIL_TO_SMEM(L::cA, L::bufA);
     NHA_TRIL_TO_SMEM(L::cAv, L::bufB);
     NHA_SMEM_TO_MMA();
-    if (tid == 0) {
+    round([&](uint32_t sb, uint32_t tb) {
 #pragma unroll
       for (int nb = 0; nb < KT; ++nb) {
         // dk' += tril(E)^T q,  dv' += tril(Bv)^T do      (64 output columns at a time)
-        mma_tile_ex(tbase + L::cDK + 64 * nb, aA, 0, 1, aQ + nb * L::kATile, 0, 1, 64, 64, R / 16, ht > 0);
-        mma_tile_ex(tbase + L::cDV + 64 * nb, aB, 0, 1, aDO + nb * L::kATile, 0, 1, 64, 64, R / 16, ht > 0);
+        mma_tile_ex(tb + L::cDK + 64 * nb, sb + L::bufA, 0, 1, sb + L::tQ + nb * L::kATile, 0, 1, 64, 64, R / 16, ht > 0);
+        mma_tile_ex(tb + L::cDV + 64 * nb, sb + L::bufB, 0, 1, sb + L::tDO + nb * L::kATile, 0, 1, 64, 64, R / 16, ht > 0);
       }
-    }
+    });
     NHA_MMA_WAIT();
     tc_fence_before();
     __syncthreads();
@@ -426,18 +432,18 @@ __global__ void __launch_bounds__(kColsThreads, 1) nha_bwd_cols_umma_kernel(cons
     *reinterpret_cast<uint4*>(sm + L::tSB + sw_off(r, c8)) = sbe[j];
   }
   NHA_SMEM_TO_MMA();
-  if (!failed) {
-    if (tid == 0) {
+  {
+    round([&](uint32_t sb, uint32_t tb) {
 #pragma unroll
       for (int nb = 0; nb < KT; ++nb) {
         // dk' += sbe DK^T (DK rows kk as the N rows of a K-major operand), dv' += sbe DV (DV as MN-major, k = slot)
-        mma_tile(tbase + L::cDK + 64 * nb, aSB, 0, aDK + nb * 8192, 0, 64, 64, 4, 0, true);
-        mma_tile(tbase + L::cDV + 64 * nb, aSB, 0, aDV + nb * 8192, 0, 64, 64, 4, 1, true);
+        mma_tile(tb + L::cDK + 64 * nb, sb + L::tSB, 0, sb + L::tDK + nb * 8192, 0, 64, 64, 4, 0, true);
+        mma_tile(tb + L::cDV + 64 * nb, sb + L::tSB, 0, sb + L::tDV + nb * 8192, 0, 64, 64, 4, 1, true);
       }
       // DS2 = k' DK + v' DV^T
-      mma_tile(tbase + L::cDS2, aK, 8192, aDK, 0, 64, 64, D / 16, 1, false);
-      mma_tile(tbase + L::cDS2, aV, 8192, aDV, 8192, 64, 64, D / 16, 0, true);
-    }
+      mma_tile(tb + L::cDS2, sb + L::tK, 8192, sb + L::tDK, 0, 64, 64, D / 16, 1, false);
+      mma_tile(tb + L::cDS2, sb + L::tV, 8192, sb + L::tDV, 8192, 64, 64, D / 16, 0, true);
+    });
     NHA_MMA_WAIT();
   }
   cp_wait_all();

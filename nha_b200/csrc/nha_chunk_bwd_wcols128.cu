@@ -36,6 +36,7 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_wcols128_kernel(const nha
   const int wl = seq_window(d, rc.n);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int quarter = warp & 3, half = warp >> 2, gq = lane >> 2, tq = lane & 3;
+  const bool issuer = uniform(threadIdx.x >> 5) == 0;          // the warp whose elected lane issues the products
 
   extern __shared__ __align__(1024) unsigned char sm[];
   uint64_t* mbar = (uint64_t*)(sm + oBar);
@@ -92,7 +93,6 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_wcols128_kernel(const nha
   uint32_t phase = 0;
   bool failed = false;
   auto mma_wait = [&]() {
-    if (tid == 0) commit(mbar);
     if (!failed && !mbar_wait(mbar, phase)) failed = true;
     phase ^= 1;
     tc_fence_after();
@@ -105,19 +105,28 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_wcols128_kernel(const nha
   };
   const uint32_t sbase = smem_u32(sm);
   auto at = [&](int t, uint32_t off) { return sbase + (uint32_t)(t * kTile) + off; };
-  auto desc = [&](int t) { return make_desc(sbase + t * kTile); };
-  auto desc2 = [&](int t) { return make_desc_lbo(sbase + t * kTile, kTile); };    // MN-major operand of two 64-column tiles
+  // one round of products by the elected lane of warp 0, committed to the barrier of mma_wait(): f(descriptor of a tile, of an MN-major
+  // operand of two 64-column tiles, tensor memory)
+  auto round = [&](auto f) {
+    if (issuer) {
+      const uint32_t sb = uniform(sbase), tb = uniform(tbase);
+      if (elect_one()) {
+        f([&](int t) { return make_desc(sb + t * kTile); }, [&](int t) { return make_desc_lbo(sb + t * kTile, kTile); }, tb);
+        commit(mbar);
+      }
+    }
+  };
   const uint32_t iKK = idesc64(0, 0), iMM = make_idesc(128, 64, 1) | (1u << 15);
-  auto issue_s = [&](int set) {
+  auto issue_s = [&](auto desc, uint32_t tb, int set) {
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-      mma64<0, 0>(tbase + cS, desc(tQ + set + k), desc(tK + k), iKK, k > 0);
-      mma64<0, 0>(tbase + cDP, desc(tDO + set + k), desc(tV + k), iKK, k > 0);
+      mma64<0, 0>(tb + cS, desc(tQ + set + k), desc(tK + k), iKK, k > 0);
+      mma64<0, 0>(tb + cDP, desc(tDO + set + k), desc(tV + k), iKK, k > 0);
     }
   };
   const uint32_t fo0 = frag_off(quarter, half, lane, 0), fo1 = frag_off(quarter, half, lane, 1);
   const float sc2 = d.scale * kLog2e;
-  if (tid == 0) issue_s(0);
+  round([&](auto desc, auto desc2, uint32_t tb) { issue_s(desc, tb, 0); });
   mma_wait();
   for (int i = 0; i < nblk; ++i) {
     const int pq0 = (ci + i / NG) * kChunk + r0, set = (i & 1) * kSet;
@@ -151,11 +160,11 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_wcols128_kernel(const nha
     }
     cp_wait_all();
     hand_over();
-    if (tid == 0) {
-      mma64<1, 1>(tbase + cDV, desc2(tDO + set), desc(tP), iMM, i > 0);
-      mma64<1, 1>(tbase + cDK, desc2(tQ + set), desc(tZ), iMM, i > 0);
-      if (i + 1 < nblk) issue_s(kSet - set);
-    }
+    round([&](auto desc, auto desc2, uint32_t tb) {
+      mma64<1, 1>(tb + cDV, desc2(tDO + set), desc(tP), iMM, i > 0);
+      mma64<1, 1>(tb + cDK, desc2(tQ + set), desc(tZ), iMM, i > 0);
+      if (i + 1 < nblk) issue_s(desc, tb, kSet - set);
+    });
     mma_wait();
     if (i + 2 < nblk) load_block(i + 2);                       // this block's buffers are free again
   }

@@ -53,6 +53,7 @@ __global__ void __launch_bounds__(kThreads, 2) nha_fwd64_kernel(const nha_chunk_
   const int wl = seq_window(d, rc.n), shift = seq_shift(d, rc.n);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int quarter = warp & 3, half = warp >> 2, gq = lane >> 2, tq = lane & 3;
+  const bool issuer = uniform(threadIdx.x >> 5) == 0;          // the warp whose elected lane issues the products
 
   extern __shared__ unsigned char smem_raw[];
   unsigned char* sm = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -116,7 +117,6 @@ __global__ void __launch_bounds__(kThreads, 2) nha_fwd64_kernel(const nha_chunk_
   uint32_t phase = 0;
   bool failed = false;
   auto mma_wait = [&]() {
-    if (tid == 0) commit(mbar);
     if (!failed && !mbar_wait(mbar, phase)) failed = true;
     phase ^= 1;
     tc_fence_after();
@@ -127,14 +127,23 @@ __global__ void __launch_bounds__(kThreads, 2) nha_fwd64_kernel(const nha_chunk_
     __syncthreads();
     tc_fence_after();
   };
-  auto desc = [&](int t) { return make_desc(smem_u32(tile(t))); };
   const uint32_t iKK = idesc64(0, 0), iKM = idesc64(0, 1);
+  const uint32_t sbase = smem_u32(sm);
+  // one round of products: f(descriptor of a tile, tensor memory), committed to the barrier of mma_wait()
+  auto round = [&](auto f) {
+    if (issuer) {
+      const uint32_t sb = uniform(sbase), tb = uniform(tbase);
+      if (elect_one()) {
+        f([&](int t) { return make_desc(sb + t * kTile); }, tb);
+        commit(mbar);
+      }
+    }
+  };
 
   // ---- x, then a and s' .* b ------------------------------------------------------------------------------------------
-  if (tid == 0) mma64<0, 1>(tbase + cA, desc(tP1), desc(tBuf), iKM, false);
+  round([&](auto desc, uint32_t tb) { mma64<0, 1>(tb + cA, desc(tP1), desc(tBuf), iKM, false); });
   mma_wait();
   const uint32_t fo0 = frag_off(quarter, half, lane, 0), fo1 = frag_off(quarter, half, lane, 1);
-  const uint32_t sbase = smem_u32(sm);
   auto at = [&](int t, uint32_t off) { return sbase + (uint32_t)(t * kTile) + off; };
   const int r0 = 16 * quarter + gq;                            // this lane's rows: r0 and r0 + 8
   float a[16];
@@ -179,17 +188,17 @@ __global__ void __launch_bounds__(kThreads, 2) nha_fwd64_kernel(const nha_chunk_
     return;
   }
   // ---- A, QH, S of the newest step -------------------------------------------------------------------------------------
-  auto issue_s = [&](int set) { mma64<0, 0>(tbase + cS, desc(tQS), desc(set ? tWK1 : tWK), idesc64(0, 0, 128), false); };
-  auto issue_pv = [&](int set) {
+  auto issue_s = [&](auto desc, uint32_t tb, int set) { mma64<0, 0>(tb + cS, desc(tQS), desc(set ? tWK1 : tWK), idesc64(0, 0, 128), false); };
+  auto issue_pv = [&](auto desc, uint32_t tb, int set) {
     const uint64_t v = desc(set ? tWV1 : tWV);
-    mma64<0, 1>(tbase + cO, desc(tP0), v, iKM, true);
-    mma64<0, 1>(tbase + cO, desc(tP1), v + 512, iKM, true);      // the second 64 keys: 8192 bytes on
+    mma64<0, 1>(tb + cO, desc(tP0), v, iKM, true);
+    mma64<0, 1>(tb + cO, desc(tP1), v + 512, iKM, true);         // the second 64 keys: 8192 bytes on
   };
-  if (tid == 0) {
-    mma64<0, 0>(tbase + cA, desc(tQ), desc(tK), iKK, false);
-    mma64<0, 1>(tbase + cO, desc(tQ), desc(tHk), iKM, false);
-    issue_s(0);
-  }
+  round([&](auto desc, uint32_t tb) {
+    mma64<0, 0>(tb + cA, desc(tQ), desc(tK), iKK, false);
+    mma64<0, 1>(tb + cO, desc(tQ), desc(tHk), iKM, false);
+    issue_s(desc, tb, 0);
+  });
   mma_wait();
   // tril of the accumulator at cA -> bf16 tile (columns i <= row)
   auto tril_to = [&](int t) {
@@ -205,7 +214,7 @@ __global__ void __launch_bounds__(kThreads, 2) nha_fwd64_kernel(const nha_chunk_
   };
   tril_to(tBuf);
   hand_over();
-  if (tid == 0) mma64<0, 1>(tbase + cA, desc(tBuf), desc(tSB), iKM, false);
+  round([&](auto desc, uint32_t tb) { mma64<0, 1>(tb + cA, desc(tBuf), desc(tSB), iKM, false); });
   // ---- the newest step's logits and maxima while X is formed: this warp's 64 keys, two blocks of 32 ----------------------------
   const float sc2 = d.scale * kLog2e;
   const int pos0 = c0 + r0;
@@ -325,15 +334,15 @@ __global__ void __launch_bounds__(kThreads, 2) nha_fwd64_kernel(const nha_chunk_
   };
   step_probs();
   hand_over();
-  if (tid == 0) {
-    mma64<0, 1>(tbase + cO, desc(tPG), desc(tHv), iKM, false);
-    mma64<0, 0>(tbase + cA, desc(tPA), desc(tSB), iKK, false);
-    issue_pv(0);
-  }
+  round([&](auto desc, uint32_t tb) {
+    mma64<0, 1>(tb + cO, desc(tPG), desc(tHv), iKM, false);
+    mma64<0, 0>(tb + cA, desc(tPA), desc(tSB), iKK, false);
+    issue_pv(desc, tb, 0);
+  });
   mma_wait();
   tril_to(tBuf);
   hand_over();
-  if (tid == 0) mma64<0, 1>(tbase + cO, desc(tBuf), desc(tV), iKM, true);
+  round([&](auto desc, uint32_t tb) { mma64<0, 1>(tb + cO, desc(tBuf), desc(tV), iKM, true); });
   mma_wait();
   // ---- older window steps ----------------------------------------------------------------------------------------------
   if (nsteps > 1) {
@@ -343,7 +352,7 @@ __global__ void __launch_bounds__(kThreads, 2) nha_fwd64_kernel(const nha_chunk_
     cp_commit();
     cp_wait_but_one();
     hand_over();
-    if (tid == 0) issue_s(1);
+    round([&](auto desc, uint32_t tb) { issue_s(desc, tb, 1); });
     mma_wait();
     for (int p = 1; p < nsteps; ++p) {
       float mx[2];
@@ -377,10 +386,10 @@ __global__ void __launch_bounds__(kThreads, 2) nha_fwd64_kernel(const nha_chunk_
       step_probs();
       cp_wait_all();
       hand_over();
-      if (tid == 0) {
-        issue_pv(p & 1);
-        if (p + 1 < nsteps) issue_s((p + 1) & 1);
-      }
+      round([&](auto desc, uint32_t tb) {
+        issue_pv(desc, tb, p & 1);
+        if (p + 1 < nsteps) issue_s(desc, tb, (p + 1) & 1);
+      });
       mma_wait();
       if (p + 2 < nsteps) load_step(p + 2, p & 1);             // this step's buffers are free again
       cp_commit();

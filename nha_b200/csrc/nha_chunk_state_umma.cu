@@ -161,10 +161,14 @@ __global__ void __launch_bounds__(stu::kThreads) nha_state_local_umma_kernel(con
   bool failed = false;
   // every thread observes the arrival of the tiles itself (it reads the weight tile with ordinary loads later)
   if (full && !mbar_wait_limit(&bar[0], 0, kPoll)) failed = true;
-  if (tid == 0 && !failed) {
+  const bool issuer = uniform(threadIdx.x >> 5) == 0;          // the warp whose elected lane issues the products
+  if (issuer) {
     tc_fence_after();
-    mma_tile_ex(tbase, smem_u32(sU), 0, 0, smem_u32(sG), 0, 1, 64, 64, 4, false);
-    commit(&bar[1]);
+    const uint32_t u = uniform(smem_u32(sU)), g = uniform(smem_u32(sG)), tb = uniform(tbase);
+    if (elect_one()) {
+      f64::mma64<0, 1>(tb, make_desc(u), make_desc(g), f64::idesc64(0, 1), false);
+      commit(&bar[1]);
+    }
   }
   if (!failed && !mbar_wait_limit(&bar[1], 0, kPoll)) failed = true;
   tc_fence_after();
@@ -207,21 +211,23 @@ __global__ void __launch_bounds__(stu::kThreads) nha_state_local_umma_kernel(con
   tc_fence_before();
   __syncthreads();
   const uint32_t cV = D == 64 ? f64::kOtherLanes : 64u;
-  if (tid == 0 && !failed) {
+  if (issuer) {
     tc_fence_after();
     // L_k [D x 64] = k'^T sb: both operands MN-major, 16 tokens per k step; with D = 128 the A operand spans two
     // 64-column tiles, kTile bytes apart (LBO).  L_v [64 x D] = sb^T v', 64 columns to an accumulator.
     const uint32_t idk = make_idesc(D, 64, 1) | (1u << 15);
     const uint32_t idv = make_idesc(64, 64, 1) | (1u << 15);
+    const uint32_t ak = uniform(smem_u32(sK)), as = uniform(smem_u32(sS)), av = uniform(smem_u32(sV)), tb = uniform(tbase);
+    if (elect_one()) {
 #pragma unroll
-    for (int ks = 0; ks < 4; ++ks) {
-      mma_f16(tbase, make_desc_lbo(smem_u32(sK) + ks * 2048, kTile), make_desc(smem_u32(sS) + ks * 2048), idk, ks > 0);
+      for (int ks = 0; ks < 4; ++ks) {
+        mma_f16(tb, make_desc_lbo(ak + ks * 2048, kTile), make_desc(as + ks * 2048), idk, ks > 0);
 #pragma unroll
-      for (int t = 0; t < DT; ++t)
-        mma_f16(tbase + cV + t * f64::kOtherLanes, make_desc(smem_u32(sS) + ks * 2048), make_desc(smem_u32(sV) + t * kTile + ks * 2048), idv,
-                ks > 0);
+        for (int t = 0; t < DT; ++t)
+          mma_f16(tb + cV + t * f64::kOtherLanes, make_desc(as + ks * 2048), make_desc(av + t * kTile + ks * 2048), idv, ks > 0);
+      }
+      commit(&bar[1]);
     }
-    commit(&bar[1]);
   }
   if (!failed && !mbar_wait_limit(&bar[1], 1, kPoll)) failed = true;
   tc_fence_after();
