@@ -717,7 +717,8 @@ __global__ void __launch_bounds__(kBwThreads) nha_bwd_flagged_kernel(const nha_c
 // One thread owns four consecutive state elements and fetches kScanBatch chunks ahead of the serial
 // recurrence so that enough loads are in flight to cover the memory latency.
 constexpr int kScanBatch = 8;
-// win: the sums are stored at the last chunk of every `win` and where no sequence ends (1: everywhere): what the walk over runs of chunks starts from.
+// win > 0: for a walk over runs of `win` chunks.  The sums are stored where a run ends inside a sequence, and no terms are read of the
+// chunks whose sequence starts in their own run (the walk itself goes on from there).  0: stored at every chunk.
 __global__ void __launch_bounds__(256) nha_bwd_state_scan_kernel(const nha_chunk_desc d, const BwdWs w, const int win) {
   grid_dep_wait();
   grid_dep_launch();
@@ -735,15 +736,16 @@ __global__ void __launch_bounds__(256) nha_bwd_state_scan_kernel(const nha_chunk
   const int m = is_k ? e % M : e / V;
   const size_t per = is_k ? KM : MV;
   float* buf = is_k ? w.dkc : w.dvc;
+  const int first = win > 0 ? (chunk0 / win + 1) * win - chunk0 : 0;   // first chunk behind the run in which the sequence starts
   float4 run = make_float4(0.f, 0.f, 0.f, 0.f);
   const float* dht = is_k ? d.d_hkt : d.d_hvt;
   if (dht) run = *(const float4*)(dht + nh * per + e);
-  for (int hi = nchunks - 1; hi >= 0; hi -= kScanBatch) {
+  for (int hi = nchunks - 1; hi >= first - 1 && hi >= 0; hi -= kScanBatch) {
     float4 local[kScanBatch], decay[kScanBatch];
 #pragma unroll
     for (int u = 0; u < kScanBatch; ++u) {
       const int ci = hi - u;
-      if (ci >= 0) {
+      if (ci >= first) {
         const size_t cgi = (size_t)(chunk0 + ci) * H + h;
         local[u] = __ldcs((const float4*)(buf + cgi * per + e));
         if (is_k) decay[u] = *(const float4*)(w.gend + cgi * M + m);
@@ -753,9 +755,10 @@ __global__ void __launch_bounds__(256) nha_bwd_state_scan_kernel(const nha_chunk
 #pragma unroll
     for (int u = 0; u < kScanBatch; ++u) {
       const int ci = hi - u;
-      if (ci >= 0) {
+      if (ci >= 0 && ci >= first - 1) {
         const size_t cgi = (size_t)(chunk0 + ci) * H + h;
-        if (win == 1 || ((chunk0 + ci) % win == win - 1 && ci + 1 < nchunks)) __stcs((float4*)(buf + cgi * per + e), run);
+        if (win == 0 || ((chunk0 + ci) % win == win - 1 && ci + 1 < nchunks)) __stcs((float4*)(buf + cgi * per + e), run);
+        if (ci < first) continue;
         float4 a;
         if (is_k) a = make_float4(__expf(decay[u].x), __expf(decay[u].y), __expf(decay[u].z), __expf(decay[u].w));
         else { const float x = __expf(decay[u].x); a = make_float4(x, x, x, x); }
@@ -767,7 +770,7 @@ __global__ void __launch_bounds__(256) nha_bwd_state_scan_kernel(const nha_chunk
     }
   }
   float* d0 = is_k ? d.dhk0 : d.dhv0;
-  if (d0) *(float4*)(d0 + nh * per + e) = run;
+  if (d0 && (win == 0 || nchunks == 0)) *(float4*)(d0 + nh * per + e) = run;   // (else the walk's)
 }
 
 // ================================================================================================
@@ -1136,7 +1139,7 @@ static int bwd_run(const nha_chunk_desc* d, int dense_T, int stage_mask, void* s
       st = check_launch();
       if (st != NHA_OK) return st;
     }
-    bwd_state_scan_launch(d, w, 1, cs);
+    bwd_state_scan_launch(d, w, 0, cs);
     st = check_launch();
     if (st != NHA_OK) return st;
   }

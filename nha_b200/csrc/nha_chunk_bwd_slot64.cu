@@ -271,10 +271,11 @@ __device__ __forceinline__ void mma_step(uint32_t d, uint64_t a, uint64_t b, uin
   mma_f16(d, a + (uint64_t)(ks * (AMN ? 128 : 2)), b + (uint64_t)(ks * (BMN ? 128 : 2)), idesc, acc || ks > 0);
 }
 
-// win: chunks per CTA (TERMS: one).  have_stats: delta and the joint log-sum-exp are in memory already (the terms kernel ran).
+// scanned: the terms kernel ran.  It has left delta and the joint log-sum-exp of the chunks that it took: those whose sequence starts in an
+// earlier run (nothing starts from the others' terms).
 // STEEP: some chunk of the run may be steep; DL: a gradient arrives on lse_gsa.  (Bodies of their own, so that the usual one is small.)
 template <bool ONE, bool TERMS, bool STEEP, bool DL, bool M64>
-__device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs& w, int* __restrict__ err, const SlotMaps& maps, const int have_stats,
+__device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs& w, int* __restrict__ err, const SlotMaps& maps, const int scanned,
                                            const int h, const int lo, const int top) {
   typedef SlotSm<ONE, TERMS> S;
   const int H = d.H, HQ = d.HQ, M = M64 ? 64 : d.M, NG = ONE ? 1 : HQ / H;
@@ -334,7 +335,7 @@ __device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs&
   // row statistics of a head: delta = <do, o> by the threads of a row (do from its tile) and the joint log-sum-exp.  Rows past the end
   // read the last one's.
   struct RowIn { uint4 o[2]; float lsw, lgs, dl; };
-  auto row_request = [&](const ChunkRec& r, int hq) {
+  auto row_request = [&](const ChunkRec& r, int hq, bool have_stats) {
     const int row = tid >> 2, part = tid & 3, pos = min(r.ci * kChunk + row, r.len - 1);
     const size_t i = (size_t)(r.t0 + pos) * HQ + hq;
     RowIn x;
@@ -350,7 +351,7 @@ __device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs&
     }
     return x;
   };
-  auto row_stats = [&](const RowIn& in, const ChunkRec& r, int hq) {
+  auto row_stats = [&](const RowIn& in, const ChunkRec& r, int hq, bool have_stats) {
     const int row = tid >> 2, part = tid & 3, pos = r.ci * kChunk + row;
     float del = __uint_as_float(in.o[0].x), lj = in.lsw;
     if (!have_stats) {
@@ -507,7 +508,7 @@ __device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs&
     const int ci = rc.ci, t0 = rc.t0, len = rc.len, c0 = ci * kChunk, shift = rec_shift(cg);
     const size_t ch = (size_t)cg * H + h, nh = (size_t)rc.n * H + h;
     const bool steep = STEEP && recs[2 * (cg & 3) + 1].y != 0;
-    const bool more = cg > lo, last = c0 + kChunk >= len;
+    const bool more = cg > lo, last = c0 + kChunk >= len, have_stats = !TERMS && scanned && cg - ci < lo;
     float* part = (float*)(sm + S::oPart) + par * 512;
     float* part_next = (float*)(sm + S::oPart) + (par ^ 1) * 512;
     // the state gradient at this chunk's end where it does not come from the chunk behind
@@ -555,7 +556,7 @@ __device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs&
     for (int ht = 0; ht < NG; ++ht) {
       const int hq = h * NG + ht;
       const bool first = ONE || ht == 0, fin = ONE || ht + 1 == NG;
-      const RowIn rows = row_request(rc, hq);
+      const RowIn rows = row_request(rc, hq, have_stats);
       if (!first) {
         ask(rc, shift, cg, hq, kInQ, kInDO);
         cp_commit();
@@ -577,7 +578,7 @@ __device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs&
         }
       }
       if (!TERMS) flush();
-      row_stats(rows, rc, hq);
+      row_stats(rows, rc, hq, have_stats);
       mma_wait(0);
       if (first) {
         frag_ld(tl + S::cC, a);
@@ -586,13 +587,13 @@ __device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs&
           for (int j = 0; j < 4; ++j) {
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-              const float R = a[4 * j + 2 + e], n = steep ? 0.f : rintf(R * kLog2e);
+              const float R = a[4 * j + 2 + e], n = steep ? 0.f : rintf(__fmul_rn(R, kLog2e));   // (explicit roundings: the two kernels agree)
               const int m = cbase + 8 * j + e;
               tab[kTabP + m] = __int_as_float((127 + (int)n) << 23);
-              tab[kTabC + m] = R * kLog2e - n;
+              tab[kTabC + m] = fmaf(R, kLog2e, -n);
               if (!TERMS) {
                 tab[kTabIP + m] = __int_as_float((127 - (int)n) << 23);
-                tab[kTabF + m] = steep ? 1.f : exp2f(2.f * R * kLog2e - n);
+                tab[kTabF + m] = steep ? 1.f : exp2f(fmaf(2.f * R, kLog2e, -n));
                 tab[kTabD + m] = __expf(2.f * R);
               }
             }
@@ -704,11 +705,11 @@ __device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs&
           const int i = (k >> 1) & 1, K = 8 * jp + k;
           const bool mlive = M == 64 || cbase + 16 * jp + 2 * (k & 4) < M;
           const float L = mlive ? nLj[i] : -INFINITY;
-          const uint64_t a2 = pack2(a[K], a[K + 1]), ok = fmul2(a2, pack2(z[k], z[k + 1])), dps = fmul2(a2, pack2(y[k], y[k + 1]));
+          const uint64_t a2 = pack2(a[K], a[K + 1]), ok = fmul2(a2, pack2(z[k], z[k + 1])), y2 = pack2(y[k], y[k + 1]);
           float e0, e1;
           unpack2(ffma2(ok, sc22, pack2(L, L)), e0, e1);
           const uint64_t ps = pack2(exp2f(e0), exp2f(e1));
-          uint64_t dz = fmul2(ps, fadd2(dps, pack2(nd[i], nd[i])));
+          uint64_t dz = fmul2(ps, ffma2(a2, y2, pack2(nd[i], nd[i])));   // (one operation: the two kernels of a call agree to the bit)
           if (DL && d.d_lse_gsa) {
             const float g = mlive ? rowv[128 + r0 + 8 * i] : -INFINITY, dl = rowv[192 + r0 + 8 * i];
             unpack2(ffma2(ok, sc22, pack2(g, g)), e0, e1);
@@ -716,7 +717,7 @@ __device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs&
           }
           const uint64_t zs = fmul2(dz, scale2);
           if (!TERMS) {
-            const uint64_t g = ffma2(ps, dps, ffma2(ok, zs, pack2(ga[K], ga[K + 1])));
+            const uint64_t g = ffma2(ps, fmul2(a2, y2), ffma2(ok, zs, pack2(ga[K], ga[K + 1])));
             unpack2(g, ga[K], ga[K + 1]);
           }
           unpack2(fmul2(zs, a2), z[k], z[k + 1]);              // scale dz a
@@ -768,7 +769,7 @@ __device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs&
         if (i == kInHv && lane == 0) rec_put(cg - 1, rn);
         if (maps.use && elect_one()) {
           prefetch_tile(maps.in[i], 0, i < kInK ? h * NG : i < kInHk ? h : 0, i < kInHk ? row : (int)((ch - H) * 64));
-          if (i == 1 && !have_stats) prefetch_tile(maps.o, 0, h * NG, row);
+          if (i == 1 && !(scanned && cg - 1 - rn.ci < lo)) prefetch_tile(maps.o, 0, h * NG, row);
         }
       }
       mma_wait(2);
@@ -967,32 +968,32 @@ __device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs&
 template <bool ONE, bool TERMS>
 __global__ void __launch_bounds__(kThreads, SlotSm<ONE, TERMS>::kCtas)
 nha_bwd_slot64_kernel(const __grid_constant__ nha_chunk_desc d, const __grid_constant__ BwdWs w, int* __restrict__ err,
-                      const __grid_constant__ SlotMaps maps, const int win,
-                      const int have_stats) {
+                      const __grid_constant__ SlotMaps maps, const int win, const int scanned) {
   grid_dep_wait();
   grid_dep_launch();
   const int ncb = (int)((d.Ttot + kChunk - 1) / kChunk + d.N);
-  const int wi = blockIdx.x / d.H, h = blockIdx.x - wi * d.H, lo = wi * win;
-  int top = min(ncb, lo + win) - 1;
+  const int wi = blockIdx.x / d.H, h = blockIdx.x - wi * d.H, lo = TERMS ? wi : wi * win;
+  int top = TERMS ? wi : min(ncb, lo + win) - 1;
   while (top >= lo && d.plan[d.N + 1 + top] < 0) --top;         // chunks that the plan does not use are the last ones
   if (top < lo) return;
+  if (TERMS && d.plan[d.plan[d.N + 1 + top]] >= top / win * win) return;   // its sequence starts in the chunk's own run
   int steep = 0;
   for (int c = lo + threadIdx.x; c <= top; c += kThreads) steep |= w.flags[(size_t)c * d.H + h];
-  if (__syncthreads_or(steep)) slot64_run<ONE, TERMS, true, true, false>(d, w, err, maps, have_stats, h, lo, top);
-  else if (d.M != 64) slot64_run<ONE, TERMS, false, true, false>(d, w, err, maps, have_stats, h, lo, top);
-  else if (!ONE || d.d_lse_gsa) slot64_run<ONE, TERMS, false, true, true>(d, w, err, maps, have_stats, h, lo, top);
-  else slot64_run<ONE, TERMS, false, false, true>(d, w, err, maps, have_stats, h, lo, top);
+  if (__syncthreads_or(steep)) slot64_run<ONE, TERMS, true, true, false>(d, w, err, maps, scanned, h, lo, top);
+  else if (d.M != 64) slot64_run<ONE, TERMS, false, true, false>(d, w, err, maps, scanned, h, lo, top);
+  else if (!ONE || d.d_lse_gsa) slot64_run<ONE, TERMS, false, true, true>(d, w, err, maps, scanned, h, lo, top);
+  else slot64_run<ONE, TERMS, false, false, true>(d, w, err, maps, scanned, h, lo, top);
 }
 
 bool bwd64_supported(const nha_chunk_desc* d) { return d->K == 64 && d->V == 64 && d->M <= 64 && d->scale > 0.f; }
 
 template <bool ONE, bool TERMS>
-static int slot64_launch(const nha_chunk_desc* d, const BwdWs& w, int* err, const SlotMaps& maps, int win, bool stats, cudaStream_t cs) {
+static int slot64_launch(const nha_chunk_desc* d, const BwdWs& w, int* err, const SlotMaps& maps, int win, bool scanned, cudaStream_t cs) {
   typedef SlotSm<ONE, TERMS> S;
   cudaError_t e = set_max_smem((const void*)nha_bwd_slot64_kernel<ONE, TERMS>, S::total);
   if (e != cudaSuccess) return record_cuda_error(e);
   const int64_t ncb = nha_chunk_count_bound(d->Ttot, d->N);
-  launch_after(nha_bwd_slot64_kernel<ONE, TERMS>, dim3((unsigned)((ncb + win - 1) / win * d->H)), kThreads, S::total, cs, *d, w, err, maps, win, (int)stats);
+  launch_after(nha_bwd_slot64_kernel<ONE, TERMS>, dim3((unsigned)((TERMS ? ncb : (ncb + win - 1) / win) * d->H)), kThreads, S::total, cs, *d, w, err, maps, win, (int)scanned);
   return check_launch();
 }
 
@@ -1029,7 +1030,7 @@ int bwd_slot64_launch(const nha_chunk_desc* d, const BwdWs& w, int dense_T, int*
   const SlotPlan p = slot64_plan(d, dense_T);
   const bool one = d->HQ == d->H;
   if (p.scan) {
-    const int st = one ? slot64_launch<true, true>(d, w, err, maps, 1, false, cs) : slot64_launch<false, true>(d, w, err, maps, 1, false, cs);
+    const int st = one ? slot64_launch<true, true>(d, w, err, maps, p.win, false, cs) : slot64_launch<false, true>(d, w, err, maps, p.win, false, cs);
     if (st != NHA_OK) return st;
     bwd_state_scan_launch(d, w, p.win, cs);
     const int sc = check_launch();
