@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows128_kernel(const nha_
   const bool issuer = uniform(threadIdx.x >> 5) == 0;          // the warp whose elected lane issues the products
 
   extern __shared__ unsigned char smem_raw[];
-  unsigned char* sm = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  unsigned char* sm = align_1024(smem_raw);
   float* ER = (float*)(sm + oER);
   float* rowv = (float*)(sm + oRow);
   uint64_t* mbar = (uint64_t*)(sm + oBar);

@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(kColsThreads, 1) nha_bwd_cols_umma_kernel(cons
   const size_t ch = (size_t)cg * H + h;
 
   extern __shared__ unsigned char smem_raw[];
-  unsigned char* sm = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  unsigned char* sm = align_1024(smem_raw);
   float* Bs = (float*)(sm + L::oG);                   // cumulative gates, then b = exp(R - G)
   float* ER = (float*)(sm + L::oR);                   // exp(R)
   float* cgv = ER + 64;

@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(kThreads, 3) nha_bwd_win64_kernel(const nha_ch
   const bool issuer = uniform(threadIdx.x >> 5) == 0;          // the warp whose elected lane issues the products
 
   extern __shared__ unsigned char smem_raw[];
-  unsigned char* sm = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  unsigned char* sm = align_1024(smem_raw);
   uint64_t* mbar = (uint64_t*)(sm + oBar);
   uint32_t* tslot = (uint32_t*)(mbar + 1);
   auto tile = [&](int i) { return sm + i * kTile; };

@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(pipe::kThreads, 2)
   const bool two = 2 * z + 1 < NG;
 
   extern __shared__ unsigned char smem_raw[];
-  unsigned char* sm = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  unsigned char* sm = align_1024(smem_raw);
   float* ER = (float*)(sm + oER);
   float* xch = (float*)(sm + oX);
   uint64_t* bar = (uint64_t*)(sm + oBar);

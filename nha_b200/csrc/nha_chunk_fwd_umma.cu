@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(UmmaLayout<R>::kThreads, 1) nha_fwd_umma_kerne
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   extern __shared__ unsigned char smem_raw[];
-  unsigned char* sm = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  unsigned char* sm = align_1024(smem_raw);
   float* As = (float*)(sm + L::oA);
   float* ER = (float*)(sm + L::oR);
   uint64_t* mbar = (uint64_t*)(sm + L::oBar);

@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(stu::kThreads) nha_state_local_umma_kernel(con
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   extern __shared__ unsigned char smem_raw[];
-  unsigned char* sm = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  unsigned char* sm = align_1024(smem_raw);
   unsigned char* sU = sm;                         // strictly upper triangular ones [64][64], K-major
   unsigned char* sG = sm + kTile;                 // g' [64 rows][64 slots]
   unsigned char* sS = sm + 2 * kTile;             // s', overwritten by sb
