@@ -286,7 +286,7 @@ __device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs&
   const bool issuer = uwarp == 0;                              // the warp whose elected lane issues the products
 
   extern __shared__ unsigned char smem_raw[];
-  unsigned char* sm = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  unsigned char* sm = align_1024(smem_raw);
   float* tab = (float*)(sm + S::oTab);
   float* rowv = (float*)(sm + S::oRow);
   float* tot = (float*)(sm + S::oTot);
@@ -430,37 +430,37 @@ __device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs&
       if (cbase + 8 * (k >> 2) + (k & 1) > r0 + 4 * (k & 2)) v[k] = 0.f;
     to_tile(t, v);
   };
-  // fp32 rows of a [64][M] or [M][64] state: this thread's part
-  auto state_k = [&](const float* p, float (&v)[16]) {
+  // fp32 rows of a [64][M] or [M][64] state: this thread's part of block jp of 16 columns
+  auto state_k8 = [&](const float* p, int jp, float (&v)[8]) {
 #pragma unroll
-    for (int k = 0; k < 16; k += 2) {
-      const int m = cbase + 2 * (k & ~3);
+    for (int k = 0; k < 8; k += 2) {
+      const int m = cbase + 16 * jp + 2 * (k & 4);
       const float2 x = p && m < M ? *reinterpret_cast<const float2*>(p + (r0 + 4 * (k & 2)) * M + m) : make_float2(0.f, 0.f);
       v[k] = x.x;
       v[k + 1] = x.y;
     }
   };
-  auto state_v = [&](const float* p, float (&v)[16]) {
+  auto state_v8 = [&](const float* p, int jp, float (&v)[8]) {
 #pragma unroll
-    for (int k = 0; k < 16; k += 2) {
+    for (int k = 0; k < 8; k += 2) {
       const int m = r0 + 4 * (k & 2);
-      const float2 x = p && m < M ? *reinterpret_cast<const float2*>(p + m * 64 + cbase + 2 * (k & ~3)) : make_float2(0.f, 0.f);
+      const float2 x = p && m < M ? *reinterpret_cast<const float2*>(p + m * 64 + cbase + 16 * jp + 2 * (k & 4)) : make_float2(0.f, 0.f);
       v[k] = x.x;
       v[k + 1] = x.y;
     }
   };
-  auto put_k = [&](float* p, const float (&v)[16]) {
+  auto put_k8 = [&](float* p, int jp, const float (&v)[8]) {
 #pragma unroll
-    for (int k = 0; k < 16; k += 2) {
-      const int m = cbase + 2 * (k & ~3);
+    for (int k = 0; k < 8; k += 2) {
+      const int m = cbase + 16 * jp + 2 * (k & 4);
       if (m < M) *reinterpret_cast<float2*>(p + (r0 + 4 * (k & 2)) * M + m) = make_float2(v[k], v[k + 1]);
     }
   };
-  auto put_v = [&](float* p, const float (&v)[16]) {
+  auto put_v8 = [&](float* p, int jp, const float (&v)[8]) {
 #pragma unroll
-    for (int k = 0; k < 16; k += 2) {
+    for (int k = 0; k < 8; k += 2) {
       const int m = r0 + 4 * (k & 2);
-      if (m < M) *reinterpret_cast<float2*>(p + m * 64 + cbase + 2 * (k & ~3)) = make_float2(v[k], v[k + 1]);
+      if (m < M) *reinterpret_cast<float2*>(p + m * 64 + cbase + 16 * jp + 2 * (k & 4)) = make_float2(v[k], v[k + 1]);
     }
   };
   // dot products of the carry from a thread's products: columns m of DK . hk over the rows (one part per quarter), rows m of DV . hv
@@ -515,42 +515,49 @@ __device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs&
     const float* endk = last ? (d.d_hkt ? d.d_hkt + nh * 64 * M : nullptr) : w.dkc + ch * 64 * M;
     const float* endv = last ? (d.d_hvt ? d.d_hvt + nh * M * 64 : nullptr) : w.dvc + ch * M * 64;
     if (!TERMS && (last || cg == top)) {
-      float v[16], x[16], c[8], cv[2] = {0.f, 0.f};
+      float v[8], x[8], c[8], cv[2] = {0.f, 0.f};
       auto next = [&](const bf16* p, bool ok) { return ok ? pair_f32(*reinterpret_cast<const uint32_t*>(p)) : make_float2(0.f, 0.f); };
-      state_k(endk, v);
-      if (ONE) frag_st(tl + S::cSK, v);
-      if (last) state_k(d.d_hkt ? d.hkt + nh * 64 * M : nullptr, x);
 #pragma unroll
-      for (int k = 0; k < 16 && !last; k += 2) {
-        const int m = cbase + 2 * (k & ~3);
-        const float2 f = next((const bf16*)d.hk_chunks + (ch + H) * 64 * M + (r0 + 4 * (k & 2)) * M + m, m < M);
-        x[k] = f.x;
-        x[k + 1] = f.y;
-      }
+      for (int jp = 0; jp < 2; ++jp) {
+        state_k8(endk, jp, v);
+        if (ONE) frag_st8(tl + S::cSK + 16 * jp, v);
+        if (last) state_k8(d.d_hkt ? d.hkt + nh * 64 * M : nullptr, jp, x);
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) c[2 * j + e] = fmaf(v[4 * j + e], x[4 * j + e], v[4 * j + 2 + e] * x[4 * j + 2 + e]);
-      part_k(c, part, false);
-      state_v(endv, v);
-      if (ONE) frag_st(tl + S::cSV, v);
-      if (last) state_v(d.d_hkt ? d.hvt + nh * M * 64 : nullptr, x);
-#pragma unroll
-      for (int k = 0; k < 16; k += 2) {
-        const int m = r0 + 4 * (k & 2);
-        if (!last) {
-          const float2 f = next((const bf16*)d.hv_chunks + (ch + H) * M * 64 + m * 64 + cbase + 2 * (k & ~3), m < M);
+        for (int k = 0; k < 8 && !last; k += 2) {
+          const int m = cbase + 16 * jp + 2 * (k & 4);
+          const float2 f = next((const bf16*)d.hk_chunks + (ch + H) * 64 * M + (r0 + 4 * (k & 2)) * M + m, m < M);
           x[k] = f.x;
           x[k + 1] = f.y;
         }
-        cv[(k >> 1) & 1] = fmaf(v[k + 1], x[k + 1], fmaf(v[k], x[k], cv[(k >> 1) & 1]));
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) c[4 * jp + 2 * j + e] = fmaf(v[4 * j + e], x[4 * j + e], v[4 * j + 2 + e] * x[4 * j + 2 + e]);
+      }
+      part_k(c, part, false);
+#pragma unroll
+      for (int jp = 0; jp < 2; ++jp) {
+        state_v8(endv, jp, v);
+        if (ONE) frag_st8(tl + S::cSV + 16 * jp, v);
+        if (last) state_v8(d.d_hkt ? d.hvt + nh * M * 64 : nullptr, jp, x);
+#pragma unroll
+        for (int k = 0; k < 8; k += 2) {
+          const int m = r0 + 4 * (k & 2);
+          if (!last) {
+            const float2 f = next((const bf16*)d.hv_chunks + (ch + H) * M * 64 + m * 64 + cbase + 16 * jp + 2 * (k & 4), m < M);
+            x[k] = f.x;
+            x[k + 1] = f.y;
+          }
+          cv[(k >> 1) & 1] = fmaf(v[k + 1], x[k + 1], fmaf(v[k], x[k], cv[(k >> 1) & 1]));
+        }
       }
       part_v(cv, part, false);
+      if (ONE) tmem_st_wait();
     }
     SteepCtx sx;
     if (steep) sx = SteepCtx{(const bf16*)d.g + (size_t)h * M, (const bf16*)d.s + (size_t)h * M, rm, t0, c0, len, shift, M};
     float a[16], ga[16], dsum[16];
-    uint32_t s[8];
+    uint32_t s[8];                                              // SB, as its tile has it
 #pragma unroll
     for (int k = 0; k < 16; ++k) ga[k] = dsum[k] = 0.f;
     for (int ht = 0; ht < NG; ++ht) {
@@ -631,8 +638,9 @@ __device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs&
             a[e + 1] = exp2f(x1);
             hk[q] = times(hk[q], pair_bf16(p2.x, p2.y));
             hv[q] = times(hv[q], (q & 1) ? pv1 : pv0);
-            s[4 * jp + q] = sv[q];
           }
+#pragma unroll
+          for (int q = 0; q < 4; ++q) s[4 * jp + q] = sb[q];
           stm4(at(S::tSB, fo[jp]), sb[0], sb[1], sb[2], sb[3]);
           stm4(at(S::tHk, fo[jp]), hk[0], hk[1], hk[2], hk[3]);
           stm4(at(S::tHv, fo[jp]), hv[0], hv[1], hv[2], hv[3]);
@@ -667,26 +675,29 @@ __device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs&
       }
       if (!TERMS && fin) {                                     // DK' and DV'
         const float f0 = tab[kTabF + r0], f1 = tab[kTabF + r0 + 8];
-        float g[16], v[16];
-        if (ONE) {
-          frag_ld_nowait(tl + S::cSK, g);
-          frag_ld_nowait(tl + S::cSV, v);
-          tmem_ld_wait();
-        } else {
-          state_k(endk, g);
-          state_v(endv, v);
-        }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 f = *reinterpret_cast<const float2*>(tab + kTabF + cbase + 8 * j);
-#pragma unroll
-          for (int k = 4 * j; k < 4 * j + 4; ++k) {
-            g[k] *= (k & 1) ? f.y : f.x;
-            v[k] *= (k & 2) ? f1 : f0;
+        for (int jp = 0; jp < 2; ++jp) {
+          float g[8], v[8];
+          if (ONE) {
+            frag_ld8_nowait(tl + S::cSK + 16 * jp, g);
+            frag_ld8_nowait(tl + S::cSV + 16 * jp, v);
+            tmem_ld_wait();
+          } else {
+            state_k8(endk, jp, g);
+            state_v8(endv, jp, v);
           }
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const float2 f = *reinterpret_cast<const float2*>(tab + kTabF + cbase + 16 * jp + 8 * j);
+#pragma unroll
+            for (int k = 4 * j; k < 4 * j + 4; ++k) {
+              g[k] *= (k & 1) ? f.y : f.x;
+              v[k] *= (k & 2) ? f1 : f0;
+            }
+          }
+          frag8_to_tile(at(S::tDK, fo[jp]), g);
+          frag8_to_tile(at(S::tDV, fo[jp]), v);
         }
-        to_tile(S::tDK, g);
-        to_tile(S::tDV, v);
       }
       const float nd[2] = {rowv[r0], rowv[r0 + 8]}, nLj[2] = {rowv[64 + r0], rowv[64 + r0 + 8]};   // -delta, -Lj
       const float sc2 = d.scale * kLog2e;
@@ -697,6 +708,7 @@ __device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs&
 #pragma unroll
       for (int jp = 0; jp < 2; ++jp) {
         float z[8], y[8];
+        uint32_t pa[4];
         frag_ld8_nowait(tl + S::cC + 16 * jp, z);
         frag_ld8_nowait(tl + S::cD + 16 * jp, y);
         tmem_ld_wait();
@@ -716,15 +728,16 @@ __device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs&
             dz = ffma2(pack2(dl, dl), pack2(exp2f(e0), exp2f(e1)), dz);
           }
           const uint64_t zs = fmul2(dz, scale2);
+          unpack2(fmul2(ps, a2), e0, e1);                      // p a
+          pa[k >> 1] = pair_bf16(e0, e1);
           if (!TERMS) {
-            const uint64_t g = ffma2(ps, fmul2(a2, y2), ffma2(ok, zs, pack2(ga[K], ga[K + 1])));
-            unpack2(g, ga[K], ga[K + 1]);
+            const float2 r = pair_f32(pa[k >> 1]);             // gate terms ok dz + p dp, the latter as (p a) Y: see below
+            unpack2(ffma2(pack2(r.x, r.y), y2, ffma2(ok, zs, pack2(ga[K], ga[K + 1]))), ga[K], ga[K + 1]);
           }
           unpack2(fmul2(zs, a2), z[k], z[k + 1]);              // scale dz a
-          unpack2(fmul2(ps, a2), y[k], y[k + 1]);              // p a
         }
         frag8_to_tile(at(S::tZA, fo[jp]), z);
-        frag8_to_tile(at(S::tPA, fo[jp]), y);
+        stm4(at(S::tPA, fo[jp]), pa[0], pa[1], pa[2], pa[3]);
       }
       if (steep) {
         __syncthreads();
@@ -817,59 +830,76 @@ __device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs&
         if (steep) steep_ds(sx, tl + S::cD, w.dsp + ((size_t)(t0 + c0) * H + h) * M, rm, r0, cbase);
         float v[16];
         frag_ld(tl + S::cD, v);
+        // The gate terms less s' ds', as SB times what is divided by a for ds'.  A pair of rows adds (p a)[t] Av[t,i] SB[i] to the terms of
+        // row t and takes it off those of row i; with the operands as the products had them, rounded, on both sides the pairs cancel to the
+        // last bit in the sums over the rows behind (error of dg against 64 bits 2.07e-2 with p dp and s' ds' formed in fp32, 4.3e-3 so).
 #pragma unroll
-        for (int k = 0; k < 16; k += 2) {
-          const int i = (k >> 1) & 1;
-          if (!ONE) { v[k] += dsum[k]; v[k + 1] += dsum[k + 1]; }
-          const float d0 = __fdividef(v[k], a[k]), d1 = __fdividef(v[k + 1], a[k + 1]);
-          const float2 sv = pair_f32(s[k >> 1]);
-          ga[k] = keep[i] ? ga[k] - sv.x * d0 : 0.f;
-          ga[k + 1] = keep[i] ? ga[k + 1] - sv.y * d1 : 0.f;
-          dsp[k >> 1] = pair_bf16(d0, d1);
+        for (int jp = 0; jp < 2; ++jp) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int k = 8 * jp + 2 * q, i = q & 1;
+            if (!ONE) { v[k] += dsum[k]; v[k + 1] += dsum[k + 1]; }
+            float2 sv = pair_f32(s[4 * jp + q]);
+            if (steep) {                                       // (a is 1)
+              const bf16* sr = steep_row(sx, sx.s, r0 + 8 * i);
+              const int m = cbase + 16 * jp + 8 * (q >> 1);
+              sv = sr && m < M ? steep_pair(sr, m) : make_float2(0.f, 0.f);
+            }
+            ga[k] = keep[i] ? ga[k] - sv.x * v[k] : 0.f;
+            ga[k + 1] = keep[i] ? ga[k + 1] - sv.y * v[k + 1] : 0.f;
+            dsp[k >> 1] = pair_bf16(__fdividef(v[k], a[k]), __fdividef(v[k + 1], a[k + 1]));
+          }
         }
         // the state gradient at the chunk's start, and its dot products with the chunk's start state: the next chunk's carry
         {
-          float g[16], c[8], cv[2] = {0.f, 0.f};
-          uint32_t x[4];
-          if (ONE) frag_ld_nowait(tl + S::cSK, g); else state_k(endk, g);
-          frag_ld(tl + S::cLK, v);
+          // (16 columns at a time: with whole fragments the registers do not suffice)
+          float c[8], cv[2] = {0.f, 0.f};
 #pragma unroll
           for (int jp = 0; jp < 2; ++jp) {
+            float g[8], l[8];
+            uint32_t x[4];
+            if (ONE) frag_ld8_nowait(tl + S::cSK + 16 * jp, g); else state_k8(endk, jp, g);
+            frag_ld8_nowait(tl + S::cLK + 16 * jp, l);
             ldm4(at(S::tHk, fo[jp]), x);
+            tmem_ld_wait();
 #pragma unroll
-            for (int j = 2 * jp; j < 2 * jp + 2; ++j) {
-              const int m = cbase + 8 * j;
+            for (int j = 0; j < 2; ++j) {
+              const int m = cbase + 16 * jp + 8 * j;
               const float2 dec = *reinterpret_cast<const float2*>(tab + kTabD + m), p2 = *reinterpret_cast<const float2*>(tab + kTabP + m);
-              const float2 h0 = pair_f32(x[2 * (j & 1)]), h1 = pair_f32(x[2 * (j & 1) + 1]);
+              const float2 h0 = pair_f32(x[2 * j]), h1 = pair_f32(x[2 * j + 1]);
 #pragma unroll
-              for (int k = 4 * j; k < 4 * j + 4; ++k) g[k] = fmaf(g[k], (k & 1) ? dec.y : dec.x, v[k] * ((k & 1) ? p2.y : p2.x));
-              c[2 * j] = fmaf(g[4 * j], h0.x, g[4 * j + 2] * h1.x);
-              c[2 * j + 1] = fmaf(g[4 * j + 1], h0.y, g[4 * j + 3] * h1.y);
+              for (int k = 4 * j; k < 4 * j + 4; ++k) g[k] = fmaf(g[k], (k & 1) ? dec.y : dec.x, __fmul_rn(l[k], (k & 1) ? p2.y : p2.x));
+              c[4 * jp + 2 * j] = fmaf(g[4 * j], h0.x, g[4 * j + 2] * h1.x);
+              c[4 * jp + 2 * j + 1] = fmaf(g[4 * j + 1], h0.y, g[4 * j + 3] * h1.y);
             }
+            if (ONE) frag_st8(tl + S::cSK + 16 * jp, g);
+            else if (more && ci > 0) put_k8(w.dkc + (ch - H) * 64 * M, jp, g);
+            if (ci == 0 && d.dhk0) put_k8(d.dhk0 + nh * 64 * M, jp, g);
           }
-          if (ONE) frag_st(tl + S::cSK, g);
-          else if (more && ci > 0) put_k(w.dkc + (ch - H) * 64 * M, g);
-          if (ci == 0 && d.dhk0) put_k(d.dhk0 + nh * 64 * M, g);
           part_k(c, part_next, true);
-          if (ONE) frag_ld_nowait(tl + S::cSV, g); else state_v(endv, g);
-          frag_ld(tl + S::cLV, v);
           const float d0 = tab[kTabD + r0], d1 = tab[kTabD + r0 + 8], p0 = tab[kTabP + r0], p1 = tab[kTabP + r0 + 8];
 #pragma unroll
           for (int jp = 0; jp < 2; ++jp) {
+            float g[8], l[8];
+            uint32_t x[4];
+            if (ONE) frag_ld8_nowait(tl + S::cSV + 16 * jp, g); else state_v8(endv, jp, g);
+            frag_ld8_nowait(tl + S::cLV + 16 * jp, l);
             ldm4(at(S::tHv, fo[jp]), x);
+            tmem_ld_wait();
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-              const int k = 8 * jp + 2 * q, i = q & 1;
+              const int k = 2 * q, i = q & 1;
               const float2 hv = pair_f32(x[q]);
-              g[k] = fmaf(g[k], i ? d1 : d0, v[k] * (i ? p1 : p0));
-              g[k + 1] = fmaf(g[k + 1], i ? d1 : d0, v[k + 1] * (i ? p1 : p0));
+              g[k] = fmaf(g[k], i ? d1 : d0, __fmul_rn(l[k], i ? p1 : p0));
+              g[k + 1] = fmaf(g[k + 1], i ? d1 : d0, __fmul_rn(l[k + 1], i ? p1 : p0));
               cv[i] = fmaf(g[k + 1], hv.y, fmaf(g[k], hv.x, cv[i]));
             }
+            if (ONE) frag_st8(tl + S::cSV + 16 * jp, g);
+            else if (more && ci > 0) put_v8(w.dvc + (ch - H) * M * 64, jp, g);
+            if (ci == 0 && d.dhv0) put_v8(d.dhv0 + nh * M * 64, jp, g);
           }
-          if (ONE) frag_st(tl + S::cSV, g);
-          else if (more && ci > 0) put_v(w.dvc + (ch - H) * M * 64, g);
-          if (ci == 0 && d.dhv0) put_v(d.dhv0 + nh * M * 64, g);
           part_v(cv, part_next, true);
+          if (ONE) tmem_st_wait();
         }
         // reverse running sum over the rows: inside the blocks of eight rows over the lanes, then the later block, then the later
         // quarters and the carry
@@ -933,21 +963,24 @@ __device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs&
     }
     if (TERMS) {
       const float p0 = tab[kTabP + r0], p1 = tab[kTabP + r0 + 8];
-      float g[16], v[16];
-      frag_ld_nowait(tl + S::cLK, g);
-      frag_ld_nowait(tl + S::cLV, v);
-      tmem_ld_wait();
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 p2 = *reinterpret_cast<const float2*>(tab + kTabP + cbase + 8 * j);
+      for (int jp = 0; jp < 2; ++jp) {
+        float g[8], v[8];
+        frag_ld8_nowait(tl + S::cLK + 16 * jp, g);
+        frag_ld8_nowait(tl + S::cLV + 16 * jp, v);
+        tmem_ld_wait();
 #pragma unroll
-        for (int k = 4 * j; k < 4 * j + 4; ++k) {
-          g[k] *= (k & 1) ? p2.y : p2.x;
-          v[k] *= (k & 2) ? p1 : p0;
+        for (int j = 0; j < 2; ++j) {
+          const float2 p2 = *reinterpret_cast<const float2*>(tab + kTabP + cbase + 16 * jp + 8 * j);
+#pragma unroll
+          for (int k = 4 * j; k < 4 * j + 4; ++k) {
+            g[k] *= (k & 1) ? p2.y : p2.x;
+            v[k] *= (k & 2) ? p1 : p0;
+          }
         }
+        put_k8(w.dkc + ch * 64 * M, jp, g);
+        put_v8(w.dvc + ch * M * 64, jp, v);
       }
-      put_k(w.dkc + ch * 64 * M, g);
-      put_v(w.dvc + ch * M * 64, v);
       break;
     }
     if (!more) break;
@@ -965,6 +998,13 @@ __device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs&
   if (warp == 0) tmem_dealloc(tbase, S::kTmemCols);
 }
 
+// A body as a function of its own: the registers of the usual one are then not shared out together with those of the others.
+template <bool ONE, bool TERMS, bool STEEP, bool DL, bool M64>
+__device__ __noinline__ void slot64_apart(const nha_chunk_desc& d, const BwdWs& w, int* __restrict__ err, const SlotMaps& maps, const int scanned,
+                                          const int h, const int lo, const int top) {
+  slot64_run<ONE, TERMS, STEEP, DL, M64>(d, w, err, maps, scanned, h, lo, top);
+}
+
 template <bool ONE, bool TERMS>
 __global__ void __launch_bounds__(kThreads, SlotSm<ONE, TERMS>::kCtas)
 nha_bwd_slot64_kernel(const __grid_constant__ nha_chunk_desc d, const __grid_constant__ BwdWs w, int* __restrict__ err,
@@ -979,9 +1019,9 @@ nha_bwd_slot64_kernel(const __grid_constant__ nha_chunk_desc d, const __grid_con
   if (TERMS && d.plan[d.plan[d.N + 1 + top]] >= top / win * win) return;   // its sequence starts in the chunk's own run
   int steep = 0;
   for (int c = lo + threadIdx.x; c <= top; c += kThreads) steep |= w.flags[(size_t)c * d.H + h];
-  if (__syncthreads_or(steep)) slot64_run<ONE, TERMS, true, true, false>(d, w, err, maps, scanned, h, lo, top);
-  else if (d.M != 64) slot64_run<ONE, TERMS, false, true, false>(d, w, err, maps, scanned, h, lo, top);
-  else if (!ONE || d.d_lse_gsa) slot64_run<ONE, TERMS, false, true, true>(d, w, err, maps, scanned, h, lo, top);
+  if (__syncthreads_or(steep)) slot64_apart<ONE, TERMS, true, true, false>(d, w, err, maps, scanned, h, lo, top);
+  else if (d.M != 64) slot64_apart<ONE, TERMS, false, true, false>(d, w, err, maps, scanned, h, lo, top);
+  else if (d.d_lse_gsa) slot64_apart<ONE, TERMS, false, true, true>(d, w, err, maps, scanned, h, lo, top);
   else slot64_run<ONE, TERMS, false, false, true>(d, w, err, maps, scanned, h, lo, top);
 }
 
