@@ -73,6 +73,7 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows128_kernel(const nha_
   const int64_t rq = (int64_t)HQ * D, rp = (int64_t)H * D, rm = (int64_t)H * M;
   // nt tiles of 64 columns each: rows row .. row + 63 of a [tokens][pitch] tensor from column col on, zeros outside [0, hi)
   auto load_tokens = [&](int t, int nt, const void* base, int64_t pitch, int col, int row, int hi) {
+    const int lr = from_here(tid >> 3);
     const bf16* p = (const bf16*)base + (int64_t)t0 * pitch + col + 8 * lc;
     const bool ok0 = row + lr >= 0 && row + lr < hi, ok1 = row + lr + 32 >= 0 && row + lr + 32 < hi;
     const bf16 *p0 = p + (ok0 ? row + lr : 0) * pitch, *p1 = p + (ok1 ? row + lr + 32 : 0) * pitch;
@@ -90,9 +91,9 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows128_kernel(const nha_
   auto load_q = [&](const void* base, int t, int hq) { load_tokens(t, 2, base, rq, hq * D, c0, len); };
   auto load_kp = [&]() { load_tokens(tS0, 2, d.k_gsa, rp, h * D, c0 - shift, len - shift); };
   auto load_vp = [&]() { load_tokens(tS1, 2, d.v, rp, h * D, c0 - shift, len - shift); };
-  const bf16* hk = (const bf16*)d.hk_chunks + ((size_t)cg * H + h) * D * M;       // [D][M]
-  const bf16* hv = (const bf16*)d.hv_chunks + ((size_t)cg * H + h) * M * D;       // [M][D]
   auto load_hk = [&]() {
+    const int lr = from_here(tid >> 3);
+    const bf16* hk = (const bf16*)d.hk_chunks + ((size_t)cg * H + h) * D * M;     // [D][M]
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
       const bf16* p = hk + (64 * k + lr) * M + 8 * lc;
@@ -100,6 +101,8 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows128_kernel(const nha_
     }
   };
   auto load_hv = [&]() {
+    const int lr = from_here(tid >> 3);
+    const bf16* hv = (const bf16*)d.hv_chunks + ((size_t)cg * H + h) * M * D;     // [M][D]
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
       const bf16* p = hv + lr * D + 64 * k + 8 * lc;
@@ -111,7 +114,7 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows128_kernel(const nha_
   uint4 oreg[4];
   float lsw, lgs, dl;
   auto row_request = [&](int hq) {
-    const int r = tid >> 2, part = tid & 3, pos = c0 + r;
+    const int r = from_here(tid >> 2), part = tid & 3, pos = c0 + r;
 #pragma unroll
     for (int e = 0; e < 4; ++e) oreg[e] = make_uint4(0u, 0u, 0u, 0u);
     lsw = lgs = dl = 0.f;
@@ -128,7 +131,7 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows128_kernel(const nha_
     }
   };
   auto row_stats = [&](int hq) {
-    const int r = tid >> 2, part = tid & 3, pos = c0 + r;
+    const int r = from_here(tid >> 2), part = tid & 3, pos = c0 + r;
     float del = 0.f;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
@@ -268,7 +271,7 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows128_kernel(const nha_
     __syncwarp();
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
-      const int r = r0 + 8 * u;
+      const int r = from_here(r0) + 8 * u;
       if (c0 + r < len)
         *reinterpret_cast<uint4*>(base + (int64_t)(t0 + c0 + r) * pitch + 32 * half + 8 * tq) =
             *reinterpret_cast<const uint4*>(tile(t) + sw_off(r, 4 * half + tq));
@@ -289,17 +292,18 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows128_kernel(const nha_
   auto acc_add = [&](int col, float* base, int ld, bool add) {
     float v[16];
     frag_ld(tl + col, v);
+    const int r = from_here(r0);
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        float2* p = reinterpret_cast<float2*>(base + (size_t)(r0 + 8 * i) * ld + 32 * half + 8 * j + 2 * tq);
+        float2* p = reinterpret_cast<float2*>(base + (size_t)(r + 8 * i) * ld + 32 * half + 8 * j + 2 * tq);
         if (add) red_add2(reinterpret_cast<float*>(p), v[4 * j + 2 * i], v[4 * j + 2 * i + 1]);
         else *p = make_float2(v[4 * j + 2 * i], v[4 * j + 2 * i + 1]);
       }
   };
-  float* dkc = w.dkc + ((size_t)cg * H + h) * D * M;            // [D][M]
-  float* dvc = w.dvc + ((size_t)cg * H + h) * M * D;            // [M][D]
+  auto dkc = [&]() { return w.dkc + ((size_t)from_here(cg) * H + h) * D * M; };     // [D][M]
+  auto dvc = [&]() { return w.dvc + ((size_t)from_here(cg) * H + h) * M * D; };     // [M][D]
   float ga[16];                                                // gate terms ok dz + p dp, summed over the heads
 #pragma unroll
   for (int k = 0; k < 16; ++k) ga[k] = 0.f;
@@ -327,51 +331,61 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows128_kernel(const nha_
       mma64<0, 1>(tb + cQH, desc(tQ), desc(tS2), iKM, false);
       mma64<0, 1>(tb + cQH, desc(tQ + 1), desc(tS2 + 1), iKM, true);
     });
-    float delta[2], nLj[2], nLg[2], dls[2];
+    float delta[2], nLj[2];
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       delta[i] = rowv[r0 + 8 * i];
-      nLj[i] = rowv[64 + r0 + 8 * i];
-      nLg[i] = rowv[128 + r0 + 8 * i];
-      dls[i] = rowv[192 + r0 + 8 * i];
+      nLj[i] = pos0 + 8 * i < len ? rowv[64 + r0 + 8 * i] : -INFINITY;   // a row past the end has no weights
     }
+    const uint64_t sc22 = pack2(sc2, sc2), scale2 = pack2(d.scale, d.scale);
     mma_wait();
-    // ---- slot part of dz (16 columns at a time), decayed bf16 operands, gate terms ---------------------------------------
+    // ---- slot part of dz, decayed bf16 operands, gate terms: eight columns at a time (more do not fit the registers), two by two -----
 #pragma unroll
     for (int jp = 0; jp < 2; ++jp) {
-      float qh[8], xv[8], y0[8], x2[8];
-      frag_ld8_nowait(tl + cQH + 16 * jp, qh);
-      frag_ld8_nowait(tl + cA + 16 * jp, xv);
-      frag_ld8_nowait(tl + cY + 16 * jp, y0);
-      frag_ld8_nowait(tl + cAv + 16 * jp, x2);
-      tmem_ld_wait();
-      float pg[8];
+      uint32_t za[4], zg[4], pa[4], pg[4];
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
-        const float2 er2 = *reinterpret_cast<const float2*>(ER + 32 * half + 16 * jp + 8 * j + 2 * tq);
+        float qh[4], xv[4], y0[4], x2[4];
+        frag_ld4_nowait(tl + cQH + 16 * jp + 8 * j, qh);
+        frag_ld4_nowait(tl + cA + 16 * jp + 8 * j, xv);
+        frag_ld4_nowait(tl + cY + 16 * jp + 8 * j, y0);
+        frag_ld4_nowait(tl + cAv + 16 * jp + 8 * j, x2);
+        tmem_ld_wait();
+        const float2 erf = *reinterpret_cast<const float2*>(ER + 32 * half + 16 * jp + 8 * j + 2 * tq);
+        const uint64_t er = pack2(erf.x, erf.y);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int k = 4 * j + e, i = e >> 1;
-          const float er = (e & 1) ? er2.y : er2.x, aI = a[8 * jp + k];
-          const float ok = sc2 * aI * (er * qh[k] + xv[k]);     // log2 units
-          const float dps = aI * (er * y0[k] + x2[k]);
-          float ps = 0.f, dz = 0.f;
-          if (pos0 + 8 * i < len) {
-            ps = exp2f(ok + nLj[i]);
-            dz = ps * (dps - delta[i]) + dls[i] * exp2f(ok + nLg[i]);
+        for (int i = 0; i < 2; ++i) {
+          const int k = 2 * i, K = 8 * jp + 4 * j + k, q = 2 * j + i;
+          const uint64_t aI = pack2(a[K], a[K + 1]);
+          const uint64_t ok = fmul2(aI, ffma2(er, pack2(qh[k], qh[k + 1]), pack2(xv[k], xv[k + 1])));
+          const uint64_t dps = fmul2(aI, ffma2(er, pack2(y0[k], y0[k + 1]), pack2(x2[k], x2[k + 1])));
+          float e0, e1;
+          unpack2(ffma2(ok, sc22, pack2(nLj[i], nLj[i])), e0, e1);
+          const uint64_t ps = pack2(exp2f(e0), exp2f(e1));
+          uint64_t dz = fmul2(ps, fadd2(dps, pack2(-delta[i], -delta[i])));
+          if (d.d_lse_gsa) {
+            const float g = nLj[i] > -INFINITY ? rowv[128 + r0 + 8 * i] : -INFINITY, dl = rowv[192 + r0 + 8 * i];
+            unpack2(ffma2(ok, sc22, pack2(g, g)), e0, e1);
+            dz = ffma2(pack2(dl, dl), pack2(exp2f(e0), exp2f(e1)), dz);
           }
-          ga[8 * jp + k] += ok * kLn2 * dz + ps * dps;
-          xv[k] = d.scale * dz * aI;                            // scale dz a
-          qh[k] = xv[k] * er;                                   // scale dz e^G
-          y0[k] = ps * aI;                                      // p a
-          pg[k] = y0[k] * er;                                   // p e^G
+          const uint64_t zs = fmul2(dz, scale2);
+          unpack2(ffma2(ps, dps, ffma2(ok, zs, pack2(ga[K], ga[K + 1]))), ga[K], ga[K + 1]);
+          const uint64_t z2 = fmul2(zs, aI), p2 = fmul2(ps, aI);
+          unpack2(z2, e0, e1);
+          za[q] = pair_bf16(e0, e1);                            // scale dz a
+          unpack2(fmul2(z2, er), e0, e1);
+          zg[q] = pair_bf16(e0, e1);                            // scale dz e^G
+          unpack2(p2, e0, e1);
+          pa[q] = pair_bf16(e0, e1);                            // p a
+          unpack2(fmul2(p2, er), e0, e1);
+          pg[q] = pair_bf16(e0, e1);                            // p e^G
         }
       }
       const uint32_t fo = jp ? fo1 : fo0;
-      frag8_to_tile(at(bufB, fo), qh);
-      frag8_to_tile(at(bufA, fo), xv);
-      frag8_to_tile(at(tPA, fo), y0);
-      frag8_to_tile(at(tPG, fo), pg);
+      stm4(at(bufB, fo), zg[0], zg[1], zg[2], zg[3]);
+      stm4(at(bufA, fo), za[0], za[1], za[2], za[3]);
+      stm4(at(tPA, fo), pa[0], pa[1], pa[2], pa[3]);
+      stm4(at(tPG, fo), pg[0], pg[1], pg[2], pg[3]);
     }
     hand_over();
     round([&](auto desc, auto desc2, uint32_t tb) {
@@ -384,9 +398,9 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows128_kernel(const nha_
     block_out(tPA, w.paq + (size_t)hq * M, (int64_t)HQ * M);
     mma_wait();
     tril_to(cA, bufA);                                          // (a warp writes the blocks that it has copied out itself)
-    acc_add(cLK0, dkc, M, ht > 0);
-    acc_add(cLV, dvc, D, ht > 0);
-    acc_add(cLV + 64, dvc + 64, D, ht > 0);
+    acc_add(cLK0, dkc(), M, ht > 0);
+    acc_add(cLV, dvc(), D, ht > 0);
+    acc_add(cLV + 64, dvc() + 64, D, ht > 0);
     hand_over();
     round([&](auto desc, auto desc2, uint32_t tb) {
       mma64<0, 0>(tb + cDQ, desc(bufB), desc(tS2), iKK2, false);
@@ -401,7 +415,7 @@ __global__ void __launch_bounds__(kThreads, 2) nha_bwd_rows128_kernel(const nha_
     if (ntile > 1) load_wk(1);
     cp_commit();
     acc_out(cDQ, (bf16*)d.dq_gsa + hq * D, rq);
-    acc_add(cLK1, dkc + 64 * M, M, ht > 0);
+    acc_add(cLK1, dkc() + 64 * M, M, ht > 0);
     cp_wait_but_one();
     hand_over();
     round([&](auto desc, auto desc2, uint32_t tb) {

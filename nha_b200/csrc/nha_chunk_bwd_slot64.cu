@@ -336,7 +336,7 @@ __device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs&
   // read the last one's.
   struct RowIn { uint4 o[2]; float lsw, lgs, dl; };
   auto row_request = [&](const ChunkRec& r, int hq, bool have_stats) {
-    const int row = tid >> 2, part = tid & 3, pos = min(r.ci * kChunk + row, r.len - 1);
+    const int row = from_here(tid >> 2), part = tid & 3, pos = min(r.ci * kChunk + row, r.len - 1);
     const size_t i = (size_t)(r.t0 + pos) * HQ + hq;
     RowIn x;
     x.lgs = d.lse_gsa[i];
@@ -352,7 +352,7 @@ __device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs&
     return x;
   };
   auto row_stats = [&](const RowIn& in, const ChunkRec& r, int hq, bool have_stats) {
-    const int row = tid >> 2, part = tid & 3, pos = r.ci * kChunk + row;
+    const int row = from_here(tid >> 2), part = tid & 3, pos = r.ci * kChunk + row;
     float del = __uint_as_float(in.o[0].x), lj = in.lsw;
     if (!have_stats) {
       del = 0.f;

@@ -49,6 +49,11 @@ __device__ __forceinline__ void frag_ld8_nowait(uint32_t taddr, float (&v)[8]) {
                : "r"(taddr)
                : "memory");
 }
+// 8 columns: v[e]
+__device__ __forceinline__ void frag_ld4_nowait(uint32_t taddr, float (&v)[4]) {
+  uint32_t* r = reinterpret_cast<uint32_t*>(v);
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
+}
 __device__ __forceinline__ void frag_st8(uint32_t taddr, const float (&v)[8]) {
   const uint32_t* r = reinterpret_cast<const uint32_t*>(v);
   asm volatile("tcgen05.st.sync.aligned.16x256b.x2.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]),

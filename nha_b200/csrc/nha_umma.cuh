@@ -18,6 +18,12 @@ namespace umma {
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// A value that the compiler has to take from here: addresses formed from it are formed where they are used, and not in front of a loop
+// and kept in registers that the loop does not have.
+__device__ __forceinline__ int from_here(int x) {
+  asm volatile("" : "+r"(x));
+  return x;
+}
 // The next 1024-byte boundary of a shared array, in a form that leaves the compiler the address space (through an integer of the
 // pointer it would take the array for generic memory: 64-bit addresses, and another check for each access).
 __device__ __forceinline__ unsigned char* align_1024(unsigned char* smem) { return smem + ((1024u - (smem_u32(smem) & 1023u)) & 1023u); }
