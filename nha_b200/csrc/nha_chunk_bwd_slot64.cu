@@ -998,14 +998,14 @@ __device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs&
   if (warp == 0) tmem_dealloc(tbase, S::kTmemCols);
 }
 
-// A body as a function of its own: the registers of the usual one are then not shared out together with those of the others.
-template <bool ONE, bool TERMS, bool STEEP, bool DL, bool M64>
-__device__ __noinline__ void slot64_apart(const nha_chunk_desc& d, const BwdWs& w, int* __restrict__ err, const SlotMaps& maps, const int scanned,
+// The body for runs with steep chunks, as a function of its own: the registers of the other are then not shared out together with its.
+template <bool ONE, bool TERMS>
+__device__ __noinline__ void slot64_steep(const nha_chunk_desc& d, const BwdWs& w, int* __restrict__ err, const SlotMaps& maps, const int scanned,
                                           const int h, const int lo, const int top) {
-  slot64_run<ONE, TERMS, STEEP, DL, M64>(d, w, err, maps, scanned, h, lo, top);
+  slot64_run<ONE, TERMS, true, true, false>(d, w, err, maps, scanned, h, lo, top);
 }
 
-template <bool ONE, bool TERMS>
+template <bool ONE, bool TERMS, bool DL, bool M64>
 __global__ void __launch_bounds__(kThreads, SlotSm<ONE, TERMS>::kCtas)
 nha_bwd_slot64_kernel(const __grid_constant__ nha_chunk_desc d, const __grid_constant__ BwdWs w, int* __restrict__ err,
                       const __grid_constant__ SlotMaps maps, const int win, const int scanned) {
@@ -1019,22 +1019,27 @@ nha_bwd_slot64_kernel(const __grid_constant__ nha_chunk_desc d, const __grid_con
   if (TERMS && d.plan[d.plan[d.N + 1 + top]] >= top / win * win) return;   // its sequence starts in the chunk's own run
   int steep = 0;
   for (int c = lo + threadIdx.x; c <= top; c += kThreads) steep |= w.flags[(size_t)c * d.H + h];
-  if (__syncthreads_or(steep)) slot64_apart<ONE, TERMS, true, true, false>(d, w, err, maps, scanned, h, lo, top);
-  else if (d.M != 64) slot64_apart<ONE, TERMS, false, true, false>(d, w, err, maps, scanned, h, lo, top);
-  else if (d.d_lse_gsa) slot64_apart<ONE, TERMS, false, true, true>(d, w, err, maps, scanned, h, lo, top);
-  else slot64_run<ONE, TERMS, false, false, true>(d, w, err, maps, scanned, h, lo, top);
+  if (__syncthreads_or(steep)) slot64_steep<ONE, TERMS>(d, w, err, maps, scanned, h, lo, top);
+  else slot64_run<ONE, TERMS, false, DL, M64>(d, w, err, maps, scanned, h, lo, top);
 }
 
 bool bwd64_supported(const nha_chunk_desc* d) { return d->K == 64 && d->V == 64 && d->M <= 64 && d->scale > 0.f; }
 
-template <bool ONE, bool TERMS>
-static int slot64_launch(const nha_chunk_desc* d, const BwdWs& w, int* err, const SlotMaps& maps, int win, bool scanned, cudaStream_t cs) {
+template <bool ONE, bool TERMS, bool DL, bool M64>
+static int slot64_launch_as(const nha_chunk_desc* d, const BwdWs& w, int* err, const SlotMaps& maps, int win, bool scanned, cudaStream_t cs) {
   typedef SlotSm<ONE, TERMS> S;
-  cudaError_t e = set_max_smem((const void*)nha_bwd_slot64_kernel<ONE, TERMS>, S::total);
+  const auto kernel = nha_bwd_slot64_kernel<ONE, TERMS, DL, M64>;
+  cudaError_t e = set_max_smem((const void*)kernel, S::total);
   if (e != cudaSuccess) return record_cuda_error(e);
   const int64_t ncb = nha_chunk_count_bound(d->Ttot, d->N);
-  launch_after(nha_bwd_slot64_kernel<ONE, TERMS>, dim3((unsigned)((TERMS ? ncb : (ncb + win - 1) / win) * d->H)), kThreads, S::total, cs, *d, w, err, maps, win, (int)scanned);
+  launch_after(kernel, dim3((unsigned)((TERMS ? ncb : (ncb + win - 1) / win) * d->H)), kThreads, S::total, cs, *d, w, err, maps, win, (int)scanned);
   return check_launch();
+}
+template <bool ONE, bool TERMS>
+static int slot64_launch(const nha_chunk_desc* d, const BwdWs& w, int* err, const SlotMaps& maps, int win, bool scanned, cudaStream_t cs) {
+  const auto as = d->M == 64 ? (d->d_lse_gsa ? slot64_launch_as<ONE, TERMS, true, true> : slot64_launch_as<ONE, TERMS, false, true>)
+                             : (d->d_lse_gsa ? slot64_launch_as<ONE, TERMS, true, false> : slot64_launch_as<ONE, TERMS, false, false>);
+  return as(d, w, err, maps, win, scanned, cs);
 }
 
 void bwd_state_scan_launch(const nha_chunk_desc* d, const BwdWs& w, int win, cudaStream_t cs);
