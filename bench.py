@@ -765,9 +765,9 @@ def main():
             dist.all_reduce(t_n, op=dist.ReduceOp.MAX)
             n = int(t_n.item())
         return timed(fn, n) / n
-    # plan, state pass (2), output pass (2), backward: rows and the flagged chunks' general kernel (2), window columns (1),
-    # state-gradient scan + columns + general inter-chunk kernel (3); the general kernels run gated on the chunk flags
-    launches_per_step = 11
+    # plan, state pass (2), output pass and the flagged chunks' general kernel (2), backward: the slot branch (terms and scan, which find nothing
+    # to do where every sequence is walked whole, and the walk) and the window branch (4)
+    launches_per_step = 9
 
     # ---- per-kernel timing: every kernel of a step on its own, CUDA events on the launching stream ----
     kernels = {}
@@ -786,10 +786,8 @@ def main():
     calls = {
         'state_pass': lambda: lib.nha_chunk_state_pass(ctypes.byref(desc), stream),
         'output_pass': lambda: lib.nha_chunk_output_pass(ctypes.byref(desc), stream),
-        'bwd_rows': lambda: lib.nha_chunk_bwd_stage(ctypes.byref(desc), 0, stream),
-        'bwd_window_cols': lambda: lib.nha_chunk_bwd_stage(ctypes.byref(desc), 1, stream),
-        'bwd_state_scan': lambda: lib.nha_chunk_bwd_stage(ctypes.byref(desc), 3, stream),
-        'bwd_cols': lambda: lib.nha_chunk_bwd_stage(ctypes.byref(desc), 4, stream),
+        'bwd_slot': lambda: lib.nha_chunk_bwd_stage(ctypes.byref(desc), 0, stream),
+        'bwd_window': lambda: lib.nha_chunk_bwd_stage(ctypes.byref(desc), 1, stream),
     }
     # compulsory bytes of each stage per token (all heads): what its kernels must read once and write once,
     # scratch that one kernel hands to the next included (e = bf16, f = fp32; states per 64-token chunk)
@@ -800,17 +798,10 @@ def main():
         'state_pass': H * ((2 * D + 2 * M) * e + st * 3 * e),
         # q_gsa, q_swa, k_gsa, k_swa, v, s, g, states in; o and both log-sum-exps out
         'output_pass': H * ((5 * D + 2 * M) * e + st * e + D * e + 2 * f),
-        # q_gsa, q_swa, do, o, k_gsa, k_swa, v, s, g, states, log-sum-exps in; dq_gsa, dq_swa, delta, joint LSE,
-        # gate terms (fp32), two bf16 copies of dz / p, the chunk's state-gradient terms (fp32) out
-        'bwd_rows': H * ((7 * D + 2 * M) * e + st * e + 2 * f + 2 * D * e + 2 * f + M * f + 2 * M * e + st * f),
-        # k_swa, v, q_swa, do, joint LSE, delta in; dk_swa and the fp32 window part of dv out
-        'bwd_window_cols': H * (4 * D * e + 2 * f + D * e + D * f),
-        # general kernel of the slot branch: runs only on chunks flagged by the forward (none here)
-        # in-place scan of the chunks' fp32 state-gradient terms
-        'bwd_state_scan': H * (st * 2 * f),
-        # fp32 state gradients, next states, q_gsa, do, k_gsa, v, s, g, dz / p copies, gate terms, window dv in;
-        # dk_gsa, dv, ds, dg out
-        'bwd_cols': H * (st * (f + e) + (4 * D + 4 * M) * e + M * f + D * f + (2 * D + 2 * M) * e),
+        # q_gsa, do, o, k_gsa, v, s, g, states, log-sum-exps in; dq_gsa, dk_gsa, ds, dg, the slot part of dv (fp32), delta, joint LSE out
+        'bwd_slot': H * ((5 * D + 2 * M) * e + st * e + 2 * f + (2 * D + 2 * M) * e + D * f + 2 * f),
+        # q_swa, do, k_swa, v, the slot part of dv, delta, joint LSE in; dq_swa, dk_swa, dv out
+        'bwd_window': H * (4 * D * e + D * f + 2 * f + 3 * D * e),
     }
     for name, fn in calls.items():
         for _ in range(3):

@@ -1013,13 +1013,18 @@ nha_bwd_slot64_kernel(const __grid_constant__ nha_chunk_desc d, const __grid_con
   grid_dep_launch();
   const int ncb = (int)((d.Ttot + kChunk - 1) / kChunk + d.N);
   const int wi = blockIdx.x / d.H, h = blockIdx.x - wi * d.H, lo = TERMS ? wi : wi * win;
-  int top = TERMS ? wi : min(ncb, lo + win) - 1;
-  while (top >= lo && d.plan[d.N + 1 + top] < 0) --top;         // chunks that the plan does not use are the last ones
-  if (top < lo) return;
-  if (TERMS && d.plan[d.plan[d.N + 1 + top]] >= top / win * win) return;   // its sequence starts in the chunk's own run
-  int steep = 0;
-  for (int c = lo + threadIdx.x; c <= top; c += kThreads) steep |= w.flags[(size_t)c * d.H + h];
-  if (__syncthreads_or(steep)) slot64_steep<ONE, TERMS>(d, w, err, maps, scanned, h, lo, top);
+  int top = TERMS ? wi : min(ncb, lo + win) - 1, steep = 0;
+  if (TERMS) {
+    const ChunkRec rc = chunk_rec(d, top);
+    steep = w.flags[(size_t)top * d.H + h];
+    if (rc.n < 0 || top - rc.ci >= top / win * win) return;     // an unused chunk, or its sequence starts in the chunk's own run
+  } else {
+    while (top >= lo && d.plan[d.N + 1 + top] < 0) --top;       // chunks that the plan does not use are the last ones
+    if (top < lo) return;
+    for (int c = lo + threadIdx.x; c <= top; c += kThreads) steep |= w.flags[(size_t)c * d.H + h];
+    steep = __syncthreads_or(steep);
+  }
+  if (steep) slot64_steep<ONE, TERMS>(d, w, err, maps, scanned, h, lo, top);
   else slot64_run<ONE, TERMS, false, DL, M64>(d, w, err, maps, scanned, h, lo, top);
 }
 
@@ -1044,17 +1049,20 @@ static int slot64_launch(const nha_chunk_desc* d, const BwdWs& w, int* err, cons
 
 void bwd_state_scan_launch(const nha_chunk_desc* d, const BwdWs& w, int win, cudaStream_t cs);
 
-// Chunks per CTA of the walk, and whether the terms and the scan are needed in front of it.  dense_T: tokens of every sequence of the
-// call, or 0.
+// Chunks per CTA of the walk, and whether the terms and the scan run in front of it.  dense_T: tokens of every sequence of the call, or 0.
+// Whole sequences where they fill the machine as well as equal runs do: a run costs a step a chunk, the terms and the scan in front of runs that
+// cut sequences about half of one for every chunk and the launches of six.  Backward of B x 2048 tokens, 16 heads of 64, us, whole | cut: B = 12
+// 485 | 542, 16 535 | 677, 24 834 | 963; B x 512: 8 93 | 115, 16 149 | 176.
+// Where only the caller's max_seqlen says that all sequences are equally long, runs of that length are taken and the terms and the scan launched all the
+// same: they find nothing to do if it is so, and do the rest if it is not.
 struct SlotPlan { int win; bool scan; };
 static SlotPlan slot64_plan(const nha_chunk_desc* d, int dense_T) {
   const int64_t ncb = nha_chunk_count_bound(d->Ttot, d->N), places = 2 * (int64_t)sm_count();
   const int64_t even = (ncb * d->H + places - 1) / places;       // one wave of equal runs
-  if (dense_T > 0) {
-    const int64_t per = (dense_T + kChunk - 1) / kChunk, seqs = (int64_t)d->N * d->H;
-    // whole sequences
-    const int64_t waves = (seqs + places - 1) / places;
-    if (2 * waves * per <= 3 * even + 6) return {(int)per, false};
+  const int64_t T = dense_T > 0 ? dense_T : (int64_t)d->max_seqlen * d->N == d->Ttot ? d->max_seqlen : 0;
+  if (T > 0) {
+    const int64_t per = (T + kChunk - 1) / kChunk, waves = ((int64_t)d->N * d->H + places - 1) / places;
+    if (2 * waves * per <= 3 * even + 6) return {(int)per, dense_T <= 0};
   }
   return {(int)(even > 0 ? even : 1), true};
 }
