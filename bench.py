@@ -52,7 +52,7 @@ CFG = dict(B=16, T=2048, H=16, D=64, M=64, W=64, shift=0)
 WORKLOAD = 'nha_attn_fwd_bwd B16 T2048 H16 D64 M64 W64 chunk64 bf16 (340M-layer shape)'
 CPU_SLICE_T = 512                             # tokens of the B=1 slice both CPU measurements run (cost grows with T)
 # dram__bytes_read.sum + dram__bytes_write.sum of all kernels of one step per token, from the committed ncu captures
-NCU_STEP_TRAFFIC_PER_TOKEN = 1070.8e6 / 8192       # profiles/step_B4_T2048_H16_D64.md
+NCU_STEP_TRAFFIC_PER_TOKEN = 592.8e6 / 8192        # profiles/step_B4_T2048_H16_D64.md, without the terms and the scan that only runs need
 ALG_BYTES_PER_TOKEN = 16512 + 32832          # forward + backward, all 16 heads (each input read once per pass)
 NAMES = ('q_swa', 'k_swa', 'q_gsa', 'k_gsa', 'v', 's', 'g')
 
@@ -765,9 +765,9 @@ def main():
             dist.all_reduce(t_n, op=dist.ReduceOp.MAX)
             n = int(t_n.item())
         return timed(fn, n) / n
-    # plan, state pass (2), output pass and the flagged chunks' general kernel (2), backward: the slot branch (terms and scan, which find nothing
-    # to do where every sequence is walked whole, and the walk) and the window branch (4)
-    launches_per_step = 9
+    # plan, state pass (2), output pass and the flagged chunks' general kernel (2), backward: the walk of the slot branch and the window branch
+    # (2); too few sequences to fill the SMs (B=4): the walk is cut into runs behind its terms and their scan (2 more)
+    launches_per_step = 9 if args.small else 7
 
     # ---- per-kernel timing: every kernel of a step on its own, CUDA events on the launching stream ----
     kernels = {}

@@ -9,19 +9,19 @@ namespace nha {
 struct BwdWs {
   float* delta;   // [Ttot, HQ]      <do, o>
   float* lj;      // [Ttot, HQ]      joint log-sum-exp
-  float* dvacc;   // [Ttot, H, V]    window part of dv
+  float* dvacc;   // [Ttot, H, V]    window part of dv (head dim 64: slot part)
   float* dkp;     // [Ttot, H, K]    intra-chunk part of dk' (row = shifted position)
   float* dvp;     // [Ttot, H, V]    intra-chunk part of dv'
   float* dsp;     // [Ttot, H, M]    intra-chunk part of ds'
   float* dga;     // [Ttot, H, M]    ok .* dz + p .* dp summed over the group
-  bf16* dzg;      // [Ttot, HQ, M]   scale * dz_slot .* exp(G)   (general kernels; the tensor-core rows passes keep both on chip)
+  bf16* dzg;      // [Ttot, HQ, M]   scale * dz_slot .* exp(G)   (general kernels; the tensor-core kernels keep both on chip)
   bf16* pgq;      // [Ttot, HQ, M]   p_slot .* exp(G)
   float* dkc;     // [NC, H, K, M]   first the chunk's own term q^T (scale dz exp G), then (after the scan)
                   //                 the gradient of hk at the END of the chunk
   float* dvc;     // [NC, H, M, V]   likewise (p exp G)^T do, then the gradient of hv at the chunk end
   float* gend;    // [NC, H, M]      total shifted log gate of each chunk
-  bf16* dza;      // [Ttot, HQ, M]   scale * dz_slot .* a   (tensor-core path only)
-  bf16* paq;      // [Ttot, HQ, M]   p_slot .* a            (tensor-core path only)
+  bf16* dza;      // [Ttot, HQ, M]   scale * dz_slot .* a   (tensor-core path at head dim 128 only)
+  bf16* paq;      // [Ttot, HQ, M]   p_slot .* a            (likewise)
   bf16* dkb;      // [NC, H, K, M]   bf16 copy of the scanned dkc (tensor-core path at head dim 128 only, like the next two)
   bf16* dvb;      // [NC, H, M, V]   bf16 copy of the scanned dvc
   float* gcarry;  // [NC, H, M]      gate-gradient carry of all later chunks

@@ -21,10 +21,22 @@
 // A chunk that decays by more than 140 nats (the forward's flag) cannot have one reference.  It takes R = 0 and forms the sums
 // over pairs of rows directly in fp32 (steep_*): slow, exact for any gate, and inside the same walk.
 //
-// What bounds it: SLOT64_BOUND
+// What bounds it: the chain of a chunk, five rounds of products with the element-wise work between them, about 2000 instructions a warp.  With two
+// CTAs of eight warps on an SM the issue slots are 38 % busy, the tensor cores 26 %, HBM a quarter to a third; a warp waits, per instruction
+// issued, 1.6 for tensor memory or a global load, 1.6 for shared memory and shuffles, 1.2 at barriers.  Code beyond the SM's instruction cache of about
+// 48 KB was measured at 5.7 cycles an instruction, which is why rare cases are bodies or functions of their own.  16 warps to a CTA, half as much
+// work for each, were slower (490 us against 384 of that build): the same chain, and more code fetches.
+// Measured, B16 T2048 H16 M64: query-row pass, state-gradient scan and key-row pass of this branch, three kernels that hand dz, p, the terms and
+// the state gradients to each other through memory, 810 us with the rows' window part (about 50); this kernel 335 us, and nothing in between but delta, L
+// and the slot part of dv.  Runs that cut sequences pay the terms and the scan: 32768 packed tokens, longest sequence 8192: 340 us behind 160 + 75.
+// One reference that is a power of two, the states as they are stored, and products issued by an elected lane (see elect_one()) took
+// the walk from 384 to 335 us; dz, p and SB rounded the same way on both sides of the gate terms took dg's error against 64 bits from
+// 2.07e-2 to 4.3e-3 at no cost.
 //
 // Replaces, with nha_chunk_bwd_win64.cu, ChunkNativeHybridAttentionFunction.backward (nha_fla/ops/nha/chunk.py:491-564).
 #include <string.h>
+
+#include <algorithm>
 
 #include "nha_bwd_common.cuh"
 #include "nha_frag64.cuh"
@@ -1012,8 +1024,18 @@ nha_bwd_slot64_kernel(const __grid_constant__ nha_chunk_desc d, const __grid_con
   grid_dep_wait();
   grid_dep_launch();
   const int ncb = (int)((d.Ttot + kChunk - 1) / kChunk + d.N);
-  const int wi = blockIdx.x / d.H, h = blockIdx.x - wi * d.H, lo = TERMS ? wi : wi * win;
-  int top = TERMS ? wi : min(ncb, lo + win) - 1, steep = 0;
+  const int wi = blockIdx.x / d.H, h = blockIdx.x - wi * d.H;
+  const bool whole = !TERMS && win == 0;                       // a run is a sequence
+  const int lo = TERMS ? wi : whole ? d.plan[wi] : wi * win;
+  int top = TERMS ? wi : whole ? d.plan[wi + 1] - 1 : min(ncb, lo + win) - 1, steep = 0;
+  if (whole && top < lo) {                                     // no tokens: the initial state's gradient is the final state's
+    for (int i = threadIdx.x; i < 64 * d.M; i += kThreads) {
+      const size_t at = (size_t)blockIdx.x * 64 * d.M + i;
+      if (d.dhk0) d.dhk0[at] = d.d_hkt ? d.d_hkt[at] : 0.f;
+      if (d.dhv0) d.dhv0[at] = d.d_hvt ? d.d_hvt[at] : 0.f;
+    }
+    return;
+  }
   if (TERMS) {
     const ChunkRec rc = chunk_rec(d, top);
     steep = w.flags[(size_t)top * d.H + h];
@@ -1037,7 +1059,7 @@ static int slot64_launch_as(const nha_chunk_desc* d, const BwdWs& w, int* err, c
   cudaError_t e = set_max_smem((const void*)kernel, S::total);
   if (e != cudaSuccess) return record_cuda_error(e);
   const int64_t ncb = nha_chunk_count_bound(d->Ttot, d->N);
-  launch_after(kernel, dim3((unsigned)((TERMS ? ncb : (ncb + win - 1) / win) * d->H)), kThreads, S::total, cs, *d, w, err, maps, win, (int)scanned);
+  launch_after(kernel, dim3((unsigned)((TERMS ? ncb : win ? (ncb + win - 1) / win : d->N) * d->H)), kThreads, S::total, cs, *d, w, err, maps, win, (int)scanned);
   return check_launch();
 }
 template <bool ONE, bool TERMS>
@@ -1049,22 +1071,22 @@ static int slot64_launch(const nha_chunk_desc* d, const BwdWs& w, int* err, cons
 
 void bwd_state_scan_launch(const nha_chunk_desc* d, const BwdWs& w, int win, cudaStream_t cs);
 
-// Chunks per CTA of the walk, and whether the terms and the scan run in front of it.  dense_T: tokens of every sequence of the call, or 0.
-// Whole sequences where they fill the machine as well as equal runs do: a run costs a step a chunk, the terms and the scan in front of runs that
-// cut sequences about half of one for every chunk and the launches of six.  Backward of B x 2048 tokens, 16 heads of 64, us, whole | cut: B = 12
-// 485 | 542, 16 535 | 677, 24 834 | 963; B x 512: 8 93 | 115, 16 149 | 176.
-// Where only the caller's max_seqlen says that all sequences are equally long, runs of that length are taken and the terms and the scan launched all the
-// same: they find nothing to do if it is so, and do the rest if it is not.
-struct SlotPlan { int win; bool scan; };
-static SlotPlan slot64_plan(const nha_chunk_desc* d, int dense_T) {
+// Chunks per CTA of the walk; 0: a CTA takes a whole sequence, whatever its length, and nothing runs in front of it.  dense_T: tokens of every
+// sequence of the call, or 0.  Whole sequences where they fill the machine as well as equal runs do: a run costs a step a chunk, the terms and the
+// scan in front of runs that cut sequences about half of one for every chunk and the launches of six.  CTAs of at most `per` steps are done
+// after as many waves of them, or after the even share and one more.  Backward of B x 2048 tokens, 16 heads of 64, us, whole | cut: B = 12
+// 485 | 542, 16 535 | 677, 24 834 | 963; B x 512: 8 93 | 115, 16 149 | 176; packed, unequal: 64 sequences of 64-1024 tokens 681 | 788, sorted 618 |
+// 729, 128 of 16-512 (16 heads on 8) 720 | 776, 64 of 1-128 (4 heads) 48 | 78.
+// The caller's max_seqlen is taken at its word for this choice alone.
+static int slot64_plan(const nha_chunk_desc* d, int dense_T) {
   const int64_t ncb = nha_chunk_count_bound(d->Ttot, d->N), places = 2 * (int64_t)sm_count();
   const int64_t even = (ncb * d->H + places - 1) / places;       // one wave of equal runs
-  const int64_t T = dense_T > 0 ? dense_T : (int64_t)d->max_seqlen * d->N == d->Ttot ? d->max_seqlen : 0;
+  const int64_t T = dense_T > 0 ? dense_T : d->max_seqlen;
   if (T > 0) {
     const int64_t per = (T + kChunk - 1) / kChunk, waves = ((int64_t)d->N * d->H + places - 1) / places;
-    if (2 * waves * per <= 3 * even + 6) return {(int)per, dense_T <= 0};
+    if (2 * std::min(waves * per, even + per) <= 3 * even + 6) return 0;
   }
-  return {(int)(even > 0 ? even : 1), true};
+  return (int)std::max<int64_t>(even, 1);
 }
 
 // The caller has checked bwd64_supported().
@@ -1080,16 +1102,16 @@ int bwd_slot64_launch(const nha_chunk_desc* d, const BwdWs& w, int dense_T, int*
              make_map_rows_heads(&in[kInHv], d->hv_chunks, rows, 1, 64) && make_map_rows_heads(&maps.out[0], d->dq_gsa, d->Ttot, d->HQ, 64) &&
              make_map_rows_heads(&maps.out[1], d->dk_gsa, d->Ttot, d->H, 64) && make_map_rows_heads(&maps.out[2], d->ds, d->Ttot, d->H, 64) &&
              make_map_rows_heads(&maps.out[3], d->dg, d->Ttot, d->H, 64) && make_map_rows_heads(&maps.o, d->o, d->Ttot, d->HQ, 64);
-  const SlotPlan p = slot64_plan(d, dense_T);
+  const int win = slot64_plan(d, dense_T);
   const bool one = d->HQ == d->H;
-  if (p.scan) {
-    const int st = one ? slot64_launch<true, true>(d, w, err, maps, p.win, false, cs) : slot64_launch<false, true>(d, w, err, maps, p.win, false, cs);
+  if (win) {
+    const int st = one ? slot64_launch<true, true>(d, w, err, maps, win, false, cs) : slot64_launch<false, true>(d, w, err, maps, win, false, cs);
     if (st != NHA_OK) return st;
-    bwd_state_scan_launch(d, w, p.win, cs);
+    bwd_state_scan_launch(d, w, win, cs);
     const int sc = check_launch();
     if (sc != NHA_OK) return sc;
   }
-  return one ? slot64_launch<true, false>(d, w, err, maps, p.win, p.scan, cs) : slot64_launch<false, false>(d, w, err, maps, p.win, p.scan, cs);
+  return one ? slot64_launch<true, false>(d, w, err, maps, win, win > 0, cs) : slot64_launch<false, false>(d, w, err, maps, win, win > 0, cs);
 }
 
 }  // namespace nha

@@ -1,6 +1,6 @@
 // Backward of the chunked NHA operator on the sm_100a tensor-core path (tcgen05.mma, accumulators in
-// tensor memory).  Two chunk-parallel passes bracket the state-gradient scan of nha_chunk_bwd.cu: the rows pass
-// (nha_chunk_bwd_rows64.cu, nha_chunk_bwd_rows128.cu) and the columns pass (nha_chunk_bwd_cols64.cu; head dim 128: here).
+// tensor memory) at head dim 128 (head dim 64: nha_chunk_bwd_slot64.cu).  Two chunk-parallel passes bracket the state-gradient scan of
+// nha_chunk_bwd.cu: the rows pass (nha_chunk_bwd_rows128.cu) and the columns pass (here).
 //
 //   rows pass  (per chunk, kv head; query-row side)
 //       ok, p_slot recomputed as in the forward;  dp_slot = exp(G) .* (do Hv^T) + a .* (tril(do v'^T) SB)

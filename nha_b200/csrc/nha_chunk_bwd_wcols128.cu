@@ -1,11 +1,13 @@
 // Backward of the window branch, key side, for head dim 128: dk_swa and the window part of dv, every lane at work (nha_frag64.cuh),
-// two CTAs per SM.  As nha_chunk_bwd_wcols64.cu, which says what it computes, one round of products per block of 64 query rows:
+// two CTAs per SM.  With the joint log-sum-exp L and delta = <do, o> of the query-row pass, for every visible pair of a key and a query row
+//     p = exp(scale q_swa k - L),  dz = scale p (do v - delta),  dv += p do,  dk_swa += dz q_swa,
+// one round of products per block of 64 query rows:
 //     dv^T += do^T P,  dk^T += q_swa^T dZ  of block i   together with   S = q_swa k^T,  dP = do v^T  of block i + 1.
 // The sums are kept transposed, head dim along the 128 lanes and keys along 64 columns: as [64 keys][128] accumulators they would
 // take 384 tensor-memory columns with the scores, and only one CTA would fit an SM.
 //
 // What bounds it: the chain of rounds of a CTA.  Measured against two blocks of 64 rows to a product with two rounds per pair and
-// one CTA per SM: 2 x 1999 tokens, 32 heads on 8, window 127, 122 -> 75 us.
+// one CTA per SM: 2 x 1999 tokens, 32 heads on 8, window 127, 122 -> 75 us; issued by an elected lane 73 us.
 //
 // Replaces the third-party flash-attn varlen backward's dk / dv (call site nha_fla/ops/nha/chunk.py:333-344).
 #include "nha_bwd_common.cuh"

@@ -14,7 +14,8 @@
 // What bounds it: the chain of rounds (two CTAs of eight warps per SM; about 13 k cycles per CTA, HBM at half its rate).
 // It waits for the scan as its first instruction, although it needs only Hk and Hv from it: the early start of nha_fwd_pipe_kernel has not
 // been tried here.
-// Measured against the version with one row per lane and the gate scan in shared memory: B16 T2048 H16 W64 373 -> 230 us;
+// Measured against the version with one row per lane and the gate scan in shared memory: B16 T2048 H16 W64 373 -> 230 us, with products issued
+// by an elected lane (see elect_one()) 221-229 us;
 // 32768 packed tokens, windows 32-512, 555 -> 328 us; 8 query heads on 2, 4 x 3000 tokens, W 512, 136 -> 90 us; 32 slots
 // (general kernel before), 4 x 2000 tokens, 194 -> 33 us.
 // Decay factorisation, flags for chunks that decay too fast for one reference per chunk, and the general kernel that takes

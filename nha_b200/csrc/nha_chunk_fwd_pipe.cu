@@ -41,11 +41,12 @@
 // too fast for one reference per chunk, and the general kernel that takes those: as in nha_chunk_fwd_umma.cu.
 //
 // What bounds it: latencies that two CTAs an SM cover in part (issue slots 48 % busy, DRAM 28 %).  Clocks of a tile at W 512, two CTAs
-// an SM: 8 k to the decay factors, 13 k for the slot rounds, 2.2-2.6 k for each of nine window steps (score product, tensor-memory load,
-// exponentials, store, value product), 3 k to the end: nearly half lies in front of the window steps, and all of that but the products
+// an SM: 8 k to the decay factors, 10 k for the slot rounds, 2.0 k for each of nine window steps (400 waiting for the scores, 650 maxima,
+// 850 exponentials), 3 k to the end: nearly half lies in front of the window steps, and all of that but the products
 // with q is the same for every pair of heads of a kv head.  Against one thread a
 // row, the gates scanned in shared memory, and the tiles of a chunk far apart in the grid: 131072 tokens, 32 heads on 8, W 512,
-// 2714 -> 2600-2640 us; 2 x 1999 tokens, 32 heads on 8, W 127, 76 -> 71 us.  An L2 prefetch of a later CTA's tiles: 1 % better in
+// 2714 -> 2600-2640 us, and 2578 with products issued by an elected lane and shared memory
+// addressed as such (on a GPU where it was 2909 before); 2 x 1999 tokens, 32 heads on 8, W 127, 76 -> 71 us.  An L2 prefetch of a later CTA's tiles: 1 % better in
 // the first, 4 % worse in the second.
 //
 // Replaces chunk_nha_fused_o_kernel (nha_fla/ops/nha/chunk_fused.py:117-283) at the long-context shape.

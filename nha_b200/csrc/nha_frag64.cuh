@@ -1,4 +1,4 @@
-// Building blocks of the chunk kernels with 64-row products: all of them at head dim 64, the query-row and window-key passes of the
+// Building blocks of the chunk kernels with 64-row products: those at head dim 64, the query-row and window-key passes of the
 // backward at head dim 128.
 //
 // The accumulator of a product with M = 64 fills only the first 16 lanes of each tensor-memory quarter, so a warp that reads

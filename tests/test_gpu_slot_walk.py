@@ -17,13 +17,14 @@ def _grads(x, do, B, T, how, **kw):
     from nha_b200 import chunk_nha
     leaves = {n: (x[n][None] if how == 'packed' else x[n].view(B, T, *x[n].shape[1:])).detach().cuda().requires_grad_(True) for n in NAMES}
     if how == 'packed':
-        kw.update(cu_seqlens=torch.arange(0, (B + 1) * T, T, dtype=torch.int32, device='cuda'), max_seqlen=T)
+        kw.update(cu_seqlens=torch.arange(0, (B + 1) * T, T, dtype=torch.int32, device='cuda'), max_seqlen=B * T)
     o, _, lse = chunk_nha(*(leaves[n] for n in ('q_swa', 'k_swa', 'q_gsa', 'k_gsa', 'v', 's', 'g')), window_size_right=0, **kw)
     loss = (o.reshape(do.shape).float() * do.cuda()).sum() + 0.1 * lse.sum()
     return dict(zip(NAMES, torch.autograd.grad(loss, [leaves[n] for n in NAMES])))
 
 
-# 320 sequences give every kv head whole sequences to walk; packed, the same calls take the terms, the scan and runs that cut sequences
+# 320 sequences give every kv head whole sequences to walk; packed, with a bound on the lengths that does not say so, the same calls take the terms,
+# the scan and runs that cut sequences
 @pytest.mark.parametrize('T', [1, 63, 64, 65, 200, 449])
 def test_whole_sequences_and_runs_from_the_scan_agree_to_the_bit(T):
     B, H, M = 80, 4, 64
@@ -33,6 +34,28 @@ def test_whole_sequences_and_runs_from_the_scan_agree_to_the_bit(T):
     b = _grads(x, do, B, T, 'packed', window_size_left=64, gsa_kv_shift=0)
     for n in NAMES:
         assert torch.equal(a[n].reshape(-1), b[n].reshape(-1)), n
+
+
+# Packed sequences that the true longest length sends down the walk over whole sequences, and a looser bound through the scan: unequal lengths, empty
+# sequences (first, last and between), the states' gradients
+@pytest.mark.parametrize('HQ,H', [(4, 4), (8, 4)])
+def test_packed_whole_sequences_and_runs_agree_to_the_bit(HQ, H):
+    lens = [0, 65, 1, 0, 64, 200, 63, 0, 130, 128, 0] + [40 + 7 * i for i in range(20)] + [0]
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    N, T, M = len(lens), cu[-1], 64
+    d = gen.layer_inputs(77, 1, T, HQ, H, 64, 64, M, gate_div=1.0)
+    x, do = flat_inputs(d, 1, T), d['do'].reshape(T, HQ, 64).float()
+    torch.manual_seed(5)
+    state = (torch.randn(N, H, 64, M) * 0.5, torch.randn(N, H, M, 64) * 0.5)
+    end = (torch.randn(N, H, 64, M) * 0.1, torch.randn(N, H, M, 64) * 0.1)
+    _, a = run_gpu(x, cu, max(lens), 0.125, 64, 0, *state, do, None, *end)
+    _, b = run_gpu(x, cu, T, 0.125, 64, 0, *state, do, None, *end)
+    for n in a:
+        assert torch.equal(a[n], b[n]), n
+    empty = [i for i, n in enumerate(lens) if n == 0]
+    assert torch.equal(a['hk0'][empty].cpu().float(), end[0][empty]) and torch.equal(a['hv0'][empty].cpu().float(), end[1][empty])
 
 
 # one and several heads a kv head, fewer than 64 slots, ragged ends, a shift that is not a whole chunk, with and without a gradient on lse_gsa,
