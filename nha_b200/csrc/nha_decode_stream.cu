@@ -181,6 +181,124 @@ template <int D> __device__ __forceinline__ constexpr int key_piece(int tq, int 
   return D == 128 ? 16 * tq + 8 * (i & 1) + 64 * (i >> 1) : 8 * tq + 32 * i;
 }
 
+__device__ __forceinline__ void store_row4(bf16* o, const float4& x) {
+  uint2 pk;
+  *reinterpret_cast<__nv_bfloat162*>(&pk.x) = __floats2bfloat162_rn(x.x, x.y);
+  *reinterpret_cast<__nv_bfloat162*>(&pk.y) = __floats2bfloat162_rn(x.z, x.w);
+  *reinterpret_cast<uint2*>(o) = pk;
+}
+
+// The merges of a (sequence, kv head) that several CTAs share, as functions of their own, so that the kernel's registers and the code in front of
+// them are the same whether they run or not.  They are the last link of the call's chain: their loads are asked for together.  Us a layer in a
+// graph of 16, one load waited for at a time | so: one sequence, 16 heads of 64, W 256 (two CTAs) 5.26 | 5.26, W 512 (four) 5.48 | 4.6, W 1200
+// (eight) 7.44 | 5.6; 28 heads of 128 on 4, W 512 7.43 | 6.6, W 1200 8.60 | 6.9; through the workspace, W 1200, 12.8-14.4 | 8.1-9.6.
+
+// From the shared memory of the cluster's CTAs: ml [NG][2] maxima and sums, outp [NG][V] partial outputs; at most eight of them.
+template <int V, int NT>
+__device__ __noinline__ void merge_cluster(const float* ml, const float* outp, bf16* o, int NG, int SPL) {
+  constexpr int V4 = V / 4;
+#pragma unroll 1
+  for (int u = 0; u < NT; ++u) {
+    const int i = threadIdx.x + u * kStrThreads;
+    if (i >= NG * V4) return;
+    const int qh = i / V4, c = i - qh * V4;
+    float mx = -INFINITY, den = 0.f;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    float2 t2[8];
+#pragma unroll
+    for (int s2 = 0; s2 < 8; ++s2) t2[s2] = s2 < SPL ? ld_cluster_f2(cluster_map(ml + 2 * qh, s2)) : make_float2(-INFINITY, 0.f);
+#pragma unroll
+    for (int s2 = 0; s2 < 8; ++s2) mx = fmaxf(mx, t2[s2].x);
+#pragma unroll
+    for (int s4 = 0; s4 < 8; s4 += 4) {
+      if (s4 >= SPL) break;
+      float4 pv[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) pv[k] = s4 + k < SPL ? ld_cluster_f4(cluster_map(outp + qh * V + 4 * c, s4 + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float w2 = t2[s4 + k].x > -INFINITY ? __expf(t2[s4 + k].x - mx) : 0.f;
+        den += t2[s4 + k].y * w2;
+        acc.x += w2 * pv[k].x; acc.y += w2 * pv[k].y; acc.z += w2 * pv[k].z; acc.w += w2 * pv[k].w;
+      }
+    }
+    const float inv = 1.0f / den;
+    store_row4(o + qh * V + 4 * c, make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv));
+  }
+}
+
+// From the workspace: all_ml [SPL][NG][2], all_o [SPL][NG][V]; wgt: [SPL][NG] floats of shared memory.
+template <int V, int NT>
+__device__ __noinline__ void merge_workspace(const float* all_ml, const float* all_o, float* wgt, bf16* o, int NG, int SPL) {
+  constexpr int V4 = V / 4;
+  const int tid = threadIdx.x;
+  if (SPL <= 4) {
+    // few splits: a thread fetches the maxima, sums and partial outputs of its element in one go (one trip to L2)
+    // and forms the merge weights itself
+#pragma unroll
+    for (int u = 0; u < NT; ++u) {
+      const int i = tid + u * kStrThreads;
+      if (i < NG * V4) {
+        const int qh = i / V4, c = i - qh * V4;
+        float4 pv[4];
+        float m2[4], l2[4];
+#pragma unroll
+        for (int s2 = 0; s2 < 4; ++s2) {
+          if (s2 < SPL) {
+            pv[s2] = __ldcg(reinterpret_cast<const float4*>(all_o + ((size_t)s2 * NG + qh) * V + 4 * c));
+            const float2 t2 = __ldcg(reinterpret_cast<const float2*>(all_ml + ((size_t)s2 * NG + qh) * 2));
+            m2[s2] = t2.x; l2[s2] = t2.y;
+          } else {
+            pv[s2] = make_float4(0.f, 0.f, 0.f, 0.f);
+            m2[s2] = -INFINITY; l2[s2] = 0.f;
+          }
+        }
+        const float mx = fmaxf(fmaxf(m2[0], m2[1]), fmaxf(m2[2], m2[3]));
+        float wq[4], den = 0.f;
+#pragma unroll
+        for (int s2 = 0; s2 < 4; ++s2) {
+          wq[s2] = m2[s2] > -INFINITY ? __expf(m2[s2] - mx) : 0.f;
+          den += l2[s2] * wq[s2];
+        }
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int s2 = 0; s2 < 4; ++s2) {
+          const float w2 = wq[s2] / den;
+          acc.x += w2 * pv[s2].x; acc.y += w2 * pv[s2].y; acc.z += w2 * pv[s2].z; acc.w += w2 * pv[s2].w;
+        }
+        store_row4(o + qh * V + 4 * c, acc);
+      }
+    }
+    return;
+  }
+  // merge weights exp(m_s - m) / denominator
+  for (int qh = tid; qh < NG; qh += kStrThreads) {
+    float mx = -INFINITY;
+    for (int s2 = 0; s2 < SPL; ++s2) mx = fmaxf(mx, __ldcg(all_ml + ((size_t)s2 * NG + qh) * 2));
+    float den = 0.f;
+    for (int s2 = 0; s2 < SPL; ++s2) {
+      const float m2 = __ldcg(all_ml + ((size_t)s2 * NG + qh) * 2);
+      const float l2 = __ldcg(all_ml + ((size_t)s2 * NG + qh) * 2 + 1);
+      den += m2 > -INFINITY ? l2 * __expf(m2 - mx) : 0.f;
+    }
+    for (int s2 = 0; s2 < SPL; ++s2) {
+      const float m2 = __ldcg(all_ml + ((size_t)s2 * NG + qh) * 2);
+      wgt[s2 * NG + qh] = m2 > -INFINITY ? __expf(m2 - mx) / den : 0.f;
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < NG * V4; i += kStrThreads) {
+    const int qh = i / V4, c = i - qh * V4;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s2 = 0; s2 < SPL; ++s2) {
+      const float wq = wgt[s2 * NG + qh];
+      const float4 pv = __ldcg(reinterpret_cast<const float4*>(all_o + ((size_t)s2 * NG + qh) * V + 4 * c));
+      acc.x += wq * pv.x; acc.y += wq * pv.y; acc.z += wq * pv.z; acc.w += wq * pv.w;
+    }
+    store_row4(o + qh * V + 4 * c, acc);
+  }
+}
+
 // HB: heads that the slot part of a tile of eight is compiled for (1, 4 or 8).  The kernel is straight-line code that a CTA runs once, and
 // beyond 32 KB an SM fetches an instruction every 5.7 cycles for all of its warps together; with the padding heads out of it and the
 // loops whose length the compiler does not know kept as loops it is 49-68 KB instead of 97-105 at four heads (8 layers of 32 sequences on
@@ -764,12 +882,7 @@ __global__ void __launch_bounds__(kStrThreads, NT == 1 ? 2 : 1) nha_decode_strea
   }
   __syncthreads();
   float* po = a.part_o + ((size_t)bh * SPL + sp) * NG * V;
-  auto store_row = [&](int qh, int c, const float4& x) {
-    uint2 pk;
-    *reinterpret_cast<__nv_bfloat162*>(&pk.x) = __floats2bfloat162_rn(x.x, x.y);
-    *reinterpret_cast<__nv_bfloat162*>(&pk.y) = __floats2bfloat162_rn(x.z, x.w);
-    *reinterpret_cast<uint2*>(a.o + ((size_t)b * a.HQ + h * NG + qh) * V + 4 * c) = pk;
-  };
+  auto store_row = [&](int qh, int c, const float4& x) { store_row4(a.o + ((size_t)b * a.HQ + h * NG + qh) * V + 4 * c, x); };
 #pragma unroll 1
   for (int i = tid; i < NG * V4; i += kStrThreads) {
     const int qh = i / V4, c = i - qh * V4;
@@ -813,28 +926,7 @@ __global__ void __launch_bounds__(kStrThreads, NT == 1 ? 2 : 1) nha_decode_strea
     cluster_sync_all();
     if (sp == 0) {
       append_token();
-#pragma unroll 1
-      for (int u = 0; u < 2; ++u) {
-        const int i = tid + u * kStrThreads;
-        if (i < NG * V4) {
-          const int qh = i / V4, c = i - qh * V4;
-          float mx = -INFINITY;
-#pragma unroll 1
-          for (int s2 = 0; s2 < SPL; ++s2) mx = fmaxf(mx, ld_cluster_f2(cluster_map(ml + 2 * qh, s2)).x);
-          float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-          float den = 0.f;
-#pragma unroll 1
-          for (int s2 = 0; s2 < SPL; ++s2) {
-            const float2 t2 = ld_cluster_f2(cluster_map(ml + 2 * qh, s2));
-            const float4 pv = ld_cluster_f4(cluster_map(outp + qh * V + 4 * c, s2));
-            const float w2 = t2.x > -INFINITY ? __expf(t2.x - mx) : 0.f;
-            den += t2.y * w2;
-            acc.x += w2 * pv.x; acc.y += w2 * pv.y; acc.z += w2 * pv.z; acc.w += w2 * pv.w;
-          }
-          const float inv = 1.0f / den;
-          store_row(qh, c, make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv));
-        }
-      }
+      merge_cluster<V, NT>(ml, outp, a.o + ((size_t)b * a.HQ + h * NG) * V, NG, SPL);
     }
     cluster_sync_all();
     return;
@@ -859,77 +951,7 @@ __global__ void __launch_bounds__(kStrThreads, NT == 1 ? 2 : 1) nha_decode_strea
   append_token();
   const float* all_ml = a.part_ml + (size_t)bh * SPL * NG * 2;
   const float* all_o = a.part_o + (size_t)bh * SPL * NG * V;
-  if (SPL <= 4) {
-    // few splits: a thread fetches the maxima, sums and partial outputs of its element in one go (one trip to L2)
-    // and forms the merge weights itself
-#pragma unroll 1
-    for (int u = 0; u < 2; ++u) {
-      const int i = tid + u * kStrThreads;
-      if (i < NG * V4) {
-        const int qh = i / V4, c = i - qh * V4;
-        float4 pv[4];
-        float m2[4], l2[4];
-#pragma unroll
-        for (int s2 = 0; s2 < 4; ++s2) {
-          if (s2 < SPL) {
-            pv[s2] = __ldcg(reinterpret_cast<const float4*>(all_o + ((size_t)s2 * NG + qh) * V + 4 * c));
-            const float2 t2 = __ldcg(reinterpret_cast<const float2*>(all_ml + ((size_t)s2 * NG + qh) * 2));
-            m2[s2] = t2.x; l2[s2] = t2.y;
-          } else {
-            pv[s2] = make_float4(0.f, 0.f, 0.f, 0.f);
-            m2[s2] = -INFINITY; l2[s2] = 0.f;
-          }
-        }
-        const float mx = fmaxf(fmaxf(m2[0], m2[1]), fmaxf(m2[2], m2[3]));
-        float wq[4], den = 0.f;
-#pragma unroll
-        for (int s2 = 0; s2 < 4; ++s2) {
-          wq[s2] = m2[s2] > -INFINITY ? __expf(m2[s2] - mx) : 0.f;
-          den += l2[s2] * wq[s2];
-        }
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int s2 = 0; s2 < 4; ++s2) {
-          const float w2 = wq[s2] / den;
-          acc.x += w2 * pv[s2].x; acc.y += w2 * pv[s2].y; acc.z += w2 * pv[s2].z; acc.w += w2 * pv[s2].w;
-        }
-        store_row(qh, c, acc);
-      }
-    }
-    return;
-  }
-  float* wgt = outp;                    // [SPL][NG] merge weights exp(m_s - m) / denominator
-#pragma unroll 1
-  for (int qh = tid; qh < NG; qh += kStrThreads) {
-    float mx = -INFINITY;
-#pragma unroll 1
-    for (int s2 = 0; s2 < SPL; ++s2) mx = fmaxf(mx, __ldcg(all_ml + ((size_t)s2 * NG + qh) * 2));
-    float den = 0.f;
-#pragma unroll 1
-    for (int s2 = 0; s2 < SPL; ++s2) {
-      const float m2 = __ldcg(all_ml + ((size_t)s2 * NG + qh) * 2);
-      const float l2 = __ldcg(all_ml + ((size_t)s2 * NG + qh) * 2 + 1);
-      den += m2 > -INFINITY ? l2 * __expf(m2 - mx) : 0.f;
-    }
-#pragma unroll 1
-    for (int s2 = 0; s2 < SPL; ++s2) {
-      const float m2 = __ldcg(all_ml + ((size_t)s2 * NG + qh) * 2);
-      wgt[s2 * NG + qh] = m2 > -INFINITY ? __expf(m2 - mx) / den : 0.f;
-    }
-  }
-  __syncthreads();
-#pragma unroll 1
-  for (int i = tid; i < NG * V4; i += kStrThreads) {
-    const int qh = i / V4, c = i - qh * V4;
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 1
-    for (int s2 = 0; s2 < SPL; ++s2) {
-      const float wq = wgt[s2 * NG + qh];
-      const float4 pv = __ldcg(reinterpret_cast<const float4*>(all_o + ((size_t)s2 * NG + qh) * V + 4 * c));
-      acc.x += wq * pv.x; acc.y += wq * pv.y; acc.z += wq * pv.z; acc.w += wq * pv.w;
-    }
-    store_row(qh, c, acc);
-  }
+  merge_workspace<V, NT>(all_ml, all_o, outp, a.o + ((size_t)b * a.HQ + h * NG) * V, NG, SPL);
 }
 
 static int stream_layout(DecodeStreamArgs& a, int D) {
