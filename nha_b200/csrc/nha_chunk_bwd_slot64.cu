@@ -19,7 +19,12 @@
 // ways give the same bits: the walk updates the state gradient by the scan's arithmetic, element by element in fp32.
 //
 // A chunk that decays by more than 140 nats (the forward's flag) cannot have one reference.  It takes R = 0 and forms the sums
-// over pairs of rows directly in fp32 (steep_*): slow, exact for any gate, and inside the same walk.
+// over pairs of rows directly in fp32 (steep_*), exact for any gate, inside the same walk.  What bounds that is the sums' arithmetic: 64 x 64 / 2 pairs of
+// rows by 64 slots, five times.  Backward, us, B x 2048 tokens, 16 heads, chunks with one steep slot or all of them: general kernels beside
+// the former three passes | sums of each element by itself, its gates read for each | blocks of four rows with running products:
+// B 16: 0.2 % 1262 | 2622 | 933, 1 % 1260 | 3600 | 1025, 10 % 2303 | 11371 | 1422, all 9208 | 51862 | 3346 (none: 982 | 540 | 541);
+// B 2: 1 % 434 | 1769 | 256, all 2222 | 10774 | 592;  4 x 1999 tokens, 16 heads on 4: 1 % 948 | 5717 | 551, all 5091 | 20365 | 1043;
+// 256 tokens, 4 heads, 32 slots: all 342 | 3171 | 338.
 //
 // What bounds it: the chain of a chunk, five rounds of products with the element-wise work between them, about 2000 instructions a warp.  With two
 // CTAs of eight warps on an SM the issue slots are 38 % busy, the tensor cores 26 %, HBM a quarter to a third; a warp waits, per instruction
@@ -80,137 +85,291 @@ struct SlotSm {
 enum { kTabP = 0, kTabC = 64, kTabIP = 128, kTabF = 192, kTabD = 256 };   // 2^n, R log2e - n; 2^-n, F, exp(Gend)  (R = Gend / 2)
 
 // ---- steep chunks ---------------------------------------------------------------------------------------------------------
-// Rows of g, s of position r of the chunk: token c0 + r - shift, or nothing (g = s = 0).
+// The chunk's rows of g: row r at g + r * pitch if lo <= r < hi, or nothing (g = 0).  Handed on by value: the kernel's stack does not fit the L1 cache
+// that two CTAs' shared memory leaves, and a field read from there takes as long as the rows themselves.
 struct SteepCtx {
-  const bf16* g;      // d.g + head offset, row pitch H M
-  const bf16* s;
-  int64_t pitch;
-  int t0, c0, len, shift, M;
+  const bf16* g;      // row 0, this head
+  int pitch, lo, hi, M;
 };
-__device__ __forceinline__ const bf16* steep_row(const SteepCtx& c, const bf16* base, int r) {
-  const int p = c.c0 + r;
-  return p >= c.shift && p < c.len ? base + (int64_t)(c.t0 + p - c.shift) * c.pitch : nullptr;
-}
-__device__ __forceinline__ float tile_at(const unsigned char* t, int r, int c) {
-  return bf2f(*reinterpret_cast<const bf16*>(t + sw_off(r, c >> 3) + 2 * (c & 7)));
-}
-// log decays up to row r and behind it, columns m and m + 1: {G, G, Gend - G, Gend - G} (sums of their own, so that a gate of minus
-// infinity leaves no difference of infinities)
-__device__ float4 steep_sums(const SteepCtx& c, int r, int m) {
-  float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int i = 0; i < kChunk && m < c.M; ++i) {
-    const bf16* gr = steep_row(c, c.g, i);
-    const float2 gv = gr ? __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(gr + m)) : make_float2(0.f, 0.f);
-    if (i <= r) { x.x += gv.x; x.y += gv.y; } else { x.z += gv.x; x.w += gv.y; }
-  }
-  return x;
-}
-__device__ __forceinline__ float2 steep_pair(const bf16* row, int m) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(row + m)); }
-// tile <- tile .* exp(G) (behind: exp(Gend - G)); from: the values of g's row layout instead of the tile's own (s'), or NULL
-__device__ __noinline__ void steep_decay(const SteepCtx& c, unsigned char* t, const bf16* from, bool behind, int tid) {
-  const int r = tid >> 2, m0 = 16 * (tid & 3);
-  const bf16* fr = from ? steep_row(c, from, r) : nullptr;
-  for (int m = m0; m < m0 + 16; m += 2) {
-    __nv_bfloat162* at = reinterpret_cast<__nv_bfloat162*>(t + sw_off(r, m >> 3) + 2 * (m & 7));
-    const float4 g = steep_sums(c, r, m);
-    const float2 v = from ? (fr && m < c.M ? steep_pair(fr, m) : make_float2(0.f, 0.f)) : __bfloat1622float2(*at);
-    *at = __floats2bfloat162_rn(v.x * __expf(behind ? g.z : g.x), v.y * __expf(behind ? g.w : g.y));
+__device__ __forceinline__ const bf16* steep_row(const SteepCtx& c, int r) { return r >= c.lo && r < c.hi ? c.g + (int64_t)r * c.pitch : nullptr; }
+// In these functions a warp has two blocks of four rows, one as far from the chunk's start as the other from its end (so that all have the
+// same number of blocks in front of theirs, and behind), and a lane two slots.  Decays are products of exp(g), never differences of sums (a gate
+// of minus infinity leaves no difference of infinities): from a row outside the block the factors up to the block's edge, one run of products
+// for all four rows, times those inside it.
+__device__ __forceinline__ float2 steep_mul(float2 x, float2 y) { return make_float2(x.x * y.x, x.y * y.y); }
+__device__ __forceinline__ float2 steep_fma(float a, float2 x, float2 y) { return make_float2(fmaf(a, x.x, y.x), fmaf(a, x.y, y.y)); }
+// g of rows i .. i + 3, slots m and m + 1 (rows outside the chunk as well: those of the next block are asked for while a block is worked on), and exp of it
+__device__ __forceinline__ void steep_gates(const SteepCtx& c, int i, int m, uint32_t (&g)[4]) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const bf16* gr = m < c.M ? steep_row(c, i + k) : nullptr;
+    g[k] = gr ? *reinterpret_cast<const uint32_t*>(gr + m) : 0u;
   }
 }
-// The rows' products with the start states, in the accumulators at z and y, become what the whole chunk gives: times exp(G), plus
-// sum_{i<=t} A[t,i] s_i[m] exp(G_t - G_i) from A's tile, and Av's for y
-__device__ __noinline__ void steep_rows(const SteepCtx& c, const unsigned char* A, const unsigned char* Av, uint32_t z, uint32_t y, int r0, int cbase) {
-  float vz[16], vy[16];
-  frag_ld(z, vz);
-  frag_ld(y, vy);
+__device__ __forceinline__ void steep_factors(const uint32_t (&g)[4], float2 (&f)[4]) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const float2 x = pair_f32(g[k]);
+    f[k] = make_float2(__expf(x.x), __expf(x.y));
+  }
+}
+// two neighbouring elements, and four, of a row of a tile
+__device__ __forceinline__ float2 steep_pair(const unsigned char* t, int r, int m) { return pair_f32(*reinterpret_cast<const uint32_t*>(t + sw_off(r, m >> 3) + 2 * (m & 7))); }
+__device__ __forceinline__ void steep_quad(const unsigned char* t, int r, int i, float (&v)[4]) {
+  const uint2 x = *reinterpret_cast<const uint2*>(t + sw_off(r, i >> 3) + 2 * (i & 7));
+  const float2 a = pair_f32(x.x), b = pair_f32(x.y);
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+__device__ __forceinline__ void steep_put(unsigned char* t, int r, int m, float2 v) { *reinterpret_cast<uint32_t*>(t + sw_off(r, m >> 3) + 2 * (m & 7)) = pair_bf16(v.x, v.y); }
+// element pair of an fp32 [64][64] array in two tiles, turned so that a warp's accumulator fragments and its rows both are free of conflicts
+__device__ __forceinline__ float2* steep_at(unsigned char* stage, int r, int m) { return reinterpret_cast<float2*>(stage) + r * 32 + ((m >> 1) ^ ((r & 7) << 2)); }
+__device__ __forceinline__ void steep_stage_in(unsigned char* stage, uint32_t acc, int r0, int cbase) {
+  float v[16];
+  frag_ld(acc, v);
+#pragma unroll
+  for (int k = 0; k < 16; k += 2) *steep_at(stage, r0 + 4 * (k & 2), cbase + 2 * (k & 12)) = make_float2(v[k], v[k + 1]);
+  __syncthreads();
+}
+__device__ __forceinline__ void steep_stage_out(unsigned char* stage, uint32_t acc, int r0, int cbase) {
+  float v[16];
+  __syncthreads();
 #pragma unroll
   for (int k = 0; k < 16; k += 2) {
-    const int r = r0 + 4 * (k & 2), m = cbase + 2 * (k & 12);
-    float w0 = 1.f, w1 = 1.f, a0 = 0.f, a1 = 0.f, b0 = 0.f, b1 = 0.f;
+    const float2 x = *steep_at(stage, r0 + 4 * (k & 2), cbase + 2 * (k & 12));
+    v[k] = x.x;
+    v[k + 1] = x.y;
+  }
+  frag_st(acc, v);
+  __syncthreads();
+}
+// The rows' products with a start state, in the accumulator, become what the whole chunk gives: times exp(G), plus sum_{i<=t} A[t,i] s_i[m]
+// exp(G_t - G_i) from the tiles of tril(q k'^T) (or tril(do v'^T)) and s'.  Through the two tiles at `stage`.
+__device__ __noinline__ void steep_rows(const SteepCtx c, int A, int S, int stage_tile, uint32_t acc, int r0, int cbase) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* sm = align_1024(smem_raw);
+  const unsigned char *tA = sm + A * kTile, *tS = sm + S * kTile;
+  unsigned char* stage = sm + stage_tile * kTile;
+  steep_stage_in(stage, acc, r0, cbase);
+  const int warp = threadIdx.x >> 5, m = 2 * (threadIdx.x & 31);
 #pragma unroll 1
-    for (int i = r; i >= 0 && m < c.M; --i) {
-      const bf16* sr = steep_row(c, c.s, i);
-      if (!sr) continue;
-      const float2 sv = steep_pair(sr, m), gv = steep_pair(steep_row(c, c.g, i), m);
-      const float ai = tile_at(A, r, i), vi = tile_at(Av, r, i);
-      a0 += ai * (sv.x * w0); a1 += ai * (sv.y * w1);
-      b0 += vi * (sv.x * w0); b1 += vi * (sv.y * w1);
-      w0 *= __expf(gv.x); w1 *= __expf(gv.y);
-    }
-    const float4 g = steep_sums(c, r, m);
-    vz[k] = fmaf(vz[k], __expf(g.x), a0); vz[k + 1] = fmaf(vz[k + 1], __expf(g.y), a1);
-    vy[k] = fmaf(vy[k], __expf(g.x), b0); vy[k + 1] = fmaf(vy[k + 1], __expf(g.y), b1);
-  }
-  frag_st(z, vz);
-  frag_st(y, vy);
-}
-// dS[i,m] (+)= sum_{t>=i} (A[t,i] dz_t[m] + Av[t,i] p_t[m]) exp(G_t - G_i) into scratch; then E[t,i] = sum_m dz_t[m] s_i[m]
-// exp(G_t - G_i) and Bv likewise, into A's and Av's tiles (zeros above the diagonal); then the tiles of dz and p are decayed
-__device__ __noinline__ void steep_grads(const SteepCtx& c, unsigned char* A, unsigned char* Av, unsigned char* dz, unsigned char* p, float* ds,
-                                         int64_t dpitch, bool add, int tid) {
-  {
-    const int r = tid >> 2, m0 = 16 * (tid & 3);
-    if (m0 < c.M && c.c0 + r < c.len) {
-      for (int mm = m0; mm < m0 + 16; mm += 2) {
-        float w0 = 1.f, w1 = 1.f, a0 = 0.f, a1 = 0.f;
-        for (int t = r; t < kChunk; ++t) {
-          if (t > r) {
-            const bf16* gr = steep_row(c, c.g, t);
-            const float2 gv = gr ? steep_pair(gr, mm) : make_float2(0.f, 0.f);
-            w0 *= __expf(gv.x); w1 *= __expf(gv.y);
-          }
-          const float ai = tile_at(A, t, r), vi = tile_at(Av, t, r);
-          a0 += (ai * tile_at(dz, t, mm) + vi * tile_at(p, t, mm)) * w0;
-          a1 += (ai * tile_at(dz, t, mm + 1) + vi * tile_at(p, t, mm + 1)) * w1;
-        }
-        float2* o = reinterpret_cast<float2*>(ds + (int64_t)r * dpitch + mm);
-        const float2 old = add ? *o : make_float2(0.f, 0.f);
-        *o = make_float2(old.x + a0, old.y + a1);
-      }
-    }
-  }
-  __syncthreads();
-  const int warp = tid >> 5, lane = tid & 31, m = 2 * lane;
-  for (int t = warp; t < kChunk; t += kThreads / 32) {
-    const float2 zv = make_float2(tile_at(dz, t, m), tile_at(dz, t, m + 1)), pv = make_float2(tile_at(p, t, m), tile_at(p, t, m + 1));
-    float w0 = 1.f, w1 = 1.f;
-    for (int i = kChunk - 1; i >= 0; --i) {
-      float e = 0.f, b = 0.f;
-      if (i <= t) {                                            // (the same for all lanes)
-        const bf16* sr = steep_row(c, c.s, i);
-        if (sr && m < c.M) {
-          const float2 sv = steep_pair(sr, m), gv = steep_pair(steep_row(c, c.g, i), m);
-          e = zv.x * (sv.x * w0) + zv.y * (sv.y * w1);
-          b = pv.x * (sv.x * w0) + pv.y * (sv.y * w1);
-          w0 *= __expf(gv.x); w1 *= __expf(gv.y);
-        }
-        e = warp_sum(e);
-        b = warp_sum(b);
-      }
-      if (lane == 0) {
-        const int at = sw_off(t, i >> 3) + 2 * (i & 7);
-        *reinterpret_cast<bf16*>(A + at) = f2bf(e);
-        *reinterpret_cast<bf16*>(Av + at) = f2bf(b);
-      }
-    }
-  }
-  __syncthreads();
-  steep_decay(c, dz, nullptr, false, tid);
-  steep_decay(c, p, nullptr, false, tid);
-}
-// the products with the state gradient at the chunk's end, in the accumulator at v, become ds': times exp(Gend - G), plus dS
-__device__ __noinline__ void steep_ds(const SteepCtx& c, uint32_t v, const float* ds, int64_t dpitch, int r0, int cbase) {
-  float x[16];
-  frag_ld(v, x);
+  for (int x = 0; x < 2; ++x) {
+    const int b = x ? 15 - warp : warp;
+    float2 v[4], u = make_float2(1.f, 1.f), f[4];
+    uint32_t g[4], own[4];
+    steep_gates(c, 4 * b - 4, m, g);
+    steep_gates(c, 4 * b, m, own);
 #pragma unroll
-  for (int k = 0; k < 16; k += 2) {
-    const int r = r0 + 4 * (k & 2), m = cbase + 2 * (k & 12);
-    const float4 g = steep_sums(c, r, m);
-    const float2 f = m < c.M && c.c0 + r < c.len ? *reinterpret_cast<const float2*>(ds + (int64_t)r * dpitch + m) : make_float2(0.f, 0.f);
-    x[k] = fmaf(x[k], __expf(g.z), f.x);
-    x[k + 1] = fmaf(x[k + 1], __expf(g.w), f.y);
+    for (int t = 0; t < 4; ++t) v[t] = make_float2(0.f, 0.f);
+#pragma unroll 1
+    for (int ib = b - 1; ib >= 0; --ib) {
+      steep_factors(g, f);
+      steep_gates(c, 4 * ib - 4, m, g);
+      float w[4][4];
+#pragma unroll
+      for (int t = 0; t < 4; ++t) steep_quad(tA, 4 * b + t, 4 * ib, w[t]);
+#pragma unroll
+      for (int i = 3; i >= 0; --i) {
+        const float2 sv = steep_mul(steep_pair(tS, 4 * ib + i, m), u);
+#pragma unroll
+        for (int t = 0; t < 4; ++t) v[t] = steep_fma(w[t][i], sv, v[t]);
+        u = steep_mul(u, f[i]);
+      }
+    }
+    steep_factors(own, f);
+    float2 sv[4], pr = make_float2(1.f, 1.f);
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      float w[4];
+      steep_quad(tA, 4 * b + t, 4 * b, w);
+      pr = steep_mul(pr, f[t]);
+#pragma unroll
+      for (int i = 0; i < t; ++i) sv[i] = steep_mul(sv[i], f[t]);
+      sv[t] = steep_pair(tS, 4 * b + t, m);
+      float2* at = steep_at(stage, 4 * b + t, m);
+      const float2 h = steep_mul(*at, u);
+      float2 y = steep_mul(make_float2(v[t].x + h.x, v[t].y + h.y), pr);
+#pragma unroll
+      for (int i = 0; i <= t; ++i) y = steep_fma(w[i], sv[i], y);
+      *at = y;
+    }
   }
-  frag_st(v, x);
+  steep_stage_out(stage, acc, r0, cbase);
+}
+// dS[i,m] (+)= sum_{t>=i} (A[t,i] dz_t[m] + Av[t,i] p_t[m]) exp(G_t - G_i) into scratch
+__device__ __noinline__ void steep_keys(const SteepCtx c, int A, int Av, int dz, int p, float* ds, int64_t dpitch, bool add) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* sm = align_1024(smem_raw);
+  const unsigned char *tA = sm + A * kTile, *tAv = sm + Av * kTile, *tz = sm + dz * kTile, *tp = sm + p * kTile;
+  const int warp = threadIdx.x >> 5, m = 2 * (threadIdx.x & 31);
+#pragma unroll 1
+  for (int x = 0; x < 2; ++x) {
+    const int b = x ? 15 - warp : warp;
+    float2 v[4], u = make_float2(1.f, 1.f), f[4];
+    uint32_t g[4], own[4];
+    steep_gates(c, 4 * b + 4, m, g);
+    steep_gates(c, 4 * b, m, own);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = make_float2(0.f, 0.f);
+#pragma unroll 1
+    for (int tb = b + 1; tb < 16; ++tb) {
+      steep_factors(g, f);
+      steep_gates(c, 4 * tb + 4, m, g);
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        float wa[4], wv[4];
+        steep_quad(tA, 4 * tb + t, 4 * b, wa);
+        steep_quad(tAv, 4 * tb + t, 4 * b, wv);
+        u = steep_mul(u, f[t]);
+        const float2 zv = steep_mul(steep_pair(tz, 4 * tb + t, m), u), pv = steep_mul(steep_pair(tp, 4 * tb + t, m), u);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = steep_fma(wv[i], pv, steep_fma(wa[i], zv, v[i]));
+      }
+    }
+    steep_factors(own, f);
+    // from the block's last row to its first: what the rows behind have left for row t is carried on to the rows in front of it
+#pragma unroll
+    for (int t = 3; t >= 0; --t) {
+      float wa[4], wv[4];
+      steep_quad(tA, 4 * b + t, 4 * b, wa);
+      steep_quad(tAv, 4 * b + t, 4 * b, wv);
+      const float2 zv = steep_pair(tz, 4 * b + t, m), pv = steep_pair(tp, 4 * b + t, m);
+#pragma unroll
+      for (int i = 0; i <= t; ++i) v[i] = steep_fma(wv[i], pv, steep_fma(wa[i], zv, v[i]));
+#pragma unroll
+      for (int i = 0; i < t; ++i) v[i] = steep_mul(v[i], f[t]);
+      if (m < c.M && 4 * b + t < c.hi) {
+        float2* o = reinterpret_cast<float2*>(ds + (int64_t)(4 * b + t) * dpitch + m);
+        const float2 old = add ? *o : make_float2(0.f, 0.f);
+        *o = make_float2(old.x + v[t].x, old.y + v[t].y);
+      }
+    }
+  }
+}
+// The tiles of dz and p become dz exp(G) and p exp(G).  PAIRS: before that E[t,i] = sum_m dz_t[m] s_i[m] exp(G_t - G_i) and Bv likewise from p,
+// into the tiles E and Bv (zeros above the diagonal).
+template <bool PAIRS>
+__device__ __noinline__ void steep_pairs(const SteepCtx c, int E, int Bv, int dz, int p, int S) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* sm = align_1024(smem_raw);
+  const unsigned char* tS = sm + S * kTile;
+  unsigned char *tz = sm + dz * kTile, *tp = sm + p * kTile;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, m = 2 * lane;
+  // this lane's element of the 32 sums of a block: E or Bv, row, column
+  unsigned char* const te = sm + (lane & 16 ? Bv : E) * kTile;
+  const int lt = (lane >> 2) & 3, li = lane & 3;
+  auto sums_out = [&](float (&v)[32], int r, int i) {
+#pragma unroll
+    for (int n = 16; n > 0; n >>= 1) {
+      const bool up = lane & n;
+#pragma unroll
+      for (int k = 0; k < n; ++k) {
+        const float keep = up ? v[k + n] : v[k], give = up ? v[k] : v[k + n];
+        v[k] = keep + __shfl_xor_sync(0xffffffffu, give, n);
+      }
+    }
+    *reinterpret_cast<bf16*>(te + sw_off(r + lt, i >> 3) + 2 * ((i & 7) + li)) = f2bf(v[0]);
+  };
+#pragma unroll 1
+  for (int x = 0; x < 2; ++x) {
+    const int b = x ? 15 - warp : warp;
+    float2 zv[4], pv[4], f[4], u = make_float2(1.f, 1.f);
+    uint32_t g[4];
+    steep_gates(c, 4 * b, m, g);
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      zv[t] = steep_pair(tz, 4 * b + t, m);
+      pv[t] = steep_pair(tp, 4 * b + t, m);
+    }
+    steep_factors(g, f);
+    steep_gates(c, 4 * b - 4, m, g);
+    if (PAIRS) {
+      float v[32];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float2 sv = steep_pair(tS, 4 * b + i, m);
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          if (t > i) sv = steep_mul(sv, f[t]);
+          v[4 * t + i] = t >= i ? fmaf(zv[t].x, sv.x, zv[t].y * sv.y) : 0.f;
+          v[16 + 4 * t + i] = t >= i ? fmaf(pv[t].x, sv.x, pv[t].y * sv.y) : 0.f;
+        }
+      }
+      sums_out(v, 4 * b, 4 * b);
+      for (int k = lane; k < 8 * (15 - b); k += 32) {          // the blocks above the diagonal
+        const int i = 4 * (b + 1 + (k >> 3)), r = 4 * b + (k & 3);
+        *reinterpret_cast<uint2*>(sm + (k & 4 ? Bv : E) * kTile + sw_off(r, i >> 3) + 2 * (i & 7)) = make_uint2(0u, 0u);
+      }
+    }
+    float2 pr = make_float2(1.f, 1.f);
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      pr = steep_mul(pr, f[t]);
+      zv[t] = steep_mul(zv[t], pr);
+      pv[t] = steep_mul(pv[t], pr);
+    }
+#pragma unroll 1
+    for (int ib = b - 1; ib >= 0; --ib) {
+      steep_factors(g, f);
+      steep_gates(c, 4 * ib - 4, m, g);
+      float v[32];
+#pragma unroll
+      for (int i = 3; i >= 0; --i) {
+        if (PAIRS) {
+          const float2 sv = steep_mul(steep_pair(tS, 4 * ib + i, m), u);
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            v[4 * t + i] = fmaf(zv[t].x, sv.x, zv[t].y * sv.y);
+            v[16 + 4 * t + i] = fmaf(pv[t].x, sv.x, pv[t].y * sv.y);
+          }
+        }
+        u = steep_mul(u, f[i]);
+      }
+      if (PAIRS) sums_out(v, 4 * b, 4 * ib);
+    }
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      steep_put(tz, 4 * b + t, m, steep_mul(zv[t], u));
+      steep_put(tp, 4 * b + t, m, steep_mul(pv[t], u));
+    }
+  }
+}
+// With the factors exp(Gend - G): the tile of s' times them (stage_tile < 0), or the products with the state gradient at the chunk's end, in the
+// accumulator, times them plus dS from scratch: ds', through the two tiles at `stage`.
+__device__ __noinline__ void steep_ends(const SteepCtx c, int S, int stage_tile, uint32_t acc, const float* ds, int64_t dpitch, int r0, int cbase) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* sm = align_1024(smem_raw);
+  unsigned char *tS = sm + S * kTile, *stage = sm + stage_tile * kTile;
+  const bool tile = stage_tile < 0;
+  if (!tile) steep_stage_in(stage, acc, r0, cbase);
+  const int warp = threadIdx.x >> 5, m = 2 * (threadIdx.x & 31);
+#pragma unroll 1
+  for (int x = 0; x < 2; ++x) {
+    const int b = x ? 15 - warp : warp;
+    float2 u = make_float2(1.f, 1.f), f[4];
+    uint32_t g[4];
+    steep_gates(c, 60, m, g);
+#pragma unroll 1
+    for (int tb = 15; tb >= b; --tb) {
+      steep_factors(g, f);
+      steep_gates(c, 4 * tb - 4, m, g);
+#pragma unroll
+      for (int t = 3; t >= 0; --t) {
+        if (tb == b) {
+          const int r = 4 * b + t;
+          if (tile) {
+            steep_put(tS, r, m, steep_mul(steep_pair(tS, r, m), u));
+          } else {
+            float2* at = steep_at(stage, r, m);
+            const float2 d = m < c.M && r < c.hi ? *reinterpret_cast<const float2*>(ds + (int64_t)r * dpitch + m) : make_float2(0.f, 0.f);
+            const float2 h = steep_mul(*at, u);
+            *at = make_float2(h.x + d.x, h.y + d.y);
+          }
+        }
+        u = steep_mul(u, f[t]);
+      }
+    }
+  }
+  if (!tile) steep_stage_out(stage, acc, r0, cbase);
 }
 
 // ---- rows that are not whole tiles ------------------------------------------------------------------------------------------
@@ -567,7 +726,7 @@ __device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs&
       if (ONE) tmem_st_wait();
     }
     SteepCtx sx;
-    if (steep) sx = SteepCtx{(const bf16*)d.g + (size_t)h * M, (const bf16*)d.s + (size_t)h * M, rm, t0, c0, len, shift, M};
+    if (steep) sx = SteepCtx{(const bf16*)d.g + (int64_t)(t0 + c0 - shift) * rm + h * M, (int)rm, shift - c0, len - c0, M};
     float a[16], ga[16], dsum[16];
     uint32_t s[8];                                              // SB, as its tile has it
 #pragma unroll
@@ -645,7 +804,7 @@ __device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs&
             const float2 c2 = *reinterpret_cast<const float2*>(tab + kTabC + m), p2 = *reinterpret_cast<const float2*>(tab + kTabP + m);
             const float x0 = fmaf(a[e], kLog2e, c2.x), x1 = fmaf(a[e + 1], kLog2e, c2.y);
             const float2 f = pair_f32(sv[q]);
-            sb[q] = pair_bf16(f.x * exp2f(-x0), f.y * exp2f(-x1));
+            sb[q] = steep ? sv[q] : pair_bf16(f.x * exp2f(-x0), f.y * exp2f(-x1));
             a[e] = exp2f(x0);
             a[e + 1] = exp2f(x1);
             hk[q] = times(hk[q], pair_bf16(p2.x, p2.y));
@@ -660,8 +819,6 @@ __device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs&
         if (steep) {                                           // no factors on the rows: the steep_ functions put them in
 #pragma unroll
           for (int k = 0; k < 16; ++k) a[k] = 1.f;
-          __syncthreads();
-          steep_decay(sx, tile(S::tSB), sx.s, true, tid);
         }
       }
       if (!TERMS) flushed();
@@ -715,7 +872,10 @@ __device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs&
       const float sc2 = d.scale * kLog2e;
       const uint64_t sc22 = pack2(sc2, sc2), scale2 = pack2(d.scale, d.scale);
       mma_wait(1);
-      if (steep) steep_rows(sx, tile(S::tA), tile(S::tB), tl + S::cC, tl + S::cD, r0, cbase);
+      if (steep) {                                             // (the results that waited in ZA and PA have left)
+        steep_rows(sx, S::tA, S::tSB, S::tZA, tl + S::cC, r0, cbase);
+        steep_rows(sx, S::tB, S::tSB, S::tZA, tl + S::cD, r0, cbase);
+      }
       // ---- slot part of dz, decayed bf16 operands, gate terms --------------------------------------------------------------
 #pragma unroll
       for (int jp = 0; jp < 2; ++jp) {
@@ -753,7 +913,15 @@ __device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs&
       }
       if (steep) {
         __syncthreads();
-        steep_grads(sx, tile(S::tA), tile(S::tB), tile(S::tZA), tile(S::tPA), w.dsp + ((size_t)(t0 + c0) * H + h) * M, rm, !first, tid);
+        if (!TERMS) {
+          steep_keys(sx, S::tA, S::tB, S::tZA, S::tPA, w.dsp + ((size_t)(t0 + c0) * H + h) * M, rm, !first);
+          __syncthreads();
+        }
+        steep_pairs<!TERMS>(sx, S::tA, S::tB, S::tZA, S::tPA, S::tSB);
+        if (!TERMS && fin) {
+          __syncthreads();
+          steep_ends(sx, S::tSB, -1, 0, nullptr, 0, r0, cbase);
+        }
       }
       hand_over();
       if (issuer) {
@@ -839,7 +1007,7 @@ __device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs&
           const int p = c0 + r0 + 8 * i;
           keep[i] = p >= shift && p < len;                     // rows of this lane that are a token's
         }
-        if (steep) steep_ds(sx, tl + S::cD, w.dsp + ((size_t)(t0 + c0) * H + h) * M, rm, r0, cbase);
+        if (steep) steep_ends(sx, 0, S::tZA, tl + S::cD, w.dsp + ((size_t)(t0 + c0) * H + h) * M, rm, r0, cbase);
         float v[16];
         frag_ld(tl + S::cD, v);
         // The gate terms less s' ds', as SB times what is divided by a for ds'.  A pair of rows adds (p a)[t] Av[t,i] SB[i] to the terms of
@@ -851,12 +1019,7 @@ __device__ __forceinline__ void slot64_run(const nha_chunk_desc& d, const BwdWs&
           for (int q = 0; q < 4; ++q) {
             const int k = 8 * jp + 2 * q, i = q & 1;
             if (!ONE) { v[k] += dsum[k]; v[k + 1] += dsum[k + 1]; }
-            float2 sv = pair_f32(s[4 * jp + q]);
-            if (steep) {                                       // (a is 1)
-              const bf16* sr = steep_row(sx, sx.s, r0 + 8 * i);
-              const int m = cbase + 16 * jp + 8 * (q >> 1);
-              sv = sr && m < M ? steep_pair(sr, m) : make_float2(0.f, 0.f);
-            }
+            const float2 sv = pair_f32(s[4 * jp + q]);         // (a steep chunk's is s' itself, and a is 1)
             ga[k] = keep[i] ? ga[k] - sv.x * v[k] : 0.f;
             ga[k + 1] = keep[i] ? ga[k + 1] - sv.y * v[k + 1] : 0.f;
             dsp[k >> 1] = pair_bf16(__fdividef(v[k], a[k]), __fdividef(v[k + 1], a[k + 1]));
