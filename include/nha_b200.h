@@ -243,7 +243,8 @@ int64_t nha_chunk_desc_size(void);
 int64_t nha_chunk_count_bound(int64_t Ttot, int64_t N);
 /* number of int32 of desc->plan */
 int64_t nha_chunk_plan_ints(int64_t Ttot, int64_t N, int64_t H);
-/* bytes of desc->workspace for the forward (state pass + output pass) / the backward */
+/* bytes of desc->workspace for the forward (state pass + output pass) / the backward (of the kernels that the descriptor and the
+   environment select: scale and the sizes as the call will have them) */
 int64_t nha_chunk_fwd_workspace_bytes(const nha_chunk_desc* d);
 int64_t nha_chunk_bwd_workspace_bytes(const nha_chunk_desc* d);
 

@@ -1040,9 +1040,17 @@ int bwd_wcols_umma_launch(const nha_chunk_desc* d, const BwdWs& w, int* err, cud
 
 using namespace nha;
 
+// NHA_B200_NO_UMMA=1: the general kernels for every shape
+static bool bwd_tensor_cores() {
+  const char* off = getenv("NHA_B200_NO_UMMA");
+  return !(off && off[0] == '1');
+}
+// Head dim 64: the slot branch as a walk that takes the flagged chunks too, then the window branch.
+static bool bwd_walks(const nha_chunk_desc* d) { return bwd_tensor_cores() && bwd64_supported(d); }
+
 extern "C" int64_t nha_chunk_bwd_workspace_bytes(const nha_chunk_desc* d) {
   if (!d) return 0;
-  return bwd_ws_layout(d, nullptr, nullptr);
+  return bwd_ws_layout(d, bwd_walks(d), nullptr, nullptr);
 }
 
 static int bwd_run(const nha_chunk_desc* d, int dense_T, int stage_mask, void* stream) {
@@ -1055,23 +1063,21 @@ static int bwd_run(const nha_chunk_desc* d, int dense_T, int stage_mask, void* s
   if (d->d_hkt && (!d->hkt || !d->hvt)) return NHA_ERR_BAD_ARG;
   if (d->V % 32 || d->K % 32) return NHA_ERR_UNSUPPORTED;
   if (d->q_offset != 0) return NHA_ERR_UNSUPPORTED;        // late-starting queries exist in the forward only
-  const int64_t need = bwd_ws_layout(d, nullptr, nullptr);
+  const bool tensor_cores = bwd_tensor_cores(), walk = bwd_walks(d);
+  const int64_t need = bwd_ws_layout(d, walk, nullptr, nullptr);
   if (!d->workspace || (int64_t)d->workspace_bytes < need) return NHA_ERR_WORKSPACE;
   BwdWs w;
-  bwd_ws_layout(d, &w, d->workspace);
+  bwd_ws_layout(d, walk, &w, d->workspace);
   const WRowLayout L1 = wrow_layout(d->K, d->V);
   const WColLayout L2 = wcol_layout(d->K, d->V);
   const SlotLayout L3 = slot_layout(d->K, d->V, d->M);
   const MarchLayout L4 = march_layout(d->K, d->V, d->M);
   if (L1.total > kMaxSmem || L2.total > kMaxSmem || L3.total > kMaxSmem || L4.total > kMaxSmem) return NHA_ERR_SMEM;
   cudaStream_t cs = (cudaStream_t)stream;
-  const char* off = getenv("NHA_B200_NO_UMMA");
-  const bool tensor_cores = !(off && off[0] == '1');
   const int NCB = (int)nha_chunk_count_bound(d->Ttot, d->N);
   int* flags = d->plan + d->N + 1 + NCB;
   int* err = flags + (size_t)NCB * d->H;
-  // Head dim 64: the slot branch as a walk that takes the flagged chunks too, then the window branch.
-  if (tensor_cores && bwd64_supported(d)) {
+  if (walk) {
     w.flags = flags;
     if (stage_mask & 1) {
       st = bwd_slot64_launch(d, w, dense_T, err, cs);
