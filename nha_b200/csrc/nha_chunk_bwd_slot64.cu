@@ -16,7 +16,8 @@
 //
 // A run has to know the state gradient at its end.  Where it ends with a sequence that is the caller's (or zero); otherwise it
 // comes from the scan over the terms LK, LV of every chunk (TERMS: the same kernel, one chunk a CTA, the first two rounds).  Both
-// ways give the same bits: the walk updates the state gradient by the scan's arithmetic, element by element in fp32.
+// ways give the same bits: the walk updates the state gradient by the scan's arithmetic, element by element in fp32.  (All but the carry of dg where a
+// chunk comes within about a nat of the limit below: products with its start state, which the walk has scaled by exp(R), may then underflow.)
 //
 // A chunk that decays by more than 140 nats (the forward's flag) cannot have one reference.  It takes R = 0 and forms the sums
 // over pairs of rows directly in fp32 (steep_*), exact for any gate, inside the same walk.  What bounds that is the sums' arithmetic: 64 x 64 / 2 pairs of
@@ -1238,19 +1239,27 @@ static int slot64_launch(const nha_chunk_desc* d, const BwdWs& w, int* err, cons
 void bwd_state_scan_launch(const nha_chunk_desc* d, const BwdWs& w, int win, cudaStream_t cs);
 
 // Chunks per CTA of the walk; 0: a CTA takes a whole sequence, whatever its length, and nothing runs in front of it.  dense_T: tokens of every
-// sequence of the call, or 0.  Whole sequences where they fill the machine as well as equal runs do: a run costs a step a chunk, the terms and the
-// scan in front of runs that cut sequences about half of one for every chunk and the launches of six.  CTAs of at most `per` steps are done
-// after as many waves of them, or after the even share and one more.  Backward of B x 2048 tokens, 16 heads of 64, us, whole | cut: B = 12
-// 485 | 542, 16 535 | 677, 24 834 | 963; B x 512: 8 93 | 115, 16 149 | 176; packed, unequal: 64 sequences of 64-1024 tokens 681 | 788, sorted 618 |
-// 729, 128 of 16-512 (16 heads on 8) 720 | 776, 64 of 1-128 (4 heads) 48 | 78.
-// The caller's max_seqlen is taken at its word for this choice alone.
+// sequence of the call, or 0 (the caller's max_seqlen is then taken at its word, for this choice alone).  With whole sequences the longest chain has
+// `steps` chunks: as many waves of CTAs as there are, or the even share and one sequence more.  Equal runs have `even`, and cost the terms and the
+// scan besides, about half as much again, and two launches.  A chunk takes a CTA that has its SM to itself two thirds of the time that it takes one of
+// two with one head a kv head (8.5 us | 12.8), four fifths with several, whose chain fills an SM better (four heads 37 | 45, seven 60 | 71).  Where
+// the line lies, us, whole | cut, 148 SMs; backward of B x T tokens, or with * forward and backward in a graph; the tenths below stand for these:
+//   one head, a CTA an SM:  16 heads, 4 x 2048 285 | 216, 6 x 311 | 308, 7 x 322 | 350, 9 x 347 | 427; 8 x 8192 1285 | 1407; 4 x 1024 150 | 120, 6 x 165 | 172;
+//                           * 1 x 192 49 | 47, 1 x 256 56 | 47, 1 x 384 70 | 49, 3 x 512 103 | 90, 6 x 512 136 | 144
+//                           (four chunks go whole all the same: such calls wait for the host, whom two launches cost more)
+//   one head, two:          16 heads, 10 x 2048 459 | 459, 11 x 476 | 496, 16 x 535 | 677; 10 x 8192 1779 | 1748; 10 x 1024 237 | 254
+//   several, a CTA an SM:   2, 4, 7 heads on each of 4, 36 x 512 217 | 243, 361 | 379, 582 | 583; 36 x 1024 417 | 437, 698 | 689, 1145 | 1069;
+//                           * 1 x 128 65 | 62, 92 | 84, 133 | 119; 1 x 256 99 | 66, 147 | 88, 219 | 127; 30 x 128 92 | 103, 139 | 149, 225 | 222
+//   several, two:           40 x 512 262 | 253, 421 | 391, 662 | 599; 44 x 512 270 | 280, 439 | 440, 697 | 685; 60 x 1024 579 | 655, 949 | 1037, 1499 | 1604
+// Packed sequences of unequal length leave the whole ones ahead for longer than the bound on their chain says: 20 of 64-1024 tokens, 16 heads, 240 | 287.
 static int slot64_plan(const nha_chunk_desc* d, int dense_T) {
-  const int64_t ncb = nha_chunk_count_bound(d->Ttot, d->N), places = 2 * (int64_t)sm_count();
+  const int64_t ncb = nha_chunk_count_bound(d->Ttot, d->N), sms = sm_count(), places = 2 * sms, ctas = (int64_t)d->N * d->H;
   const int64_t even = (ncb * d->H + places - 1) / places;       // one wave of equal runs
   const int64_t T = dense_T > 0 ? dense_T : d->max_seqlen;
   if (T > 0) {
-    const int64_t per = (T + kChunk - 1) / kChunk, waves = ((int64_t)d->N * d->H + places - 1) / places;
-    if (2 * std::min(waves * per, even + per) <= 3 * even + 6) return 0;
+    const int64_t per = (T + kChunk - 1) / kChunk, waves = (ctas + places - 1) / places, steps = std::min(waves * per, even + per);
+    const int64_t most = d->HQ == d->H ? (ctas <= sms ? 24 * even + 16 : 15 * even + 25) : (ctas <= sms ? 17 * even : 15 * even + 2);
+    if (10 * steps <= most) return 0;
   }
   return (int)std::max<int64_t>(even, 1);
 }

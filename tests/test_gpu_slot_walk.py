@@ -92,3 +92,14 @@ def test_gate_gradients_are_as_precise_as_the_others():
     _, want = run_oracle(x, [0, T, 2 * T], 0.125, 64, 0, None, None, do, None)
     _, got = run_gpu(x, [0, T, 2 * T], T, 0.125, 64, 0, None, None, do, None, batched_B=B)
     assert_close(got['g'], want['g'], 4 * 2.0 ** -9, 'g')
+
+
+# Several query heads a kv head walk whole sequences where those fill the SMs (a CTA an SM, and two), runs from the scan elsewhere
+@pytest.mark.parametrize('B,HQ,H,T', [(37, 8, 4, 130), (74, 8, 4, 257), (74, 28, 4, 65)])
+def test_grouped_whole_sequences_and_runs_agree_to_the_bit(B, HQ, H, T):
+    d = gen.layer_inputs(67 + T, B, T, HQ, H, 64, 64, 64, gate_div=1.0)
+    x, do = flat_inputs(d, B, T), d['do'].reshape(B * T, HQ, 64).float()
+    a = _grads(x, do, B, T, 'dense', window_size_left=64, gsa_kv_shift=0)
+    b = _grads(x, do, B, T, 'packed', window_size_left=64, gsa_kv_shift=0)
+    for n in NAMES:
+        assert torch.equal(a[n].reshape(-1), b[n].reshape(-1)), n
