@@ -188,14 +188,17 @@ __device__ __forceinline__ void store_row4(bf16* o, const float4& x) {
   *reinterpret_cast<uint2*>(o) = pk;
 }
 
-// The merges of a (sequence, kv head) that several CTAs share, as functions of their own, so that the kernel's registers and the code in front of
-// them are the same whether they run or not.  They are the last link of the call's chain: their loads are asked for together.  Us a layer in a
-// graph of 16, one load waited for at a time | so: one sequence, 16 heads of 64, W 256 (two CTAs) 5.26 | 5.26, W 512 (four) 5.48 | 4.6, W 1200
-// (eight) 7.44 | 5.6; 28 heads of 128 on 4, W 512 7.43 | 6.6, W 1200 8.60 | 6.9; through the workspace, W 1200, 12.8-14.4 | 8.1-9.6.
+// The merges of a (sequence, kv head) that several CTAs share.  They are the last link of the call's chain: their loads are asked for together.  Us a
+// layer in a graph of 16, one load waited for at a time | so: one sequence, 16 heads of 64, W 256 (two CTAs) 5.26 | 5.1, W 512 (four) 5.5 | 4.7,
+// W 1200 (eight) 7.4 | 5.5; 28 heads of 128 on 4, W 512 7.43 | 6.7, W 1200 8.60 | 6.9; through the workspace, W 1200, 12.6-14.6 | 7.8-9.4.
+// INLINE where the rest of the kernel is small (one head a kv head): as functions they cost 0.2-0.3 us there (5.3, 5.0, 5.8 us of the first three
+// above; 4 sequences, 16 heads of 128, W 64, not shared, 7.05 us beside the functions, 6.75 without).  Elsewhere functions, so that the registers and
+// the code in front of them are the same whether they run or not: 8 layers of 32 sequences on rings, HQ 32, H 8, W 512, not shared either, 26.3 us
+// a layer with the merges inline, 25.6 so.
 
 // From the shared memory of the cluster's CTAs: ml [NG][2] maxima and sums, outp [NG][V] partial outputs; at most eight of them.
 template <int V, int NT>
-__device__ __noinline__ void merge_cluster(const float* ml, const float* outp, bf16* o, int NG, int SPL) {
+__device__ __forceinline__ void merge_cluster_inline(const float* ml, const float* outp, bf16* o, int NG, int SPL) {
   constexpr int V4 = V / 4;
 #pragma unroll 1
   for (int u = 0; u < NT; ++u) {
@@ -229,7 +232,7 @@ __device__ __noinline__ void merge_cluster(const float* ml, const float* outp, b
 
 // From the workspace: all_ml [SPL][NG][2], all_o [SPL][NG][V]; wgt: [SPL][NG] floats of shared memory.
 template <int V, int NT>
-__device__ __noinline__ void merge_workspace(const float* all_ml, const float* all_o, float* wgt, bf16* o, int NG, int SPL) {
+__device__ __forceinline__ void merge_workspace_inline(const float* all_ml, const float* all_o, float* wgt, bf16* o, int NG, int SPL) {
   constexpr int V4 = V / 4;
   const int tid = threadIdx.x;
   if (SPL <= 4) {
@@ -297,6 +300,23 @@ __device__ __noinline__ void merge_workspace(const float* all_ml, const float* a
     }
     store_row4(o + qh * V + 4 * c, acc);
   }
+}
+
+template <int V, int NT>
+__device__ __noinline__ void merge_cluster_call(const float* ml, const float* outp, bf16* o, int NG, int SPL) { merge_cluster_inline<V, NT>(ml, outp, o, NG, SPL); }
+template <int V, int NT>
+__device__ __noinline__ void merge_workspace_call(const float* all_ml, const float* all_o, float* wgt, bf16* o, int NG, int SPL) {
+  merge_workspace_inline<V, NT>(all_ml, all_o, wgt, o, NG, SPL);
+}
+template <int V, int NT, bool INLINE>
+__device__ __forceinline__ void merge_cluster(const float* ml, const float* outp, bf16* o, int NG, int SPL) {
+  if constexpr (INLINE) merge_cluster_inline<V, NT>(ml, outp, o, NG, SPL);
+  else merge_cluster_call<V, NT>(ml, outp, o, NG, SPL);
+}
+template <int V, int NT, bool INLINE>
+__device__ __forceinline__ void merge_workspace(const float* all_ml, const float* all_o, float* wgt, bf16* o, int NG, int SPL) {
+  if constexpr (INLINE) merge_workspace_inline<V, NT>(all_ml, all_o, wgt, o, NG, SPL);
+  else merge_workspace_call<V, NT>(all_ml, all_o, wgt, o, NG, SPL);
 }
 
 // HB: heads that the slot part of a tile of eight is compiled for (1, 4 or 8).  The kernel is straight-line code that a CTA runs once, and
@@ -926,7 +946,7 @@ __global__ void __launch_bounds__(kStrThreads, NT == 1 ? 2 : 1) nha_decode_strea
     cluster_sync_all();
     if (sp == 0) {
       append_token();
-      merge_cluster<V, NT>(ml, outp, a.o + ((size_t)b * a.HQ + h * NG) * V, NG, SPL);
+      merge_cluster<V, NT, HB == 1>(ml, outp, a.o + ((size_t)b * a.HQ + h * NG) * V, NG, SPL);
     }
     cluster_sync_all();
     return;
@@ -951,7 +971,7 @@ __global__ void __launch_bounds__(kStrThreads, NT == 1 ? 2 : 1) nha_decode_strea
   append_token();
   const float* all_ml = a.part_ml + (size_t)bh * SPL * NG * 2;
   const float* all_o = a.part_o + (size_t)bh * SPL * NG * V;
-  merge_workspace<V, NT>(all_ml, all_o, outp, a.o + ((size_t)b * a.HQ + h * NG) * V, NG, SPL);
+  merge_workspace<V, NT, HB == 1>(all_ml, all_o, outp, a.o + ((size_t)b * a.HQ + h * NG) * V, NG, SPL);
 }
 
 static int stream_layout(DecodeStreamArgs& a, int D) {
