@@ -52,7 +52,7 @@ CFG = dict(B=16, T=2048, H=16, D=64, M=64, W=64, shift=0)
 WORKLOAD = 'nha_attn_fwd_bwd B16 T2048 H16 D64 M64 W64 chunk64 bf16 (340M-layer shape)'
 CPU_SLICE_T = 512                             # tokens of the B=1 slice both CPU measurements run (cost grows with T)
 # dram__bytes_read.sum + dram__bytes_write.sum of all kernels of one step per token, from the committed ncu captures
-NCU_STEP_TRAFFIC_PER_TOKEN = 592.8e6 / 8192        # profiles/step_B4_T2048_H16_D64.md, without the terms and the scan that only runs need
+NCU_STEP_TRAFFIC_PER_TOKEN = 592.8e6 / 8192        # 8192 tokens, without the terms and the scan that only runs need
 ALG_BYTES_PER_TOKEN = 16512 + 32832          # forward + backward, all 16 heads (each input read once per pass)
 NAMES = ('q_swa', 'k_swa', 'q_gsa', 'k_gsa', 'v', 's', 'g')
 
@@ -812,8 +812,7 @@ def main():
     stage_sum = sum(k['ms'] for k in kernels.values())
     peak, how = peaks()
     # DRAM bytes of one step: dram__bytes_read.sum + dram__bytes_write.sum of every kernel of a step, one ncu capture
-    # per kernel on the B=4 case (8192 tokens; traffic grows in proportion to the tokens), summed; the per-kernel
-    # figures are in profiles/step_B4_T2048_H16_D64.md
+    # per kernel on the B=4 case (8192 tokens; traffic grows in proportion to the tokens), summed
     traffic = NCU_STEP_TRAFFIC_PER_TOKEN * tokens if NCU_STEP_TRAFFIC_PER_TOKEN else None
     step_gbs = ALG_BYTES_PER_TOKEN * tokens * args.steps / (ms * 1e-3) / 1e9
     roofline = {'bound': 'hbm', 'achieved': step_gbs, 'peak': peak, 'unit': 'GB/s', 'frac': step_gbs / peak,

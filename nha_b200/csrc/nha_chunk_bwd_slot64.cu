@@ -29,8 +29,8 @@
 //
 // What bounds it: the chain of a chunk, five rounds of products with the element-wise work between them, about 2000 instructions a warp.  With two
 // CTAs of eight warps on an SM the issue slots are 38 % busy, the tensor cores 26 %, HBM a quarter to a third; a warp waits, per instruction
-// issued, 1.6 for tensor memory or a global load, 1.6 for shared memory and shuffles, 1.2 at barriers.  Code beyond the SM's instruction cache of about
-// 48 KB was measured at 5.7 cycles an instruction, which is why rare cases are bodies or functions of their own.  16 warps to a CTA, half as much
+// issued, 1.6 for tensor memory or a global load, 1.6 for shared memory and shuffles, 1.2 at barriers.  A body beyond 64 KB of
+// code waits for its instructions (2.4 cycles for each at 96-128 KB, 6 at 192), which is why rare cases are bodies or functions of their own.  16 warps to a CTA, half as much
 // work for each, were slower (490 us against 384 of that build): the same chain, and more code fetches.
 // Measured, B16 T2048 H16 M64: query-row pass, state-gradient scan and key-row pass of this branch, three kernels that hand dz, p, the terms and
 // the state gradients to each other through memory, 810 us with the rows' window part (about 50); this kernel 335 us, and nothing in between but delta, L
